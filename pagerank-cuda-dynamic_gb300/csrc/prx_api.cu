@@ -226,7 +226,7 @@ SolveArgs make_args(prx_context* c, const GraphDev& g, const prx_options& o) {
   a.pf_tab = c->pf ? c->pf + c->ws_n : nullptr;
   a.acc64 = c->acc64;
   a.acc32 = c->acc32;
-  // expand by pulling once more than 1/16 of the vertices changed by > D
+  // 0: push or pull, chosen on the device each iteration (expand_by_pull)
   a.pull_threshold = o.expansion == 1 ? 0xffffffffu : (o.expansion == 2 ? 0u : g.n / 16);
   // int_adds: the option, else the autotuner's pick, else the library default
   const int ia = o.int_adds ? o.int_adds : (g.tuned_int_adds ? g.tuned_int_adds : (int)kDefaultIntAdds);
@@ -599,14 +599,19 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   // Hot sources (the FP64 sweeps of every mode): a layout whose edges from
   // the highest out-degree vertices gather from a dense copy of their
   // contributions
-  const bool hot_ok = o.hot_sources >= 0;
+  // A graph of up to kPersistEdges edges runs its FP64 loop as one cooperative
+  // kernel on the plain rows (no hot copy, no source chunks); see there.
+  const bool persist = !refine && o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase &&
+                       g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) &&
+                       g.m <= (mode >= PRX_DYNAMIC_FRONTIER ? kPersistFrontierEdges : kPersistEdges);
+  const bool hot_ok = o.hot_sources >= 0 && !persist;
   if (hot_ok) {
     TRY_CUDA_ST(ensure_hot(gr->g, o.hot_sources > 0 ? (uint32_t)o.hot_sources : kDefaultHotCap, c->sms,
                            c->stream));
     if (g.hot_n && (st = ensure_ch(c, g.hot_n))) return st;
   }
   const ChunkLayout *lay64 = nullptr, *lay32 = nullptr;
-  TRY_CUDA_ST(ensure_chunks(gr->g, w64, c->sms, c->stream, &lay64, hot_ok && g.hot_n > 0));
+  if (!persist) TRY_CUDA_ST(ensure_chunks(gr->g, w64, c->sms, c->stream, &lay64, hot_ok && g.hot_n > 0));
   if (refine) TRY_CUDA_ST(ensure_chunks(gr->g, w32, c->sms, c->stream, &lay32));
   cudaStream_t s = c->stream;
   SolveArgs a = make_args(c, g, o);
@@ -643,6 +648,14 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
     TRY_CUDA_ST(cudaEventRecord(c->ev[2], s));
     // iterations of `m` until done: one CUDA graph, or host-driven batches
     auto iterate = [&](int m, const ChunkLayout* lay) -> int {
+      if (persist) {
+        TRY_CUDA_ST(launch_persist(a, g, m, c->sms, c->persist_per_sm, s));
+        c->launches += 1;
+        TRY_CUDA_ST(cudaMemcpyAsync(&c->st_host[1], c->st, sizeof(State), cudaMemcpyDeviceToHost, s));
+        TRY_CUDA_ST(cudaStreamSynchronize(s));
+        if (c->st_host[1].err & kErrGridWait) FAIL(PRX_ETIMEOUT, "prx_solve: a bounded grid wait ran out");
+        return PRX_OK;
+      }
       if (o.loop != PRX_LOOP_HOST && !timing) return run_graph_loop(c, gr, a, m, lay, o.max_iterations);
       for (int k = 1;; k = std::min(2 * k, 16)) {
         for (int i = 0; i < k; ++i) {

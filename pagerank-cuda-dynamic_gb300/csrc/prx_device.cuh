@@ -110,6 +110,57 @@ __device__ __forceinline__ void block_sum_u64(unsigned long long x, unsigned lon
   }
 }
 
+__device__ __forceinline__ void block_sum_u32(uint32_t x, uint32_t* dst) {
+  __shared__ uint32_t ssum[32];
+  x = __reduce_add_sync(0xffffffffu, x);
+  __syncthreads();
+  if (lane_id() == 0) ssum[threadIdx.x >> 5] = x;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    x = __reduce_add_sync(0xffffffffu, lane_id() < (blockDim.x >> 5) ? ssum[lane_id()] : 0u);
+    if (lane_id() == 0 && x) atomicAdd(dst, x);
+  }
+}
+
+// Barrier over all blocks of a cooperative launch (st->bar zero before it).
+// Thread 0 counts the block in and polls; every write of the block before the
+// barrier is visible to every block after it (the fences order thread 0's
+// arrival and the block barriers order the other threads).  The wait is
+// bounded: after kGridSpin polls (seconds; a phase takes well under a
+// millisecond), or when another block gave up, sync returns false in every
+// thread and the kernel must return.  after(): run by thread 0 once all
+// blocks have arrived, before the block continues.
+constexpr int kGridSpin = 1 << 23;
+struct GridBarrier {
+  State* st;
+  uint32_t target = 0;
+  __device__ explicit GridBarrier(State* s) : st(s) {}
+  template <class F>
+  __device__ bool sync(F after) {
+    __shared__ int ok;
+    target += gridDim.x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(&st->bar, 1u);
+      volatile uint32_t* arrived = &st->bar;
+      int good = 1;
+      for (int spin = 0; (int)(*arrived - target) < 0;) {
+        if (++spin > kGridSpin || ((spin & 1023) == 0 && (*(volatile uint32_t*)&st->err & kErrGridWait))) {
+          atomicOr(&st->err, kErrGridWait);
+          good = 0;
+          break;
+        }
+      }
+      __threadfence();
+      if (good) after();
+      ok = good;
+    }
+    __syncthreads();
+    return ok != 0;
+  }
+};
+
 __device__ __forceinline__ unsigned long long dbits(double x) {
   return (unsigned long long)__double_as_longlong(x);
 }
@@ -203,9 +254,13 @@ __device__ __forceinline__ uint32_t layout_id(const uint32_t* __restrict__ hot_i
 
 // The contribution of edge id u: with `hot` (a layout whose hot sources are
 // encoded, kHotFlag | number) from the dense hot copy ch, else c[u].
-template <class T>
-__device__ __forceinline__ T gather(const T* __restrict__ c, const T* __restrict__ ch, bool hot, uint32_t u) {
-  return __ldg((hot && (u & kHotFlag)) ? ch + (u ^ kHotFlag) : c + u);
+// COH: c is written by other blocks of the same launch (between grid
+// barriers), so the load is an ordinary one, not the read-only path.
+template <class T, bool COH = false>
+__device__ __forceinline__ T gather(const T* c, const T* ch, bool hot, uint32_t u) {
+  const T* at = (hot && (u & kHotFlag)) ? ch + (u ^ kHotFlag) : c + u;
+  if constexpr (COH) return *at;
+  else return __ldg(at);
 }
 
 // Sum of c[edg[j]] for j in [s, e) added front to back onto acc.  The edge
@@ -271,9 +326,10 @@ __device__ __forceinline__ double add_alt(double acc, double x, bool alt) {
 // acc (a sum of non-negative terms from +0) unchanged.  int_adds (0 .. 4)
 // of every four adds of a full step run on the integer pipes (add_alt), so
 // the FP64 pipe, the sweep's bound, carries fewer of them.
-__device__ __forceinline__ double warp_row_sums(const double* __restrict__ c, const uint32_t* __restrict__ edg,
-                                                uint32_t s, uint32_t e, double acc,
-                                                const double* __restrict__ ch, bool hot, uint32_t int_adds) {
+template <bool COH = false>
+__device__ __forceinline__ double warp_row_sums(const double* c, const uint32_t* __restrict__ edg, uint32_t s,
+                                                uint32_t e, double acc, const double* ch, bool hot,
+                                                uint32_t int_adds) {
   const uint32_t len = e - s;
   const uint32_t L = __reduce_max_sync(0xffffffffu, len);
   if (L == 0) return acc;
@@ -288,10 +344,10 @@ __device__ __forceinline__ double warp_row_sums(const double* __restrict__ c, co
     const uint32_t a0 = o1 ? g0.y : g0.x, a1 = o1 ? g0.z : g0.y, a2 = o1 ? g0.w : g0.z, a3 = o1 ? g1.x : g0.w,
                    a4 = o1 ? g1.y : g1.x, a5 = o1 ? g1.z : g1.y;
     const uint32_t u0 = o2 ? a2 : a0, u1 = o2 ? a3 : a1, u2 = o2 ? a4 : a2, u3 = o2 ? a5 : a3;
-    double x0 = t < len ? gather(c, ch, hot, u0) : 0.0;
-    double x1 = t + 1 < len ? gather(c, ch, hot, u1) : 0.0;
-    double x2 = t + 2 < len ? gather(c, ch, hot, u2) : 0.0;
-    const double x3 = t + 3 < len ? gather(c, ch, hot, u3) : 0.0;
+    double x0 = t < len ? gather<double, COH>(c, ch, hot, u0) : 0.0;
+    double x1 = t + 1 < len ? gather<double, COH>(c, ch, hot, u1) : 0.0;
+    double x2 = t + 2 < len ? gather<double, COH>(c, ch, hot, u2) : 0.0;
+    const double x3 = t + 3 < len ? gather<double, COH>(c, ch, hot, u3) : 0.0;
     if (t + 4 <= L) {
       acc = add_alt(acc, x0, int_adds >= 4);
       acc = add_alt(acc, x1, int_adds >= 2);

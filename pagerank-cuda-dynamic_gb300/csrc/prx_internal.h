@@ -51,6 +51,7 @@ struct State {
   unsigned long long affected;    // vertices marked before the first iteration
   uint32_t nfcnt;                 // DF / DF-P: vertices whose change exceeded D this iteration
   uint32_t xbcnt;                 // high out-degree vertices queued for block-wide expansion
+  uint32_t marked;                // DF / DF-P: vertices affected in this iteration
   // FP32 refinement
   int k32;                        // FP32 sweeps in the current round (parity of e / ce)
   int inner_done;                 // the current round's FP32 sweeps have converged / hit the cap
@@ -62,10 +63,17 @@ struct State {
   unsigned int el32_prev[2];      // FP32 rounds: the changes of the round's two previous sweeps (bits, 0: none)
   uint32_t q_head;                // DT closure queue (fr[0], length fcnt[0]): items claimed
   uint32_t q_done;                // ... and items whose out-neighbours are marked
+  // persistent loop (prx_persist.cu), its slots rotating over iterations
+  uint32_t bar;                   // grid barrier: blocks arrived since the reset
+  unsigned long long pel[3];      // L-inf change (bits)
+  uint32_t pnf[3];                // DF / DF-P: vertices whose change exceeded D
+  uint32_t pxb[3];                // ... of them of out-degree > kWarpExpand, queued in xb
+  uint32_t pmarked[3];            // vertices affected in it
 };
 
 // Device error codes (State::err bits).
 constexpr uint32_t kErrClosureWait = 1u << 4;  // the DT closure's bounded wait ran out
+constexpr uint32_t kErrGridWait = 1u << 5;     // a persistent loop's grid barrier ran out
 
 // Internal mode of the update kernels: the FP64 residual sweep of the FP32
 // refinement (reads the base ranks r[0] / c[0], writes the next iterate to
@@ -227,7 +235,7 @@ struct SolveArgs {
   State* st;
   uint32_t n;
   uint32_t mid_max;
-  uint32_t pull_threshold;        // expand by pulling when more than this many vertices changed by > D
+  uint32_t pull_threshold;        // prx_options.expansion: 0xffffffff push, 0 pull, else see expand_by_pull
   uint32_t int_adds;              // FP64 LOW sweeps: adds of every four run on the integer pipes (0..4)
   double C0, P, D, C;
 };
@@ -262,6 +270,19 @@ constexpr uint32_t kDefaultHotCap = 4u << 20;
 // Source-chunk width of the FP64 sweeps when prx_options.chunk_vertices is 0
 // and the graph is untuned: 200 MB of FP64 contributions per chunk.
 constexpr uint32_t kDefaultChunk64 = (200u << 20) / sizeof(double);
+
+// The whole FP64 iteration loop of a plain graph (one row segment) as one
+// cooperative kernel from the ranks in parity 0 (prx_persist.cu); per_sm
+// caches each mode's resident blocks per SM (0: not known yet).
+// The largest graphs it takes, by what was measured (us an iteration, graph
+// loop against this; R-MAT 2^16 / 2^18 / 2^20 / 2^21, web-like 1.5M, grids of
+// 2000^2 and 3400^2): Static 46 / 77 / 242 / 402, 213, 116, 314 against 18 /
+// 55 / 183 / 348, 184, 105, 287.  DF and DF-P pay a second barrier and have
+// fewer blocks resident than the launched sweep: DF-P 65 / 98 / 273 / 547, 234,
+// 127, 262 against 24 / 60 / 185 / 432, 238, 130, 288.
+constexpr uint64_t kPersistEdges = 64ull << 20;
+constexpr uint64_t kPersistFrontierEdges = 32ull << 20;
+cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, int per_sm[4], cudaStream_t s);
 
 // ---- FP32 refinement (prx_refine.cu) --------------------------------------
 // FP64 residual sweep of one in-degree class (update kernels in MODE_REFINE64).

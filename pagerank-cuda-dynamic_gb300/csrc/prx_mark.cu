@@ -282,6 +282,7 @@ __global__ void k_state_reset(State* st, int max_iter, double tol) {
   st->affected = 0;
   st->nfcnt = 0;
   st->xbcnt = 0;
+  st->marked = 0;
   st->k32 = 0;
   st->inner_done = 0;
   st->rounds = 0;
@@ -292,6 +293,11 @@ __global__ void k_state_reset(State* st, int max_iter, double tol) {
   st->q_head = 0;
   st->q_done = 0;
   st->el32_prev[0] = st->el32_prev[1] = 0;
+  st->bar = 0;
+  for (int k = 0; k < 3; ++k) {
+    st->pel[k] = 0;
+    st->pnf[k] = st->pxb[k] = st->pmarked[k] = 0;
+  }
 }
 
 // ---- launchers ------------------------------------------------------------------

@@ -34,114 +34,9 @@
 // prev (k-1); the LOW kernel clears prev after reading it, which makes it the
 // empty nxt of iteration k+1.
 #include <algorithm>
-#include <type_traits>
-#include "prx_device.cuh"
+#include "prx_update.cuh"
 
 namespace prx {
-
-template <int MODE> struct ModeTraits {
-  static constexpr bool F32 = (MODE & MODE_F32) != 0;
-  static constexpr int BASE = MODE & ~MODE_F32;
-  static constexpr bool REFINE = BASE == MODE_REFINE64;
-  static constexpr bool DYN = !REFINE && BASE >= PRX_DYNAMIC_TRAVERSAL;
-  static constexpr bool FRONTIER = DYN && BASE >= PRX_DYNAMIC_FRONTIER;
-  static constexpr bool PRUNE = BASE == PRX_PRUNE_DYNAMIC_FRONTIER;
-  using V = typename std::conditional<F32, float, double>::type;  // rank / contribution type
-  // resident blocks of 256 per SM the LOW kernel is compiled (register
-  // budget) and launched for: the dynamic modes' bookkeeping needs more than
-  // 32 registers a thread
-  static constexpr int LOW_BLOCKS = (DYN || F32) ? 6 : 8;
-};
-
-// Rank, contribution and carried-sum arrays of a mode: FP64 r / c / acc64,
-// or for the FP32 dynamic phase e / ce / acc32.
-template <int MODE>
-__device__ __forceinline__ typename ModeTraits<MODE>::V* ranks_of(const SolveArgs& a, int p) {
-  if constexpr (ModeTraits<MODE>::F32) return a.e[p];
-  else return a.r[p];
-}
-template <int MODE>
-__device__ __forceinline__ typename ModeTraits<MODE>::V* contribs_of(const SolveArgs& a, int p) {
-  if constexpr (ModeTraits<MODE>::F32) return a.ce[p];
-  else return a.c[p];
-}
-template <int MODE>
-__device__ __forceinline__ typename ModeTraits<MODE>::V* carried_of(const SolveArgs& a) {
-  if constexpr (ModeTraits<MODE>::F32) return a.acc32;
-  else return a.acc64;
-}
-
-// Data parity read by an iteration: the refinement's FP64 sweep always reads
-// the base ranks (parity 0) and writes parity 1.
-template <int MODE>
-__device__ __forceinline__ int data_parity(const State* st) {
-  return ModeTraits<MODE>::REFINE ? 0 : (st->iter & 1);
-}
-
-__device__ __forceinline__ void set_bit(uint32_t* bm, uint32_t w) {
-  const uint32_t bit = 1u << (w & 31u);
-  if (!(bm[w >> 5] & bit)) atomicOr(&bm[w >> 5], bit);
-}
-
-// Finish vertex v given its contribution sum.  Returns |a_v - r_v| as bits
-// (of a double; an FP32 change converts exactly).  survive (dynamic): v stays
-// affected next iteration; changed (DF / DF-P): its relative change exceeded
-// the frontier tolerance, so its out-neighbours become affected (:106-107,
-// expanded after the sweep as at :686-687).  FP32 phase: *mag is raised to
-// |a_v| (bits of a float).
-template <int MODE>
-__device__ __forceinline__ unsigned long long finish_vertex(const SolveArgs& a, uint32_t v,
-                                                            typename ModeTraits<MODE>::V cv, int p, bool& survive,
-                                                            bool& changed, unsigned int& mag) {
-  using T = ModeTraits<MODE>;
-  const uint32_t d = a.xtdat[v];
-  if constexpr (T::F32) {
-    const float P = (float)a.P, C0 = (float)a.C0, df = (float)d;
-    const float rv = a.e[p][v];
-    float av;
-    // ce[p][v] is rv / df, formed when rv was (the same division)
-    if (T::PRUNE) av = fmaf(P, cv - a.ce[p][v], C0) * (1.f / (1.f - P / df));
-    else          av = fmaf(P, cv, C0);
-    const float ev = fabsf(av - rv);
-    a.e[p ^ 1][v] = av;
-    a.ce[p ^ 1][v] = av / df;
-    mag = max(mag, __float_as_uint(fabsf(av)));
-    survive = true;
-    changed = false;
-    if (T::FRONTIER) {  // relative change against the tolerances, without the division
-      const float m = fmaxf(rv, av);
-      if (T::PRUNE && ev <= (float)a.C * m) survive = false;
-      changed = ev > (float)a.D * m;
-    }
-    return dbits((double)ev);
-  } else {
-    const double y = a.rcp[v];
-    const double rv = a.r[p][v];
-    double av;
-    // c[p][v] is div_count(rv, d, y), formed when rv was; pf: 1 / (1 - P/d)
-    if (T::PRUNE) av = fma(a.P, cv - a.c[p][v], a.C0) * a.pf[v];
-    else          av = fma(a.P, cv, a.C0);
-    const double ev = fabs(av - rv);
-    a.r[p ^ 1][v] = av;
-    if (T::REFINE) {
-      // residual of the base ranks, the first FP32 correction and its contribution
-      const float rho = (float)(av - rv);
-      a.rho[v] = rho;
-      a.e[0][v] = rho;
-      a.ce[0][v] = __fdividef(rho, (float)d);
-    } else {
-      a.c[p ^ 1][v] = div_count(av, d, y);
-    }
-    survive = true;
-    changed = false;
-    if constexpr (T::FRONTIER) {  // rel = ev / max(rv, av) compared with C and D
-      const RelChange rc = rel_change(av, rv);
-      if (T::PRUNE && quot_le(rc, a.C)) survive = false;  // :106
-      changed = quot_gt(rc, a.D);                          // :107
-    }
-    return dbits(ev);
-  }
-}
 
 // ---- LOW: one warp per 32 consecutive vertex ids ------------------------------
 // One launch per source chunk (PASS_ONLY when the row-major CSR is used
@@ -177,6 +72,7 @@ __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
   // rows [vb, ve) (vb a multiple of 32); off is indexed from row vb
   const uint32_t words = (uint32_t)(((uint64_t)ve + 31) >> 5);
   unsigned long long emax = 0, edges = 0;
+  uint32_t marked = 0;
   unsigned int mag = 0;
   for (uint32_t w = (vb >> 5) + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < words;
        w += (gridDim.x * blockDim.x) >> 5) {
@@ -185,6 +81,7 @@ __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
     if (T::DYN) {
       const uint32_t cw = cur[w];
       if (FIRST) {
+        if (T::FRONTIER && lane == 0) marked += __popc(cw);
         const uint32_t pw = prev[w];
         if (((pw & ~cw) >> lane) & 1u) {  // updated last iteration, not this one: refresh parity p^1
           ranks_of<MODE>(a, p ^ 1)[v] = ranks_of<MODE>(a, p)[v];
@@ -234,7 +131,7 @@ __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
       if (lane == 0 && keep) atomicOr(&nxt[w], keep);
     }
     if (LAST && T::FRONTIER) {
-      const unsigned ch = __ballot_sync(0xffffffffu, mine && changed);
+      const unsigned ch = fresh_changes<T::PRUNE>(a.naff, w, __ballot_sync(0xffffffffu, mine && changed), lane);
       if (lane == 0 && ch) {
         atomicOr(&a.nf[p][w], ch);
         atomicAdd(&st->nfcnt, (uint32_t)__popc(ch));
@@ -244,6 +141,7 @@ __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
   if (LAST) block_max_bits(emax, &st->el_bits[iter & 1]);
   if (LAST && T::F32) block_max_u32(mag, &st->e32max_bits[iter & 1]);
   if (T::DYN) block_sum_u64(edges, &st->edges);
+  if (FIRST && T::FRONTIER) block_sum_u32(marked, &st->marked);
 }
 
 // MID / HIGH lists: Static and ND use the graph's class lists; the dynamic
@@ -267,7 +165,7 @@ __device__ __forceinline__ void finish_listed(const SolveArgs& a, uint32_t v, ty
   const unsigned long long ev = finish_vertex<MODE>(a, v, x, p, survive, changed, mag);
   emax = ev > emax ? ev : emax;
   if (ModeTraits<MODE>::DYN && survive) atomicOr(&a.bm[(a.st->iter + 1) % 3][v >> 5], 1u << (v & 31u));
-  if (ModeTraits<MODE>::FRONTIER && changed) {
+  if (ModeTraits<MODE>::FRONTIER && changed && (ModeTraits<MODE>::PRUNE || test_and_set(a.naff, v))) {
     atomicOr(&a.nf[p][v >> 5], 1u << (v & 31u));
     atomicAdd(&a.st->nfcnt, 1u);
   }
@@ -294,29 +192,7 @@ __global__ void __launch_bounds__(kThreads) k_update_mid(SolveArgs a, uint32_t b
     const uint64_t iv = seg_index(v, a.seg_shift);
     const uint32_t s = a.xtoff[iv], d = a.xtoff[iv + 1] - s;
     const uint32_t* __restrict__ ed = seg_edges(a.xtedg, a.xtbase, a.seg_shift, v) + s;
-    V ps[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) ps[k] = V(0);
-    for (uint32_t base = 0; base < d; base += 256) {
-      uint32_t u[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t t = base + lane + 32u * k;
-        u[k] = t < d ? __ldg(ed + t) : 0u;
-      }
-      V x[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) x[k] = (base + lane + 32u * k < d) ? __ldg(c + u[k]) : V(0);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) ps[k] += x[k];
-    }
-    // halving tree over virtual thread t = lane + 32k
-    ps[0] += ps[4]; ps[1] += ps[5]; ps[2] += ps[6]; ps[3] += ps[7];  // t < 128: += t+128
-    ps[0] += ps[2]; ps[1] += ps[3];                                  // t < 64:  += t+64
-    ps[0] += ps[1];                                                  // t < 32:  += t+32
-    V x = ps[0];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    const V x = mid_row_sum<V, false>(c, ed, d, lane);
     if (lane == 0) {
       finish_listed<MODE>(a, v, x, p, emax, mag);
       edges += d;
@@ -347,35 +223,11 @@ __global__ void __launch_bounds__(256) k_update_high(SolveArgs a, uint32_t begin
     const uint64_t iv = seg_index(v, a.seg_shift);
     const uint32_t s = a.xtoff[iv], d = a.xtoff[iv + 1] - s;
     const uint32_t* __restrict__ ed = seg_edges(a.xtedg, a.xtbase, a.seg_shift, v) + s;
-    V acc = V(0);
-    uint32_t j = t;
-    for (; j + 7 * 256 < d; j += 8 * 256) {
-      uint32_t u[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) u[k] = __ldg(ed + j + 256 * k);
-      V x[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) x[k] = __ldg(c + u[k]);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc += x[k];
+    const V x = high_row_sum<V, false>(c, ed, d, t, part);
+    if (t == 0) {
+      finish_listed<MODE>(a, v, x, p, emax, mag);
+      edges += d;
     }
-    for (; j < d; j += 256) acc += __ldg(c + __ldg(ed + j));
-    part[t] = acc;
-    __syncthreads();
-    if (t < 128) part[t] += part[t + 128];
-    __syncthreads();
-    if (t < 64) part[t] += part[t + 64];
-    __syncthreads();
-    if (t < 32) {
-      V x = part[t] + part[t + 32];
-#pragma unroll
-      for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (t == 0) {
-        finish_listed<MODE>(a, v, x, p, emax, mag);
-        edges += d;
-      }
-    }
-    __syncthreads();
   }
   block_max_bits(emax, &a.st->el_bits[a.st->iter & 1]);
   if (T::F32) block_max_u32(mag, &a.st->e32max_bits[a.st->iter & 1]);
@@ -392,7 +244,7 @@ __device__ __forceinline__ bool expansion_needed(const State* st) {
 // the thread, larger ones are queued for k_expand_big.
 __global__ void __launch_bounds__(kThreads) k_expand_push(SolveArgs a) {
   State* st = a.st;
-  if (!expansion_needed(st) || st->nfcnt > a.pull_threshold) return;
+  if (!expansion_needed(st) || !st->nfcnt || expand_by_pull(st->nfcnt, st->marked, a.n, a.pull_threshold)) return;
   const int p = st->iter & 1;
   uint32_t* nxt = a.bm[(st->iter + 1) % 3];
   const uint32_t* nf = a.nf[p];
@@ -416,7 +268,7 @@ __global__ void __launch_bounds__(kThreads) k_expand_push(SolveArgs a) {
 // changed (the same set as the push; cheaper when most vertices changed).
 __global__ void __launch_bounds__(kThreads) k_expand_pull(SolveArgs a) {
   State* st = a.st;
-  if (!expansion_needed(st) || st->nfcnt <= a.pull_threshold) return;
+  if (!expansion_needed(st) || !st->nfcnt || !expand_by_pull(st->nfcnt, st->marked, a.n, a.pull_threshold)) return;
   const int p = st->iter & 1;
   uint32_t* nxt = a.bm[(st->iter + 1) % 3];
   const uint32_t* nf = a.nf[p];
@@ -497,6 +349,7 @@ __global__ void k_finalize(State* st) {
     st->xcnt = 0;
     st->nfcnt = 0;
     st->xbcnt = 0;
+    st->marked = 0;
   }
 }
 
@@ -565,6 +418,7 @@ __global__ void k_commit_dyn32(SolveArgs a, int parity) {
     st->cnt[0][MID] = st->cnt[0][HIGH] = 0;
     st->nfcnt = 0;
     st->xbcnt = 0;
+    st->marked = 0;
   }
 }
 

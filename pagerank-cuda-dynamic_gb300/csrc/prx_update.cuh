@@ -1,0 +1,216 @@
+// prx_update.cuh -- the rank update of one vertex and the row sums of the
+// MID and HIGH classes, shared by the launched sweeps (prx_update.cu) and the
+// persistent loop (prx_persist.cu).
+#pragma once
+#include <type_traits>
+#include "prx_device.cuh"
+
+namespace prx {
+
+template <int MODE> struct ModeTraits {
+  static constexpr bool F32 = (MODE & MODE_F32) != 0;
+  static constexpr int BASE = MODE & ~MODE_F32;
+  static constexpr bool REFINE = BASE == MODE_REFINE64;
+  static constexpr bool DYN = !REFINE && BASE >= PRX_DYNAMIC_TRAVERSAL;
+  static constexpr bool FRONTIER = DYN && BASE >= PRX_DYNAMIC_FRONTIER;
+  static constexpr bool PRUNE = BASE == PRX_PRUNE_DYNAMIC_FRONTIER;
+  using V = typename std::conditional<F32, float, double>::type;  // rank / contribution type
+  // resident blocks of 256 per SM the LOW kernel is compiled (register
+  // budget) and launched for: the dynamic modes' bookkeeping needs more than
+  // 32 registers a thread
+  static constexpr int LOW_BLOCKS = (DYN || F32) ? 6 : 8;
+};
+
+// Rank, contribution and carried-sum arrays of a mode: FP64 r / c / acc64,
+// or for the FP32 dynamic phase e / ce / acc32.
+template <int MODE>
+__device__ __forceinline__ typename ModeTraits<MODE>::V* ranks_of(const SolveArgs& a, int p) {
+  if constexpr (ModeTraits<MODE>::F32) return a.e[p];
+  else return a.r[p];
+}
+template <int MODE>
+__device__ __forceinline__ typename ModeTraits<MODE>::V* contribs_of(const SolveArgs& a, int p) {
+  if constexpr (ModeTraits<MODE>::F32) return a.ce[p];
+  else return a.c[p];
+}
+template <int MODE>
+__device__ __forceinline__ typename ModeTraits<MODE>::V* carried_of(const SolveArgs& a) {
+  if constexpr (ModeTraits<MODE>::F32) return a.acc32;
+  else return a.acc64;
+}
+
+// Data parity read by an iteration: the refinement's FP64 sweep always reads
+// the base ranks (parity 0) and writes parity 1.
+template <int MODE>
+__device__ __forceinline__ int data_parity(const State* st) {
+  return ModeTraits<MODE>::REFINE ? 0 : (st->iter & 1);
+}
+
+__device__ __forceinline__ void set_bit(uint32_t* bm, uint32_t w) {
+  const uint32_t bit = 1u << (w & 31u);
+  if (!(bm[w >> 5] & bit)) atomicOr(&bm[w >> 5], bit);
+}
+
+// Finish vertex v given its contribution sum.  Returns |a_v - r_v| as bits
+// (of a double; an FP32 change converts exactly).  survive (dynamic): v stays
+// affected next iteration; changed (DF / DF-P): its relative change exceeded
+// the frontier tolerance, so its out-neighbours become affected (:106-107,
+// expanded after the sweep as at :686-687).  FP32 phase: *mag is raised to
+// |a_v| (bits of a float).
+template <int MODE>
+__device__ __forceinline__ unsigned long long finish_vertex(const SolveArgs& a, uint32_t v,
+                                                            typename ModeTraits<MODE>::V cv, int p, bool& survive,
+                                                            bool& changed, unsigned int& mag) {
+  using T = ModeTraits<MODE>;
+  const uint32_t d = a.xtdat[v];
+  if constexpr (T::F32) {
+    const float P = (float)a.P, C0 = (float)a.C0, df = (float)d;
+    const float rv = a.e[p][v];
+    float av;
+    // ce[p][v] is rv / df, formed when rv was (the same division)
+    if (T::PRUNE) av = fmaf(P, cv - a.ce[p][v], C0) * (1.f / (1.f - P / df));
+    else          av = fmaf(P, cv, C0);
+    const float ev = fabsf(av - rv);
+    a.e[p ^ 1][v] = av;
+    a.ce[p ^ 1][v] = av / df;
+    mag = max(mag, __float_as_uint(fabsf(av)));
+    survive = true;
+    changed = false;
+    if (T::FRONTIER) {  // relative change against the tolerances, without the division
+      const float m = fmaxf(rv, av);
+      if (T::PRUNE && ev <= (float)a.C * m) survive = false;
+      changed = ev > (float)a.D * m;
+    }
+    return dbits((double)ev);
+  } else {
+    const double y = a.rcp[v];
+    const double rv = a.r[p][v];
+    double av;
+    // c[p][v] is div_count(rv, d, y), formed when rv was; pf: 1 / (1 - P/d)
+    if (T::PRUNE) av = fma(a.P, cv - a.c[p][v], a.C0) * a.pf[v];
+    else          av = fma(a.P, cv, a.C0);
+    const double ev = fabs(av - rv);
+    a.r[p ^ 1][v] = av;
+    if (T::REFINE) {
+      // residual of the base ranks, the first FP32 correction and its contribution
+      const float rho = (float)(av - rv);
+      a.rho[v] = rho;
+      a.e[0][v] = rho;
+      a.ce[0][v] = __fdividef(rho, (float)d);
+    } else {
+      a.c[p ^ 1][v] = div_count(av, d, y);
+    }
+    survive = true;
+    changed = false;
+    if constexpr (T::FRONTIER) {  // rel = ev / max(rv, av) compared with C and D
+      const RelChange rc = rel_change(av, rv);
+      if (T::PRUNE && quot_le(rc, a.C)) survive = false;  // :106
+      changed = quot_gt(rc, a.D);                          // :107
+    }
+    return dbits(ev);
+  }
+}
+
+// DF keeps every vertex it ever marked affected (only DF-P prunes), so a
+// vertex whose out-neighbours were marked once -- as a seed of the batch or by
+// an earlier iteration's expansion -- need not be expanded again: the bitmap
+// naff, which the marking leaves with its seeds, collects them, and only the
+// vertices new to it are.  DF on R-MAT 2^18 in the persistent loop (50
+// iterations, nearly every vertex changing in most of them): 5.5 -> 3.0 ms.
+// chg: the changed
+// vertices of word w (the same in every lane); returns those to expand.
+template <bool PRUNE>
+__device__ __forceinline__ unsigned fresh_changes(uint32_t* naff, uint32_t w, unsigned chg, uint32_t lane) {
+  if (PRUNE || !chg) return chg;
+  const unsigned fresh = chg & ~naff[w];
+  __syncwarp();
+  if (lane == 0 && fresh) atomicOr(&naff[w], fresh);
+  return fresh;
+}
+
+// Whether to expand nf changed vertices by pulling, when `marked` of the n
+// vertices are affected.  A push reads every out-edge of the nf vertices, a
+// pull the in-edges of the unmarked ones up to the first changed source: pull
+// when more than 1/16 of the vertices changed (pull_threshold) or when more
+// changed than are unmarked.  Without the second rule DF on a web-like graph
+// of 1.5M vertices, most of them marked from the start, took 1.57 ms of
+// launched iterations; with it 1.33 ms.
+__device__ __forceinline__ bool expand_by_pull(uint32_t nf, uint32_t marked, uint32_t n, uint32_t pull_threshold) {
+  if (pull_threshold == 0xffffffffu) return false;
+  return nf > pull_threshold || nf > n - marked;
+}
+
+// A contribution: through the read-only path, or with COH (the array is
+// written by other blocks of the same launch, between grid barriers) by an
+// ordinary load.
+template <bool COH, class V>
+__device__ __forceinline__ V load_c(const V* c) {
+  if constexpr (COH) return *c;
+  else return __ldg(c);
+}
+
+// MID: the reference's 256-way sum of c over the d ids at ed, by one warp.
+// Lane l owns virtual threads l + 32k (k = 0..7); the sum is in lane 0.
+template <class V, bool COH>
+__device__ __forceinline__ V mid_row_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t lane) {
+  V ps[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) ps[k] = V(0);
+  for (uint32_t base = 0; base < d; base += 256) {
+    uint32_t u[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t t = base + lane + 32u * k;
+      u[k] = t < d ? __ldg(ed + t) : 0u;
+    }
+    V x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = (base + lane + 32u * k < d) ? load_c<COH>(c + u[k]) : V(0);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) ps[k] += x[k];
+  }
+  // halving tree over virtual thread t = lane + 32k
+  ps[0] += ps[4]; ps[1] += ps[5]; ps[2] += ps[6]; ps[3] += ps[7];  // t < 128: += t+128
+  ps[0] += ps[2]; ps[1] += ps[3];                                  // t < 64:  += t+64
+  ps[0] += ps[1];                                                  // t < 32:  += t+32
+  V x = ps[0];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  return x;
+}
+
+// HIGH: the same sum by a block of 256 (thread t of the reference's block);
+// part: 256 values of shared memory.  The sum is in thread 0.
+template <class V, bool COH>
+__device__ __forceinline__ V high_row_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t t,
+                                          V* part) {
+  V acc = V(0);
+  uint32_t j = t;
+  for (; j + 7 * 256 < d; j += 8 * 256) {
+    uint32_t u[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) u[k] = __ldg(ed + j + 256 * k);
+    V x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = load_c<COH>(c + u[k]);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc += x[k];
+  }
+  for (; j < d; j += 256) acc += load_c<COH>(c + __ldg(ed + j));
+  part[t] = acc;
+  __syncthreads();
+  if (t < 128) part[t] += part[t + 128];
+  __syncthreads();
+  if (t < 64) part[t] += part[t + 64];
+  __syncthreads();
+  V x = V(0);
+  if (t < 32) {
+    x = part[t] + part[t + 32];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  }
+  __syncthreads();  // part is free for the next row
+  return x;
+}
+
+}  // namespace prx
