@@ -75,6 +75,8 @@ int prx_context_create(int device, prx_context** out) {
   if (e == cudaSuccess) e = cudaMalloc(&c->st, sizeof(State));
   if (e == cudaSuccess) e = cudaMallocHost(&c->st_host, 2 * sizeof(State));
   for (int i = 0; i < 4 && e == cudaSuccess; ++i) e = cudaEventCreate(&c->ev[i]);
+  if (e == cudaSuccess) e = degree_tables(&c->qtab, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     set_error(std::string("prx_context_create: ") + cudaGetErrorString(e));
     prx_context_destroy(c);
@@ -221,6 +223,7 @@ SolveArgs make_args(prx_context* c, const GraphDev& g, const prx_options& o) {
   for (int p = 0; p < 2; ++p) { a.e[p] = c->e32[p]; a.ce[p] = c->ce32[p]; }
   a.low_bm = g.low_bm;
   a.rcp = g.rcp;
+  a.qtab = c->qtab;
   a.ever = c->ever;
   a.pf = c->pf;
   a.pf_tab = c->pf ? c->pf + c->ws_n : nullptr;
@@ -599,11 +602,11 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   // Hot sources (the FP64 sweeps of every mode): a layout whose edges from
   // the highest out-degree vertices gather from a dense copy of their
   // contributions
-  // A graph of up to kPersistEdges edges runs its FP64 loop as one cooperative
-  // kernel on the plain rows (no hot copy, no source chunks); see there.
+  // A small or medium graph runs its FP64 loop as one cooperative kernel on
+  // the plain rows (no hot copy, no source chunks); see launch_persist.
   const bool persist = !refine && o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase &&
-                       g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) &&
-                       g.m <= (mode >= PRX_DYNAMIC_FRONTIER ? kPersistFrontierEdges : kPersistEdges);
+                       g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) && persist_fits(g);
+  if (persist) TRY_CUDA_ST(ensure_plan(gr->g, c->sms, c->stream));
   const bool hot_ok = o.hot_sources >= 0 && !persist;
   if (hot_ok) {
     TRY_CUDA_ST(ensure_hot(gr->g, o.hot_sources > 0 ? (uint32_t)o.hot_sources : kDefaultHotCap, c->sms,
@@ -649,7 +652,7 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
     // iterations of `m` until done: one CUDA graph, or host-driven batches
     auto iterate = [&](int m, const ChunkLayout* lay) -> int {
       if (persist) {
-        TRY_CUDA_ST(launch_persist(a, g, m, c->sms, c->persist_per_sm, s));
+        TRY_CUDA_ST(launch_persist(a, g, m, c->sms, s));
         c->launches += 1;
         TRY_CUDA_ST(cudaMemcpyAsync(&c->st_host[1], c->st, sizeof(State), cudaMemcpyDeviceToHost, s));
         TRY_CUDA_ST(cudaStreamSynchronize(s));
@@ -1058,7 +1061,8 @@ int prx_graph_destroy(prx_graph* gr) {
   if (!gr) return PRX_OK;
   cudaSetDevice(gr->g.device);
   GraphDev& g = gr->g;
-  graph_free({g.xoff, g.xedg, g.xtoff, g.xtedg, g.xtdat, g.cls_list, g.xbase, g.xtbase, g.low_bm, g.rcp, g.rcp32});
+  graph_free({g.xoff, g.xedg, g.xtoff, g.xtedg, g.xtdat, g.cls_list, g.plan_list, g.xbase, g.xtbase,
+              g.low_bm, g.rcp, g.rcp32});
   drop_weights(g);
   cudaFree(g.ocls_list);
   free_chunks(g);

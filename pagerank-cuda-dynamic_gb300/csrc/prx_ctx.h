@@ -56,7 +56,7 @@ struct prx_context {
   prx::PprWs* ppr = nullptr;  // batched personalized PageRank workspace (prx_ppr.cu)
   double* wk = nullptr;       // weighted solves and the adjoint: 3 n-vectors + partial sums (prx_weighted.cu)
   size_t wk_cap = 0;          // in doubles
-  int persist_per_sm[4] = {0, 0, 0, 0};  // resident blocks per SM of the persistent loops (launch_persist)
+  const uint64_t* qtab = nullptr;  // degree_tables of the device
 };
 
 struct prx_graph {

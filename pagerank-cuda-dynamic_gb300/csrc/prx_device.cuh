@@ -56,6 +56,12 @@ __device__ __forceinline__ void push(uint32_t* list, uint32_t* cnt, uint32_t v) 
   list[base + __popc(peers & ((1u << lane) - 1u))] = v;
 }
 
+// *cnt += 1 by every active lane, one atomic for them together.
+__device__ __forceinline__ void count_one(uint32_t* cnt) {
+  const unsigned active = __activemask();
+  if ((int)lane_id() == __ffs(active) - 1) atomicAdd(cnt, (uint32_t)__popc(active));
+}
+
 // Block-wide max of a non-negative double given as its bit pattern (for
 // x >= 0 the IEEE-754 bit patterns order like the values), folded into *dst
 // with one atomicMax per block.  Every thread of the block must call it; the
@@ -124,8 +130,8 @@ __device__ __forceinline__ void block_sum_u32(uint32_t x, uint32_t* dst) {
 
 // Barrier over all blocks of a cooperative launch (st->bar zero before it).
 // Thread 0 counts the block in and polls; every write of the block before the
-// barrier is visible to every block after it (the fences order thread 0's
-// arrival and the block barriers order the other threads).  The wait is
+// barrier is visible to every block after it (thread 0's release and acquire
+// order the blocks, the block barriers the other threads).  The wait is
 // bounded: after kGridSpin polls (seconds; a phase takes well under a
 // millisecond), or when another block gave up, sync returns false in every
 // thread and the kernel must return.  after(): run by thread 0 once all
@@ -141,18 +147,20 @@ struct GridBarrier {
     target += gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
-      __threadfence();
-      atomicAdd(&st->bar, 1u);
-      volatile uint32_t* arrived = &st->bar;
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar) : "memory");
+      auto arrived = [&] {
+        uint32_t n;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&st->bar) : "memory");
+        return n;
+      };
       int good = 1;
-      for (int spin = 0; (int)(*arrived - target) < 0;) {
+      for (int spin = 0; (int)(arrived() - target) < 0;) {
         if (++spin > kGridSpin || ((spin & 1023) == 0 && (*(volatile uint32_t*)&st->err & kErrGridWait))) {
           atomicOr(&st->err, kErrGridWait);
           good = 0;
           break;
         }
       }
-      __threadfence();
       if (good) after();
       ok = good;
     }
@@ -301,68 +309,134 @@ __device__ __forceinline__ T lane_row_sum(const T* __restrict__ c, const uint32_
   return acc;
 }
 
-// acc + x for the whole warp (all lanes converged): with `alt`, and when
-// every lane's operands are in add_nonneg_bits's range (sign clear, below
-// 2^977: a warp-uniform test), on the integer pipes; otherwise a DADD.  The
-// bits are the same either way.
-__device__ __forceinline__ double add_alt(double acc, double x, bool alt) {
-  if (alt) {
-    const uint32_t ha = (uint32_t)__double2hiint(acc), hx = (uint32_t)__double2hiint(x);
-    if (__all_sync(0xffffffffu, (ha > hx ? ha : hx) < kSoftAddHiLimit))
-      return __longlong_as_double((long long)add_nonneg_bits((uint64_t)__double_as_longlong(acc),
-                                                             (uint64_t)__double_as_longlong(x)));
+// a / d correctly rounded for an integer d >= 1: in integer operations
+// (quot_bits) with R = the table's reciprocal (0: no entry), otherwise -- a
+// not a positive normal of the middle range, or the estimate undecided -- by
+// div_count with y = RN(1/d) loaded from *y.
+__device__ __forceinline__ double div_outdeg(double a, uint32_t d, uint64_t R, const double* y) {
+  bool undecided;
+  const uint64_t q = quot_bits((uint64_t)__double_as_longlong(a), d, R, &undecided);
+  if (undecided || R == 0 || (uint32_t)__double2hiint(a) - kQuotMinHi >= kQuotHiRange) return div_count(a, d, *y);
+  return __longlong_as_double((long long)q);
+}
+
+// Whether soft_add takes every lane's sum and terms (one vote).
+__device__ __forceinline__ bool soft_step(double acc, const double x[4]) {
+  const uint32_t h0 = (uint32_t)__double2hiint(x[0]), h1 = (uint32_t)__double2hiint(x[1]),
+                 h2 = (uint32_t)__double2hiint(x[2]), h3 = (uint32_t)__double2hiint(x[3]);
+  const uint32_t top = max(max(h0, h1), max(h2, h3)), ha = (uint32_t)__double2hiint(acc);
+  return __all_sync(0xffffffffu, ha - kSoftMinHi < kSoftAddHiLimit - kSoftMinHi && top < kSoftAddHiLimit);
+}
+
+// The adds of a step, x[LO .. m) in order (m, at most 4, the same in every
+// lane), the first K of them by soft_add where it takes them, the others
+// DADDs.  The bits are the same.
+template <int K, int LO>
+__device__ __forceinline__ double add_step(double acc, const double x[4], uint32_t m) {
+  if (K > 0 && soft_step(acc, x)) {
+    SoftAcc u = soft_unpack((uint64_t)__double_as_longlong(acc));
+#pragma unroll
+    for (int i = LO; i < LO + K && i < 4; ++i)
+      if (m > (uint32_t)i) u = soft_add(u, (uint64_t)__double_as_longlong(x[i]));
+    acc = __longlong_as_double((long long)soft_pack(u));
+#pragma unroll
+    for (int i = LO + K; i < 4; ++i)
+      if (m > (uint32_t)i) acc += x[i];
+  } else {
+#pragma unroll
+    for (int i = LO; i < 4; ++i)
+      if (m > (uint32_t)i) acc += x[i];
   }
-  return acc + x;
+  return acc;
 }
 
 // FP64 row sums, one row per lane, for a whole warp: every lane calls it
 // (lanes with nothing to add pass s == e).  Each lane adds c[edg[j]] for j in
-// [s, e) onto acc front to back, as lane_row_sum does, but the warp issues
+// [s, e) onto init front to back, as lane_row_sum does, but the warp issues
 // exactly L adds, L the longest row: lane_row_sum's aligned head and tail
 // groups take up to three predicated adds each, and predicated-off FP64
 // instructions cost the warp as much as live ones.  Step k reads ids
 // s+4k .. s+4k+3 out of the two aligned 16-byte groups they span (the lane's
-// offset s & 3 picks them); a lane past its row's end adds +0.0, which leaves
-// acc (a sum of non-negative terms from +0) unchanged.  int_adds (0 .. 4)
-// of every four adds of a full step run on the integer pipes (add_alt), so
-// the FP64 pipe, the sweep's bound, carries fewer of them.
-template <bool COH = false>
+// offset s & 3 picks them), loaded a step ahead; a lane past its row's end
+// adds +0.0, which leaves the sum (of non-negative terms from +0) unchanged.
+// ZERO: init is +0, so the first term is the first sum and is not added.
+// K of every step's four adds are soft_adds, so that the FP64 pipe carries
+// fewer of them.
+// AHEAD: steps whose gathers are in flight beyond the one being added, for
+// launches with few warps a scheduler, where a step's latency (ids, gathers
+// and four dependent adds) is what counts; 8 registers each.
+template <bool COH, bool ZERO, int AHEAD, int K>
 __device__ __forceinline__ double warp_row_sums(const double* c, const uint32_t* __restrict__ edg, uint32_t s,
-                                                uint32_t e, double acc, const double* ch, bool hot,
-                                                uint32_t int_adds) {
+                                                uint32_t e, double init, const double* ch, bool hot) {
   const uint32_t len = e - s;
   const uint32_t L = __reduce_max_sync(0xffffffffu, len);
-  if (L == 0) return acc;
+  if (L == 0) return init;
   const uint32_t j0 = s & ~3u, o = s & 3u;
-  const uint4 z = make_uint4(0, 0, 0, 0);
-  uint4 g0 = len ? __ldg(reinterpret_cast<const uint4*>(edg + j0)) : z;
-  for (uint32_t t = 0; t < L; t += 4) {
-    const uint32_t jn = j0 + t + 4;
-    const uint4 g1 = jn < e ? __ldg(reinterpret_cast<const uint4*>(edg + jn)) : z;
+  auto ids = [&](uint32_t t) {  // the group at step t of this lane's row
+    const uint32_t j = j0 + t;
+    return len && j < e ? __ldg(reinterpret_cast<const uint4*>(edg + j)) : make_uint4(0, 0, 0, 0);
+  };
+  auto terms = [&](uint32_t t, const uint4& g0, const uint4& g1, double x[4]) {
     // ids at s+t+i, i < 4: the 8 words of g0:g1 shifted by o
     const bool o1 = o & 1u, o2 = o & 2u;
     const uint32_t a0 = o1 ? g0.y : g0.x, a1 = o1 ? g0.z : g0.y, a2 = o1 ? g0.w : g0.z, a3 = o1 ? g1.x : g0.w,
                    a4 = o1 ? g1.y : g1.x, a5 = o1 ? g1.z : g1.y;
     const uint32_t u0 = o2 ? a2 : a0, u1 = o2 ? a3 : a1, u2 = o2 ? a4 : a2, u3 = o2 ? a5 : a3;
-    double x0 = t < len ? gather<double, COH>(c, ch, hot, u0) : 0.0;
-    double x1 = t + 1 < len ? gather<double, COH>(c, ch, hot, u1) : 0.0;
-    double x2 = t + 2 < len ? gather<double, COH>(c, ch, hot, u2) : 0.0;
-    const double x3 = t + 3 < len ? gather<double, COH>(c, ch, hot, u3) : 0.0;
-    if (t + 4 <= L) {
-      acc = add_alt(acc, x0, int_adds >= 4);
-      acc = add_alt(acc, x1, int_adds >= 2);
-      acc = add_alt(acc, x2, int_adds >= 3);
-      acc = add_alt(acc, x3, int_adds >= 1);
-    } else {  // the last 1..3 adds; the trip count is the same in every lane
-      for (uint32_t r = L - t; r; --r) {
-        acc += x0;
-        x0 = x1;
-        x1 = x2;
-      }
+    x[0] = t < len ? gather<double, COH>(c, ch, hot, u0) : 0.0;
+    x[1] = t + 1 < len ? gather<double, COH>(c, ch, hot, u1) : 0.0;
+    x[2] = t + 2 < len ? gather<double, COH>(c, ch, hot, u2) : 0.0;
+    x[3] = t + 3 < len ? gather<double, COH>(c, ch, hot, u3) : 0.0;
+  };
+  // lanes without terms sum from 1 (in soft_add's range) and return init
+  double acc = len ? init : 1.0;
+  auto first = [&](const double x[4]) {  // step 0
+    const uint32_t m = min(4u, L);
+    if (!ZERO) return add_step<K, 0>(acc, x, m);
+    const double x0 = __double_as_longlong(x[0]) == (long long)(1ull << 63) ? 0.0 : x[0];  // +0 + -0 = +0
+    return add_step<K, 1>(len ? x0 : 1.0, x, m);
+  };
+  uint4 g0 = ids(0), g1 = ids(4);
+  if constexpr (AHEAD > 0) {
+    uint4 g2 = ids(8);
+    double x[AHEAD + 1][4];  // x[i]: the terms of step t / 4 + i
+    auto next = [&](uint32_t t, double y[4]) {  // the terms at t; g0 : g1 hold its ids, g2 the group after
+      terms(t, g0, g1, y);
+      g0 = g1;
+      g1 = g2;
+      g2 = ids(t + 12);
+    };
+#pragma unroll
+    for (int i = 0; i <= AHEAD; ++i) next(4 * i, x[i]);
+    acc = first(x[0]);
+    uint32_t t = 4;
+    for (; t + 4 <= L; t += 4) {
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[k][i] = x[k + 1][i];
+      next(t + 4 * AHEAD, x[AHEAD]);
+      acc = add_step<K, 0>(acc, x[0], 4);
     }
-    g0 = g1;
+    if (t < L) acc = add_step<K, 0>(acc, x[1], L - t);
+  } else {
+    double x[4];
+    terms(0, g0, g1, x);
+    uint4 g2 = ids(8);
+    acc = first(x);
+    uint32_t t = 4;
+    for (; t + 4 <= L; t += 4) {
+      g0 = g1;
+      g1 = g2;
+      terms(t, g0, g1, x);
+      g2 = ids(t + 8);
+      acc = add_step<K, 0>(acc, x, 4);
+    }
+    if (t < L) {
+      terms(t, g1, g2, x);
+      acc = add_step<K, 0>(acc, x, L - t);
+    }
   }
-  return acc;
+  return len ? acc : init;
 }
 
 }  // namespace prx

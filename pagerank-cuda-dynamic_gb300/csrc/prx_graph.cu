@@ -187,35 +187,52 @@ __global__ void __launch_bounds__(256) k_cls_scatter(const uint32_t* __restrict_
   }
 }
 
-// In-edges per class (statistics for the roofline): one u64 atomic per block
-// and class.
+// In-edges per class, out[0 .. NCLS), and out[NCLS]: 32 times the longest LOW
+// row of each 32-id word, summed (what a warp per word makes of them): one u64
+// atomic per block each.
 __global__ void __launch_bounds__(256) k_cls_edges(const uint32_t* __restrict__ xtoff, uint32_t shift, uint32_t n, uint32_t mid_max,
                                                    unsigned long long* __restrict__ out) {
-  __shared__ unsigned long long acc[NCLS];
-  if (threadIdx.x < NCLS) acc[threadIdx.x] = 0;
+  __shared__ unsigned long long acc[NCLS + 1];
+  if (threadIdx.x <= NCLS) acc[threadIdx.x] = 0;
   __syncthreads();
-  unsigned long long mine[NCLS] = {0, 0, 0};
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    mine[in_class(xtoff, shift, v, mid_max)] += row_len(xtoff, shift, v);
-  for (int c = 0; c < NCLS; ++c)
+  unsigned long long mine[NCLS + 1] = {0, 0, 0, 0};
+  const uint32_t words = (uint32_t)(((uint64_t)n + 31) >> 5);
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t v = (w << 5) | lane_id();
+    const uint32_t d = v < n ? row_len(xtoff, shift, v) : 0u;
+    mine[d <= kLowMax ? LOW : (d <= mid_max ? MID : HIGH)] += d;
+    mine[NCLS] += __reduce_max_sync(0xffffffffu, d <= kLowMax ? d : 0u);
+  }
+  for (int c = 0; c <= NCLS; ++c)
     if (mine[c]) atomicAdd(&acc[c], mine[c]);
   __syncthreads();
-  if (threadIdx.x < NCLS && acc[threadIdx.x]) atomicAdd(&out[threadIdx.x], acc[threadIdx.x]);
+  if (threadIdx.x <= NCLS && acc[threadIdx.x]) atomicAdd(&out[threadIdx.x], acc[threadIdx.x]);
 }
 
 // RN(1/d) for every out-degree below kRcpTable, formed by the same divisions
 // as k_reciprocals (FP64 division is many FP64 instructions on this part, and
-// 50M vertices share a few thousand degrees).  Filled before each use on the
-// stream that reads it.
+// 50M vertices share a few thousand degrees), and the 64-bit reciprocals of
+// quot_bits.  Filled when a context is created (again by a later one, with
+// the same values).
 constexpr uint32_t kRcpTable = 1u << 16;
 __device__ double g_rcp_table[kRcpTable];
 __device__ float g_rcp32_table[kRcpTable];
+__device__ uint64_t g_quot_table[kQuotTable];
+static_assert(kQuotTable == kRcpTable, "filled together");
+
 
 __global__ void k_rcp_table() {
   for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < kRcpTable; d += gridDim.x * blockDim.x) {
     g_rcp_table[d] = 1.0 / (double)d;
     g_rcp32_table[d] = 1.0f / (float)d;
+    g_quot_table[d] = d ? quot_table_entry(d) : 0ull;
   }
+}
+
+cudaError_t degree_tables(const uint64_t** out, cudaStream_t s) {
+  k_rcp_table<<<kRcpTable / 256, 256, 0, s>>>();
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetSymbolAddress((void**)out, g_quot_table);
 }
 
 __global__ void k_reciprocals(const uint32_t* __restrict__ deg, uint32_t n, double* __restrict__ rcp,
@@ -242,6 +259,7 @@ __global__ void k_selftest_div(uint32_t dmax, uint32_t per, unsigned long long* 
     const double a = __longlong_as_double((long long)(((uint64_t)ex << 52) | (z & 0xFFFFFFFFFFFFFull)));
     const double y = 1.0 / (double)d;
     if (dbits(div_count(a, d, y)) != dbits(a / (double)d)) ++mine;
+    if (dbits(div_outdeg(a, d, quot_table_entry(d), &y)) != dbits(a / (double)d)) ++mine;
     if (dbits(u32_to_f64(d)) != dbits((double)d) || (i == 0 && dbits(u32_to_f64(0)) != 0)) ++mine;
     // the tolerance comparisons of a relative change |m - b| / max(m, b)
     // around their tie band: b = m -+ c*m*(1 + t 2^-50) for t in [-2^8, 2^8)
@@ -777,6 +795,7 @@ cudaError_t ensure_hot(GraphDev& g, uint32_t cap, int sms, cudaStream_t s) {
 
 cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layouts) {
   const uint32_t n = g.n;
+  g.plan_built = false;
   if (!keep_layouts) {
     free_chunks(g);
     free_hot(g);
@@ -798,19 +817,63 @@ cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layout
     cudaError_t e = graph_alloc(&g.cls_list, sizeof(uint32_t) * (n ? n : 1), s);
     if (e != cudaSuccess) return e;
   }
-  return build_class_lists(g.xtoff, g.seg_shift, n, g.mid_max, g.cls_list, g.cls_begin, g.cls_edges, sms, s);
+  return build_class_lists(g.xtoff, g.seg_shift, n, g.mid_max, g.cls_list, g.cls_begin, g.cls_edges, sms, s,
+                           &g.low_padded);
 }
 
 void launch_vertex_tables(const uint32_t* xtoff, uint32_t shift, const uint32_t* xtdat, uint32_t n, uint32_t* low_bm,
                           double* rcp, float* rcp32, int sms, cudaStream_t s) {
   if (!n) return;
   k_low_bitmap<<<sms * 4, 256, 0, s>>>(xtoff, shift, n, low_bm);
-  k_rcp_table<<<kRcpTable / 256, 256, 0, s>>>();
   k_reciprocals<<<sms * 4, 256, 0, s>>>(xtdat, n, rcp, rcp32);
 }
 
+__global__ void k_len_keys(const uint32_t* __restrict__ off, const uint32_t* __restrict__ list, uint32_t count,
+                           unsigned long long* __restrict__ key) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    const uint32_t v = list[i];
+    key[i] = ((unsigned long long)(off[v + 1] - off[v]) << 32) | v;
+  }
+}
+__global__ void k_key_ids(const unsigned long long* __restrict__ key, uint32_t count, uint32_t* __restrict__ list) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    list[i] = (uint32_t)key[i];
+}
+
+cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s) {
+  if (g.plan_built || g.n == 0) return cudaSuccess;
+  cudaError_t e = cudaSuccess;
+  if (!g.plan_list) e = graph_alloc(&g.plan_list, sizeof(uint32_t) * g.n, s);
+  uint64_t edges[NCLS];
+  if (e == cudaSuccess)
+    e = build_class_lists(g.xtoff, g.seg_shift, g.n, kPlanMid, g.plan_list, g.plan_begin, edges, sms, s);
+  if (e != cudaSuccess) return e;
+  if (mixed_lengths(g)) {
+    const uint32_t low = g.plan_begin[MID];
+    unsigned long long *key = nullptr, *tmp = nullptr, *sorted = nullptr;
+    uint32_t* hist = nullptr;
+    e = graph_alloc(&key, sizeof(*key) * ((size_t)low + 2), s);
+    if (e == cudaSuccess) e = graph_alloc(&tmp, sizeof(*tmp) * ((size_t)low + 2), s);
+    if (e == cudaSuccess) e = graph_alloc(&hist, sizeof(uint32_t) * radix_hist_words(low), s);
+    if (e == cudaSuccess) {
+      k_len_keys<<<sms * 4, 256, 0, s>>>(g.xtoff, g.plan_list, low, key);
+      e = radix_sort_u64(key, tmp, low, 32, 39, hist, sms, s, &sorted);
+      if (e == cudaSuccess) k_key_ids<<<sms * 4, 256, 0, s>>>(sorted, low, g.plan_list);
+    }
+    if (key) cudaFreeAsync(key, s);
+    if (tmp) cudaFreeAsync(tmp, s);
+    if (hist) cudaFreeAsync(hist, s);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  g.plan_built = true;
+  return cudaSuccess;
+}
+
 cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, uint32_t mid_max, uint32_t* list,
-                              uint32_t begin[NCLS + 1], uint64_t edges_out[NCLS], int sms, cudaStream_t s) {
+                              uint32_t begin[NCLS + 1], uint64_t edges_out[NCLS], int sms, cudaStream_t s,
+                              uint64_t* low_padded) {
+  if (low_padded) *low_padded = 0;
   if (n == 0) {
     for (int c = 0; c <= NCLS; ++c) begin[c] = 0;
     for (int c = 0; c < NCLS; ++c) edges_out[c] = 0;
@@ -818,20 +881,20 @@ cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, u
   }
   const uint32_t ntiles = (n + kTileV - 1) / kTileV;
   uint32_t* cnt = nullptr;
-  // [class-major tile counts | 4 bounds | pad | 3 u64 edge sums]
+  // [class-major tile counts | 4 bounds | pad | 4 u64 sums]
   const size_t words = (size_t)NCLS * ntiles + NCLS + 1;
-  const size_t bytes = ((words * sizeof(uint32_t) + 7) & ~(size_t)7) + NCLS * sizeof(unsigned long long);
+  const size_t bytes = ((words * sizeof(uint32_t) + 7) & ~(size_t)7) + (NCLS + 1) * sizeof(unsigned long long);
   cudaError_t e = graph_alloc(&cnt, bytes, s);
   if (e != cudaSuccess) return e;
   uint32_t* bounds = cnt + (size_t)NCLS * ntiles;
   unsigned long long* edges = (unsigned long long*)((char*)cnt + ((words * sizeof(uint32_t) + 7) & ~(size_t)7));
-  e = cudaMemsetAsync(edges, 0, NCLS * sizeof(unsigned long long), s);
+  e = cudaMemsetAsync(edges, 0, (NCLS + 1) * sizeof(unsigned long long), s);
   k_cls_count<<<ntiles, 256, 0, s>>>(off, shift, n, mid_max, ntiles, cnt);
   k_cls_scan<<<1, 1024, 0, s>>>(cnt, ntiles, bounds);
   k_cls_scatter<<<ntiles, 256, 0, s>>>(off, shift, n, mid_max, ntiles, cnt, list);
   k_cls_edges<<<sms * 4, 256, 0, s>>>(off, shift, n, mid_max, edges);
   uint32_t hb[NCLS + 1];
-  unsigned long long he[NCLS];
+  unsigned long long he[NCLS + 1];
   if (e == cudaSuccess) e = cudaMemcpyAsync(hb, bounds, sizeof(hb), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(he, edges, sizeof(he), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -839,6 +902,7 @@ cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, u
   if (e != cudaSuccess) return e;
   for (int c = 0; c <= NCLS; ++c) begin[c] = hb[c];
   for (int c = 0; c < NCLS; ++c) edges_out[c] = he[c];
+  if (low_padded) *low_padded = he[NCLS];
   return cudaGetLastError();
 }
 

@@ -130,12 +130,13 @@ struct GraphDev {
   uint32_t* cls_list = nullptr;   // n ids: LOW ids, then MID, then HIGH (each ascending)
   uint32_t cls_begin[NCLS + 1] = {0, 0, 0, 0};
   uint64_t cls_edges[NCLS] = {0, 0, 0};  // in-edges per class
+  uint64_t low_padded = 0;        // the LOW edges, had every row of a 32-id word its longest one's length
   uint32_t mid_max = kDefaultMidMax;
   uint32_t tuned_w64 = 0;         // source-chunk widths picked by prx_autotune (0: library default)
   uint32_t tuned_w32 = 0;
   int tuned_fetch = 0;            // L2 fetch granularity picked by prx_autotune (0: none)
-  int tuned_int_adds = 0;         // integer-pipe adds of the FP64 sweep picked by prx_autotune (-1 none,
-                                  // 1 .. 4; 0: not tuned)
+  int tuned_int_adds = 0;         // integer-pipe adds of the FP64 sweep picked by prx_autotune (-1 none, 1 some;
+                                  // 0: not tuned)
   uint32_t* low_bm = nullptr;     // bitmap of the LOW class
   double* rcp = nullptr;          // RN(1 / outdeg) per vertex, for div_count
   float* rcp32 = nullptr;         // the same in FP32 (personalized PageRank sweeps)
@@ -155,6 +156,12 @@ struct GraphDev {
   uint32_t hot_n = 0;
   uint32_t hot_cap = 0;
   bool hot_built = false;
+  // Rows of the persistent loop (prx_persist.cu), built on first use per graph
+  // version: plan_list holds the LOW ids (by length when mixed_lengths, else
+  // ascending), then those of 65 to kPlanMid in-edges, then the longer ones.
+  uint32_t* plan_list = nullptr;
+  uint32_t plan_begin[NCLS + 1] = {0, 0, 0, 0};
+  bool plan_built = false;
   // batched personalized PageRank picks of prx_autotune_ppr (0: defaults):
   // rows of in-degree above ppr_low_max are cut into ppr_seg-edge segments
   uint32_t ppr_low_max = 0;
@@ -183,6 +190,10 @@ cudaError_t build_default_layout_pipelined(GraphDev& g, uint32_t width, bool hot
                                            const uint32_t* piece_rows, const cudaEvent_t* piece_ready, int sms,
                                            cudaStream_t s);
 
+constexpr uint32_t kQuotTable = 1u << 16;  // out-degrees whose 64-bit reciprocal is tabulated
+// Fills the device's per-degree tables on stream s (one set per process and
+// device); *out: the 64-bit reciprocals.
+cudaError_t degree_tables(const uint64_t** out, cudaStream_t s);
 constexpr uint32_t kPfTable = 1u << 16;  // out-degrees whose DF-P factor is tabulated
 constexpr uint32_t kHotFlag = 0x80000000u;
 // The hot sources of g for a cap of `cap` vertices (0: none); graphs of 2^31
@@ -227,6 +238,7 @@ struct SolveArgs {
   float* ce[2];                   // FP32 refinement: correction / outdeg, ping-pong
   const uint32_t* low_bm;         // LOW-class bitmap
   const double* rcp;              // RN(1 / outdeg)
+  const uint64_t* qtab;           // 64-bit reciprocals of the out-degrees below kQuotTable (quot_table_entry)
   uint32_t* ever;                 // FP32 dynamic phase: vertices updated at least once
   double* pf;                     // DF-P: 1 / (1 - P/d) per vertex (launch_prune_factor)
   double* pf_tab;                 // the same per out-degree d < kPfTable, formed once per solve
@@ -236,7 +248,7 @@ struct SolveArgs {
   uint32_t n;
   uint32_t mid_max;
   uint32_t pull_threshold;        // prx_options.expansion: 0xffffffff push, 0 pull, else see expand_by_pull
-  uint32_t int_adds;              // FP64 LOW sweeps: adds of every four run on the integer pipes (0..4)
+  uint32_t int_adds;              // FP64 LOW sweeps: some adds run on the integer pipes (0: none)
   double C0, P, D, C;
 };
 
@@ -259,11 +271,10 @@ void launch_finalize(const SolveArgs& a, int mode, cudaStream_t s);
 // ch[p] <- the hot sources' c[p] (parity < 0: the parity the running
 // iteration wrote); false when the solve uses no hot copy.
 bool launch_hot_copy(const SolveArgs& a, int parity, int sms, cudaStream_t s);
-// Adds of every four in a full step of the FP64 LOW sweep that run on the
-// integer pipes when prx_options.int_adds is 0 and the graph is not tuned:
-// one.  Static measured 0.4-7% faster on the 50M web-like graph (whose sweep
-// DRAM and L1 also hold back; two or more cost more there than they save)
-// and 5% faster on the 4096^2 grid (three: 17%), DF and DF-P within 2%.
+// prx_options.int_adds when it is 0 and the graph is not tuned: one of every
+// four adds of the launched FP64 LOW sweep on the integer pipes.  Static, us a
+// sweep with none | one: web-like 20M 2440 | 2310, 3M 356 | 323, grid 4096^2
+// 345 | 342; two cost more issue slots there than they unload (2566, 355, 412).
 constexpr uint32_t kDefaultIntAdds = 1;
 // Hot-source cap when prx_options.hot_sources is 0: 32 MB of FP64 values.
 constexpr uint32_t kDefaultHotCap = 4u << 20;
@@ -271,18 +282,30 @@ constexpr uint32_t kDefaultHotCap = 4u << 20;
 // and the graph is untuned: 200 MB of FP64 contributions per chunk.
 constexpr uint32_t kDefaultChunk64 = (200u << 20) / sizeof(double);
 
+// LOW rows go by length when a word's longest row is on average more than
+// twice its mean: an R-MAT graph's words hold rows of 1 and of 60 in-edges
+// side by side (8 lanes of 9 wait), web-like ones and grids stay in id order
+// (1.35), whose rows and ranks lie side by side in memory.
+inline bool mixed_lengths(const GraphDev& g) { return g.low_padded > 2 * g.cls_edges[LOW]; }
+// The persistent loop's rows of g (GraphDev::plan_list).
+constexpr uint32_t kPlanMid = 1024;
+// Largest graphs it takes, in units of a MID row or 32 LOW rows: in id order
+// and by length.
+// Static, us an iteration, launched | persistent: in id order web-like 200k 40 |
+// 28, 1.5M (46,900 units) 179 | 167, 2.5M (78,000) 277 | 272, grid 1000^2
+// (31,000) 30 | 25, 1400^2 (61,000) 51 | 58; by length R-MAT 2^16 47 | 14, 2^18
+// 78 | 29, 2^21 (145,000) 375 | 219, 2^23 (630,000) 1254 | 991.
+constexpr uint64_t kPersistUnits = 48u << 10, kPersistSortedUnits = 1u << 20;
+inline bool persist_fits(const GraphDev& g) {
+  const uint32_t low = g.cls_begin[1] - g.cls_begin[0];
+  return ((uint64_t)(mixed_lengths(g) ? low : g.n) + 31) / 32 + (g.n - low) <=
+         (mixed_lengths(g) ? kPersistSortedUnits : kPersistUnits);
+}
+cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s);
 // The whole FP64 iteration loop of a plain graph (one row segment) as one
-// cooperative kernel from the ranks in parity 0 (prx_persist.cu); per_sm
-// caches each mode's resident blocks per SM (0: not known yet).
-// The largest graphs it takes, by what was measured (us an iteration, graph
-// loop against this; R-MAT 2^16 / 2^18 / 2^20 / 2^21, web-like 1.5M, grids of
-// 2000^2 and 3400^2): Static 46 / 77 / 242 / 402, 213, 116, 314 against 18 /
-// 55 / 183 / 348, 184, 105, 287.  DF and DF-P pay a second barrier and have
-// fewer blocks resident than the launched sweep: DF-P 65 / 98 / 273 / 547, 234,
-// 127, 262 against 24 / 60 / 185 / 432, 238, 130, 288.
-constexpr uint64_t kPersistEdges = 64ull << 20;
-constexpr uint64_t kPersistFrontierEdges = 32ull << 20;
-cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, int per_sm[4], cudaStream_t s);
+// cooperative kernel from the ranks in parity 0 (prx_persist.cu); ensure_plan
+// first.
+cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, cudaStream_t s);
 
 // ---- FP32 refinement (prx_refine.cu) --------------------------------------
 // FP64 residual sweep of one in-degree class (update kernels in MODE_REFINE64).
@@ -342,7 +365,8 @@ cudaError_t tune_apply_cached(GraphDev& g, int sms, cudaStream_t s);
 // Ids of the rows of `off` by length class (LOW, MID, HIGH; each ascending)
 // into list (n), their bounds and the edges of each class.
 cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, uint32_t mid_max, uint32_t* list,
-                              uint32_t begin[NCLS + 1], uint64_t edges[NCLS], int sms, cudaStream_t s);
+                              uint32_t begin[NCLS + 1], uint64_t edges[NCLS], int sms, cudaStream_t s,
+                              uint64_t* low_padded = nullptr);
 // b: device array [du | dv | iu | iv | tdk | tdv | tik | tiv]; t* = batch sorted by (v, u)
 cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd, uint64_t ni, int sms, cudaStream_t s);
 // The arrays of one graph version (a plain CSR pair and the out-degrees).

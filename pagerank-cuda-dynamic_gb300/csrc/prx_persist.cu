@@ -13,12 +13,15 @@
 // What bounds it: latency (offsets -> ids -> contributions -> the row's adds
 // -> barrier), then the FP64 pipe.
 //
-// Work split: HIGH rows by block (block b takes rows b, b + blocks, ...),
-// MID rows and 32-id words of LOW rows by warp, counted from the last warp
-// backwards so that the blocks that hold HIGH rows get the units of the last
-// round.  Static and ND need no bitmaps; the dynamic modes look their MID and
-// HIGH rows up in the static class lists (a bit test each) instead of
-// queueing them.
+// Work split (GraphDev::plan_list): rows of more than kPlanMid in-edges by
+// block (row i to block i mod blocks), the others by warp as units of one
+// MID row or 32 LOW rows, counted from the last warp backwards so that the
+// blocks that hold long rows get the units of the last round.  LOW rows of
+// graphs whose 32-id words mix lengths come in order of length; the words'
+// bookkeeping of the dynamic modes is then a pass of its own.  A
+// warp keeps what it knows of its first unit (row
+// bounds, out-degrees, reciprocals) in registers over the iterations.  Static and ND need no bitmaps; the dynamic
+// modes look their rows up with a bit test each instead of queueing them.
 //
 // Memory: contributions and ranks are written by one block and read by
 // others after a grid barrier, so they are read by ordinary loads (never the
@@ -31,8 +34,9 @@
 namespace prx {
 
 struct PersistRows {
-  uint32_t mid, nmid;    // MID rows: cls_list[mid .. mid + nmid)
-  uint32_t high, nhigh;  // HIGH rows
+  const uint32_t* list;  // GraphDev::plan_list: nlow LOW ids, nmid MID ids, nlong longer ones
+  uint32_t nlow, nmid, nlong;
+  bool sorted;           // the LOW ids are in order of length
 };
 
 // Expansion of the changed vertices (nf[p]) into nxt, whichever way
@@ -86,9 +90,8 @@ __device__ __forceinline__ void persist_push(const SolveArgs& a, const uint32_t*
 __device__ __forceinline__ void persist_pull(const SolveArgs& a, const PersistRows& rows, const uint32_t* nf,
                                              uint32_t* nxt, uint32_t warp, uint32_t warps) {
   const uint32_t words = (a.n + 31) >> 5, lane = lane_id();
-  // MID and HIGH lie side by side in cls_list
-  for (uint32_t i = warp; i < rows.nmid + rows.nhigh; i += warps) {
-    const uint32_t v = a.cls_list[rows.mid + i];
+  for (uint32_t i = warp; i < rows.nmid + rows.nlong; i += warps) {
+    const uint32_t v = rows.list[rows.nlow + i];
     if ((nxt[v >> 5] >> (v & 31u)) & 1u) continue;
     const uint32_t e = a.xtoff[v + 1];
     bool hit = false;
@@ -124,8 +127,19 @@ __device__ __forceinline__ void persist_pull(const SolveArgs& a, const PersistRo
   }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kThreads, 4) k_persist(SolveArgs a, PersistRows rows) {
+// A unit's rows as a warp knows them: the MID row in every lane, or lane i's
+// LOW row.
+struct Unit {
+  uint32_t v, s, e;   // row v, its in-edges [s, e)
+  bool row;           // this lane has one
+  uint32_t d;         // out-degree
+  uint64_t R;         // its reciprocal (load_vertex)
+};
+
+// Three blocks per SM (80 registers): what a unit waits for counts more here
+// than how many are in flight.  K: see warp_row_sums.
+template <int MODE, int K>
+__global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRows rows) {
   using T = ModeTraits<MODE>;
   __shared__ double part[256];
   __shared__ unsigned long long s_el;
@@ -136,10 +150,36 @@ __global__ void __launch_bounds__(kThreads, 4) k_persist(SolveArgs a, PersistRow
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t warp = warps - 1 - ((blockIdx.x * blockDim.x + t) >> 5);
   const uint32_t words = (a.n + 31) >> 5;
-  const uint32_t w0 = (warp + warps - rows.nmid % warps) % warps;
+  const uint32_t units = rows.nmid + (rows.sorted ? (rows.nlow + 31) / 32 : words);
   const int max_iter = st->max_iter;
   const double tol = st->tol;
   unsigned long long edges = 0;
+  auto load_unit = [&](uint32_t u) {
+    Unit x{};
+    if (u < rows.nmid) {
+      x.v = __ldg(rows.list + rows.nlow + u);
+      x.row = true;
+    } else if (rows.sorted) {
+      const uint32_t i = 32 * (u - rows.nmid) + lane;
+      x.row = i < rows.nlow;
+      x.v = x.row ? __ldg(rows.list + i) : 0u;
+    } else {
+      const uint32_t w = u - rows.nmid;
+      x.v = (w << 5) | lane;
+      x.row = x.v < a.n && ((__ldg(a.low_bm + w) >> lane) & 1u);
+    }
+    if (x.row) {
+      x.s = __ldg(a.xtoff + x.v);
+      x.e = __ldg(a.xtoff + x.v + 1);
+      x.d = __ldg(a.xtdat + x.v);
+      x.R = x.d < kQuotTable ? __ldg(a.qtab + x.d) : 0ull;
+    }
+    return x;
+  };
+  // this warp's first unit of LOW rows
+  const uint32_t low0 = warp < rows.nmid ? warp + (rows.nmid - warp + warps - 1) / warps * warps : warp;
+  Unit first{};
+  if (warp < units) first = load_unit(warp);
   GridBarrier bar(st);
   for (int it = 0;; ++it) {
     const int p = it & 1;
@@ -150,62 +190,79 @@ __global__ void __launch_bounds__(kThreads, 4) k_persist(SolveArgs a, PersistRow
     unsigned long long emax = 0;
     unsigned int mag = 0;
     uint32_t marked = 0;
-    // one MID / HIGH vertex, by the thread that holds its sum
-    auto finish_one = [&](uint32_t v, double x, uint32_t d) {
+    auto affected = [&](uint32_t v) { return !T::DYN || ((cur[v >> 5] >> (v & 31u)) & 1u); };
+    // one vertex, by the thread that holds its sum
+    auto finish_one = [&](uint32_t v, double x, uint32_t len, const VertexIn& in) {
       bool survive, changed;
-      const unsigned long long ev = finish_vertex<MODE>(a, v, x, p, survive, changed, mag);
+      const unsigned long long ev = finish_vertex<MODE>(a, v, x, p, survive, changed, mag, in);
       emax = ev > emax ? ev : emax;
-      edges += d;
+      edges += len;
       if (T::DYN && survive) atomicOr(&nxt[v >> 5], 1u << (v & 31u));
       if (T::FRONTIER && changed && (T::PRUNE || test_and_set(a.naff, v))) {  // see fresh_changes
         atomicOr(&a.nf[p][v >> 5], 1u << (v & 31u));
-        atomicAdd(&st->pnf[it % 3], 1u);
-        if (a.xtdat[v] > kWarpExpand) a.xb[atomicAdd(&st->pxb[it % 3], 1u)] = v;
+        count_one(&st->pnf[it % 3]);
+        if (in.d > kWarpExpand) a.xb[atomicAdd(&st->pxb[it % 3], 1u)] = v;
       }
     };
-    for (uint32_t i = blockIdx.x; i < rows.nhigh; i += gridDim.x) {
-      const uint32_t v = a.cls_list[rows.high + i];
-      if (T::DYN && !((cur[v >> 5] >> (v & 31u)) & 1u)) continue;
-      const uint32_t s = a.xtoff[v], d = a.xtoff[v + 1] - s;
-      const double x = high_row_sum<double, true>(c, a.xtedg + s, d, t, part);
-      if (t == 0) finish_one(v, x, d);
-    }
-    for (uint32_t i = warp; i < rows.nmid; i += warps) {
-      const uint32_t v = a.cls_list[rows.mid + i];
-      if (T::DYN && !((cur[v >> 5] >> (v & 31u)) & 1u)) continue;
-      const uint32_t s = a.xtoff[v], d = a.xtoff[v + 1] - s;
-      const double x = mid_row_sum<double, true>(c, a.xtedg + s, d, lane);
-      if (lane == 0) finish_one(v, x, d);
-    }
-    for (uint32_t w = w0; w < words; w += warps) {
+    // a word's bookkeeping in the dynamic modes; returns its affected vertices
+    auto word_pass = [&](uint32_t w) -> uint32_t {
       const uint32_t v = (w << 5) | lane;
-      bool mine = v < a.n && ((a.low_bm[w] >> lane) & 1u);
+      const uint32_t cw = cur[w], pw = prev[w];
+      if (T::FRONTIER && lane == 0) marked += __popc(cw);
+      if (((pw & ~cw) >> lane) & 1u) {  // updated last iteration, not this one: refresh parity p^1
+        a.r[p ^ 1][v] = a.r[p][v];
+        a.c[p ^ 1][v] = c[v];
+      }
+      if (lane == 0) {
+        if (pw) prev[w] = 0;  // becomes the empty nxt of the next iteration
+        if (T::FRONTIER && a.nf[p ^ 1][w]) a.nf[p ^ 1][w] = 0;
+      }
+      return cw;
+    };
+    for (uint32_t i = blockIdx.x; i < rows.nlong; i += gridDim.x) {
+      const uint32_t v = __ldg(rows.list + rows.nlow + rows.nmid + i);
+      if (!affected(v)) continue;
+      const uint32_t s = __ldg(a.xtoff + v), d = __ldg(a.xtoff + v + 1) - s;
+      const VertexIn in = load_vertex(a, v, p);
+      const double x = high_row_sum<double, true, true>(c, a.xtedg + s, d, t, part);
+      if (t == 0) finish_one(v, x, d, in);
+    }
+    for (uint32_t u = warp; u < rows.nmid; u += warps) {
+      const Unit x = u == warp ? first : load_unit(u);
+      if (!affected(x.v)) continue;
+      const VertexIn in = {x.d, x.R, a.r[p][x.v]};
+      const double sum = mid_row_sum<double, true, true>(c, a.xtedg + x.s, x.e - x.s, lane);
+      if (lane == 0) finish_one(x.v, sum, x.e - x.s, in);
+    }
+    for (uint32_t u = low0; u < units; u += warps) {
+      const Unit x = u == warp ? first : load_unit(u);
+      bool mine = x.row;
       if (T::DYN) {
-        const uint32_t cw = cur[w], pw = prev[w];
-        if (T::FRONTIER && lane == 0) marked += __popc(cw);
-        if (((pw & ~cw) >> lane) & 1u) {  // updated last iteration, not this one: refresh parity p^1
-          a.r[p ^ 1][v] = a.r[p][v];
-          a.c[p ^ 1][v] = c[v];
+        if (rows.sorted) {
+          mine = mine && affected(x.v);
+        } else {
+          const uint32_t cw = word_pass(u - rows.nmid);  // every lane: MID rows have stale copies too
+          mine = mine && ((cw >> lane) & 1u);
         }
-        if (lane == 0) {
-          if (pw) prev[w] = 0;  // becomes the empty nxt of the next iteration
-          if (T::FRONTIER && a.nf[p ^ 1][w]) a.nf[p ^ 1][w] = 0;
-        }
-        mine = mine && ((cw >> lane) & 1u);
         if (!__any_sync(0xffffffffu, mine)) continue;
       }
-      const uint32_t s = mine ? a.xtoff[v] : 0, e = mine ? a.xtoff[v + 1] : 0;
-      const double sum = warp_row_sums<true>(c, a.xtedg, s, e, 0.0, nullptr, false, a.int_adds);
+      VertexIn in = {x.d, x.R, 0.0};
+      if (mine) in.r = a.r[p][x.v];
+      const double sum = warp_row_sums<true, true, 1, K>(c, a.xtedg, x.s, mine ? x.e : x.s, 0.0, nullptr, false);
+      if (!T::DYN || rows.sorted) {
+        if (mine) finish_one(x.v, sum, x.e - x.s, in);
+        continue;
+      }
+      // the lanes are one word: its bits go out together
       bool survive = false, changed = false;
       if (mine) {
-        const unsigned long long ev = finish_vertex<MODE>(a, v, sum, p, survive, changed, mag);
+        const unsigned long long ev = finish_vertex<MODE>(a, x.v, sum, p, survive, changed, mag, in);
         emax = ev > emax ? ev : emax;
-        edges += e - s;
+        edges += x.e - x.s;
       }
-      if (T::DYN) {
-        const unsigned keep = __ballot_sync(0xffffffffu, mine && survive);
-        if (lane == 0 && keep) atomicOr(&nxt[w], keep);
-      }
+      const uint32_t w = u - rows.nmid;
+      const unsigned keep = __ballot_sync(0xffffffffu, mine && survive);
+      if (lane == 0 && keep) atomicOr(&nxt[w], keep);
       if (T::FRONTIER) {
         const unsigned chg = fresh_changes<T::PRUNE>(a.naff, w, __ballot_sync(0xffffffffu, mine && changed), lane);
         if (chg) {
@@ -213,10 +270,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_persist(SolveArgs a, PersistRow
             atomicOr(&a.nf[p][w], chg);
             atomicAdd(&st->pnf[it % 3], (uint32_t)__popc(chg));
           }
-          if (((chg >> lane) & 1u) && a.xtdat[v] > kWarpExpand) push(a.xb, &st->pxb[it % 3], v);
+          if (((chg >> lane) & 1u) && in.d > kWarpExpand) push(a.xb, &st->pxb[it % 3], x.v);
         }
       }
     }
+    if (T::DYN && rows.sorted)
+      for (uint32_t w = warp; w < words; w += warps) word_pass(w);
     block_max_bits(emax, &st->pel[it % 3]);
     if (T::FRONTIER) block_sum_u32(marked, &st->pmarked[it % 3]);
     if (blockIdx.x == 0 && t == 0) {  // the next iteration's slots (last read two barriers ago)
@@ -250,36 +309,48 @@ __global__ void __launch_bounds__(kThreads, 4) k_persist(SolveArgs a, PersistRow
   if (T::DYN) block_sum_u64(edges, &st->edges);
 }
 
-template <int MODE>
-static cudaError_t persist_t(const SolveArgs& a, const PersistRows& rows, int sms, int* per_sm, cudaStream_t s) {
-  if (!*per_sm) {
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_persist<MODE>, kThreads, 0);
-    if (e != cudaSuccess) return e;
-  }
-  // a warp per MID row and 32-id word, a block per HIGH row; no more blocks than are resident
-  const uint64_t units = (uint64_t)rows.nmid + ((uint64_t)a.n + 31) / 32;
-  const uint64_t want = rows.nhigh + (units + kThreads / 32 - 1) / (kThreads / 32);
-  const int grid = (int)std::min<uint64_t>(std::max<uint64_t>(want, 1), (uint64_t)*per_sm * sms);
+template <int MODE, int K>
+static cudaError_t persist_k(const SolveArgs& a, const PersistRows& rows, uint64_t want, int threads, int sms,
+                             cudaStream_t s) {
+  int per_sm = 0;  // resident blocks per SM of this build
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist<MODE, K>, threads, 0);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
+  cfg.gridDim = dim3((unsigned)std::min<uint64_t>(want, (uint64_t)per_sm * sms));
+  cfg.blockDim = dim3(threads);
   cfg.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeCooperative;
   at.val.cooperative = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_persist<MODE>, a, rows);
+  return cudaLaunchKernelEx(&cfg, k_persist<MODE, K>, a, rows);
 }
 
-cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, int per_sm[4], cudaStream_t s) {
-  const PersistRows rows = {g.cls_begin[MID], g.cls_begin[HIGH] - g.cls_begin[MID], g.cls_begin[HIGH],
-                            g.cls_begin[NCLS] - g.cls_begin[HIGH]};
+template <int MODE>
+static cudaError_t persist_t(const SolveArgs& a, const PersistRows& rows, int sms, cudaStream_t s) {
+  // a warp per unit and a block per long row; no more blocks than are resident
+  const uint64_t units = (uint64_t)rows.nmid + ((uint64_t)(rows.sorted ? rows.nlow : a.n) + 31) / 32;
+  // A few units go to more SMs in smaller blocks (long rows need 256
+  // threads): the warps of an SM share its FP64 pipe.
+  const int threads = rows.nlong || units > 4ull * sms ? kThreads : units > 2ull * sms ? 128 : 64;
+  const uint64_t per = threads / 32;
+  const uint64_t want = std::max<uint64_t>(1, rows.nlong + (units + per - 1) / per);
+  // two of four adds on the integer pipes (one gives 2% less on a web-like
+  // graph of 1.5M vertices); four warps an SM leave its FP64 pipe idle for
+  // the latency of their adds (R-MAT 2^13: 6.4 us an iteration without, 7.2 with)
+  return a.int_adds && units > 4ull * sms ? persist_k<MODE, 2>(a, rows, want, threads, sms, s)
+                                          : persist_k<MODE, 0>(a, rows, want, threads, sms, s);
+}
+
+cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, cudaStream_t s) {
+  const PersistRows rows = {g.plan_list, g.plan_begin[MID], g.plan_begin[HIGH] - g.plan_begin[MID],
+                            g.plan_begin[NCLS] - g.plan_begin[HIGH], mixed_lengths(g)};
   switch (mode) {
-    case PRX_DYNAMIC_TRAVERSAL: return persist_t<PRX_DYNAMIC_TRAVERSAL>(a, rows, sms, &per_sm[1], s);
-    case PRX_DYNAMIC_FRONTIER: return persist_t<PRX_DYNAMIC_FRONTIER>(a, rows, sms, &per_sm[2], s);
-    case PRX_PRUNE_DYNAMIC_FRONTIER: return persist_t<PRX_PRUNE_DYNAMIC_FRONTIER>(a, rows, sms, &per_sm[3], s);
-    default: return persist_t<PRX_STATIC>(a, rows, sms, &per_sm[0], s);
+    case PRX_DYNAMIC_TRAVERSAL: return persist_t<PRX_DYNAMIC_TRAVERSAL>(a, rows, sms, s);
+    case PRX_DYNAMIC_FRONTIER: return persist_t<PRX_DYNAMIC_FRONTIER>(a, rows, sms, s);
+    case PRX_PRUNE_DYNAMIC_FRONTIER: return persist_t<PRX_PRUNE_DYNAMIC_FRONTIER>(a, rows, sms, s);
+    default: return persist_t<PRX_STATIC>(a, rows, sms, s);
   }
 }
 

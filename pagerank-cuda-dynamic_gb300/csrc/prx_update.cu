@@ -48,7 +48,8 @@ enum Pass { PASS_ONLY = 0, PASS_FIRST = 1, PASS_INNER = 2, PASS_LAST = 3 };
 
 // hot: the layout encodes hot sources (the FP64 modes); their contributions
 // are gathered from a.ch[p].
-template <int MODE, int PASS>
+// K: adds of every step by soft_add (the FP64 modes).
+template <int MODE, int PASS, int K>
 __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
     k_update_low(SolveArgs a, uint32_t vb, uint32_t ve, const unsigned long long* __restrict__ base, uint32_t shift,
                  const uint32_t* __restrict__ off, const uint32_t* __restrict__ edg, bool hot) {
@@ -115,12 +116,14 @@ __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
       if (mine) acc = lane_row_sum(c, seg_edges(edg, base, shift, v), s, e, FIRST ? V(0) : carried_of<MODE>(a)[v]);
     } else {  // the whole warp sums together
       const V init = (mine && !FIRST) ? carried_of<MODE>(a)[v] : V(0);
-      acc = warp_row_sums(c, seg_edges(edg, base, shift, v), s, mine ? e : s, init, ch, hot, a.int_adds);
+      acc = warp_row_sums<false, FIRST, 0, K>(c, seg_edges(edg, base, shift, v), s, mine ? e : s, init, ch, hot);
     }
     if (mine) {
       edges += e - s;
       if (LAST) {
-        const unsigned long long ev = finish_vertex<MODE>(a, v, acc, p, survive, changed, mag);
+        VertexIn in{};
+        if constexpr (!T::F32) in = load_vertex(a, v, p);
+        const unsigned long long ev = finish_vertex<MODE>(a, v, acc, p, survive, changed, mag, in);
         emax = ev > emax ? ev : emax;
       } else {
         carried_of<MODE>(a)[v] = acc;
@@ -162,7 +165,9 @@ template <int MODE>
 __device__ __forceinline__ void finish_listed(const SolveArgs& a, uint32_t v, typename ModeTraits<MODE>::V x, int p,
                                               unsigned long long& emax, unsigned int& mag) {
   bool survive, changed;
-  const unsigned long long ev = finish_vertex<MODE>(a, v, x, p, survive, changed, mag);
+  VertexIn in{};
+  if constexpr (!ModeTraits<MODE>::F32) in = load_vertex(a, v, p);
+  const unsigned long long ev = finish_vertex<MODE>(a, v, x, p, survive, changed, mag, in);
   emax = ev > emax ? ev : emax;
   if (ModeTraits<MODE>::DYN && survive) atomicOr(&a.bm[(a.st->iter + 1) % 3][v >> 5], 1u << (v & 31u));
   if (ModeTraits<MODE>::FRONTIER && changed && (ModeTraits<MODE>::PRUNE || test_and_set(a.naff, v))) {
@@ -192,7 +197,7 @@ __global__ void __launch_bounds__(kThreads) k_update_mid(SolveArgs a, uint32_t b
     const uint64_t iv = seg_index(v, a.seg_shift);
     const uint32_t s = a.xtoff[iv], d = a.xtoff[iv + 1] - s;
     const uint32_t* __restrict__ ed = seg_edges(a.xtedg, a.xtbase, a.seg_shift, v) + s;
-    const V x = mid_row_sum<V, false>(c, ed, d, lane);
+    const V x = mid_row_sum<V, false, false>(c, ed, d, lane);
     if (lane == 0) {
       finish_listed<MODE>(a, v, x, p, emax, mag);
       edges += d;
@@ -223,7 +228,7 @@ __global__ void __launch_bounds__(256) k_update_high(SolveArgs a, uint32_t begin
     const uint64_t iv = seg_index(v, a.seg_shift);
     const uint32_t s = a.xtoff[iv], d = a.xtoff[iv + 1] - s;
     const uint32_t* __restrict__ ed = seg_edges(a.xtedg, a.xtbase, a.seg_shift, v) + s;
-    const V x = high_row_sum<V, false>(c, ed, d, t, part);
+    const V x = high_row_sum<V, false, false>(c, ed, d, t, part);
     if (t == 0) {
       finish_listed<MODE>(a, v, x, p, emax, mag);
       edges += d;
@@ -447,6 +452,16 @@ void launch_commit_dyn32(const SolveArgs& a, int parity, cudaStream_t s) {
   k_commit_dyn32<<<cap_grid((a.n + kThreads - 1) / kThreads, 152 * 16), kThreads, 0, s>>>(a, parity);
 }
 
+template <int MODE, int PASS>
+static void low_pass(int grid, cudaStream_t s, const SolveArgs& a, uint32_t vb, uint32_t ve,
+                     const unsigned long long* base, uint32_t shift, const uint32_t* off, const uint32_t* edg,
+                     bool hot) {
+  if (a.int_adds && !ModeTraits<MODE>::F32)
+    k_update_low<MODE, PASS, ModeTraits<MODE>::F32 ? 0 : 1><<<grid, kThreads, 0, s>>>(a, vb, ve, base, shift, off, edg, hot);
+  else
+    k_update_low<MODE, PASS, 0><<<grid, kThreads, 0, s>>>(a, vb, ve, base, shift, off, edg, hot);
+}
+
 template <int MODE>
 static bool update_class_t(const SolveArgs& a, const GraphDev& g, int cls, const ChunkLayout* lay, int sms,
                            cudaStream_t s) {
@@ -458,8 +473,7 @@ static bool update_class_t(const SolveArgs& a, const GraphDev& g, int cls, const
     if (!lay || (lay->K <= 1 && !lay->hot)) {
       const uint64_t words = ((uint64_t)g.n + 31) / 32;
       const int grid = cap_grid((words + 7) / 8, sms * ModeTraits<MODE>::LOW_BLOCKS);
-      k_update_low<MODE, PASS_ONLY>
-          <<<grid, kThreads, 0, s>>>(a, 0, g.n, g.xtbase, g.seg_shift, g.xtoff, g.xtedg, false);
+      low_pass<MODE, PASS_ONLY>(grid, s, a, 0, g.n, g.xtbase, g.seg_shift, g.xtoff, g.xtedg, false);
       return true;
     }
     const bool hot = lay->hot && a.hot_n > 0;
@@ -475,13 +489,13 @@ static bool update_class_t(const SolveArgs& a, const GraphDev& g, int cls, const
       for (int k = 0; k < lay->K; ++k) {
         const uint32_t* off = offs + k * row;
         if (lay->K == 1)
-          k_update_low<MODE, PASS_ONLY><<<grid, kThreads, 0, s>>>(a, v0, v1, nullptr, 32, off, edg, hot);
+          low_pass<MODE, PASS_ONLY>(grid, s, a, v0, v1, nullptr, 32, off, edg, hot);
         else if (k == 0)
-          k_update_low<MODE, PASS_FIRST><<<grid, kThreads, 0, s>>>(a, v0, v1, nullptr, 32, off, edg, hot);
+          low_pass<MODE, PASS_FIRST>(grid, s, a, v0, v1, nullptr, 32, off, edg, hot);
         else if (k == lay->K - 1)
-          k_update_low<MODE, PASS_LAST><<<grid, kThreads, 0, s>>>(a, v0, v1, nullptr, 32, off, edg, hot);
+          low_pass<MODE, PASS_LAST>(grid, s, a, v0, v1, nullptr, 32, off, edg, hot);
         else
-          k_update_low<MODE, PASS_INNER><<<grid, kThreads, 0, s>>>(a, v0, v1, nullptr, 32, off, edg, hot);
+          low_pass<MODE, PASS_INNER>(grid, s, a, v0, v1, nullptr, 32, off, edg, hot);
       }
     }
     return true;

@@ -15,10 +15,10 @@ template <int MODE> struct ModeTraits {
   static constexpr bool FRONTIER = DYN && BASE >= PRX_DYNAMIC_FRONTIER;
   static constexpr bool PRUNE = BASE == PRX_PRUNE_DYNAMIC_FRONTIER;
   using V = typename std::conditional<F32, float, double>::type;  // rank / contribution type
-  // resident blocks of 256 per SM the LOW kernel is compiled (register
-  // budget) and launched for: the dynamic modes' bookkeeping needs more than
-  // 32 registers a thread
-  static constexpr int LOW_BLOCKS = (DYN || F32) ? 6 : 8;
+  // resident blocks of 256 per SM the LOW kernel is compiled (40 registers a
+  // thread) and launched for.  Static, us a sweep at 7 | 6 | 5: web-like 20M
+  // 2591 | 2310 | 2297, 3M 351 | 323 | 318, grid 4096^2 342 | 342 | 380.
+  static constexpr int LOW_BLOCKS = 6;
 };
 
 // Rank, contribution and carried-sum arrays of a mode: FP64 r / c / acc64,
@@ -51,6 +51,21 @@ __device__ __forceinline__ void set_bit(uint32_t* bm, uint32_t w) {
   if (!(bm[w >> 5] & bit)) atomicOr(&bm[w >> 5], bit);
 }
 
+// What an FP64 update of a vertex reads besides its row (loaded before the
+// row where latency counts).
+struct VertexIn {
+  uint32_t d;      // out-degree
+  uint64_t R;      // its reciprocal from the table (0: none)
+  double r;        // rank before the update
+};
+__device__ __forceinline__ VertexIn load_vertex(const SolveArgs& a, uint32_t v, int p) {
+  VertexIn x;
+  x.d = __ldg(a.xtdat + v);
+  x.r = a.r[p][v];
+  x.R = x.d < kQuotTable ? __ldg(a.qtab + x.d) : 0ull;
+  return x;
+}
+
 // Finish vertex v given its contribution sum.  Returns |a_v - r_v| as bits
 // (of a double; an FP32 change converts exactly).  survive (dynamic): v stays
 // affected next iteration; changed (DF / DF-P): its relative change exceeded
@@ -60,10 +75,10 @@ __device__ __forceinline__ void set_bit(uint32_t* bm, uint32_t w) {
 template <int MODE>
 __device__ __forceinline__ unsigned long long finish_vertex(const SolveArgs& a, uint32_t v,
                                                             typename ModeTraits<MODE>::V cv, int p, bool& survive,
-                                                            bool& changed, unsigned int& mag) {
+                                                            bool& changed, unsigned int& mag, const VertexIn& in) {
   using T = ModeTraits<MODE>;
-  const uint32_t d = a.xtdat[v];
   if constexpr (T::F32) {
+    const uint32_t d = a.xtdat[v];
     const float P = (float)a.P, C0 = (float)a.C0, df = (float)d;
     const float rv = a.e[p][v];
     float av;
@@ -83,10 +98,10 @@ __device__ __forceinline__ unsigned long long finish_vertex(const SolveArgs& a, 
     }
     return dbits((double)ev);
   } else {
-    const double y = a.rcp[v];
-    const double rv = a.r[p][v];
+    const uint32_t d = in.d;
+    const double rv = in.r;
     double av;
-    // c[p][v] is div_count(rv, d, y), formed when rv was; pf: 1 / (1 - P/d)
+    // c[p][v] is RN(rv / d), formed when rv was; pf: 1 / (1 - P/d)
     if (T::PRUNE) av = fma(a.P, cv - a.c[p][v], a.C0) * a.pf[v];
     else          av = fma(a.P, cv, a.C0);
     const double ev = fabs(av - rv);
@@ -98,7 +113,7 @@ __device__ __forceinline__ unsigned long long finish_vertex(const SolveArgs& a, 
       a.e[0][v] = rho;
       a.ce[0][v] = __fdividef(rho, (float)d);
     } else {
-      a.c[p ^ 1][v] = div_count(av, d, y);
+      a.c[p ^ 1][v] = div_outdeg(av, d, in.R, a.rcp + v);
     }
     survive = true;
     changed = false;
@@ -149,54 +164,164 @@ __device__ __forceinline__ V load_c(const V* c) {
   else return __ldg(c);
 }
 
+// The integer pipes take about half of the FP64 adds of the MID and HIGH sums
+// (soft_add): GB300's FP64 pipe needs 20 cycles a warp-wide add, soft_add 14
+// of the integer pipes'.  It needs every term to be normal and below 2^977;
+// sums that meet another one (zero, negative, subnormal, huge: a caller's
+// ranks) are formed again by FP64 adds.  A slot without a term holds +0.0,
+// whose unpacked form vanishes against any term; two empty slots give 2^-1022
+// and more, which vanishes too, and the sum asked for has at least one term.
+__device__ __forceinline__ double soft_plus(double a, double b) {
+  return __longlong_as_double((long long)soft_pack(
+      soft_add(soft_unpack((uint64_t)__double_as_longlong(a)), (uint64_t)__double_as_longlong(b))));
+}
+__device__ __forceinline__ bool soft_out_of_range(double x) {
+  return (uint32_t)__double2hiint(x) - kSoftMinHi >= kSoftAddHiLimit - kSoftMinHi;
+}
+
+// a + b by the FP64 pipe or, with SOFT, the integer pipes.
+template <bool SOFT, class V>
+__device__ __forceinline__ V plus(V a, V b) {
+  if constexpr (SOFT) return soft_plus(a, b);
+  else return a + b;
+}
+
 // MID: the reference's 256-way sum of c over the d ids at ed, by one warp.
-// Lane l owns virtual threads l + 32k (k = 0..7); the sum is in lane 0.
-template <class V, bool COH>
-__device__ __forceinline__ V mid_row_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t lane) {
+// Lane l owns virtual threads l + 32k (k = 0..7); the sum is in lane 0.  The
+// first 256 terms are not added (to +0) but are the partial sums, and neither
+// the second terms' adds nor the tree's first level run for slots that hold
+// none: of 28 warp-wide adds for a row of 275 terms, 12 are left.
+// PRE: the ids of the next 256 terms are loaded behind the gathers of these
+// (few warps, where the latency of the two loads counts; 8 more registers).
+template <class V, bool COH, bool SOFT, bool PRE>
+__device__ __forceinline__ V mid_row_sum_t(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t lane,
+                                           bool& bad) {
   V ps[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) ps[k] = V(0);
-  for (uint32_t base = 0; base < d; base += 256) {
-    uint32_t u[8];
+  uint32_t u[8];
+  auto ids = [&](uint32_t base) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const uint32_t t = base + lane + 32u * k;
       u[k] = t < d ? __ldg(ed + t) : 0u;
     }
+  };
+  if (PRE) ids(0);
+  for (uint32_t base = 0; base < d; base += 256) {
+    if (!PRE) ids(base);
     V x[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = (base + lane + 32u * k < d) ? load_c<COH>(c + u[k]) : V(0);
+    for (int k = 0; k < 8; ++k) x[k] = base + lane + 32u * k < d ? load_c<COH>(c + u[k]) : V(0);
+    if (PRE) ids(base + 256);
+    if (SOFT) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) ps[k] += x[k];
+      for (int k = 0; k < 8; ++k) bad = bad || (base + lane + 32u * k < d && soft_out_of_range(x[k]));
+    }
+    if (base == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) ps[k] = SOFT ? x[k] : V(0) + x[k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        if (base + 32u * k < d) ps[k] += x[k];
+        if (base + 32u * (k + 1) < d) ps[k + 1] = plus<SOFT>(ps[k + 1], x[k + 1]);
+      }
+    }
   }
-  // halving tree over virtual thread t = lane + 32k
-  ps[0] += ps[4]; ps[1] += ps[5]; ps[2] += ps[6]; ps[3] += ps[7];  // t < 128: += t+128
-  ps[0] += ps[2]; ps[1] += ps[3];                                  // t < 64:  += t+64
-  ps[0] += ps[1];                                                  // t < 32:  += t+32
-  V x = ps[0];
-#pragma unroll
+  // halving tree over virtual thread t = lane + 32k; d > 64
+  if (d > 128) ps[0] += ps[4];                            // t < 128: += t+128
+  if (d > 160) ps[1] = plus<SOFT>(ps[1], ps[5]);
+  if (d > 192) ps[2] += ps[6];
+  if (d > 224) ps[3] = plus<SOFT>(ps[3], ps[7]);
+  ps[0] += ps[2];                                         // t < 64:  += t+64
+  ps[1] = plus<SOFT>(ps[1], ps[3]);
+  V x = ps[0] + ps[1];                                    // t < 32:  += t+32
+  x = plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 16));
+  x += __shfl_down_sync(0xffffffffu, x, 8);
+  x = plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 4));
+  x += __shfl_down_sync(0xffffffffu, x, 2);
+  x = plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 1));
+  return x;
+}
+// The same by FP64 adds alone, rolled up: it runs on terms out of
+// soft_add's range only, and must not add to the sweep's registers.
+template <bool COH>
+__device__ __forceinline__ double mid_row_sum_plain(const double* c, const uint32_t* __restrict__ ed, uint32_t d,
+                                                    uint32_t lane) {
+  double ps[8];
+#pragma unroll 1
+  for (int k = 0; k < 8; ++k) {
+    double sum = 0.0;
+#pragma unroll 1
+    for (uint32_t t = lane + 32u * k; t < d; t += 256) sum += load_c<COH>(c + __ldg(ed + t));
+    ps[k] = sum;
+  }
+#pragma unroll 1
+  for (int o = 4; o; o >>= 1)
+#pragma unroll 1
+    for (int k = 0; k < o; ++k) ps[k] += ps[k + o];
+  double x = ps[0];
+#pragma unroll 1
   for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  return x;
+}
+template <class V, bool COH, bool PRE>
+__device__ __forceinline__ V mid_row_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t lane) {
+  constexpr bool SOFT = std::is_same<V, double>::value;
+  bool bad = false;
+  const V x = mid_row_sum_t<V, COH, SOFT, PRE>(c, ed, d, lane, bad);
+  if constexpr (SOFT) {
+    if (__any_sync(0xffffffffu, bad)) return mid_row_sum_plain<COH>(c, ed, d, lane);
+  }
   return x;
 }
 
 // HIGH: the same sum by a block of 256 (thread t of the reference's block);
-// part: 256 values of shared memory.  The sum is in thread 0.
-template <class V, bool COH>
-__device__ __forceinline__ V high_row_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t t,
-                                          V* part) {
+// part: 256 values of shared memory.  The sum is in thread 0.  Eight gathers
+// are in flight, in the last batch too (empty slots add +0.0).
+template <class V, bool COH, bool SOFT, bool PRE>
+__device__ __forceinline__ V high_thread_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t t,
+                                             bool& bad) {
   V acc = V(0);
-  uint32_t j = t;
-  for (; j + 7 * 256 < d; j += 8 * 256) {
-    uint32_t u[8];
+  uint32_t u[8];
+  auto ids = [&](uint32_t base) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) u[k] = __ldg(ed + j + 256 * k);
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t j = base + 256 * k + t;
+      u[k] = j < d ? __ldg(ed + j) : 0u;
+    }
+  };
+  if (PRE) ids(0);
+  for (uint32_t base = 0; base < d; base += 8 * 256) {
+    if (!PRE) ids(base);
     V x[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = load_c<COH>(c + u[k]);
+    for (int k = 0; k < 8; ++k) x[k] = base + 256 * k + t < d ? load_c<COH>(c + u[k]) : V(0);
+    if (PRE) ids(base + 8 * 256);
+    if (SOFT) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc += x[k];
+      for (int k = 0; k < 8; ++k) bad = bad || (base + 256 * k + t < d && soft_out_of_range(x[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (base + 256 * k < d) {
+        if (SOFT && k < 4) acc = plus<SOFT>(acc, x[k]);
+        else acc += x[k];
+      }
   }
-  for (; j < d; j += 256) acc += load_c<COH>(c + __ldg(ed + j));
+  return acc;
+}
+template <class V, bool COH, bool PRE>
+__device__ __forceinline__ V high_row_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t t, V* part) {
+  constexpr bool SOFT = std::is_same<V, double>::value;
+  bool bad = false;
+  V acc = high_thread_sum<V, COH, SOFT, PRE>(c, ed, d, t, bad);
+  if constexpr (SOFT) {
+    if (__syncthreads_or(bad)) {
+      acc = 0.0;
+#pragma unroll 1
+      for (uint32_t j = t; j < d; j += 256) acc += load_c<COH>(c + __ldg(ed + j));
+    }
+  }
   part[t] = acc;
   __syncthreads();
   if (t < 128) part[t] += part[t + 128];
