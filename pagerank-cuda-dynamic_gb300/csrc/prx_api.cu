@@ -1061,7 +1061,7 @@ int prx_graph_destroy(prx_graph* gr) {
   if (!gr) return PRX_OK;
   cudaSetDevice(gr->g.device);
   GraphDev& g = gr->g;
-  graph_free({g.xoff, g.xedg, g.xtoff, g.xtedg, g.xtdat, g.cls_list, g.plan_list, g.xbase, g.xtbase,
+  graph_free({g.xoff, g.xedg, g.xtoff, g.xtedg, g.xtdat, g.cls_list, g.plan_list, g.len_list, g.xbase, g.xtbase,
               g.low_bm, g.rcp, g.rcp32});
   drop_weights(g);
   cudaFree(g.ocls_list);

@@ -795,7 +795,7 @@ cudaError_t ensure_hot(GraphDev& g, uint32_t cap, int sms, cudaStream_t s) {
 
 cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layouts) {
   const uint32_t n = g.n;
-  g.plan_built = false;
+  g.plan_built = g.len_built = false;
   if (!keep_layouts) {
     free_chunks(g);
     free_hot(g);
@@ -840,34 +840,41 @@ __global__ void k_key_ids(const unsigned long long* __restrict__ key, uint32_t c
     list[i] = (uint32_t)key[i];
 }
 
+cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s) {
+  const uint32_t low = g.cls_begin[MID];
+  if (g.len_built || low == 0) return cudaSuccess;
+  unsigned long long *key = nullptr, *tmp = nullptr, *sorted = nullptr;
+  uint32_t* hist = nullptr;
+  cudaError_t e = g.len_list ? cudaSuccess : graph_alloc(&g.len_list, sizeof(uint32_t) * g.n, s);
+  if (e == cudaSuccess) e = graph_alloc(&key, sizeof(*key) * ((size_t)low + 2), s);
+  if (e == cudaSuccess) e = graph_alloc(&tmp, sizeof(*tmp) * ((size_t)low + 2), s);
+  if (e == cudaSuccess) e = graph_alloc(&hist, sizeof(uint32_t) * radix_hist_words(low), s);
+  if (e == cudaSuccess) {
+    k_len_keys<<<sms * 4, 256, 0, s>>>(g.xtoff, g.cls_list, low, key);
+    e = radix_sort_u64(key, tmp, low, 32, 39, hist, sms, s, &sorted);
+    if (e == cudaSuccess) k_key_ids<<<sms * 4, 256, 0, s>>>(sorted, low, g.len_list);
+    if (e == cudaSuccess) e = cudaGetLastError();
+  }
+  if (key) cudaFreeAsync(key, s);
+  if (tmp) cudaFreeAsync(tmp, s);
+  if (hist) cudaFreeAsync(hist, s);
+  g.len_built = e == cudaSuccess;
+  return e;
+}
+
 cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s) {
-  if (g.plan_built || g.n == 0) return cudaSuccess;
-  cudaError_t e = cudaSuccess;
-  if (!g.plan_list) e = graph_alloc(&g.plan_list, sizeof(uint32_t) * g.n, s);
+  if (g.n == 0) return cudaSuccess;
+  if (mixed_lengths(g)) {
+    const cudaError_t e = ensure_len_list(g, sms, s);
+    if (e != cudaSuccess) return e;
+  }
+  if (g.plan_built) return cudaSuccess;
+  cudaError_t e = g.plan_list ? cudaSuccess : graph_alloc(&g.plan_list, sizeof(uint32_t) * g.n, s);
   uint64_t edges[NCLS];
   if (e == cudaSuccess)
     e = build_class_lists(g.xtoff, g.seg_shift, g.n, kPlanMid, g.plan_list, g.plan_begin, edges, sms, s);
-  if (e != cudaSuccess) return e;
-  if (mixed_lengths(g)) {
-    const uint32_t low = g.plan_begin[MID];
-    unsigned long long *key = nullptr, *tmp = nullptr, *sorted = nullptr;
-    uint32_t* hist = nullptr;
-    e = graph_alloc(&key, sizeof(*key) * ((size_t)low + 2), s);
-    if (e == cudaSuccess) e = graph_alloc(&tmp, sizeof(*tmp) * ((size_t)low + 2), s);
-    if (e == cudaSuccess) e = graph_alloc(&hist, sizeof(uint32_t) * radix_hist_words(low), s);
-    if (e == cudaSuccess) {
-      k_len_keys<<<sms * 4, 256, 0, s>>>(g.xtoff, g.plan_list, low, key);
-      e = radix_sort_u64(key, tmp, low, 32, 39, hist, sms, s, &sorted);
-      if (e == cudaSuccess) k_key_ids<<<sms * 4, 256, 0, s>>>(sorted, low, g.plan_list);
-    }
-    if (key) cudaFreeAsync(key, s);
-    if (tmp) cudaFreeAsync(tmp, s);
-    if (hist) cudaFreeAsync(hist, s);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  g.plan_built = true;
-  return cudaSuccess;
+  g.plan_built = e == cudaSuccess;
+  return e;
 }
 
 cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, uint32_t mid_max, uint32_t* list,

@@ -69,6 +69,7 @@ struct State {
   uint32_t pnf[3];                // DF / DF-P: vertices whose change exceeded D
   uint32_t pxb[3];                // ... of them of out-degree > kWarpExpand, queued in xb
   uint32_t pmarked[3];            // vertices affected in it
+  uint32_t work;                  // personalized PageRank: units of a sweep taken
 };
 
 // Device error codes (State::err bits).
@@ -156,9 +157,11 @@ struct GraphDev {
   uint32_t hot_n = 0;
   uint32_t hot_cap = 0;
   bool hot_built = false;
-  // Rows of the persistent loop (prx_persist.cu), built on first use per graph
-  // version: plan_list holds the LOW ids (by length when mixed_lengths, else
-  // ascending), then those of 65 to kPlanMid in-edges, then the longer ones.
+  // Built on first use per graph version: the LOW ids in order of in-degree
+  // (ties ascending), and the ids by class with kPlanMid as the MID / HIGH
+  // boundary (the persistent loop's rows).
+  uint32_t* len_list = nullptr;
+  bool len_built = false;
   uint32_t* plan_list = nullptr;
   uint32_t plan_begin[NCLS + 1] = {0, 0, 0, 0};
   bool plan_built = false;
@@ -287,7 +290,9 @@ constexpr uint32_t kDefaultChunk64 = (200u << 20) / sizeof(double);
 // side by side (8 lanes of 9 wait), web-like ones and grids stay in id order
 // (1.35), whose rows and ranks lie side by side in memory.
 inline bool mixed_lengths(const GraphDev& g) { return g.low_padded > 2 * g.cls_edges[LOW]; }
-// The persistent loop's rows of g (GraphDev::plan_list).
+// GraphDev::len_list (plain graphs), and the persistent loop's rows: plan_list,
+// and len_list where the lengths mix.
+cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s);
 constexpr uint32_t kPlanMid = 1024;
 // Largest graphs it takes, in units of a MID row or 32 LOW rows: in id order
 // and by length.

@@ -294,6 +294,7 @@ __global__ void k_state_reset(State* st, int max_iter, double tol) {
   st->q_done = 0;
   st->el32_prev[0] = st->el32_prev[1] = 0;
   st->bar = 0;
+  st->work = 0;
   for (int k = 0; k < 3; ++k) {
     st->pel[k] = 0;
     st->pnf[k] = st->pxb[k] = st->pmarked[k] = 0;

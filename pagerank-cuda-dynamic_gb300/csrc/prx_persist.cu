@@ -13,7 +13,7 @@
 // What bounds it: latency (offsets -> ids -> contributions -> the row's adds
 // -> barrier), then the FP64 pipe.
 //
-// Work split (GraphDev::plan_list): rows of more than kPlanMid in-edges by
+// Work split: rows of more than kPlanMid in-edges by
 // block (row i to block i mod blocks), the others by warp as units of one
 // MID row or 32 LOW rows, counted from the last warp backwards so that the
 // blocks that hold long rows get the units of the last round.  LOW rows of
@@ -34,9 +34,10 @@
 namespace prx {
 
 struct PersistRows {
-  const uint32_t* list;  // GraphDev::plan_list: nlow LOW ids, nmid MID ids, nlong longer ones
+  const uint32_t* low;   // LOW ids in order of length (GraphDev::len_list)
+  const uint32_t* list;  // nmid MID ids, then nlong longer ones (GraphDev::plan_list)
   uint32_t nlow, nmid, nlong;
-  bool sorted;           // the LOW ids are in order of length
+  bool sorted;           // whether the LOW rows go by `low`, or word by word
 };
 
 // Expansion of the changed vertices (nf[p]) into nxt, whichever way
@@ -91,7 +92,7 @@ __device__ __forceinline__ void persist_pull(const SolveArgs& a, const PersistRo
                                              uint32_t* nxt, uint32_t warp, uint32_t warps) {
   const uint32_t words = (a.n + 31) >> 5, lane = lane_id();
   for (uint32_t i = warp; i < rows.nmid + rows.nlong; i += warps) {
-    const uint32_t v = rows.list[rows.nlow + i];
+    const uint32_t v = rows.list[i];
     if ((nxt[v >> 5] >> (v & 31u)) & 1u) continue;
     const uint32_t e = a.xtoff[v + 1];
     bool hit = false;
@@ -157,12 +158,12 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
   auto load_unit = [&](uint32_t u) {
     Unit x{};
     if (u < rows.nmid) {
-      x.v = __ldg(rows.list + rows.nlow + u);
+      x.v = __ldg(rows.list + u);
       x.row = true;
     } else if (rows.sorted) {
       const uint32_t i = 32 * (u - rows.nmid) + lane;
       x.row = i < rows.nlow;
-      x.v = x.row ? __ldg(rows.list + i) : 0u;
+      x.v = x.row ? __ldg(rows.low + i) : 0u;
     } else {
       const uint32_t w = u - rows.nmid;
       x.v = (w << 5) | lane;
@@ -220,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
       return cw;
     };
     for (uint32_t i = blockIdx.x; i < rows.nlong; i += gridDim.x) {
-      const uint32_t v = __ldg(rows.list + rows.nlow + rows.nmid + i);
+      const uint32_t v = __ldg(rows.list + rows.nmid + i);
       if (!affected(v)) continue;
       const uint32_t s = __ldg(a.xtoff + v), d = __ldg(a.xtoff + v + 1) - s;
       const VertexIn in = load_vertex(a, v, p);
@@ -344,7 +345,8 @@ static cudaError_t persist_t(const SolveArgs& a, const PersistRows& rows, int sm
 }
 
 cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, cudaStream_t s) {
-  const PersistRows rows = {g.plan_list, g.plan_begin[MID], g.plan_begin[HIGH] - g.plan_begin[MID],
+  const PersistRows rows = {g.len_list, g.plan_list + g.plan_begin[MID], g.plan_begin[MID],
+                            g.plan_begin[HIGH] - g.plan_begin[MID],
                             g.plan_begin[NCLS] - g.plan_begin[HIGH], mixed_lengths(g)};
   switch (mode) {
     case PRX_DYNAMIC_TRAVERSAL: return persist_t<PRX_DYNAMIC_TRAVERSAL>(a, rows, sms, s);

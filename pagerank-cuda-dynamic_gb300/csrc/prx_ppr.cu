@@ -8,10 +8,20 @@
 // vertices and vectors of one sweep is below the tolerance (the reference's
 // convergence test, :680,689, taken over the whole block).
 //
-// Layout: ranks are vertex-major, 64 values per vertex (one 512-byte FP64 or
-// 256-byte FP32 row), so every in-edge is one coalesced row gather; lane l of
-// a warp owns columns 2l and 2l+1.  Contributions are not stored: each
-// gathered row is scaled by the source's reciprocal out-degree in the fma.
+// Layout: ranks are vertex-major, C values per vertex, where C is the smallest
+// of 8, 16, 24, 32, 48 and 64 that holds the block's vectors.  A lane owns 16
+// bytes of a row (three columns, strided, for 24 and 48), so a row is a
+// coalesced gather by 2 to 32 lanes, and a warp works on 1 to 16 vertices side
+// by side.
+// Contributions are not stored: each gathered row is scaled by the source's
+// reciprocal out-degree in the fma.
+//
+// What bounds the sweeps: the FP64 ones GB300's FP64 pipe (16 to 17 cycles a
+// warp-wide fma, 93% busy), the FP32 ones the way from L2 (about 10 TB/s).
+// Measured, us a sweep, 64 columns with a vertex per warp and a block per
+// 512-edge segment | so: R-MAT 2^20, 64 vectors, FP32 914 | 790; R-MAT 2^18, 64
+// vectors, FP64 760 | 643; web-like 200k, 24 vectors, FP64 895 | 370, 10
+// vectors, FP32 240 | 94, 64 vectors, FP32 253 | 251.
 //
 // Precision:
 //  - PRX_FP64: FP64 rows, FP64 sums.
@@ -23,11 +33,11 @@
 //    below 2^-18 of the correction's size (FP32 cannot resolve more), or at
 //    the iteration cap.
 //
-// Rows of in-degree up to low_max (64 by default): one warp per vertex.
-// Longer rows are cut into segments of `seg` in-edges (512 by default); a
-// block sums a segment (warp w a contiguous eighth of it) into a partial
-// row, and a warp per long vertex adds its segments' partials in order and
-// finishes the vertex.  Every sum has a fixed order for given low_max / seg,
+// Rows of in-degree up to low_max (64 by default): a row's lanes per vertex.
+// Longer rows are cut into segments of `seg` in-edges (512 by default) of
+// eight contiguous parts; a part's sum is a partial row, and a second kernel
+// adds a segment's parts, and a vertex's segments, in order and finishes the
+// vertex.  Every sum has a fixed order for given low_max / seg,
 // so results are deterministic; prx_autotune_ppr picks both per graph.
 //
 // Loop: by default the whole iteration loop of a column block is one CUDA
@@ -38,15 +48,16 @@
 // kernels from a host loop that reads the control block back between batches
 // of sweeps.  Both run the same kernels in the same order (same results).
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 #include "prx_ctx.h"
 #include "prx_device.cuh"
 
 namespace prx {
 
-constexpr int kCols = 64;         // vectors per column block
+constexpr int kCols = 64;         // vectors per column block at most
 constexpr uint32_t kSeg = 512;    // default in-edges per segment of a long row
-constexpr int kSegWarps = 8;      // warps per segment block
+constexpr uint32_t kSegParts = 8; // parts of a segment, summed side by side
 
 enum PprMode { PPR_J64 = 0, PPR_R64 = 1, PPR_S32 = 2 };
 
@@ -57,18 +68,20 @@ struct PprWs {
   double* x[2] = {nullptr, nullptr};   // FP64 ranks, [n][64], ping-pong (refinement: base, sweep output)
   float* rho = nullptr;                // FP32 refinement: residual [n][64]
   float* e[2] = {nullptr, nullptr};    // FP32 corrections, ping-pong
-  double* part = nullptr;              // partial rows of the segments [nseg][64]
-  size_t part_cap = 0;                 // in segments
-  uint32_t* seg = nullptr;             // [2][seg_cap]: vertex, first edge
-  size_t seg_cap = 0;
-  uint32_t* segstart = nullptr;        // first segment of each long vertex (+ total)
-  size_t segstart_cap = 0;
+  double* part = nullptr;              // partial rows of the long rows' parts [nparts][C]
+  size_t part_cap = 0;
+  uint2* parts = nullptr;              // vertex, first edge
+  size_t parts_cap = 0;
+  uint32_t* partstart = nullptr;       // first part of each long vertex (+ total)
+  size_t partstart_cap = 0;
   uint32_t* big = nullptr;             // vertices above a low_max other than 64, and their scan
   size_t big_cap = 0;
   uint32_t* toff = nullptr;            // teleport entries by vertex: offsets (n+1)
   uint32_t* tent = nullptr;            // entries: vertex, column (sorted)
   double* tmass = nullptr;             // entry mass 1/|S_k|
   size_t t_cap = 0, tm_cap = 0;
+  uint2* pair = nullptr;               // the graph's in-edges as pairs (PprArgs::pair), for one call
+  size_t pair_cap = 0;
   double* out = nullptr;               // device staging of the host output
   size_t out_cap = 0;
 };
@@ -82,23 +95,25 @@ void ppr_free(PprWs* w) {
   }
   cudaFree(w->rho);
   cudaFree(w->part);
-  cudaFree(w->seg);
-  cudaFree(w->segstart);
+  cudaFree(w->parts);
+  cudaFree(w->partstart);
   cudaFree(w->big);
   cudaFree(w->toff);
   cudaFree(w->tent);
   cudaFree(w->tmass);
+  cudaFree(w->pair);
   cudaFree(w->out);
   delete w;
 }
 
 struct PprArgs {
   const uint32_t* xtoff;
-  const uint32_t* xtedg;
   const unsigned long long* xtbase;  // row segments (see GraphDev); null: one segment
   uint32_t seg_shift;
   const double* rcp;
   const float* rcp32;
+  const uint32_t* xtedg;
+  const uint2* pair;              // per in-edge, laid out like xtedg: source, bits of its FP32 reciprocal out-degree
   const uint32_t* toff;
   const uint32_t* tcol;           // column of each teleport entry
   const double* tmass;
@@ -108,19 +123,82 @@ struct PprArgs {
   const uint32_t* big;            // vertices with in-degree > low_max
   uint32_t nbig;
   uint32_t low_max;               // rows up to this in-degree: one warp per vertex
-  uint32_t seg;                   // in-edges per segment of a longer row (a multiple of kSegWarps)
-  const uint32_t* segstart;       // [nbig + 1]
-  const uint32_t* seg_v;
-  const uint32_t* seg_e;
-  uint32_t nseg;
-  double* part;
+  uint32_t seg;                   // in-edges per segment of a longer row (a multiple of kSegParts)
+  uint32_t per;                   // in-edges per part: seg / kSegParts
+  const uint32_t* partstart;      // [nbig + 1]: each long row's first part
+  const uint2* parts;             // vertex, first edge (relative to its row segment)
+  uint32_t nparts;
+  double* part;                   // the parts' partial rows
   State* st;
   uint32_t n;
+  const uint32_t* rows;           // the vertices of the short rows in the order they are taken (null: by id)
+  uint32_t nrows;
+  uint32_t batch;                 // vertices of a unit, whose bounds a warp loads at once (at most 32)
+  int cols;                       // C: columns stored per vertex
+  bool share;                     // a fixed share of the units per warp
+  bool flat;                      // 64 FP32 columns: the short rows by k_ppr_flat
   double P, Q;                    // damping, 1 - damping
+  float P32;                      // (float)P: a conversion in the kernel runs on the FP64 pipe
 };
 
-template <int MODE> struct PprType { using S = double; using V2 = double2; };
-template <> struct PprType<PPR_S32> { using S = float; using V2 = float2; };
+template <int MODE> struct PprType { using S = double; };
+template <> struct PprType<PPR_S32> { using S = float; };
+
+// How a warp holds rows of C columns: LPR lanes per row, G rows side by side,
+// N columns per lane -- columns N sub .. N sub + N - 1 of lane sub, read as one
+// 16-byte vector, or (VEC false) columns sub + LPR i.
+template <int MODE, int C> struct PprShape {
+  using S = typename PprType<MODE>::S;
+  static constexpr bool VEC = C % 3 != 0;
+  static constexpr int N = VEC ? 16 / (int)sizeof(S) : 3;
+  static constexpr int LPR = C / N;
+  static constexpr int G = 32 / LPR;
+  static constexpr int U = 4;       // rows a lane has in flight
+  static constexpr int BLOCKS = 4;  // resident blocks of 256 per SM
+  using Raw = typename std::conditional<sizeof(S) == 8, double2, float4>::type;
+  struct V {
+    S c[N];
+    __device__ __forceinline__ S& operator[](int i) { return c[i]; }
+    __device__ __forceinline__ S operator[](int i) const { return c[i]; }
+  };
+  static_assert(LPR * G == 32, "a warp's lanes");
+  // row r of an array of rows, this lane's columns; LDG: by the read-only path
+  template <bool LDG>
+  __device__ static __forceinline__ V load(const S* rows, size_t r, uint32_t sub) {
+    V x;
+    if constexpr (VEC) {
+      const Raw* at = reinterpret_cast<const Raw*>(rows) + r * LPR + sub;
+      const Raw y = LDG ? __ldg(at) : *at;
+      x[0] = y.x;
+      x[1] = y.y;
+      if constexpr (N == 4) {
+        x[2] = y.z;
+        x[3] = y.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) x[i] = LDG ? __ldg(rows + r * C + sub + LPR * i) : rows[r * C + sub + LPR * i];
+    }
+    return x;
+  }
+  __device__ static __forceinline__ void store(S* rows, size_t r, uint32_t sub, const V& x) {
+    if constexpr (VEC) {
+      Raw y;
+      y.x = x[0];
+      y.y = x[1];
+      if constexpr (N == 4) {
+        y.z = x[2];
+        y.w = x[3];
+      }
+      reinterpret_cast<Raw*>(rows)[r * LPR + sub] = y;
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) rows[r * C + sub + LPR * i] = x[i];
+    }
+  }
+  // the lane's i-th column
+  __device__ static __forceinline__ uint32_t column(uint32_t sub, int i) { return VEC ? sub * N + i : sub + LPR * i; }
+};
 
 template <int MODE>
 __device__ __forceinline__ bool ppr_skip(const State* st) {
@@ -129,88 +207,153 @@ __device__ __forceinline__ bool ppr_skip(const State* st) {
 
 // Source rows of this sweep.
 template <int MODE>
-__device__ __forceinline__ const typename PprType<MODE>::V2* ppr_src(const PprArgs& a, const State* st) {
-  using V2 = typename PprType<MODE>::V2;
-  if (MODE == PPR_J64) return reinterpret_cast<const V2*>(a.x[st->iter & 1]);
-  if (MODE == PPR_R64) return reinterpret_cast<const V2*>(a.x[0]);
-  return reinterpret_cast<const V2*>(a.e[st->k32 & 1]);
+__device__ __forceinline__ const typename PprType<MODE>::S* ppr_src(const PprArgs& a, const State* st) {
+  if constexpr (MODE == PPR_J64) return a.x[st->iter & 1];
+  else if constexpr (MODE == PPR_R64) return a.x[0];
+  else return a.e[st->k32 & 1];
 }
-
-// acc += row(u) / outdeg(u) over the in-edges [s, e) of edg (v's segment of
-// the in-CSR; lane: its two columns).
-template <int MODE>
-__device__ __forceinline__ void ppr_gather(const PprArgs& a, const typename PprType<MODE>::V2* __restrict__ src,
-                                           const uint32_t* __restrict__ edg, uint32_t s, uint32_t e,
-                                           typename PprType<MODE>::V2& acc) {
-  using S = typename PprType<MODE>::S;
-  using V2 = typename PprType<MODE>::V2;
-  const S* __restrict__ rc;
-  if constexpr (MODE == PPR_S32) rc = a.rcp32;
-  else rc = a.rcp;
-  const uint32_t lane = lane_id();
-  uint32_t j = s;
-  for (; j + 4 <= e; j += 4) {
-    const uint32_t u0 = __ldg(edg + j), u1 = __ldg(edg + j + 1), u2 = __ldg(edg + j + 2), u3 = __ldg(edg + j + 3);
-    const V2 g0 = __ldg(src + (size_t)u0 * (kCols / 2) + lane), g1 = __ldg(src + (size_t)u1 * (kCols / 2) + lane);
-    const V2 g2 = __ldg(src + (size_t)u2 * (kCols / 2) + lane), g3 = __ldg(src + (size_t)u3 * (kCols / 2) + lane);
-    const S y0 = __ldg(rc + u0), y1 = __ldg(rc + u1), y2 = __ldg(rc + u2), y3 = __ldg(rc + u3);
-    acc.x = fma(g0.x, y0, acc.x); acc.y = fma(g0.y, y0, acc.y);
-    acc.x = fma(g1.x, y1, acc.x); acc.y = fma(g1.y, y1, acc.y);
-    acc.x = fma(g2.x, y2, acc.x); acc.y = fma(g2.y, y2, acc.y);
-    acc.x = fma(g3.x, y3, acc.x); acc.y = fma(g3.y, y3, acc.y);
-  }
-  for (; j < e; ++j) {
-    const uint32_t u = __ldg(edg + j);
-    const V2 g = __ldg(src + (size_t)u * (kCols / 2) + lane);
-    const S y = __ldg(rc + u);
-    acc.x = fma(g.x, y, acc.x);
-    acc.y = fma(g.y, y, acc.y);
-  }
+// acc += row(u) / outdeg(u) over the edges [s, s + len) of pair, by the LPR
+// lanes of a row (every lane of the warp calls it; rows may differ in
+// length), one edge after the other.  A pair is an edge's source and the bits
+// of its FP32 reciprocal, read by all lanes of the row at once: for the FP32
+// sweeps, which the L1 bounds, half the wavefronts of an id, a reciprocal
+// gather and the row.  first: the pairs of the first U edges, loaded by the
+// caller.  Up to U rows are in flight.
+template <int MODE, int C>
+__device__ __forceinline__ void ppr_pairs(const uint2* __restrict__ ed, uint32_t len, uint2 pr[PprShape<MODE, C>::U]) {
+#pragma unroll
+  for (int k = 0; k < PprShape<MODE, C>::U; ++k) pr[k] = (uint32_t)k < len ? __ldg(ed + k) : make_uint2(0, 0);
 }
-
-// Finish vertex v from its gathered sum (lane: columns 2l, 2l+1); returns the
-// lane's L-inf term (bits of a double, or of a float for PPR_S32) and, for
-// PPR_S32, the size of the new correction in *emag.
-template <int MODE>
-__device__ __forceinline__ unsigned long long ppr_finish(const PprArgs& a, const State* st, uint32_t v,
-                                                         typename PprType<MODE>::V2 acc, unsigned int* emag) {
-  const uint32_t lane = lane_id();
-  const size_t at = (size_t)v * (kCols / 2) + lane;
-  if constexpr (MODE == PPR_S32) {
-    const int q = st->k32 & 1;
-    const float2 r = reinterpret_cast<const float2*>(a.rho)[at];
-    const float2 old = reinterpret_cast<const float2*>(a.e[q])[at];
-    const float P = (float)a.P;
-    float2 en;
-    en.x = fmaf(P, acc.x, r.x);
-    en.y = fmaf(P, acc.y, r.y);
-    reinterpret_cast<float2*>(a.e[q ^ 1])[at] = en;
-    *emag = __float_as_uint(fmaxf(fabsf(en.x), fabsf(en.y)));
-    return __float_as_uint(fmaxf(fabsf(en.x - old.x), fabsf(en.y - old.y)));
-  } else {
-    double tx = 0.0, ty = 0.0;
-    for (uint32_t i = __ldg(a.toff + v), ie = __ldg(a.toff + v + 1); i < ie; ++i) {
-      const uint32_t col = __ldg(a.tcol + i);
-      if ((col >> 1) == lane) {
-        if (col & 1u) ty += __ldg(a.tmass + i);
-        else tx += __ldg(a.tmass + i);
+template <int MODE, int C>
+__device__ __forceinline__ void ppr_gather(const typename PprType<MODE>::S* __restrict__ src,
+                                           const double* __restrict__ rcp, const uint2* __restrict__ ed, uint32_t len,
+                                           uint2 pr[PprShape<MODE, C>::U], uint32_t sub,
+                                           typename PprShape<MODE, C>::V& acc) {
+  using Sh = PprShape<MODE, C>;
+  using S = typename Sh::S;
+  using V = typename Sh::V;
+  constexpr int U = PprShape<MODE, C>::U;
+  const uint32_t longest = Sh::G == 1 ? len : __reduce_max_sync(0xffffffffu, len);
+  for (uint32_t base = 0; base < longest; base += U) {
+    V g[U];
+    S w[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (base + k < len) {
+        g[k] = Sh::template load<true>(src, pr[k].x, sub);
+        if constexpr (MODE == PPR_S32) w[k] = __uint_as_float(pr[k].y);
+        else w[k] = __ldg(rcp + pr[k].x);
+      } else {  // + 0 * 0 leaves the sum
+#pragma unroll
+        for (int i = 0; i < Sh::N; ++i) g[k][i] = S(0);
+        w[k] = S(0);
       }
     }
-    double2 an;
-    an.x = fma(a.P, acc.x, a.Q * tx);
-    an.y = fma(a.P, acc.y, a.Q * ty);
-    const int p = MODE == PPR_J64 ? (st->iter & 1) : 0;
-    const double2 old = reinterpret_cast<const double2*>(a.x[p])[at];
-    reinterpret_cast<double2*>(a.x[p ^ 1])[at] = an;
-    const double dx = an.x - old.x, dy = an.y - old.y;
-    if (MODE == PPR_R64) {
-      float2 r;
-      r.x = (float)dx;
-      r.y = (float)dy;
-      reinterpret_cast<float2*>(a.rho)[at] = r;
-      reinterpret_cast<float2*>(a.e[0])[at] = r;
+    if (base + U < longest) ppr_pairs<MODE, C>(ed + base + U, len > base + U ? len - base - U : 0u, pr);
+    auto add = [&](int k) {
+#pragma unroll
+      for (int i = 0; i < Sh::N; ++i) acc[i] = fma(g[k][i], w[k], acc[i]);
+    };
+    if constexpr (MODE == PPR_S32) {
+#pragma unroll
+      for (int k = 0; k < U; ++k) add(k);
+    } else {
+      // an FP64 fma issued for no row costs as much as one: branches, not
+      // predicates, over the rows the warp has
+      const uint32_t n = longest - base;
+      if (n >= 4) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) add(k);
+        if constexpr (U == 8) {
+          if (n >= 8) {
+#pragma unroll
+            for (int k = 4; k < 8; ++k) add(k);
+          } else {
+            switch (n) {
+              case 5: add(4); break;
+              case 6: add(4); add(5); break;
+              case 7: add(4); add(5); add(6); break;
+              default: break;
+            }
+          }
+        }
+      } else {
+        switch (n) {
+          case 1: add(0); break;
+          case 2: add(0); add(1); break;
+          default: add(0); add(1); add(2); break;
+        }
+      }
     }
-    return dbits(fmax(fabs(dx), fabs(dy)));
+  }
+}
+
+// Finish vertex v from its gathered sum (sub: which 16 bytes of the row);
+// returns the lane's L-inf term (bits of a double, or of a float for PPR_S32)
+// and, for PPR_S32, the size of the new correction in *emag.
+template <int MODE, int C>
+__device__ __forceinline__ unsigned long long ppr_finish(const PprArgs& a, const State* st, uint32_t v,
+                                                         const typename PprShape<MODE, C>::V& acc, uint32_t sub,
+                                                         unsigned int* emag) {
+  using Sh = PprShape<MODE, C>;
+  using V = typename Sh::V;
+  if constexpr (MODE == PPR_S32) {
+    const int q = st->k32 & 1;
+    const V r = Sh::template load<false>(a.rho, v, sub), old = Sh::template load<false>(a.e[q], v, sub);
+    V en;
+    const float P = a.P32;
+    float big = 0.f, chg = 0.f;
+#pragma unroll
+    for (int i = 0; i < Sh::N; ++i) {
+      en[i] = fmaf(P, acc[i], r[i]);
+      big = fmaxf(big, fabsf(en[i]));
+      chg = fmaxf(chg, fabsf(en[i] - old[i]));
+    }
+    Sh::store(a.e[q ^ 1], v, sub, en);
+    *emag = __float_as_uint(big);
+    return __float_as_uint(chg);
+  } else {
+    const int p = MODE == PPR_J64 ? (st->iter & 1) : 0;
+    const V old = Sh::template load<false>(a.x[p], v, sub);
+    V t;
+#pragma unroll
+    for (int i = 0; i < Sh::N; ++i) t[i] = 0.0;
+    const uint32_t t0 = __ldg(a.toff + v), t1 = __ldg(a.toff + v + 1);
+    if (t0 < t1) {  // few vertices are seeds; Q * 0 is 0
+      for (uint32_t i = t0; i < t1; ++i) {
+        const uint32_t col = __ldg(a.tcol + i);
+#pragma unroll
+        for (int k = 0; k < Sh::N; ++k)
+          if (col == Sh::column(sub, k)) t[k] += __ldg(a.tmass + i);
+      }
+#pragma unroll
+      for (int i = 0; i < Sh::N; ++i) t[i] = a.Q * t[i];
+    }
+    V an;
+    unsigned long long chg = 0;  // |change| as bits (non-negative doubles order as their bits)
+    float r[Sh::N];
+#pragma unroll
+    for (int i = 0; i < Sh::N; ++i) {
+      an[i] = fma(a.P, acc[i], t[i]);
+      const double d = an[i] - old[i];
+      if (MODE == PPR_R64) r[i] = (float)d;
+      const unsigned long long b = dbits(d) & ~(1ull << 63);
+      chg = b > chg ? b : chg;
+    }
+    Sh::store(a.x[p ^ 1], v, sub, an);
+    if constexpr (MODE == PPR_R64 && Sh::VEC) {
+      const float2 r2 = make_float2(r[0], r[1]);
+      reinterpret_cast<float2*>(a.rho)[(size_t)v * Sh::LPR + sub] = r2;
+      reinterpret_cast<float2*>(a.e[0])[(size_t)v * Sh::LPR + sub] = r2;
+    } else if constexpr (MODE == PPR_R64) {
+#pragma unroll
+      for (int i = 0; i < Sh::N; ++i) {
+        const size_t at = (size_t)v * C + Sh::column(sub, i);
+        a.rho[at] = r[i];
+        a.e[0][at] = r[i];
+      }
+    }
+    return chg;
   }
 }
 
@@ -224,90 +367,191 @@ __device__ __forceinline__ void ppr_reduce(State* st, unsigned long long dmax, u
   }
 }
 
-// In-degree <= 64: one warp per vertex.
-template <int MODE>
-__global__ void __launch_bounds__(256) k_ppr_low(PprArgs a) {
-  using V2 = typename PprType<MODE>::V2;
+// One sweep's rows.  A warp takes units: first G parts of long rows (partial
+// sums of a.per in-edges each, added up by k_ppr_combine), then batches of
+// short rows (in-degree <= low_max), LPR lanes per vertex and G vertices side
+// by side; a batch's bounds are loaded by a lane each, and the first pairs of
+// the next G vertices while it sums these.  No warp waits for another.
+template <int MODE, int C>
+__global__ void __launch_bounds__(256, PprShape<MODE, C>::BLOCKS) k_ppr_rows(PprArgs a) {
+  using Sh = PprShape<MODE, C>;
+  using S = typename Sh::S;
+  using V = typename Sh::V;
+  constexpr uint32_t LPR = Sh::LPR, G = Sh::G;
+  constexpr int U = Sh::U;
   State* st = a.st;
   if (ppr_skip<MODE>(st)) return;
-  const V2* __restrict__ src = ppr_src<MODE>(a, st);
+  const S* __restrict__ src = ppr_src<MODE>(a, st);
+  const uint32_t lane = lane_id(), sub = lane % LPR, grp = lane / LPR;
   unsigned long long dmax = 0;
   unsigned int emag = 0;
+  const uint32_t nb = (uint32_t)(((uint64_t)a.nrows + a.batch - 1) / a.batch);
+  const uint32_t np = (a.nparts + G - 1) / G;
+  auto zero = [](V& x) {
+#pragma unroll
+    for (int k = 0; k < Sh::N; ++k) x[k] = S(0);
+  };
+  // units are taken from a counter (reset by the sweep's finalize kernel), the
+  // next one while this one is summed: they differ in length and in what the
+  // caches hold, and a fixed share per warp left a seventh of the warps idle
+  // (with few units the counter's latency is what counts: a.share)
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < a.n; v += warps) {
-    const uint64_t iv = seg_index(v, a.seg_shift);
-    const uint32_t s = __ldg(a.xtoff + iv), e = __ldg(a.xtoff + iv + 1);
-    if (e - s > a.low_max) continue;
-    V2 acc;
-    acc.x = 0;
-    acc.y = 0;
-    ppr_gather<MODE>(a, src, seg_edges(a.xtedg, a.xtbase, a.seg_shift, v), s, e, acc);
-    unsigned int em = 0;
-    const unsigned long long d = ppr_finish<MODE>(a, st, v, acc, &em);
-    dmax = d > dmax ? d : dmax;
-    emag = em > emag ? em : emag;
+  uint32_t next = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  auto take = [&] {
+    if (a.share) next += warps;
+    else if (lane == 0) next = atomicAdd(&st->work, 1u);
+  };
+  if (!a.share) take();
+  uint2 pr[U];
+  for (;;) {
+    const uint32_t b = __shfl_sync(0xffffffffu, next, 0);
+    if (b >= np + nb) break;
+    take();
+    if (b < np) {
+      const uint32_t i = b * G + grp;
+      uint32_t len = 0;
+      const uint2* ed = a.pair;
+      if (i < a.nparts) {
+        const uint2 w = __ldg(a.parts + i);  // vertex, first edge
+        const uint32_t end = __ldg(a.xtoff + seg_index(w.x, a.seg_shift) + 1);
+        len = min(a.per, end - w.y);
+        ed += w.y + (a.xtbase ? a.xtbase[(uint64_t)w.x >> a.seg_shift] : 0ull);
+      }
+      ppr_pairs<MODE, C>(ed, len, pr);
+      V acc;
+      zero(acc);
+      ppr_gather<MODE, C>(src, a.rcp, ed, len, pr, sub, acc);
+      if (i < a.nparts) Sh::store(reinterpret_cast<S*>(a.part), i, sub, acc);
+      continue;
+    }
+    const uint32_t i0 = (np + nb - 1 - b) * a.batch;  // the longest rows first
+    // lane i: vertex i of the batch (len 0xffffffff: none, or a long row)
+    uint32_t mv = 0, ml = 0xffffffffu;
+    unsigned long long ms = 0;
+    if (lane < a.batch && i0 + lane < a.nrows) {
+      mv = a.rows ? __ldg(a.rows + i0 + lane) : i0 + lane;
+      const uint64_t iv = seg_index(mv, a.seg_shift);
+      const uint32_t s = __ldg(a.xtoff + iv), len = __ldg(a.xtoff + iv + 1) - s;
+      ms = s + (a.xtbase ? a.xtbase[(uint64_t)mv >> a.seg_shift] : 0ull);
+      if (len <= a.low_max) ml = len;
+    }
+    const uint32_t cnt = min(a.batch, a.nrows - i0);
+    uint32_t v, len;
+    const uint2* ed;
+    auto fetch = [&](uint32_t i) {  // vertex i + grp of the batch and its first edges
+      const uint32_t k = i + grp;
+      v = __shfl_sync(0xffffffffu, mv, k & 31);
+      ed = a.pair + __shfl_sync(0xffffffffu, ms, k & 31);
+      len = __shfl_sync(0xffffffffu, ml, k & 31);
+      if (k >= cnt) len = 0xffffffffu;
+      ppr_pairs<MODE, C>(ed, len == 0xffffffffu ? 0u : len, pr);
+    };
+    fetch(0);
+    for (uint32_t i = 0; i < cnt; i += G) {
+      const uint32_t cv = v, cl = len;
+      V acc;
+      zero(acc);
+      ppr_gather<MODE, C>(src, a.rcp, ed, cl == 0xffffffffu ? 0u : cl, pr, sub, acc);
+      if (i + G < cnt) fetch(i + G);
+      if (cl == 0xffffffffu) continue;
+      unsigned int em = 0;
+      const unsigned long long d = ppr_finish<MODE, C>(a, st, cv, acc, sub, &em);
+      dmax = d > dmax ? d : dmax;
+      emag = em > emag ? em : emag;
+    }
   }
   ppr_reduce<MODE>(st, dmax, emag);
 }
 
-// Segments of the long rows: block per segment, warp w sums the w-th eighth;
-// the partial row is the warps' sums added in warp order.
-template <int MODE>
-__global__ void __launch_bounds__(kSegWarps * 32) k_ppr_seg(PprArgs a) {
-  using V2 = typename PprType<MODE>::V2;
-  __shared__ V2 sh[kSegWarps][32];
-  const State* st = a.st;
-  if (ppr_skip<MODE>(st)) return;
-  const V2* __restrict__ src = ppr_src<MODE>(a, st);
-  const uint32_t w = threadIdx.x >> 5, lane = lane_id();
-  V2* part = reinterpret_cast<V2*>(a.part);
-  for (uint32_t g = blockIdx.x; g < a.nseg; g += gridDim.x) {
-    const uint32_t v = a.seg_v[g], s0 = a.seg_e[g];
-    const uint32_t end = min(s0 + a.seg, a.xtoff[seg_index(v, a.seg_shift) + 1]);
-    const uint32_t per = a.seg / kSegWarps;
-    const uint32_t s = min(s0 + w * per, end), e = min(s + per, end);
-    V2 acc;
-    acc.x = 0;
-    acc.y = 0;
-    ppr_gather<MODE>(a, src, seg_edges(a.xtedg, a.xtbase, a.seg_shift, v), s, e, acc);
-    sh[w][lane] = acc;
-    __syncthreads();
-    if (w == 0) {
-      V2 t = sh[0][lane];
-#pragma unroll
-      for (int k = 1; k < kSegWarps; ++k) {
-        t.x += sh[k][lane].x;
-        t.y += sh[k][lane].y;
-      }
-      part[(size_t)g * (kCols / 2) + lane] = t;
+// The short rows of a 64-column FP32 sweep, a warp per vertex in id order, two
+// columns per lane: 32 registers, so 64 warps an SM, and 4-byte ids (their
+// reciprocals hit the L1), which web-like graphs -- rows of one length, bound
+// by the L1 and the way to it -- need more than the side-by-side rows: 174
+// against 192 us a sweep on 200k vertices.  The same sums.
+__global__ void __launch_bounds__(256) k_ppr_flat(PprArgs a) {
+  State* st = a.st;
+  if (ppr_skip<PPR_S32>(st)) return;
+  const int q = st->k32 & 1;
+  const float2* __restrict__ src = reinterpret_cast<const float2*>(a.e[q]);
+  const float* __restrict__ rc = a.rcp32;
+  const uint32_t lane = lane_id(), warps = (gridDim.x * blockDim.x) >> 5;
+  unsigned int dmax = 0, emag = 0;
+  for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < a.n; v += warps) {
+    const uint64_t iv = seg_index(v, a.seg_shift);
+    const uint32_t s = __ldg(a.xtoff + iv), e = __ldg(a.xtoff + iv + 1);
+    if (e - s > a.low_max) continue;
+    const uint32_t* __restrict__ edg = seg_edges(a.xtedg, a.xtbase, a.seg_shift, v);
+    float2 acc = make_float2(0.f, 0.f);
+    uint32_t j = s;
+    for (; j + 4 <= e; j += 4) {
+      const uint32_t u0 = __ldg(edg + j), u1 = __ldg(edg + j + 1), u2 = __ldg(edg + j + 2), u3 = __ldg(edg + j + 3);
+      const float2 g0 = __ldg(src + (size_t)u0 * 32 + lane), g1 = __ldg(src + (size_t)u1 * 32 + lane);
+      const float2 g2 = __ldg(src + (size_t)u2 * 32 + lane), g3 = __ldg(src + (size_t)u3 * 32 + lane);
+      const float y0 = __ldg(rc + u0), y1 = __ldg(rc + u1), y2 = __ldg(rc + u2), y3 = __ldg(rc + u3);
+      acc.x = fma(g0.x, y0, acc.x); acc.y = fma(g0.y, y0, acc.y);
+      acc.x = fma(g1.x, y1, acc.x); acc.y = fma(g1.y, y1, acc.y);
+      acc.x = fma(g2.x, y2, acc.x); acc.y = fma(g2.y, y2, acc.y);
+      acc.x = fma(g3.x, y3, acc.x); acc.y = fma(g3.y, y3, acc.y);
     }
-    __syncthreads();
+    for (; j < e; ++j) {
+      const uint32_t u = __ldg(edg + j);
+      const float2 g = __ldg(src + (size_t)u * 32 + lane);
+      const float y = __ldg(rc + u);
+      acc.x = fma(g.x, y, acc.x);
+      acc.y = fma(g.y, y, acc.y);
+    }
+    const size_t at = (size_t)v * 32 + lane;
+    const float2 r = reinterpret_cast<const float2*>(a.rho)[at], old = src[at];
+    const float P = a.P32;
+    const float2 en = make_float2(fmaf(P, acc.x, r.x), fmaf(P, acc.y, r.y));
+    reinterpret_cast<float2*>(a.e[q ^ 1])[at] = en;
+    emag = max(emag, __float_as_uint(fmaxf(fabsf(en.x), fabsf(en.y))));
+    dmax = max(dmax, __float_as_uint(fmaxf(fabsf(en.x - old.x), fabsf(en.y - old.y))));
   }
+  ppr_reduce<PPR_S32>(st, dmax, emag);
 }
 
-// Long rows: warp per vertex adds its segments' partial rows in order.
-template <int MODE>
+// Long rows: a row's lanes per vertex add its segments in order, a segment
+// being its kSegParts parts (fewer in the last) added in order.
+template <int MODE, int C>
 __global__ void __launch_bounds__(256) k_ppr_combine(PprArgs a) {
-  using V2 = typename PprType<MODE>::V2;
+  using Sh = PprShape<MODE, C>;
+  using S = typename Sh::S;
+  using V = typename Sh::V;
+  constexpr uint32_t LPR = Sh::LPR;
   State* st = a.st;
   if (ppr_skip<MODE>(st)) return;
-  const V2* part = reinterpret_cast<const V2*>(a.part);
-  const uint32_t lane = lane_id();
+  const S* part = reinterpret_cast<const S*>(a.part);
+  const uint32_t sub = threadIdx.x % LPR;
   unsigned long long dmax = 0;
   unsigned int emag = 0;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.nbig; i += warps) {
-    const uint32_t v = a.big[i];
-    V2 acc;
-    acc.x = 0;
-    acc.y = 0;
-    for (uint32_t g = a.segstart[i]; g < a.segstart[i + 1]; ++g) {
-      const V2 t = part[(size_t)g * (kCols / 2) + lane];
-      acc.x += t.x;
-      acc.y += t.y;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / LPR; i < a.nbig; i += gridDim.x * blockDim.x / LPR) {
+    V acc;
+#pragma unroll
+    for (int k = 0; k < Sh::N; ++k) acc[k] = S(0);
+    const uint32_t end = a.partstart[i + 1];
+    for (uint32_t g = a.partstart[i]; g < end; g += kSegParts) {
+      V x[kSegParts];
+#pragma unroll
+      for (uint32_t k = 0; k < kSegParts; ++k) {
+        if (g + k < end) {
+          x[k] = Sh::template load<false>(part, g + k, sub);
+        } else {
+#pragma unroll
+          for (int j = 0; j < Sh::N; ++j) x[k][j] = S(0);
+        }
+      }
+#pragma unroll
+      for (uint32_t k = 1; k < kSegParts; ++k)
+        if (g + k < end) {
+#pragma unroll
+          for (int j = 0; j < Sh::N; ++j) x[0][j] += x[k][j];
+        }
+#pragma unroll
+      for (int k = 0; k < Sh::N; ++k) acc[k] += x[0][k];
     }
     unsigned int em = 0;
-    const unsigned long long d = ppr_finish<MODE>(a, st, v, acc, &em);
+    const unsigned long long d = ppr_finish<MODE, C>(a, st, a.big[i], acc, sub, &em);
     dmax = d > dmax ? d : dmax;
     emag = em > emag ? em : emag;
   }
@@ -317,6 +561,7 @@ __global__ void __launch_bounds__(256) k_ppr_combine(PprArgs a) {
 // ---- loop control ------------------------------------------------------------
 __global__ void k_ppr_fin64(State* st) {  // Jacobi FP64 sweep
   if (st->done) return;
+  st->work = 0;
   const int p = st->iter & 1;
   const double el = __longlong_as_double((long long)st->el_bits[p]);
   st->last_delta = el;
@@ -327,6 +572,7 @@ __global__ void k_ppr_fin64(State* st) {  // Jacobi FP64 sweep
 
 __global__ void k_ppr_fin_r64(State* st) {  // refinement: FP64 residual sweep
   if (st->done) return;
+  st->work = 0;
   const double el = __longlong_as_double((long long)st->el_bits[st->iter & 1]);
   st->last_delta = el;
   st->iter += 1;
@@ -345,6 +591,7 @@ __global__ void k_ppr_fin_r64(State* st) {  // refinement: FP64 residual sweep
 
 __global__ void k_ppr_fin32(State* st) {  // refinement: FP32 correction sweep
   if (st->done || st->inner_done) return;
+  st->work = 0;
   const int q = st->k32 & 1;
   const float dl = __uint_as_float(st->el32_bits[q]);
   const float em = __uint_as_float(st->e32max_bits[q]);
@@ -365,7 +612,7 @@ __global__ void k_ppr_fin32(State* st) {  // refinement: FP32 correction sweep
 __global__ void k_ppr_commit(PprArgs a) {
   if (a.st->done) return;
   const float* __restrict__ e = a.e[a.st->k32 & 1];
-  const size_t total = (size_t)a.n * kCols;
+  const size_t total = (size_t)a.n * a.cols;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
     a.x[0][i] += (double)e[i];
 }
@@ -404,14 +651,14 @@ __global__ void k_ppr_toff(const uint32_t* __restrict__ ent_v, uint32_t nent, ui
 // x0 = t (rows zeroed before): each vertex adds its own entries.
 __global__ void k_ppr_init(PprArgs a) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.n; v += gridDim.x * blockDim.x)
-    for (uint32_t i = a.toff[v]; i < a.toff[v + 1]; ++i) a.x[0][(size_t)v * kCols + a.tcol[i]] += a.tmass[i];
+    for (uint32_t i = a.toff[v]; i < a.toff[v + 1]; ++i) a.x[0][(size_t)v * a.cols + a.tcol[i]] += a.tmass[i];
 }
 
-// Segment counts of the long vertices (ceil(indeg / seg)), then the segments.
-__global__ void k_ppr_segcount(const uint32_t* __restrict__ xtoff, uint32_t shift, const uint32_t* __restrict__ big,
-                               uint32_t nbig, uint32_t seg, uint32_t* __restrict__ cnt) {
+// Part counts of the long vertices (ceil(indeg / per)), then the parts.
+__global__ void k_ppr_partcount(const uint32_t* __restrict__ xtoff, uint32_t shift, const uint32_t* __restrict__ big,
+                                uint32_t nbig, uint32_t per, uint32_t* __restrict__ cnt) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += gridDim.x * blockDim.x)
-    cnt[i] = (row_len(xtoff, shift, big[i]) + seg - 1) / seg;
+    cnt[i] = (row_len(xtoff, shift, big[i]) + per - 1) / per;
 }
 
 // Vertices of in-degree above t: flags (n + 1 entries, the last 0) for the
@@ -427,28 +674,32 @@ __global__ void k_ppr_biglist(const uint32_t* __restrict__ xtoff, uint32_t shift
     if (row_len(xtoff, shift, v) > t) big[pos[v]] = v;
 }
 
-// seg_e: the segment's first in-edge, relative to v's row segment like the
-// offsets.
-__global__ void k_ppr_segfill(const uint32_t* __restrict__ xtoff, uint32_t shift, const uint32_t* __restrict__ big,
-                              uint32_t nbig, uint32_t seg, const uint32_t* __restrict__ start,
-                              uint32_t* __restrict__ seg_v, uint32_t* __restrict__ seg_e) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += gridDim.x * blockDim.x) {
-    const uint32_t v = big[i];
+// A warp per long vertex writes its parts.
+__global__ void k_ppr_partfill(const uint32_t* __restrict__ xtoff, uint32_t shift, const uint32_t* __restrict__ big,
+                               uint32_t nbig, uint32_t per, const uint32_t* __restrict__ start,
+                               uint2* __restrict__ parts) {
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nbig; i += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t v = big[i], g0 = start[i], n = start[i + 1] - g0;
     const uint32_t s0 = xtoff[seg_index(v, shift)];
-    for (uint32_t g = start[i], k = 0; g < start[i + 1]; ++g, ++k) {
-      seg_v[g] = v;
-      seg_e[g] = s0 + k * seg;
-    }
+    for (uint32_t k = lane_id(); k < n; k += 32) parts[g0 + k] = make_uint2(v, s0 + k * per);
   }
 }
 
-// out[v * nvec + c0 + k] = x[v][k] for k < w.
-__global__ void k_ppr_out(const double* __restrict__ x, uint32_t n, uint32_t nvec, uint32_t c0, uint32_t w,
-                          double* __restrict__ out) {
+__global__ void k_ppr_pairs(const uint32_t* __restrict__ edg, uint64_t slots, uint32_t n,
+                            const float* __restrict__ rcp32, uint2* __restrict__ pair) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < slots; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t u = edg[i];  // the slots between row segments hold no edge
+    pair[i] = make_uint2(u, u < n ? __float_as_uint(__ldg(rcp32 + u)) : 0u);
+  }
+}
+
+// out[v * nvec + c0 + k] = x[v][k] for k < w (x has cols columns).
+__global__ void k_ppr_out(const double* __restrict__ x, uint32_t n, uint32_t cols, uint32_t nvec, uint32_t c0,
+                          uint32_t w, double* __restrict__ out) {
   const size_t total = (size_t)n * w;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t v = i / w, k = i % w;
-    out[v * nvec + c0 + k] = x[v * kCols + k];
+    out[v * nvec + c0 + k] = x[v * cols + k];
   }
 }
 
@@ -457,14 +708,43 @@ static inline int grid_for(uint64_t work, int threads, int cap) {
   return (int)(b < 1 ? 1 : (b < (uint64_t)cap ? b : cap));
 }
 
+template <int MODE, int C>
+static void ppr_sweep_c(const PprArgs& a, int sms, cudaStream_t s, uint64_t& launches) {
+  constexpr uint32_t G = PprShape<MODE, C>::G;
+  PprArgs b = a;
+  // Vertices per unit: what the last warps wait for, and what the counter is
+  // asked for.  FP64 units are long (a 64-column row takes the pipe 32 cycles
+  // an edge): four per group of lanes, R-MAT 2^18 738 us a sweep at 16, 643 at
+  // four; FP32 ones eight, R-MAT 2^20 784 at 16 vertices, 830 at four.
+  b.batch = std::min<uint32_t>(32, (MODE == PPR_S32 ? 8 : 4) * G);
+  while (b.batch > G && (uint64_t)a.nrows / b.batch < 2ull * 32 * sms) b.batch /= 2;
+  // few units in all: no counter (R-MAT 2^16, 5 vectors: 41 us a sweep, 52 with it)
+  b.share = (uint64_t)a.nrows / b.batch + a.nparts / G < 2ull * 32 * sms;
+  if (MODE == PPR_S32 && C == 64 && a.flat) {
+    k_ppr_flat<<<grid_for((uint64_t)a.n * 32, 256, sms * 8), 256, 0, s>>>(a);
+    ++launches;
+    b.nrows = 0;  // the long rows are left
+  }
+  const uint64_t units = ((uint64_t)b.nrows + b.batch - 1) / b.batch + (a.nparts + G - 1) / G;
+  if (units) {
+    k_ppr_rows<MODE, C><<<grid_for(units * 32, 256, sms * PprShape<MODE, C>::BLOCKS), 256, 0, s>>>(b);
+    ++launches;
+  }
+  if (a.nparts) {
+    k_ppr_combine<MODE, C><<<grid_for((uint64_t)a.nbig * (32 / G), 256, sms * 8), 256, 0, s>>>(a);
+    ++launches;
+  }
+}
+
 template <int MODE>
 static void ppr_sweep(const PprArgs& a, int sms, cudaStream_t s, uint64_t& launches) {
-  k_ppr_low<MODE><<<grid_for((uint64_t)a.n * 32, 256, sms * 8), 256, 0, s>>>(a);
-  ++launches;
-  if (a.nseg) {
-    k_ppr_seg<MODE><<<(int)std::min<uint64_t>(a.nseg, (uint64_t)sms * 8), kSegWarps * 32, 0, s>>>(a);
-    k_ppr_combine<MODE><<<grid_for((uint64_t)a.nbig * 32, 256, sms * 8), 256, 0, s>>>(a);
-    launches += 2;
+  switch (a.cols) {
+    case 8: return ppr_sweep_c<MODE, 8>(a, sms, s, launches);
+    case 16: return ppr_sweep_c<MODE, 16>(a, sms, s, launches);
+    case 24: return ppr_sweep_c<MODE, 24>(a, sms, s, launches);
+    case 32: return ppr_sweep_c<MODE, 32>(a, sms, s, launches);
+    case 48: return ppr_sweep_c<MODE, 48>(a, sms, s, launches);
+    default: return ppr_sweep_c<MODE, 64>(a, sms, s, launches);
   }
 }
 
@@ -511,8 +791,8 @@ static int ppr_ws(prx_context* c, uint32_t n, bool fp32) {
   return PRX_OK;
 }
 
-// The long rows of graph g (in-degree above a.low_max) and their segments of
-// a.seg edges into the workspace; returns the counts.
+// The long rows of graph g (in-degree above a.low_max) and their parts of
+// a.per edges into the workspace.
 static int ppr_segments(prx_context* c, const GraphDev& g, PprArgs& a) {
   PprWs& w = *c->ppr;
   cudaStream_t s = c->stream;
@@ -531,22 +811,21 @@ static int ppr_segments(prx_context* c, const GraphDev& g, PprArgs& a) {
     a.big = w.big;
   }
   a.nbig = nbig;
-  a.nseg = 0;
+  a.nparts = 0;
   if (!nbig) return PRX_OK;
-  TRY_CUDA_ST(grow(&w.segstart, w.segstart_cap, (size_t)nbig + 1));
-  const int grid = grid_for(nbig, 256, c->sms * 4);
-  k_ppr_segcount<<<grid, 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, nbig, a.seg, w.segstart);
-  TRY_CUDA_ST(exclusive_scan_u32(w.segstart, nbig + 1, s));
-  uint32_t nseg = 0;
-  TRY_CUDA_ST(cudaMemcpyAsync(&nseg, w.segstart + nbig, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  TRY_CUDA_ST(grow(&w.partstart, w.partstart_cap, (size_t)nbig + 1));
+  k_ppr_partcount<<<grid_for(nbig, 256, c->sms * 4), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, nbig, a.per, w.partstart);
+  TRY_CUDA_ST(exclusive_scan_u32(w.partstart, nbig + 1, s));
+  uint32_t nparts = 0;
+  TRY_CUDA_ST(cudaMemcpyAsync(&nparts, w.partstart + nbig, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   TRY_CUDA_ST(cudaStreamSynchronize(s));
-  TRY_CUDA_ST(grow(&w.seg, w.seg_cap, 2 * (size_t)nseg));
-  TRY_CUDA_ST(grow(&w.part, w.part_cap, (size_t)nseg * kCols));
-  k_ppr_segfill<<<grid, 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, nbig, a.seg, w.segstart, w.seg, w.seg + nseg);
-  a.segstart = w.segstart;
-  a.seg_v = w.seg;
-  a.seg_e = w.seg + nseg;
-  a.nseg = nseg;
+  TRY_CUDA_ST(grow(&w.parts, w.parts_cap, (size_t)nparts));
+  TRY_CUDA_ST(grow(&w.part, w.part_cap, (size_t)nparts * kCols));
+  k_ppr_partfill<<<grid_for((uint64_t)nbig * 32, 256, c->sms * 8), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, nbig, a.per,
+                                                                                w.partstart, w.parts);
+  a.partstart = w.partstart;
+  a.parts = w.parts;
+  a.nparts = nparts;
   a.part = w.part;
   return PRX_OK;
 }
@@ -662,7 +941,7 @@ static int ppr_block_graph(prx_context* c, PprArgs& a, const prx_options& o, boo
         if (ec == cudaSuccess) ec = el;
       }
       if (ec == cudaSuccess) {
-        k_ppr_commit<<<grid_for((size_t)a.n * kCols, 256, c->sms * 16), 256, 0, s>>>(a);
+        k_ppr_commit<<<grid_for((size_t)a.n * a.cols, 256, c->sms * 16), 256, 0, s>>>(a);
         k_ppr_cond<<<1, 1, 0, s>>>(ho, a.st, cap, 1);
       }
     }
@@ -700,7 +979,7 @@ static int ppr_block(prx_context* c, const GraphDev& g, PprArgs& a, const prx_op
                      const double** answer, prx_ppr_result* res) {
   cudaStream_t s = c->stream;
   uint64_t& L = c->launches;
-  const size_t rows = (size_t)g.n * kCols;
+  const size_t rows = (size_t)g.n * a.cols;
   TRY_CUDA_ST(cudaMemsetAsync(a.x[0], 0, sizeof(double) * rows, s));
   k_ppr_init<<<grid_for(g.n, 256, c->sms * 16), 256, 0, s>>>(a);
   launch_state_reset(c->st, o.max_iterations, o.tolerance, s);
@@ -816,13 +1095,18 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   if (st) return st;
   PprWs& w = *c->ppr;
   cudaStream_t s = c->stream;
+  const uint64_t slots = g.nseg > 1 ? g.xtpos.back() + (g.m - g.xtseg0.back()) : g.m;
+  TRY_CUDA_ST(grow(&w.pair, w.pair_cap, slots));
+  k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, w.pair);
+  c->launches += 1;
   PprArgs a{};
   a.xtoff = g.xtoff;
-  a.xtedg = g.xtedg;
   a.xtbase = g.xtbase;
   a.seg_shift = g.seg_shift;
   a.rcp = g.rcp;
   a.rcp32 = g.rcp32;
+  a.xtedg = g.xtedg;
+  a.pair = w.pair;
   a.x[0] = w.x[0];
   a.x[1] = w.x[1];
   a.rho = w.rho;
@@ -832,11 +1116,20 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   a.n = g.n;
   a.P = o.damping;
   a.Q = 1.0 - o.damping;
+  a.P32 = (float)o.damping;
   a.low_max = g.ppr_low_max ? g.ppr_low_max : kLowMax;
   a.seg = g.ppr_seg ? g.ppr_seg : kSeg;
   r.low_max = a.low_max;
   r.seg_edges = a.seg;
+  a.per = a.seg / kSegParts;
   if ((st = ppr_segments(c, g, a))) return st;
+  // The LOW rows in order of length (rows side by side in a warp then end
+  // together); by id with another bound or with row segments.
+  const bool by_length = a.low_max == kLowMax && g.nseg == 1;
+  if (by_length) TRY_CUDA_ST(ensure_len_list(gr->g, c->sms, s));
+  a.rows = by_length ? g.len_list : nullptr;
+  a.nrows = by_length ? g.cls_begin[MID] : g.n;
+  a.flat = !mixed_lengths(g);
   double* out = ranks_out;
   const size_t total = (size_t)g.n * nvec;
   if (!device_out) {
@@ -847,10 +1140,12 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   TRY_CUDA_ST(cudaEventRecord(c->ev[0], s));
   for (uint32_t c0 = 0; c0 < nvec; c0 += kCols) {
     const uint32_t cols = std::min<uint32_t>(kCols, nvec - c0);
+    for (int w : {64, 48, 32, 24, 16, 8})
+      if ((int)cols <= w) a.cols = w;
     if ((st = ppr_teleport(c, g.n, seed_off, seeds, c0, cols, a))) return st;
     const double* answer = nullptr;
     if ((st = ppr_block(c, g, a, o, fp32, &answer, &r))) return st;
-    k_ppr_out<<<grid_for((uint64_t)g.n * cols, 256, c->sms * 16), 256, 0, s>>>(answer, g.n, nvec, c0, cols, out);
+    k_ppr_out<<<grid_for((uint64_t)g.n * cols, 256, c->sms * 16), 256, 0, s>>>(answer, g.n, (uint32_t)a.cols, nvec, c0, cols, out);
     c->launches += 1;
   }
   TRY_CUDA_ST(cudaEventRecord(c->ev[1], s));
