@@ -1065,6 +1065,7 @@ int prx_graph_destroy(prx_graph* gr) {
               g.low_bm, g.rcp, g.rcp32});
   drop_weights(g);
   cudaFree(g.ocls_list);
+  cudaFree(g.oplan_list);
   free_chunks(g);
   free_hot(g);
   delete gr;

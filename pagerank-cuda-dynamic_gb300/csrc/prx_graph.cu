@@ -795,7 +795,7 @@ cudaError_t ensure_hot(GraphDev& g, uint32_t cap, int sms, cudaStream_t s) {
 
 cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layouts) {
   const uint32_t n = g.n;
-  g.plan_built = g.len_built = false;
+  g.plan_built = g.len_built = g.oplan_built = g.tpos_built = false;
   if (!keep_layouts) {
     free_chunks(g);
     free_hot(g);
@@ -828,11 +828,11 @@ void launch_vertex_tables(const uint32_t* xtoff, uint32_t shift, const uint32_t*
   k_reciprocals<<<sms * 4, 256, 0, s>>>(xtdat, n, rcp, rcp32);
 }
 
-__global__ void k_len_keys(const uint32_t* __restrict__ off, const uint32_t* __restrict__ list, uint32_t count,
-                           unsigned long long* __restrict__ key) {
+__global__ void k_len_keys(const uint32_t* __restrict__ off, uint32_t shift, const uint32_t* __restrict__ list,
+                           uint32_t count, uint32_t top, unsigned long long* __restrict__ key) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
     const uint32_t v = list[i];
-    key[i] = ((unsigned long long)(off[v + 1] - off[v]) << 32) | v;
+    key[i] = ((unsigned long long)(top - row_len(off, shift, v)) << 32) | v;
   }
 }
 __global__ void k_key_ids(const unsigned long long* __restrict__ key, uint32_t count, uint32_t* __restrict__ list) {
@@ -840,24 +840,33 @@ __global__ void k_key_ids(const unsigned long long* __restrict__ key, uint32_t c
     list[i] = (uint32_t)key[i];
 }
 
-cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s) {
-  const uint32_t low = g.cls_begin[MID];
-  if (g.len_built || low == 0) return cudaSuccess;
+cudaError_t sort_by_length(const uint32_t* off, uint32_t shift, const uint32_t* list, uint32_t count, uint32_t top,
+                           uint32_t* out, int sms, cudaStream_t s) {
+  if (count == 0) return cudaSuccess;
   unsigned long long *key = nullptr, *tmp = nullptr, *sorted = nullptr;
   uint32_t* hist = nullptr;
-  cudaError_t e = g.len_list ? cudaSuccess : graph_alloc(&g.len_list, sizeof(uint32_t) * g.n, s);
-  if (e == cudaSuccess) e = graph_alloc(&key, sizeof(*key) * ((size_t)low + 2), s);
-  if (e == cudaSuccess) e = graph_alloc(&tmp, sizeof(*tmp) * ((size_t)low + 2), s);
-  if (e == cudaSuccess) e = graph_alloc(&hist, sizeof(uint32_t) * radix_hist_words(low), s);
+  cudaError_t e = graph_alloc(&key, sizeof(*key) * ((size_t)count + 2), s);
+  if (e == cudaSuccess) e = graph_alloc(&tmp, sizeof(*tmp) * ((size_t)count + 2), s);
+  if (e == cudaSuccess) e = graph_alloc(&hist, sizeof(uint32_t) * radix_hist_words(count), s);
   if (e == cudaSuccess) {
-    k_len_keys<<<sms * 4, 256, 0, s>>>(g.xtoff, g.cls_list, low, key);
-    e = radix_sort_u64(key, tmp, low, 32, 39, hist, sms, s, &sorted);
-    if (e == cudaSuccess) k_key_ids<<<sms * 4, 256, 0, s>>>(sorted, low, g.len_list);
+    k_len_keys<<<sms * 4, 256, 0, s>>>(off, shift, list, count, top, key);
+    int bits = 0;
+    while (top >> bits) ++bits;
+    e = radix_sort_u64(key, tmp, count, 32, 32 + bits, hist, sms, s, &sorted);
+    if (e == cudaSuccess) k_key_ids<<<sms * 4, 256, 0, s>>>(sorted, count, out);
     if (e == cudaSuccess) e = cudaGetLastError();
   }
   if (key) cudaFreeAsync(key, s);
   if (tmp) cudaFreeAsync(tmp, s);
   if (hist) cudaFreeAsync(hist, s);
+  return e;
+}
+
+cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s) {
+  if (g.len_built || g.n == 0) return cudaSuccess;
+  cudaError_t e = g.len_list ? cudaSuccess : graph_alloc(&g.len_list, sizeof(uint32_t) * g.n, s);
+  if (e == cudaSuccess) e = sort_by_length(g.xtoff, g.seg_shift, g.cls_list, g.cls_begin[MID], kLowMax, g.len_list,
+                                           sms, s);
   g.len_built = e == cudaSuccess;
   return e;
 }
@@ -873,6 +882,9 @@ cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s) {
   uint64_t edges[NCLS];
   if (e == cudaSuccess)
     e = build_class_lists(g.xtoff, g.seg_shift, g.n, kPlanMid, g.plan_list, g.plan_begin, edges, sms, s);
+  uint32_t* mid = g.plan_list + g.plan_begin[MID];
+  if (e == cudaSuccess)
+    e = sort_by_length(g.xtoff, g.seg_shift, mid, g.plan_begin[HIGH] - g.plan_begin[MID], kPlanMid, mid, sms, s);
   g.plan_built = e == cudaSuccess;
   return e;
 }

@@ -157,9 +157,10 @@ struct GraphDev {
   uint32_t hot_n = 0;
   uint32_t hot_cap = 0;
   bool hot_built = false;
-  // Built on first use per graph version: the LOW ids in order of in-degree
-  // (ties ascending), and the ids by class with kPlanMid as the MID / HIGH
-  // boundary (the persistent loop's rows).
+  // Built on first use per graph version: the LOW ids by in-degree, the
+  // longest rows first (ties ascending), and the ids by class with kPlanMid as
+  // the MID / HIGH boundary, MID ones longest first (the persistent loop's
+  // rows: a sweep's last units are its shortest).
   uint32_t* len_list = nullptr;
   bool len_built = false;
   uint32_t* plan_list = nullptr;
@@ -174,9 +175,18 @@ struct GraphDev {
   double* pt = nullptr;           // the same in in-CSR (xtedg) order
   double* wsum = nullptr;         // W_u = sum of u's out-edge weights
   unsigned long long* wseg = nullptr;  // row segments: each out-CSR segment's compact start (weights, dL/dw)
-  uint32_t* ocls_list = nullptr;  // ids by out-degree class (rows of the out-CSR)
+  // of the out-CSR, built on the first weights of a graph version: ids by
+  // row-length class with mid_max and (oplan) with kPlanMid as the MID / HIGH
+  // boundary, LOW ids by length where they mix; each out-edge's position among
+  // the in-edges
+  uint32_t* ocls_list = nullptr;
   uint32_t ocls_begin[NCLS + 1] = {0, 0, 0, 0};
   uint64_t ocls_edges[NCLS] = {0, 0, 0};
+  uint32_t* oplan_list = nullptr;
+  uint32_t oplan_begin[NCLS + 1] = {0, 0, 0, 0};
+  bool oplan_built = false, oplan_fits = false;
+  uint32_t* tpos = nullptr;       // laid out like xedg; positions relative to the in-CSR's row segment
+  bool tpos_built = false;
 };
 
 // Frees the edge weights of g (after a batch, or with the graph).
@@ -290,7 +300,11 @@ constexpr uint32_t kDefaultChunk64 = (200u << 20) / sizeof(double);
 // side by side (8 lanes of 9 wait), web-like ones and grids stay in id order
 // (1.35), whose rows and ranks lie side by side in memory.
 inline bool mixed_lengths(const GraphDev& g) { return g.low_padded > 2 * g.cls_edges[LOW]; }
-// GraphDev::len_list (plain graphs), and the persistent loop's rows: plan_list,
+// The ids list[0 .. count) of rows of at most `top` entries, the longest rows
+// first (ties in the given order), into out (may be list).
+cudaError_t sort_by_length(const uint32_t* off, uint32_t shift, const uint32_t* list, uint32_t count, uint32_t top,
+                           uint32_t* out, int sms, cudaStream_t s);
+// GraphDev::len_list, and the persistent loop's rows: plan_list,
 // and len_list where the lengths mix.
 cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s);
 constexpr uint32_t kPlanMid = 1024;
@@ -301,11 +315,10 @@ constexpr uint32_t kPlanMid = 1024;
 // (31,000) 30 | 25, 1400^2 (61,000) 51 | 58; by length R-MAT 2^16 47 | 14, 2^18
 // 78 | 29, 2^21 (145,000) 375 | 219, 2^23 (630,000) 1254 | 991.
 constexpr uint64_t kPersistUnits = 48u << 10, kPersistSortedUnits = 1u << 20;
-inline bool persist_fits(const GraphDev& g) {
-  const uint32_t low = g.cls_begin[1] - g.cls_begin[0];
-  return ((uint64_t)(mixed_lengths(g) ? low : g.n) + 31) / 32 + (g.n - low) <=
-         (mixed_lengths(g) ? kPersistSortedUnits : kPersistUnits);
+inline bool plan_fits(uint32_t n, uint32_t low, bool mixed) {
+  return ((uint64_t)(mixed ? low : n) + 31) / 32 + (n - low) <= (mixed ? kPersistSortedUnits : kPersistUnits);
 }
+inline bool persist_fits(const GraphDev& g) { return plan_fits(g.n, g.cls_begin[MID], mixed_lengths(g)); }
 cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s);
 // The whole FP64 iteration loop of a plain graph (one row segment) as one
 // cooperative kernel from the ranks in parity 0 (prx_persist.cu); ensure_plan

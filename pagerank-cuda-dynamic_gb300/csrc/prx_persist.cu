@@ -143,11 +143,13 @@ template <int MODE, int K>
 __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRows rows) {
   using T = ModeTraits<MODE>;
   __shared__ double part[256];
+  __shared__ double s_tree[kThreads / 32][RowTree::kSlots];
   __shared__ unsigned long long s_el;
   __shared__ uint32_t s_nf, s_xb, s_marked;
   State* st = a.st;
   if (st->done) return;
   const uint32_t lane = lane_id(), t = threadIdx.x;
+  const RowTree tree{s_tree[t >> 5]};
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t warp = warps - 1 - ((blockIdx.x * blockDim.x + t) >> 5);
   const uint32_t words = (a.n + 31) >> 5;
@@ -179,8 +181,15 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
   };
   // this warp's first unit of LOW rows
   const uint32_t low0 = warp < rows.nmid ? warp + (rows.nmid - warp + warps - 1) / warps * warps : warp;
-  Unit first{};
-  if (warp < units) first = load_unit(warp);
+  // the unit this warp takes next: loaded while the one before it is summed,
+  // over the end of an iteration too (what a unit holds does not change)
+  Unit coming{};
+  if (warp < units) coming = load_unit(warp);
+  auto take = [&](uint32_t u) {
+    const Unit x = coming;
+    if (units > warps) coming = load_unit(u + warps < units ? u + warps : warp);
+    return x;
+  };
   GridBarrier bar(st);
   for (int it = 0;; ++it) {
     const int p = it & 1;
@@ -228,15 +237,37 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
       const double x = high_row_sum<double, true, true>(c, a.xtedg + s, d, t, part);
       if (t == 0) finish_one(v, x, d, in);
     }
+    // four MID rows are folded and finished together (see RowTree); lane k
+    // keeps what row k needs
+    uint32_t qv = 0, qlen = 0, held = 0;
+    VertexIn qin{};
+    auto flush = [&] {
+      double z = tree.fold<true>(held);
+      z = __shfl_sync(0xffffffffu, z, (lane & 3u) * 8);
+      if (lane < held) finish_one(qv, z, qlen, qin);
+      held = 0;
+    };
     for (uint32_t u = warp; u < rows.nmid; u += warps) {
-      const Unit x = u == warp ? first : load_unit(u);
+      const Unit x = take(u);
       if (!affected(x.v)) continue;
-      const VertexIn in = {x.d, x.R, a.r[p][x.v]};
-      const double sum = mid_row_sum<double, true, true>(c, a.xtedg + x.s, x.e - x.s, lane);
-      if (lane == 0) finish_one(x.v, sum, x.e - x.s, in);
+      if (lane == held) {
+        qv = x.v;
+        qlen = x.e - x.s;
+        qin = {x.d, x.R, a.r[p][x.v]};
+      }
+      bool bad = false;
+      const double sum = mid_lane_sums<double, true, true, true>(c, a.xtedg + x.s, x.e - x.s, lane, bad);
+      if (__any_sync(0xffffffffu, bad)) {  // terms out of soft_add's range: this row by FP64 adds alone
+        const double y = mid_row_sum_plain<true>(c, a.xtedg + x.s, x.e - x.s, lane);
+        if (lane == 0) finish_one(x.v, y, x.e - x.s, VertexIn{x.d, x.R, a.r[p][x.v]});
+        continue;
+      }
+      tree.put(held++, sum);
+      if (held == RowTree::kRows) flush();
     }
+    if (held) flush();
     for (uint32_t u = low0; u < units; u += warps) {
-      const Unit x = u == warp ? first : load_unit(u);
+      const Unit x = take(u);
       bool mine = x.row;
       if (T::DYN) {
         if (rows.sorted) {

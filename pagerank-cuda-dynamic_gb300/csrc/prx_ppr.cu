@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(256, PprShape<MODE, C>::BLOCKS) k_ppr_rows(Ppr
       if (i < a.nparts) Sh::store(reinterpret_cast<S*>(a.part), i, sub, acc);
       continue;
     }
-    const uint32_t i0 = (np + nb - 1 - b) * a.batch;  // the longest rows first
+    const uint32_t i0 = (b - np) * a.batch;
     // lane i: vertex i of the batch (len 0xffffffff: none, or a long row)
     uint32_t mv = 0, ml = 0xffffffffu;
     unsigned long long ms = 0;

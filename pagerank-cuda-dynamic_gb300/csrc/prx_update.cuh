@@ -186,6 +186,31 @@ __device__ __forceinline__ V plus(V a, V b) {
   else return a + b;
 }
 
+// The 32 lane values of up to four rows folded together: x[l] + x[l ^ 16], then
+// 8, 4, 2, 1, as a warp's shuffles would fold one row.  Lane 8r + i adds up
+// row r's values i, i + 8, i + 16, i + 24 by itself, so four rows take six
+// warp-wide FP64 adds instead of twenty (and their epilogues run side by
+// side).  One tree per warp; its rows lie 40 doubles apart (no bank conflicts).
+struct RowTree {
+  static constexpr uint32_t kRows = 4, kStride = 40, kSlots = kRows * kStride;
+  double* s;
+  __device__ __forceinline__ void put(uint32_t row, double x) const { s[row * kStride + lane_id()] = x; }
+  // Row r's sum in lane 8r (r < rows); every lane calls it.
+  template <bool SOFT>
+  __device__ __forceinline__ double fold(uint32_t rows) const {
+    __syncwarp();
+    const uint32_t row = lane_id() >> 3;
+    const double* x = s + row * kStride + (lane_id() & 7u);
+    const bool in = row < rows;
+    const double x0 = in ? x[0] : 0.0, x1 = in ? x[8] : 0.0, x2 = in ? x[16] : 0.0, x3 = in ? x[24] : 0.0;
+    __syncwarp();
+    double z = (x0 + x2) + plus<SOFT>(x1, x3);
+    z = plus<SOFT>(z, __shfl_xor_sync(0xffffffffu, z, 4));
+    z += __shfl_xor_sync(0xffffffffu, z, 2);
+    return plus<SOFT>(z, __shfl_xor_sync(0xffffffffu, z, 1));
+  }
+};
+
 // MID: the reference's 256-way sum of c over the d ids at ed, by one warp.
 // Lane l owns virtual threads l + 32k (k = 0..7); the sum is in lane 0.  The
 // first 256 terms are not added (to +0) but are the partial sums, and neither
@@ -193,8 +218,10 @@ __device__ __forceinline__ V plus(V a, V b) {
 // none: of 28 warp-wide adds for a row of 275 terms, 12 are left.
 // PRE: the ids of the next 256 terms are loaded behind the gathers of these
 // (few warps, where the latency of the two loads counts; 8 more registers).
+// mid_lane_sums: the partial sums of virtual threads 0 .. 31 (after the halving
+// tree's first three levels), one per lane.
 template <class V, bool COH, bool SOFT, bool PRE>
-__device__ __forceinline__ V mid_row_sum_t(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t lane,
+__device__ __forceinline__ V mid_lane_sums(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t lane,
                                            bool& bad) {
   V ps[8];
   uint32_t u[8];
@@ -234,14 +261,9 @@ __device__ __forceinline__ V mid_row_sum_t(const V* c, const uint32_t* __restric
   if (d > 224) ps[3] = plus<SOFT>(ps[3], ps[7]);
   ps[0] += ps[2];                                         // t < 64:  += t+64
   ps[1] = plus<SOFT>(ps[1], ps[3]);
-  V x = ps[0] + ps[1];                                    // t < 32:  += t+32
-  x = plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 16));
-  x += __shfl_down_sync(0xffffffffu, x, 8);
-  x = plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 4));
-  x += __shfl_down_sync(0xffffffffu, x, 2);
-  x = plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 1));
-  return x;
+  return ps[0] + ps[1];                                   // t < 32:  += t+32
 }
+
 // The same by FP64 adds alone, rolled up: it runs on terms out of
 // soft_add's range only, and must not add to the sweep's registers.
 template <bool COH>
@@ -268,11 +290,15 @@ template <class V, bool COH, bool PRE>
 __device__ __forceinline__ V mid_row_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t lane) {
   constexpr bool SOFT = std::is_same<V, double>::value;
   bool bad = false;
-  const V x = mid_row_sum_t<V, COH, SOFT, PRE>(c, ed, d, lane, bad);
+  V x = mid_lane_sums<V, COH, SOFT, PRE>(c, ed, d, lane, bad);
   if constexpr (SOFT) {
     if (__any_sync(0xffffffffu, bad)) return mid_row_sum_plain<COH>(c, ed, d, lane);
   }
-  return x;
+  x = plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 16));
+  x += __shfl_down_sync(0xffffffffu, x, 8);
+  x = plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 4));
+  x += __shfl_down_sync(0xffffffffu, x, 2);
+  return plus<SOFT>(x, __shfl_down_sync(0xffffffffu, x, 1));
 }
 
 // HIGH: the same sum by a block of 256 (thread t of the reference's block);

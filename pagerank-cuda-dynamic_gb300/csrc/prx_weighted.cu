@@ -16,8 +16,12 @@
 // (dr = (I - alpha P^T)^-1 (alpha dP^T r + (P^T r - t) dalpha + (1-alpha) dt),
 // and dP_uv'/dw_uv = (delta_vv' - P_uv') / W_u.)
 //
-// Rows go by length class: <= 64 one thread per row, <= 4096 one warp, else
-// one block; every sum has a fixed order, so results are deterministic.
+// Rows go by length class: <= 64 one thread per row, then one warp, then one
+// block; every sum has a fixed order, so results are deterministic.  Graphs
+// up to the lines of persist_fits iterate in one cooperative kernel
+// (k_pull_persist), as the FP64 solves do (prx_persist.cu): a sweep of R-MAT
+// 2^18 (4.2M edges, everything in L2) took 83 us in four launches and takes
+// 31 us there.  Larger ones launch the classes one by one.
 //
 // Graphs with row segments (64-bit offsets, see GraphDev): px / pt are laid
 // out like the edge arrays they follow (the same segment bases), and the
@@ -25,7 +29,7 @@
 // of a segment at its compact start + j).
 #include <algorithm>
 #include "prx_ctx.h"
-#include "prx_device.cuh"
+#include "prx_update.cuh"
 
 namespace prx {
 
@@ -34,8 +38,11 @@ void drop_weights(GraphDev& g) {
   cudaFree(g.pt);
   cudaFree(g.wsum);
   cudaFree(g.wseg);
+  cudaFree(g.tpos);
   g.px = g.pt = g.wsum = nullptr;
   g.wseg = nullptr;
+  g.tpos = nullptr;
+  g.tpos_built = false;
 }
 
 struct PullArgs {
@@ -55,6 +62,10 @@ struct PullArgs {
   double* y;                      // single sweep output (xin set)
   State* st;                      // null: single sweep, no L-inf
   uint32_t n;
+  // the persistent loop's rows (null: not taken)
+  const uint32_t* plan;
+  const uint32_t* plan_low;
+  uint32_t plan_begin[NCLS + 1];
 };
 
 __device__ __forceinline__ const double* pull_src(const PullArgs& a) {
@@ -166,6 +177,157 @@ __global__ void k_pull_fin(State* st) {
   if (el < st->tol || st->iter >= st->max_iter) st->done = 1;
 }
 
+// ---- the loop as one cooperative kernel ------------------------------------
+// Rows of PullArgs::list by class with kPlanMid as the MID / HIGH boundary.
+// See prx_persist.cu for the split, the memory rules and the barrier; the
+// iterate is read by ordinary loads.
+struct PullRow {
+  uint32_t v, len;
+  uint64_t at;   // the row's first edge in edg and prob
+};
+__device__ __forceinline__ PullRow pull_row(const PullArgs& a, uint32_t v) {
+  const uint64_t iv = seg_index(v, a.shift);
+  const uint32_t s = __ldg(a.off + iv);
+  return {v, __ldg(a.off + iv + 1) - s, (a.seg ? a.seg[(uint64_t)v >> a.shift] : 0) + s};
+}
+
+__global__ void __launch_bounds__(256, 3) k_pull_persist(PullArgs a, const uint32_t* __restrict__ low) {
+  __shared__ double part[8];
+  __shared__ double s_tree[8][RowTree::kSlots];
+  __shared__ unsigned long long s_el;
+  State* st = a.st;
+  if (st->done) return;
+  const uint32_t lane = lane_id(), t = threadIdx.x;
+  const RowTree tree{s_tree[t >> 5]};
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t warp = warps - 1 - ((blockIdx.x * blockDim.x + t) >> 5);
+  const uint32_t nlow = a.begin[MID] - a.begin[LOW], nmid = a.begin[HIGH] - a.begin[MID];
+  const uint32_t units = nmid + (nlow + 31) / 32;
+  const uint32_t low0 = warp < nmid ? warp + (nmid - warp + warps - 1) / warps * warps : warp;
+  // unit u: a MID row in every lane, or a LOW row per lane (len 0: none)
+  auto load_unit = [&](uint32_t u) -> PullRow {
+    if (u < nmid) return pull_row(a, __ldg(a.list + a.begin[MID] + u));
+    const uint32_t i = 32 * (u - nmid) + lane;
+    return i < nlow ? pull_row(a, __ldg(low + i)) : PullRow{0, 0, 0};
+  };
+  PullRow coming{0, 0, 0};  // loaded while the unit before is summed
+  if (warp < units) coming = load_unit(warp);
+  auto take = [&](uint32_t u) {
+    const PullRow r = coming;
+    if (units > warps) coming = load_unit(u + warps < units ? u + warps : warp);
+    return r;
+  };
+  const int max_iter = st->max_iter;
+  const double tol = st->tol;
+  GridBarrier bar(st);
+  for (int it = 0;; ++it) {
+    const int p = it & 1;
+    const double* x = a.x[p];
+    unsigned long long emax = 0;
+    auto finish = [&](uint32_t v, double sum, double old, double b) {
+      const double y = fma(a.alpha, sum, b);
+      a.x[p ^ 1][v] = y;
+      const unsigned long long d = dbits(fabs(y - old));
+      emax = d > emax ? d : emax;
+    };
+    auto base = [&](uint32_t v) { return a.base_scale * (a.base ? __ldg(a.base + v) : a.base_const); };
+    // sum of a row's terms i0, i0 + step, ... below len (steps: as many as any
+    // lane has; an FP64 fma issued for no term costs as much as one): ids and
+    // probabilities of the next four are loaded behind the gathers of these
+    auto strided = [&](const PullRow& r, uint32_t i0, uint32_t step, uint32_t steps) {
+      const uint32_t* __restrict__ edg = a.edg + r.at;
+      const double* __restrict__ prob = a.prob + r.at;
+      uint32_t u[4];
+      double w[4];
+      auto load = [&](uint32_t j) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t i = j + k * step;
+          u[k] = i < r.len ? __ldg(edg + i) : 0u;
+          w[k] = i < r.len ? __ldg(prob + i) : 0.0;
+        }
+      };
+      double acc = 0.0;
+      load(i0);
+      for (uint32_t n = steps, j = i0; n; j += 4 * step) {
+        double g[4], q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          g[k] = j + k * step < r.len ? x[u[k]] : 0.0;
+          q[k] = w[k];
+        }
+        load(j + 4 * step);
+        if (n >= 4) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc = fma(q[k], g[k], acc);
+          n -= 4;
+        } else {  // lanes past their row add 0 * 0
+          switch (n) {
+            case 1: acc = fma(q[0], g[0], acc); break;
+            case 2: acc = fma(q[1], g[1], fma(q[0], g[0], acc)); break;
+            default: acc = fma(q[2], g[2], fma(q[1], g[1], fma(q[0], g[0], acc))); break;
+          }
+          n = 0;
+        }
+      }
+      return acc;
+    };
+    for (uint32_t i = a.begin[HIGH] + blockIdx.x; i < a.begin[NCLS]; i += gridDim.x) {
+      const PullRow r = pull_row(a, __ldg(a.list + i));
+      double acc = strided(r, t, 256, (r.len + 255) / 256);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) part[t >> 5] = acc;
+      __syncthreads();
+      if (t == 0) {
+        double sum = 0.0;
+        for (int k = 0; k < 8; ++k) sum += part[k];
+        finish(r.v, sum, x[r.v], base(r.v));
+      }
+      __syncthreads();
+    }
+    // four MID rows are folded and finished together (see RowTree)
+    uint32_t qv = 0, held = 0;
+    double qold = 0.0, qb = 0.0;
+    auto flush = [&] {
+      double z = tree.fold<false>(held);
+      z = __shfl_sync(0xffffffffu, z, (lane & 3u) * 8);
+      if (lane < held) finish(qv, z, qold, qb);
+      held = 0;
+    };
+    for (uint32_t u = warp; u < nmid; u += warps) {
+      const PullRow r = take(u);
+      if (lane == held) {
+        qv = r.v;
+        qold = x[r.v];
+        qb = base(r.v);
+      }
+      tree.put(held++, strided(r, lane, 32, (r.len + 31) / 32));
+      if (held == RowTree::kRows) flush();
+    }
+    if (held) flush();
+    for (uint32_t u = low0; u < units; u += warps) {
+      const PullRow r = take(u);
+      const bool mine = 32 * (u - nmid) + lane < nlow;
+      const double old = mine ? x[r.v] : 0.0, b = mine ? base(r.v) : 0.0;
+      const double sum = strided(r, 0, 1, __reduce_max_sync(0xffffffffu, r.len));
+      if (mine) finish(r.v, sum, old, b);
+    }
+    block_max_bits(emax, &st->pel[it % 3]);
+    if (blockIdx.x == 0 && t == 0) st->pel[(it + 1) % 3] = 0;
+    if (!bar.sync([&] { s_el = *(volatile unsigned long long*)&st->pel[it % 3]; })) return;
+    const double el = __longlong_as_double((long long)s_el);
+    if (el < tol || it + 1 >= max_iter) {
+      if (blockIdx.x == 0 && t == 0) {
+        st->iter = it + 1;
+        st->last_delta = el;
+        st->done = 1;
+      }
+      return;
+    }
+  }
+}
+
 static int pull_grid(uint64_t work, int per_block, int cap) {
   const uint64_t b = (work + per_block - 1) / per_block;
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(b, (uint64_t)cap));
@@ -189,61 +351,161 @@ struct WeightCsr {
   const uint32_t *xoff, *xedg, *xtoff, *xtedg;
   const unsigned long long *xbase, *xtbase, *wseg;
   uint32_t shift;
+  uint32_t* tpos;   // GraphDev::tpos
 };
 
-__global__ void __launch_bounds__(256) k_set_weights(WeightCsr c, const float* __restrict__ w, uint32_t n,
-                                                     double* __restrict__ wsum, double* __restrict__ px,
+// p = w / W_u of an out-edge to its places in px and pt; its position among
+// v's in-edges is found once per graph version (tpos, found set).
+__device__ __forceinline__ void put_weight(const WeightCsr& c, uint32_t u, uint64_t at, double p, bool found,
+                                           double* __restrict__ px, double* __restrict__ pt, uint32_t* err) {
+  px[at] = p;
+  const uint32_t v = c.xedg[at];
+  const uint64_t bv = c.xtbase ? c.xtbase[(uint64_t)v >> c.shift] : 0;
+  if (found) {
+    pt[bv + c.tpos[at]] = p;
+    return;
+  }
+  const uint64_t iv = seg_index(v, c.shift);
+  const uint32_t* row = c.xtedg + bv;
+  uint32_t lo = c.xtoff[iv], hi = c.xtoff[iv + 1];
+  const uint32_t end = hi;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (row[mid] < u) lo = mid + 1;
+    else hi = mid;
+  }
+  if (lo < end && row[lo] == u) {
+    pt[bv + lo] = p;
+    c.tpos[at] = lo;
+  } else {
+    atomicOr(err, 2u);
+  }
+}
+
+// A float as a double by integer operations (the conversion instruction runs
+// on the FP64 pipe); zeros, subnormals, infinities and NaN convert as usual.
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x), e = (b >> 23) & 0xffu;
+  if (e - 1u >= 254u) return (double)x;
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+
+// w / W correctly rounded from y = RN(1 / W), as div_count does (normal W).
+__device__ __forceinline__ double div_by(double w, double W, double y) {
+  const double q = w * y;
+  return fma(fma(-q, W, w), y, q);
+}
+
+__device__ __forceinline__ double checked_weight(float x, uint32_t* err) {
+  if (!(x > 0.f) || !(x < INFINITY)) atomicOr(err, 1u);
+  return widen(x);
+}
+
+// What bounds setting weights: the FP64 pipe.  A warp per row and a plain
+// division per edge took 0.28 ms of it on R-MAT 2^18 (rows of 16 edges on
+// average), and one hub's row kept its warp busy for 2.5 ms.  Now rows of up
+// to 64 edges go by thread (in order of length where they mix), the next ones
+// by warp, longer ones by block (k_weight_sums, k_weight_edges), with one
+// reciprocal per row and three FP64 operations per edge.  list: the row ids by
+// class, begin: their bounds.
+struct WeightRows {
+  const uint32_t* list;
+  uint32_t nlow, nmid;
+};
+
+__global__ void __launch_bounds__(256) k_set_weights(WeightCsr c, WeightRows rows, const float* __restrict__ w,
+                                                     bool found, double* __restrict__ wsum, double* __restrict__ px,
                                                      double* __restrict__ pt, uint32_t* err) {
-  const uint32_t lane = lane_id();
-  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += (gridDim.x * blockDim.x) >> 5) {
+  const uint32_t lane = lane_id(), warps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t units = rows.nmid + (rows.nlow + 31) / 32;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < units; i += warps) {
+    const bool mid = i < rows.nmid;
+    const uint32_t at = mid ? rows.nlow + i : 32 * (i - rows.nmid) + lane;
+    if (!mid && at >= rows.nlow) continue;
+    const uint32_t u = rows.list[at], first = mid ? lane : 0, step = mid ? 32 : 1;
     const uint64_t iu = seg_index(u, c.shift);
     const uint32_t s = c.xoff[iu], e = c.xoff[iu + 1];
     const uint64_t bu = c.xbase ? c.xbase[(uint64_t)u >> c.shift] : 0;  // device position of the row's segment
     const uint64_t wu = c.wseg ? c.wseg[(uint64_t)u >> c.shift] : 0;    // its compact position
     double acc = 0.0;
-    for (uint32_t j = s + lane; j < e; j += 32) {
-      const float x = w[wu + j];
-      if (!(x > 0.f) || !(x < INFINITY)) atomicOr(err, 1u);
-      acc += (double)x;
-    }
+    for (uint32_t j = s + first; j < e; j += step) acc += checked_weight(w[wu + j], err);
+    if (mid) {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) wsum[u] = acc;
-    for (uint32_t j = s + lane; j < e; j += 32) {
-      const double p = (double)w[wu + j] / acc;
-      px[bu + j] = p;
-      const uint32_t v = c.xedg[bu + j];
-      const uint64_t iv = seg_index(v, c.shift);
-      const uint64_t bv = c.xtbase ? c.xtbase[(uint64_t)v >> c.shift] : 0;
-      const uint32_t* row = c.xtedg + bv;
-      uint32_t lo = c.xtoff[iv], hi = c.xtoff[iv + 1];
-      const uint32_t end = hi;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (row[mid] < u) lo = mid + 1;
-        else hi = mid;
-      }
-      if (lo < end && row[lo] == u) pt[bv + lo] = p;
-      else atomicOr(err, 2u);
+      for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     }
+    if (!mid || lane == 0) wsum[u] = acc;
+    const double y = 1.0 / acc;
+    for (uint32_t j = s + first; j < e; j += step)
+      put_weight(c, u, bu + j, div_by(widen(w[wu + j]), acc, y), found, px, pt, err);
   }
 }
 
+// W_u of the long rows, a block each (256 strided sums, then in order).
+__global__ void __launch_bounds__(256) k_weight_sums(WeightCsr c, const float* __restrict__ w,
+                                                     const uint32_t* __restrict__ list, double* __restrict__ wsum,
+                                                     uint32_t* err) {
+  __shared__ double part[8];
+  const uint32_t u = list[blockIdx.x];
+  const uint64_t iu = seg_index(u, c.shift);
+  const uint32_t s = c.xoff[iu], e = c.xoff[iu + 1];
+  const uint64_t wu = c.wseg ? c.wseg[(uint64_t)u >> c.shift] : 0;
+  double acc = 0.0;
+  for (uint32_t j = s + threadIdx.x; j < e; j += 256) {
+    acc += checked_weight(w[wu + j], err);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane_id() == 0) part[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int k = 0; k < 8; ++k) t += part[k];
+    wsum[u] = t;
+  }
+}
+
+// The long rows' edges: block (x, y) takes every gridDim.y-th piece of row x.
+__global__ void __launch_bounds__(256) k_weight_edges(WeightCsr c, const float* __restrict__ w,
+                                                      const uint32_t* __restrict__ list, bool found,
+                                                      const double* __restrict__ wsum, double* __restrict__ px,
+                                                      double* __restrict__ pt, uint32_t* err) {
+  const uint32_t u = list[blockIdx.x];
+  const uint64_t iu = seg_index(u, c.shift);
+  const uint32_t s = c.xoff[iu], e = c.xoff[iu + 1];
+  const uint64_t bu = c.xbase ? c.xbase[(uint64_t)u >> c.shift] : 0;
+  const uint64_t wu = c.wseg ? c.wseg[(uint64_t)u >> c.shift] : 0;
+  const double W = wsum[u], y = 1.0 / W;
+  for (uint32_t j = s + blockIdx.y * 256 + threadIdx.x; j < e; j += gridDim.y * 256)
+    put_weight(c, u, bu + j, div_by(widen(w[wu + j]), W, y), found, px, pt, err);
+}
+
 // ---- gradients -------------------------------------------------------------------
-// dL/dw_uv = (r_u / W_u) (alpha lambda_v - lambda_u + g_u), warp per source u.
+// dL/dw_uv = (r_u / W_u) (alpha lambda_v - lambda_u + g_u): a warp per source
+// of up to kPlanMid edges, the pieces of the longer rows (list) by block as in
+// k_weight_edges.
+__device__ __forceinline__ void grad_row(const WeightCsr& cs, uint32_t u, uint32_t first, uint32_t step,
+                                         const double* __restrict__ wsum, const double* __restrict__ r,
+                                         const double* __restrict__ lam, const double* __restrict__ g, double alpha,
+                                         double* __restrict__ out) {
+  const double f = r[u] / wsum[u], c = g[u] - lam[u];
+  const uint64_t iu = seg_index(u, cs.shift);
+  const uint64_t bu = cs.xbase ? cs.xbase[(uint64_t)u >> cs.shift] : 0;
+  const uint64_t wu = cs.wseg ? cs.wseg[(uint64_t)u >> cs.shift] : 0;
+  const uint32_t e = cs.xoff[iu + 1];
+  for (uint32_t j = cs.xoff[iu] + first; j < e; j += step) out[wu + j] = f * fma(alpha, lam[cs.xedg[bu + j]], c);
+}
 __global__ void __launch_bounds__(256) k_grad_w(WeightCsr cs, const double* __restrict__ wsum,
                                                 const double* __restrict__ r, const double* __restrict__ lam,
                                                 const double* __restrict__ g, double alpha, uint32_t n,
                                                 double* __restrict__ out) {
-  const uint32_t lane = lane_id();
-  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += (gridDim.x * blockDim.x) >> 5) {
-    const double f = r[u] / wsum[u], c = g[u] - lam[u];
-    const uint64_t iu = seg_index(u, cs.shift);
-    const uint64_t bu = cs.xbase ? cs.xbase[(uint64_t)u >> cs.shift] : 0;
-    const uint64_t wu = cs.wseg ? cs.wseg[(uint64_t)u >> cs.shift] : 0;
-    for (uint32_t j = cs.xoff[iu] + lane; j < cs.xoff[iu + 1]; j += 32)
-      out[wu + j] = f * fma(alpha, lam[cs.xedg[bu + j]], c);
-  }
+  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += (gridDim.x * blockDim.x) >> 5)
+    if (row_len(cs.xoff, cs.shift, u) <= kPlanMid) grad_row(cs, u, lane_id(), 32, wsum, r, lam, g, alpha, out);
+}
+__global__ void __launch_bounds__(256) k_grad_w_long(WeightCsr cs, const uint32_t* __restrict__ list,
+                                                     const double* __restrict__ wsum, const double* __restrict__ r,
+                                                     const double* __restrict__ lam, const double* __restrict__ g,
+                                                     double alpha, double* __restrict__ out) {
+  grad_row(cs, list[blockIdx.x], blockIdx.y * 256 + threadIdx.x, gridDim.y * 256, wsum, r, lam, g, alpha, out);
 }
 
 __global__ void k_fill(double* __restrict__ x, double value, uint32_t n) {
@@ -292,13 +554,44 @@ static int wk_grow(prx_context* c, size_t doubles) {
 }
 
 static WeightCsr weight_csr(const GraphDev& g) {
-  return WeightCsr{g.xoff, g.xedg, g.xtoff, g.xtedg, g.xbase, g.xtbase, g.wseg, g.seg_shift};
+  return WeightCsr{g.xoff, g.xedg, g.xtoff, g.xtedg, g.xbase, g.xtbase, g.wseg, g.seg_shift, g.tpos};
 }
 
 // Device slots of one CSR's edge array (its segments' positions and counts).
 static uint64_t csr_slots(const GraphDev& g, const std::vector<uint64_t>& seg0, const std::vector<uint64_t>& pos) {
   if (g.nseg <= 1) return g.m ? g.m : 1;
   return pos.back() + (g.m - seg0.back()) + 4;
+}
+
+// Blocks per long row of k_weight_edges and k_grad_w_long.
+constexpr int kLongPieces = 8;
+
+// The persistent loop's rows of a, for graphs up to the lines of persist_fits.
+static void take_plan(PullArgs& a, const uint32_t* list, const uint32_t* low, const uint32_t begin[NCLS + 1]) {
+  a.plan = list;
+  a.plan_low = low;
+  for (int k = 0; k <= NCLS; ++k) a.plan_begin[k] = begin[k];
+}
+
+static cudaError_t launch_pull_persist(PullArgs a, int sms, cudaStream_t s) {
+  int per_sm = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pull_persist, 256, 0);
+  if (e != cudaSuccess) return e;
+  a.list = a.plan;
+  for (int k = 0; k <= NCLS; ++k) a.begin[k] = a.plan_begin[k];
+  const uint32_t nlow = a.begin[MID] - a.begin[LOW], nmid = a.begin[HIGH] - a.begin[MID],
+                 nlong = a.begin[NCLS] - a.begin[HIGH];
+  const uint64_t want = std::max<uint64_t>(1, nlong + ((uint64_t)nmid + (nlow + 31) / 32 + 7) / 8);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)std::min<uint64_t>(want, (uint64_t)per_sm * sms));
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_pull_persist, a, a.plan_low);
 }
 
 static PullArgs forward_args(const GraphDev& g, const double* t, double alpha) {
@@ -326,7 +619,13 @@ static int pull_loop(prx_context* c, PullArgs& a, const prx_options& o, int* par
   a.xin = nullptr;
   launch_state_reset(c->st, o.max_iterations, o.tolerance, s);
   c->launches += 1;
-  if (o.max_iterations > 0) {
+  if (o.max_iterations > 0 && a.plan && o.loop == PRX_LOOP_AUTO) {
+    TRY_CUDA_ST(launch_pull_persist(a, c->sms, s));
+    c->launches += 1;
+    TRY_CUDA_ST(cudaMemcpyAsync(&c->st_host[1], c->st, sizeof(State), cudaMemcpyDeviceToHost, s));
+    TRY_CUDA_ST(cudaStreamSynchronize(s));
+    if (c->st_host[1].err & kErrGridWait) FAIL(PRX_ETIMEOUT, "weighted solve: a bounded grid wait ran out");
+  } else if (o.max_iterations > 0) {
     for (int k = 1;; k = std::min(2 * k, 16)) {
       for (int i = 0; i < k; ++i) {
         pull_sweep(a, c->sms, s, c->launches);
@@ -376,24 +675,50 @@ int prx_graph_set_weights(prx_context* c, prx_graph* gr, const float* w) {
   if (!w && g.m) FAIL(PRX_EINVAL, "prx_graph_set_weights: weights are NULL");
   TRY_CUDA_ST(cudaSetDevice(c->device));
   cudaStream_t s = c->stream;
-  drop_weights(g);
-  TRY_CUDA_ST(cudaMalloc(&g.px, sizeof(double) * csr_slots(g, g.xseg0, g.xpos)));
-  TRY_CUDA_ST(cudaMalloc(&g.pt, sizeof(double) * csr_slots(g, g.xtseg0, g.xtpos)));
-  TRY_CUDA_ST(cudaMalloc(&g.wsum, sizeof(double) * (g.n ? g.n : 1)));
-  if (g.nseg > 1) {  // each out-CSR segment's compact start
-    TRY_CUDA_ST(cudaMalloc(&g.wseg, sizeof(unsigned long long) * g.nseg));
-    TRY_CUDA_ST(cudaMemcpyAsync(g.wseg, g.xseg0.data(), sizeof(unsigned long long) * g.nseg,
-                                cudaMemcpyHostToDevice, s));
+  // the arrays stay for the next weights of the same graph version (a batch drops them)
+  if (!g.px) {
+    TRY_CUDA_ST(cudaMalloc(&g.px, sizeof(double) * csr_slots(g, g.xseg0, g.xpos)));
+    TRY_CUDA_ST(cudaMalloc(&g.pt, sizeof(double) * csr_slots(g, g.xtseg0, g.xtpos)));
+    TRY_CUDA_ST(cudaMalloc(&g.wsum, sizeof(double) * (g.n ? g.n : 1)));
+    TRY_CUDA_ST(cudaMalloc(&g.tpos, sizeof(uint32_t) * csr_slots(g, g.xseg0, g.xpos)));
+    if (g.nseg > 1) {  // each out-CSR segment's compact start
+      TRY_CUDA_ST(cudaMalloc(&g.wseg, sizeof(unsigned long long) * g.nseg));
+      TRY_CUDA_ST(cudaMemcpyAsync(g.wseg, g.xseg0.data(), sizeof(unsigned long long) * g.nseg,
+                                  cudaMemcpyHostToDevice, s));
+    }
   }
-  if (!g.ocls_list) TRY_CUDA_ST(cudaMalloc(&g.ocls_list, sizeof(uint32_t) * (g.n ? g.n : 1)));
+  if (!g.oplan_built) {
+    const size_t ids = sizeof(uint32_t) * (g.n ? g.n : 1);
+    if (!g.ocls_list) TRY_CUDA_ST(cudaMalloc(&g.ocls_list, ids));
+    if (!g.oplan_list) TRY_CUDA_ST(cudaMalloc(&g.oplan_list, ids));
+    uint64_t padded = 0, edges[NCLS];
+    TRY_CUDA_ST(build_class_lists(g.xoff, g.seg_shift, g.n, g.mid_max, g.ocls_list, g.ocls_begin, g.ocls_edges,
+                                  c->sms, s, &padded));
+    TRY_CUDA_ST(build_class_lists(g.xoff, g.seg_shift, g.n, kPlanMid, g.oplan_list, g.oplan_begin, edges, c->sms, s));
+    const bool mixed = padded > 2 * edges[LOW];  // as for the in-edges
+    if (mixed)
+      TRY_CUDA_ST(sort_by_length(g.xoff, g.seg_shift, g.ocls_list, g.ocls_begin[MID], kLowMax, g.oplan_list, c->sms, s));
+    uint32_t* mid_rows = g.oplan_list + g.oplan_begin[MID];
+    TRY_CUDA_ST(sort_by_length(g.xoff, g.seg_shift, mid_rows, g.oplan_begin[HIGH] - g.oplan_begin[MID], kPlanMid,
+                               mid_rows, c->sms, s));
+    g.oplan_fits = plan_fits(g.n, g.oplan_begin[MID], mixed);
+    g.oplan_built = true;
+  }
   launch_state_reset(c->st, 0, 0.0, s);
-  if (g.n)
-    k_set_weights<<<pull_grid((uint64_t)g.n * 32, 256, c->sms * 16), 256, 0, s>>>(weight_csr(g), w, g.n, g.wsum,
-                                                                                  g.px, g.pt, &c->st->err);
+  if (g.n) {
+    const bool found = g.tpos_built;
+    const WeightRows by_class = {g.oplan_list, g.oplan_begin[MID], g.oplan_begin[HIGH] - g.oplan_begin[MID]};
+    const uint64_t units = by_class.nmid + (by_class.nlow + 31ull) / 32;
+    k_set_weights<<<pull_grid(units * 32, 256, c->sms * 8), 256, 0, s>>>(weight_csr(g), by_class, w, found, g.wsum,
+                                                                         g.px, g.pt, &c->st->err);
+    if (const uint32_t nl = g.oplan_begin[NCLS] - g.oplan_begin[HIGH]) {
+      const uint32_t* rows = g.oplan_list + g.oplan_begin[HIGH];
+      k_weight_sums<<<nl, 256, 0, s>>>(weight_csr(g), w, rows, g.wsum, &c->st->err);
+      k_weight_edges<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), w, rows, found, g.wsum, g.px, g.pt,
+                                                          &c->st->err);
+    }
+  }
   TRY_CUDA_ST(cudaGetLastError());
-  const cudaError_t e = build_class_lists(g.xoff, g.seg_shift, g.n, g.mid_max, g.ocls_list, g.ocls_begin,
-                                         g.ocls_edges, c->sms, s);
-  TRY_CUDA_ST(e);
   TRY_CUDA_ST(cudaMemcpyAsync(&c->st_host[1], c->st, sizeof(State), cudaMemcpyDeviceToHost, s));
   TRY_CUDA_ST(cudaStreamSynchronize(s));
   const uint32_t err = c->st_host[1].err;
@@ -402,6 +727,7 @@ int prx_graph_set_weights(prx_context* c, prx_graph* gr, const float* w) {
     if (err & 1u) FAIL(PRX_EINVAL, "prx_graph_set_weights: every weight must be positive and finite");
     FAIL(PRX_EINVAL, "prx_graph_set_weights: an out-edge is missing from the in-CSR");
   }
+  g.tpos_built = true;
   return PRX_OK;
 }
 
@@ -423,6 +749,10 @@ int prx_solve_weighted(prx_context* c, prx_graph* gr, const double* t, const dou
   if ((st = wk_grow(c, 2 * (size_t)g.n))) return st;
   cudaStream_t s = c->stream;
   PullArgs a = forward_args(g, t, o.damping);
+  if (persist_fits(g)) {
+    TRY_CUDA_ST(ensure_plan(gr->g, c->sms, s));
+    take_plan(a, g.plan_list, mixed_lengths(g) ? g.len_list : g.plan_list, g.plan_begin);
+  }
   a.x[0] = c->wk;
   a.x[1] = c->wk + g.n;
   const uint64_t l0 = c->launches;
@@ -479,6 +809,7 @@ int prx_adjoint(prx_context* c, prx_graph* gr, const double* t, const double* r,
   a.shift = g.seg_shift;
   a.list = g.ocls_list;
   for (int k = 0; k <= NCLS; ++k) a.begin[k] = g.ocls_begin[k];
+  if (g.oplan_fits) take_plan(a, g.oplan_list, g.oplan_list, g.oplan_begin);
   a.base = gl;
   a.base_scale = 1.0;
   a.alpha = alpha;
@@ -498,6 +829,11 @@ int prx_adjoint(prx_context* c, prx_graph* gr, const double* t, const double* r,
   if (grad_w) {
     k_grad_w<<<grid, 256, 0, s>>>(weight_csr(g), g.wsum, r, lam, gl, alpha, g.n, grad_w);
     c->launches += 1;
+    if (const uint32_t nl = g.oplan_begin[NCLS] - g.oplan_begin[HIGH]) {
+      k_grad_w_long<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), g.oplan_list + g.oplan_begin[HIGH], g.wsum, r,
+                                                         lam, gl, alpha, grad_w);
+      c->launches += 1;
+    }
   }
   if (grad_t) {
     k_scale<<<pull_grid(g.n, 256, c->sms * 16), 256, 0, s>>>(lam, 1.0 - alpha, g.n, grad_t);
