@@ -443,6 +443,12 @@ cudaError_t exclusive_scan_u32(uint32_t* data, uint32_t len, cudaStream_t s);
 uint32_t scan_ws_words(uint32_t len);
 cudaError_t exclusive_scan_u32_ws(uint32_t* data, uint32_t len, uint32_t* sums, cudaStream_t s);
 
+// Both CSRs and the out-degrees of g (n set, its arrays not allocated) from an
+// edge list in device memory (prx_ingest.cu), a loop on every vertex with
+// self_loops.  *bad_id: an id was out of range (the CSRs are incomplete then).
+cudaError_t build_csr_pair(GraphDev& g, const uint32_t* u, const uint32_t* v, uint32_t count, bool self_loops,
+                           bool* bad_id, int sms, cudaStream_t s);
+
 // Stable LSD radix sort of keys[0 .. count) on their bits [lo, hi), 8 at a
 // time, ping-ponging with tmp (both with 2 keys of slack past count: the
 // last tile's bulk copy is rounded up to 16 bytes); *out is the buffer that

@@ -602,9 +602,84 @@ static int tidy_list(prx_context* c, const GraphDev& g, const uint32_t* hu, cons
   return tidy_core(c, g, b, count, deletions, ou, ov, kept);
 }
 
+// build_csr_pair of a dense list, by radix sorts of its keys.  Device memory: 3
+// key buffers of 8 bytes per edge and 2 scan buffers of 4, then the graph.
+static cudaError_t build_csr_pair_keys(GraphDev& g, const uint32_t* u, const uint32_t* v, uint32_t count,
+                                       bool self_loops, bool* bad_id, int sms, cudaStream_t s) {
+  const uint32_t n = g.n, total = count + (self_loops ? n : 0);
+  int vbits = 1;
+  while (vbits < 32 && (1ull << vbits) < n) ++vbits;
+  TidyBufs b;  // flag, pos, hist, key, key2
+  unsigned long long *key3 = nullptr, *sorted = nullptr;
+  uint32_t *bad = nullptr, m = 0, bad_h = 0;
+  const size_t cap = total ? total : 1;
+  const uint32_t tiles = (total + kSortTile - 1) / kSortTile;
+  const int grid = grid_of(cap, sms);
+  *bad_id = false;
+  cudaError_t e = graph_alloc(&b.flag, 4ull * (cap + 1), s);
+  if (e == cudaSuccess) e = graph_alloc(&b.pos, 4ull * (cap + 1), s);
+  if (e == cudaSuccess) e = graph_alloc(&b.hist, 4ull * ((size_t)kRadix * tiles + 1), s);
+  if (e == cudaSuccess) e = graph_alloc(&b.key, 8ull * (cap + 2), s);    // + 2: radix_sort_u64's slack
+  if (e == cudaSuccess) e = graph_alloc(&b.key2, 8ull * (cap + 2), s);
+  if (e == cudaSuccess) e = graph_alloc(&key3, 8ull * (cap + 2), s);
+  if (e == cudaSuccess) e = graph_alloc(&bad, 4, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, 4, s);
+  // sorted unique (u, v): the out-CSR
+  if (e == cudaSuccess) {
+    k_ingest_keys<<<grid, 256, 0, s>>>(u, v, count, n, self_loops ? 1 : 0, vbits, b.key, bad);
+    e = radix_sort_u64(b.key, b.key2, total, 0, 2 * vbits, b.hist, sms, s, &sorted);
+  }
+  unsigned long long* uniq = sorted == b.key ? b.key2 : b.key;  // the sort's spare buffer
+  if (e == cudaSuccess) {
+    k_first_flags<<<grid, 256, 0, s>>>(sorted, total, b.flag);
+    e = cudaMemcpyAsync(b.pos, b.flag, 4ull * total, cudaMemcpyDeviceToDevice, s);
+  }
+  if (e == cudaSuccess) e = cudaMemsetAsync(b.pos + total, 0, 4, s);
+  if (e == cudaSuccess) e = exclusive_scan_u32(b.pos, total + 1, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&m, b.pos + total, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&bad_h, bad, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) k_ingest_split<<<grid, 256, 0, s>>>(sorted, b.flag, b.pos, total, vbits, 1, uniq, key3);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  *bad_id = bad_h != 0;
+  if (e == cudaSuccess && !*bad_id) {
+    g.m = g.m_cap = m;
+    e = graph_alloc(&g.xoff, 4ull * ((size_t)n + 1), s);
+    if (e == cudaSuccess) e = graph_alloc(&g.xedg, 4ull * (m ? m : 1), s);
+    if (e == cudaSuccess) e = graph_alloc(&g.xtoff, 4ull * ((size_t)n + 1), s);
+    if (e == cudaSuccess) e = graph_alloc(&g.xtedg, 4ull * edge_slots(m), s);
+    if (e == cudaSuccess) e = graph_alloc(&g.xtdat, 4ull * (n ? n : 1), s);
+    const int gm = grid_of(m, sms), gn = grid_of((uint64_t)n + 1, sms);
+    if (e == cudaSuccess) {
+      k_ingest_offsets<<<gn, 256, 0, s>>>(uniq, m, vbits, n, g.xoff);
+      k_ingest_columns<<<gm, 256, 0, s>>>(uniq, m, vbits, g.xedg);
+      k_ingest_degree<<<gn, 256, 0, s>>>(g.xoff, n, g.xtdat);
+      // the transpose: the swapped keys v * 2^b + u arrive ordered by u, so a
+      // stable sort on their high half (v) alone orders them by (v, u); the
+      // spare buffer is the old sorted one
+      e = radix_sort_u64(key3, sorted, m, vbits, 2 * vbits, b.hist, sms, s, &sorted);
+    }
+    if (e == cudaSuccess) {
+      k_ingest_offsets<<<gn, 256, 0, s>>>(sorted, m, vbits, n, g.xtoff);
+      k_ingest_columns<<<gm, 256, 0, s>>>(sorted, m, vbits, g.xtedg);
+      e = cudaStreamSynchronize(s);
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+  }
+  b.release();
+  graph_free({key3, bad});
+  return e;
+}
+
+// Rows this long on average (with duplicates) come from few vertices: the keys
+// are short, and the row sorts have the long rows that cost them most.  Random
+// lists, radix keys against counting (prx_ingest.cu): 60000 rows of 1600 7.1 and
+// 9.1 ms, 100000 of 1000 9.0 and 9.2, 60000 of 800 3.8 and 3.7, 60000 of 256 1.5
+// and 1.3, 2M of 16 3.9 and 3.2; 3000 rows of 20000, mostly duplicates, 3.0 and
+// 8.3.
+constexpr uint64_t kDenseRows = 1024;
+
 // prx_graph_create_from_edges[_device].  Device memory: the edge arrays (host
-// edges only), 3 key buffers of 8 bytes per edge, 2 scan buffers of 4 bytes
-// per edge, then the graph.
+// edges only) and what the chosen build takes.
 static int create_from_edges(prx_context* c, uint32_t n, const uint32_t* u, const uint32_t* v, uint64_t count64,
                              int self_loops, bool on_device, prx_graph** out) {
   if (!c || !out) FAIL(PRX_EINVAL, "prx_graph_create_from_edges: NULL context or output");
@@ -617,95 +692,39 @@ static int create_from_edges(prx_context* c, uint32_t n, const uint32_t* u, cons
   if (n > kMaxVertices) FAIL(PRX_ERANGE, "prx_graph_create_from_edges: more than 2^32 - 2^24 vertices");
   TRY_CUDA_ST(cudaSetDevice(c->device));
   cudaStream_t s = c->stream;
-  const uint32_t count = (uint32_t)count64, total = (uint32_t)total64;
-  int vbits = 1;
-  while (vbits < 32 && (1ull << vbits) < n) ++vbits;
+  const uint32_t count = (uint32_t)count64;
   prx_graph* gr = new prx_graph();
   gr->ctx = c;
   GraphDev& g = gr->g;
   g.device = c->device;
   g.n = n;
-  TidyBufs b;                          // u, v (host edges), flag, pos, hist, key, key2
-  unsigned long long* key3 = nullptr;
-  uint32_t* bad = nullptr;
-  auto release = [&]() {
-    b.release();
-    b = TidyBufs();
-    graph_free({key3, bad});
-    key3 = nullptr;
-    bad = nullptr;
-  };
+  uint32_t *hu = nullptr, *hv = nullptr;  // device copies of host edges
   auto fail = [&](cudaError_t e) {
-    release();
+    graph_free({hu, hv});
     prx_graph_destroy(gr);
     set_error(std::string("prx_graph_create_from_edges: ") + cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? PRX_ENOMEM : PRX_ECUDA;
   };
-  const size_t cap = total ? total : 1;
-  const uint32_t tiles = (total + kSortTile - 1) / kSortTile;
   cudaError_t e = cudaSuccess;
-  const uint32_t *du = u, *dv = v;
   if (!on_device && count) {
-    if (e == cudaSuccess) e = graph_alloc(&b.u, 4ull * count, s);
-    if (e == cudaSuccess) e = graph_alloc(&b.v, 4ull * count, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(b.u, u, 4ull * count, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(b.v, v, 4ull * count, cudaMemcpyHostToDevice, s);
-    du = b.u;
-    dv = b.v;
+    e = graph_alloc(&hu, 4ull * count, s);
+    if (e == cudaSuccess) e = graph_alloc(&hv, 4ull * count, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hu, u, 4ull * count, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hv, v, 4ull * count, cudaMemcpyHostToDevice, s);
   }
-  if (e == cudaSuccess) e = graph_alloc(&b.flag, 4ull * (cap + 1), s);
-  if (e == cudaSuccess) e = graph_alloc(&b.pos, 4ull * (cap + 1), s);
-  if (e == cudaSuccess) e = graph_alloc(&b.hist, 4ull * ((size_t)kRadix * tiles + 1), s);
-  if (e == cudaSuccess) e = graph_alloc(&b.key, 8ull * (cap + 2), s);    // + 2: radix_sort_u64's slack
-  if (e == cudaSuccess) e = graph_alloc(&b.key2, 8ull * (cap + 2), s);
-  if (e == cudaSuccess) e = graph_alloc(&key3, 8ull * (cap + 2), s);
-  if (e == cudaSuccess) e = graph_alloc(&bad, 4, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, 4, s);
+  bool bad_id = false;
+  if (e == cudaSuccess)
+    e = (total64 >= kDenseRows * n ? build_csr_pair_keys : build_csr_pair)(
+        g, on_device ? u : hu, on_device ? v : hv, count, self_loops != 0, &bad_id, c->sms, s);
+  if (hu) cudaFreeAsync(hu, s);
+  if (hv) cudaFreeAsync(hv, s);
+  hu = hv = nullptr;
   if (e != cudaSuccess) return fail(e);
-  const int grid = grid_of(cap, c->sms);
-  // sorted unique (u, v): the out-CSR
-  k_ingest_keys<<<grid, 256, 0, s>>>(du, dv, count, n, self_loops ? 1 : 0, vbits, b.key, bad);
-  unsigned long long* sorted = nullptr;
-  e = radix_sort_u64(b.key, b.key2, total, 0, 2 * vbits, b.hist, c->sms, s, &sorted);
-  if (e != cudaSuccess) return fail(e);
-  unsigned long long* uniq = sorted == b.key ? b.key2 : b.key;  // the sort's spare buffer
-  k_first_flags<<<grid, 256, 0, s>>>(sorted, total, b.flag);
-  e = cudaMemcpyAsync(b.pos, b.flag, 4ull * total, cudaMemcpyDeviceToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b.pos + total, 0, 4, s);
-  if (e == cudaSuccess) e = exclusive_scan_u32(b.pos, total + 1, s);
-  uint32_t m = 0, bad_h = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&m, b.pos + total, 4, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&bad_h, bad, 4, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) k_ingest_split<<<grid, 256, 0, s>>>(sorted, b.flag, b.pos, total, vbits, 1, uniq, key3);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e != cudaSuccess) return fail(e);
-  if (bad_h) {
-    release();
+  if (bad_id) {
     prx_graph_destroy(gr);
     FAIL(PRX_EINVAL, "prx_graph_create_from_edges: vertex id out of range");
   }
-  g.m = g.m_cap = m;
-  if (e == cudaSuccess) e = graph_alloc(&g.xoff, 4ull * ((size_t)n + 1), s);
-  if (e == cudaSuccess) e = graph_alloc(&g.xedg, 4ull * (m ? m : 1), s);
-  if (e == cudaSuccess) e = graph_alloc(&g.xtoff, 4ull * ((size_t)n + 1), s);
-  if (e == cudaSuccess) e = graph_alloc(&g.xtedg, 4ull * edge_slots(m), s);
-  if (e == cudaSuccess) e = graph_alloc(&g.xtdat, 4ull * (n ? n : 1), s);
-  if (e != cudaSuccess) return fail(e);
-  const int gm = grid_of(m, c->sms), gn = grid_of((uint64_t)n + 1, c->sms);
-  k_ingest_offsets<<<gn, 256, 0, s>>>(uniq, m, vbits, n, g.xoff);
-  k_ingest_columns<<<gm, 256, 0, s>>>(uniq, m, vbits, g.xedg);
-  k_ingest_degree<<<gn, 256, 0, s>>>(g.xoff, n, g.xtdat);
-  // the transpose: the swapped keys v * 2^b + u arrive ordered by u, so a
-  // stable sort on their high half (v) alone orders them by (v, u); the
-  // spare buffer is the old sorted one
-  e = radix_sort_u64(key3, sorted, m, vbits, 2 * vbits, b.hist, c->sms, s, &sorted);
-  if (e != cudaSuccess) return fail(e);
-  k_ingest_offsets<<<gn, 256, 0, s>>>(sorted, m, vbits, n, g.xtoff);
-  k_ingest_columns<<<gm, 256, 0, s>>>(sorted, m, vbits, g.xtedg);
-  e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) e = cudaGetLastError();
-  release();
-  if (e == cudaSuccess) e = build_classes(g, c->sms, s);
+  e = build_classes(g, c->sms, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = tune_apply_cached(g, c->sms, s);
   if (e != cudaSuccess) return fail(e);
