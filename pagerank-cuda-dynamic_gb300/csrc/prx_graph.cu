@@ -980,10 +980,51 @@ __global__ void __launch_bounds__(256) k_scan_apply(uint32_t* __restrict__ data,
   }
 }
 
+// The whole scan in one block: 8 words a thread at a time, a running total
+// between.  Three launches take 10 us of any short array, this 4 of 8192
+// words and as many again for each further 8192.
+constexpr uint32_t kScanBlock = 1u << 15;
+__global__ void __launch_bounds__(1024) k_scan_block(uint32_t* __restrict__ a, uint32_t len) {
+  __shared__ uint32_t sums[2][32];
+  const uint32_t t = threadIdx.x, w = t >> 5, lane = t & 31u;
+  uint32_t total = 0, buf = 0;
+  for (uint32_t i0 = 0; i0 < len; i0 += 8192, buf ^= 1) {
+    // warp w: the 256 words from i0 + 256 w on, a word of each 32 per lane
+    const uint32_t b = i0 + 256 * w + lane;
+    uint32_t v[8], sum = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = b + 32 * k < len ? a[b + 32 * k] : 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {  // v[k]: sum of the warp's words up to and with this one
+      uint32_t x = v[k];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+      }
+      const uint32_t all = __shfl_sync(0xffffffffu, x, 31);
+      v[k] = sum + x - v[k];
+      sum += all;
+    }
+    if (lane == 0) sums[buf][w] = sum;
+    __syncthreads();
+    const uint32_t c = sums[buf][lane];
+    const uint32_t pre = total + __reduce_add_sync(0xffffffffu, lane < w ? c : 0u);
+    total += __reduce_add_sync(0xffffffffu, c);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (b + 32 * k < len) a[b + 32 * k] = pre + v[k];
+  }
+}
+
 uint32_t scan_ws_words(uint32_t len) { return (len + kTileV - 1) / kTileV; }
 
 cudaError_t exclusive_scan_u32_ws(uint32_t* data, uint32_t len, uint32_t* sums, cudaStream_t s) {
   if (len == 0) return cudaSuccess;
+  if (len <= kScanBlock) {
+    k_scan_block<<<1, 1024, 0, s>>>(data, len);
+    return cudaGetLastError();
+  }
   const uint32_t ntiles = scan_ws_words(len);
   k_scan_tile_sums<<<ntiles, 256, 0, s>>>(data, len, sums);
   k_scan_single<<<1, 1024, 0, s>>>(sums, ntiles);
@@ -992,7 +1033,7 @@ cudaError_t exclusive_scan_u32_ws(uint32_t* data, uint32_t len, uint32_t* sums, 
 }
 
 cudaError_t exclusive_scan_u32(uint32_t* data, uint32_t len, cudaStream_t s) {
-  if (len == 0) return cudaSuccess;
+  if (len <= kScanBlock) return exclusive_scan_u32_ws(data, len, nullptr, s);
   uint32_t* sums = nullptr;
   cudaError_t e = graph_alloc(&sums, sizeof(uint32_t) * scan_ws_words(len), s);
   if (e != cudaSuccess) return e;
