@@ -36,7 +36,7 @@ __global__ void k_mark_seed(SolveArgs a, const uint32_t* __restrict__ delu, cons
 }
 
 // Mark the out-neighbours of every queued source in bitmap 0, one warp per
-// source; sources with more than 1024 out-edges go to the block-wide queue.
+// source; sources with more than 256 out-edges go to k_expand_big's queue.
 __global__ void __launch_bounds__(kThreads) k_expand_seeds(SolveArgs a) {
   const uint32_t count = a.st->xcnt;
   uint32_t* b0 = a.bm[0];
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kThreads) k_expand_seeds(SolveArgs a) {
     const uint32_t u = a.xl[i];
     const uint64_t iu = seg_index(u, a.seg_shift);
     const uint32_t b = a.xoff[iu], e = a.xoff[iu + 1];
-    if (e - b > 1024) {
+    if (e - b > 256) {
       if (lane == 0) push(a.xb, &a.st->xbcnt, u);
       continue;
     }
