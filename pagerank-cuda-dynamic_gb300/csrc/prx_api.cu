@@ -604,7 +604,8 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   // contributions
   // A small or medium graph runs its FP64 loop as one cooperative kernel on
   // the plain rows (no hot copy, no source chunks); see launch_persist.
-  const bool persist = !refine && o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase &&
+  const bool persist = (!refine || (!dyn && o.max_iterations > 0 && g.mid_max >= kPlanMid)) &&
+                       o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase &&
                        g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) && persist_fits(g);
   if (persist) TRY_CUDA_ST(ensure_plan(gr->g, c->sms, c->stream));
   const bool hot_ok = o.hot_sources >= 0 && !persist;
@@ -615,7 +616,7 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   }
   const ChunkLayout *lay64 = nullptr, *lay32 = nullptr;
   if (!persist) TRY_CUDA_ST(ensure_chunks(gr->g, w64, c->sms, c->stream, &lay64, hot_ok && g.hot_n > 0));
-  if (refine) TRY_CUDA_ST(ensure_chunks(gr->g, w32, c->sms, c->stream, &lay32));
+  if (refine && !persist) TRY_CUDA_ST(ensure_chunks(gr->g, w32, c->sms, c->stream, &lay32));
   cudaStream_t s = c->stream;
   SolveArgs a = make_args(c, g, o);
   a.hot_list = g.hot_list;
@@ -652,7 +653,7 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
     // iterations of `m` until done: one CUDA graph, or host-driven batches
     auto iterate = [&](int m, const ChunkLayout* lay) -> int {
       if (persist) {
-        TRY_CUDA_ST(launch_persist(a, g, m, c->sms, s));
+        TRY_CUDA_ST(refine ? launch_persist_refine(a, g, c->sms, s) : launch_persist(a, g, m, c->sms, s));
         c->launches += 1;
         TRY_CUDA_ST(cudaMemcpyAsync(&c->st_host[1], c->st, sizeof(State), cudaMemcpyDeviceToHost, s));
         TRY_CUDA_ST(cudaStreamSynchronize(s));
@@ -697,6 +698,9 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
       if ((st = run_refine_loop(c, gr, a, timing, o.max_iterations, lay64, lay32, &final_parity, false,
                                 o.loop != PRX_LOOP_HOST)))
         return st;
+    } else if (refine && persist) {
+      if ((st = iterate(mode, nullptr))) return st;
+      final_parity = c->st_host[1].done ? 1 : 0;
     } else if (refine) {
       // Static / ND, or a dynamic mode whose marking covers most of the
       // graph: FP32 sweeps over all vertices from the initial ranks (q for

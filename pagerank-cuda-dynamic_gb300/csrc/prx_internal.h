@@ -325,6 +325,11 @@ cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s);
 // first.
 cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, cudaStream_t s);
 
+// The same for the FP32 refinement of Static and ND (prx_refine.cu's loop from
+// round 0): the answer is in parity 1 when State::done, else the committed
+// ranks in parity 0.
+cudaError_t launch_persist_refine(const SolveArgs& a, const GraphDev& g, int sms, cudaStream_t s);
+
 // ---- FP32 refinement (prx_refine.cu) --------------------------------------
 // FP64 residual sweep of one in-degree class (update kernels in MODE_REFINE64).
 bool launch_refine_sweep64(const SolveArgs& a, const GraphDev& g, int cls, const ChunkLayout* lay, int sms,

@@ -341,11 +341,294 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
   if (T::DYN) block_sum_u64(edges, &st->edges);
 }
 
-template <int MODE, int K>
-static cudaError_t persist_k(const SolveArgs& a, const PersistRows& rows, uint64_t want, int threads, int sms,
-                             cudaStream_t s) {
+// ---- FP32 refinement ------------------------------------------------------------
+// Sum of ce[edg[j]], j in [s, e), front to back: eight gathers in flight; ids
+// outside the row in its first and last groups give +0, which changes no sum
+// that started at +0.
+__device__ __forceinline__ float lane_row_sum32(const float* ce, const uint32_t* __restrict__ edg, uint32_t s,
+                                                uint32_t e) {
+  float acc = 0.f;
+  if (s >= e) return acc;
+  auto ids = [&](uint32_t j) {
+    return j < e ? __ldg(reinterpret_cast<const uint4*>(edg + j)) : make_uint4(0, 0, 0, 0);
+  };
+  uint32_t j = s & ~3u;
+  uint4 g0 = ids(j), g1 = ids(j + 4);
+  for (; j < e; j += 8) {
+    const uint32_t u[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+    float x[8];
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) x[k] = j + k >= s && j + k < e ? ce[u[k]] : 0.f;
+    g0 = ids(j + 8);
+    g1 = ids(j + 12);
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) acc += x[k];
+  }
+  return acc;
+}
+
+// The whole loop of prx_refine.cu (round 0 on the initial ranks, then FP64
+// residual sweeps and FP32 rounds) on the same units; the sums and the tests
+// that end a round are those of the launched kernels, the same bits.  Rows of
+// 1025 to mid_max ids, which a warp of the launched sweep sums alone, have their
+// terms brought in by a block.  Whole solves, launched | here, ms: R-MAT 2^10 1.62
+// | 0.40, 2^16 2.66 | 0.67, 2^18 3.67 | 1.46, 2^20 9.0 | 5.7, 2^22 27.9 | 25.1,
+// web-like 30k 0.39 | 0.12, 200k 0.56 | 0.36, 1.5M 2.00 | 1.71, grid 500^2 0.50 |
+// 0.21, 1000^2 0.57 | 0.35.  What bounds it: as k_persist, then L1 and L2 sectors
+// of the gathers.
+constexpr uint32_t kRowVals = 2048;
+
+template <int K>
+__global__ void __launch_bounds__(kThreads, 3) k_persist_refine(SolveArgs a, PersistRows rows) {
+  __shared__ double part[256];
+  __shared__ float vals[kRowVals];
+  __shared__ double s_tree[kThreads / 32][RowTree::kSlots];
+  __shared__ unsigned long long s_el;
+  __shared__ uint32_t s_dl, s_em;
+  State* st = a.st;
+  if (st->done) return;
+  const uint32_t lane = lane_id(), t = threadIdx.x;
+  const RowTree tree{s_tree[t >> 5]};
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t warp = warps - 1 - ((blockIdx.x * blockDim.x + t) >> 5);
+  const uint32_t words = (a.n + 31) >> 5;
+  const uint32_t units = rows.nmid + (rows.sorted ? (rows.nlow + 31) / 32 : words);
+  const int max_iter = st->max_iter;
+  const double tol = st->tol;
+  const float P32 = (float)a.P, tol32 = (float)tol;
+  auto load_unit = [&](uint32_t u) {
+    Unit x{};
+    if (u < rows.nmid) {
+      x.v = __ldg(rows.list + u);
+      x.row = true;
+    } else if (rows.sorted) {
+      const uint32_t i = 32 * (u - rows.nmid) + lane;
+      x.row = i < rows.nlow;
+      x.v = x.row ? __ldg(rows.low + i) : 0u;
+    } else {
+      const uint32_t w = u - rows.nmid;
+      x.v = (w << 5) | lane;
+      x.row = x.v < a.n && ((__ldg(a.low_bm + w) >> lane) & 1u);
+    }
+    if (x.row) {
+      x.s = __ldg(a.xtoff + x.v);
+      x.e = __ldg(a.xtoff + x.v + 1);
+      x.d = __ldg(a.xtdat + x.v);
+    }
+    return x;
+  };
+  const uint32_t low0 = warp < rows.nmid ? warp + (rows.nmid - warp + warps - 1) / warps * warps : warp;
+  Unit coming{};  // as in k_persist
+  if (warp < units) coming = load_unit(warp);
+  auto take = [&](uint32_t u) {
+    const Unit x = coming;
+    if (units > warps) coming = load_unit(u + warps < units ? u + warps : warp);
+    return x;
+  };
+  GridBarrier bar(st);
+  int slot = 0;  // of the sweep's maxima
+  auto next_slot = [&] {  // cleared a sweep ahead (last read two barriers ago)
+    if (blockIdx.x == 0 && t == 0) {
+      const int z = (slot + 1) % 3;
+      st->pel[z] = 0;
+      st->pnf[z] = st->pmarked[z] = 0;
+    }
+  };
+
+  // FP64 residual sweep of the base ranks
+  auto sweep64 = [&]() -> bool {
+    const double* c = a.c[0];
+    unsigned long long emax = 0;
+    unsigned int mag = 0;
+    auto finish_one = [&](uint32_t v, double x, const VertexIn& in) {
+      bool survive, changed;
+      const unsigned long long ev = finish_vertex<MODE_REFINE64>(a, v, x, 0, survive, changed, mag, in);
+      emax = ev > emax ? ev : emax;
+    };
+    for (uint32_t i = blockIdx.x; i < rows.nlong; i += gridDim.x) {
+      const uint32_t v = __ldg(rows.list + rows.nmid + i);
+      const uint32_t s = __ldg(a.xtoff + v), d = __ldg(a.xtoff + v + 1) - s;
+      const VertexIn in{__ldg(a.xtdat + v), 0ull, a.r[0][v]};
+      const double x = high_row_sum<double, true, true>(c, a.xtedg + s, d, t, part);
+      if (t == 0) finish_one(v, x, in);
+    }
+    uint32_t qv = 0, held = 0;
+    VertexIn qin{};
+    auto flush = [&] {
+      double z = tree.fold<true>(held);
+      z = __shfl_sync(0xffffffffu, z, (lane & 3u) * 8);
+      if (lane < held) finish_one(qv, z, qin);
+      held = 0;
+    };
+    for (uint32_t u = warp; u < rows.nmid; u += warps) {
+      const Unit x = take(u);
+      const VertexIn in{x.d, 0ull, a.r[0][x.v]};
+      if (lane == held) {
+        qv = x.v;
+        qin = in;
+      }
+      bool bad = false;
+      const double sum = mid_lane_sums<double, true, true, true>(c, a.xtedg + x.s, x.e - x.s, lane, bad);
+      if (__any_sync(0xffffffffu, bad)) {
+        const double y = mid_row_sum_plain<true>(c, a.xtedg + x.s, x.e - x.s, lane);
+        if (lane == 0) finish_one(x.v, y, in);
+        continue;
+      }
+      tree.put(held++, sum);
+      if (held == RowTree::kRows) flush();
+    }
+    if (held) flush();
+    for (uint32_t u = low0; u < units; u += warps) {
+      const Unit x = take(u);
+      VertexIn in{x.d, 0ull, 0.0};
+      if (x.row) in.r = a.r[0][x.v];
+      const double sum = warp_row_sums<true, true, 1, K>(c, a.xtedg, x.s, x.e, 0.0, nullptr, false);
+      if (x.row) finish_one(x.v, sum, in);
+    }
+    block_max_bits(emax, &st->pel[slot]);
+    next_slot();
+    const bool ok = bar.sync([&] { s_el = *(volatile unsigned long long*)&st->pel[slot]; });
+    slot = (slot + 1) % 3;
+    return ok;
+  };
+
+  // FP32 sweep of the correction, parity q
+  auto sweep32 = [&](int q) -> bool {
+    const float* ce = a.ce[q];
+    unsigned int emax = 0, mag = 0;
+    auto finish_one = [&](uint32_t v, float sum, uint32_t d, float rho, float old) {
+      const float en = fmaf(P32, sum, rho);
+      a.e[q ^ 1][v] = en;
+      a.ce[q ^ 1][v] = __fdividef(en, (float)d);
+      emax = max(emax, __float_as_uint(fabsf(en - old)));
+      mag = max(mag, __float_as_uint(fabsf(en)));
+    };
+    for (uint32_t i = blockIdx.x; i < rows.nlong; i += gridDim.x) {
+      const uint32_t v = __ldg(rows.list + rows.nmid + i);
+      const uint32_t s = __ldg(a.xtoff + v), d = __ldg(a.xtoff + v + 1) - s;
+      const uint32_t* __restrict__ ed = a.xtedg + s;
+      float acc = 0.f;
+      if (d > a.mid_max) {
+#pragma unroll 8
+        for (uint32_t j = t; j < d; j += kThreads) acc += ce[__ldg(ed + j)];
+      } else {  // 32 sums, their terms brought in by the whole block
+        for (uint32_t j0 = 0; j0 < d; j0 += kRowVals) {
+#pragma unroll
+          for (uint32_t j = t; j < kRowVals; j += kThreads) vals[j] = j0 + j < d ? ce[__ldg(ed + j0 + j)] : 0.f;
+          __syncthreads();
+          if (t < 32) {
+#pragma unroll 16
+            for (uint32_t j = lane; j < kRowVals; j += 32) acc += vals[j];
+          }
+          __syncthreads();
+        }
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+      if (d > a.mid_max) {
+        if (lane == 0) vals[t >> 5] = acc;
+        __syncthreads();
+        if (t < 32) {
+          acc = t < 8 ? vals[t] : 0.f;
+#pragma unroll
+          for (int o = 4; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+        }
+        __syncthreads();
+      }
+      if (t == 0) finish_one(v, acc, __ldg(a.xtdat + v), a.rho[v], a.e[q][v]);
+    }
+    for (uint32_t u = warp; u < rows.nmid; u += warps) {
+      const Unit x = take(u);
+      const float rho = a.rho[x.v], old = a.e[q][x.v];
+      const uint32_t* __restrict__ ed = a.xtedg + x.s;
+      const uint32_t d = x.e - x.s;
+      float acc = 0.f;
+      for (uint32_t j0 = 0; j0 < d; j0 += 256) {
+        float y[8];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+          const uint32_t j = j0 + 32 * k + lane;
+          y[k] = j < d ? ce[__ldg(ed + j)] : 0.f;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) acc += y[k];
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+      if (lane == 0) finish_one(x.v, acc, x.d, rho, old);
+    }
+    for (uint32_t u = low0; u < units; u += warps) {
+      const Unit x = take(u);
+      if (!x.row) continue;
+      const float rho = a.rho[x.v], old = a.e[q][x.v];
+      finish_one(x.v, lane_row_sum32(ce, a.xtedg, x.s, x.e), x.d, rho, old);
+    }
+    block_max_u32(emax, &st->pnf[slot]);
+    block_max_u32(mag, &st->pmarked[slot]);
+    next_slot();
+    const bool ok = bar.sync([&] {
+      s_dl = *(volatile uint32_t*)&st->pnf[slot];
+      s_em = *(volatile uint32_t*)&st->pmarked[slot];
+    });
+    slot = (slot + 1) % 3;
+    return ok;
+  };
+
+  const uint32_t v0 = blockIdx.x * blockDim.x + t, stride = gridDim.x * blockDim.x;
+  const float c0 = (float)a.C0;
+  for (uint32_t v = v0; v < a.n; v += stride) {  // round 0: x_b = 0, rho = C0, e_0 = the initial ranks
+    const float x = (float)a.r[0][v];
+    a.r[0][v] = 0.0;
+    a.rho[v] = c0;
+    a.e[0][v] = x;
+    a.ce[0][v] = __fdividef(x, (float)__ldg(a.xtdat + v));
+  }
+  if (!bar.sync([] {})) return;
+  int iter = 0, rounds = 0;
+  double el = 0.0;
+  bool done = false;
+  for (;;) {
+    float prev = 0.f, prev2 = 0.f;
+    int k32 = 0;
+    for (bool more = true; more;) {
+      if (!sweep32(k32 & 1)) return;
+      const float dl = __uint_as_float(s_dl), em = __uint_as_float(s_em);
+      ++iter;
+      ++k32;
+      more = !(dl < tol32 || dl < em * 0x1p-18f || iter >= max_iter || fp32_round_done(dl, prev, prev2, tol));
+      prev2 = prev;
+      prev = dl;
+    }
+    const float* e = a.e[k32 & 1];
+    for (uint32_t v = v0; v < a.n; v += stride) {  // x_b += e
+      const double x = a.r[0][v] + (double)e[v];
+      a.r[0][v] = x;
+      a.c[0][v] = div_count(x, __ldg(a.xtdat + v), __ldg(a.rcp + v));
+    }
+    if (iter >= max_iter) break;
+    if (!bar.sync([] {}) || !sweep64()) return;
+    el = __longlong_as_double((long long)s_el);
+    ++iter;
+    ++rounds;
+    if (el < tol || iter >= max_iter) {
+      done = true;
+      break;
+    }
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    st->iter = iter;
+    st->rounds = rounds;
+    st->last_delta = el;
+    st->done = done;
+  }
+}
+
+// Cooperative launch of `want` blocks, or as many as are resident.
+template <class... A>
+static cudaError_t launch_resident(void (*kernel)(A...), uint64_t want, int threads, int sms, cudaStream_t s,
+                                   A... args) {
   int per_sm = 0;  // resident blocks per SM of this build
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist<MODE, K>, threads, 0);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)std::min<uint64_t>(want, (uint64_t)per_sm * sms));
@@ -356,9 +639,14 @@ static cudaError_t persist_k(const SolveArgs& a, const PersistRows& rows, uint64
   at.val.cooperative = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_persist<MODE, K>, a, rows);
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+template <int MODE, int K>
+static cudaError_t persist_k(const SolveArgs& a, const PersistRows& rows, uint64_t want, int threads, int sms,
+                             cudaStream_t s) {
+  return launch_resident(k_persist<MODE, K>, want, threads, sms, s, a, rows);
+}
 template <int MODE>
 static cudaError_t persist_t(const SolveArgs& a, const PersistRows& rows, int sms, cudaStream_t s) {
   // a warp per unit and a block per long row; no more blocks than are resident
@@ -375,10 +663,20 @@ static cudaError_t persist_t(const SolveArgs& a, const PersistRows& rows, int sm
                                           : persist_k<MODE, 0>(a, rows, want, threads, sms, s);
 }
 
+static PersistRows persist_rows(const GraphDev& g) {
+  return {g.len_list, g.plan_list + g.plan_begin[MID], g.plan_begin[MID], g.plan_begin[HIGH] - g.plan_begin[MID],
+          g.plan_begin[NCLS] - g.plan_begin[HIGH], mixed_lengths(g)};
+}
+
+cudaError_t launch_persist_refine(const SolveArgs& a, const GraphDev& g, int sms, cudaStream_t s) {
+  const PersistRows rows = persist_rows(g);
+  const uint64_t units = (uint64_t)rows.nmid + ((uint64_t)(rows.sorted ? rows.nlow : a.n) + 31) / 32;
+  const uint64_t want = std::max<uint64_t>(1, rows.nlong + (units + kThreads / 32 - 1) / (kThreads / 32));
+  return launch_resident(k_persist_refine<2>, want, kThreads, sms, s, a, rows);
+}
+
 cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, cudaStream_t s) {
-  const PersistRows rows = {g.len_list, g.plan_list + g.plan_begin[MID], g.plan_begin[MID],
-                            g.plan_begin[HIGH] - g.plan_begin[MID],
-                            g.plan_begin[NCLS] - g.plan_begin[HIGH], mixed_lengths(g)};
+  const PersistRows rows = persist_rows(g);
   switch (mode) {
     case PRX_DYNAMIC_TRAVERSAL: return persist_t<PRX_DYNAMIC_TRAVERSAL>(a, rows, sms, s);
     case PRX_DYNAMIC_FRONTIER: return persist_t<PRX_DYNAMIC_FRONTIER>(a, rows, sms, s);
