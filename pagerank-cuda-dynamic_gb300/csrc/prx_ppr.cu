@@ -136,7 +136,7 @@ struct PprArgs {
   uint32_t batch;                 // vertices of a unit, whose bounds a warp loads at once (at most 32)
   int cols;                       // C: columns stored per vertex
   bool share;                     // a fixed share of the units per warp
-  bool flat;                      // 64 FP32 columns: the short rows by k_ppr_flat
+  bool flat;                      // 64 columns: the short rows by k_ppr_flat
   double P, Q;                    // damping, 1 - damping
   float P32;                      // (float)P: a conversion in the kernel runs on the FP64 pipe
 };
@@ -463,31 +463,39 @@ __global__ void __launch_bounds__(256, PprShape<MODE, C>::BLOCKS) k_ppr_rows(Ppr
   ppr_reduce<MODE>(st, dmax, emag);
 }
 
-// The short rows of a 64-column FP32 sweep, a warp per vertex in id order, two
-// columns per lane: 32 registers, so 64 warps an SM, and 4-byte ids (their
-// reciprocals hit the L1), which web-like graphs -- rows of one length, bound
-// by the L1 and the way to it -- need more than the side-by-side rows: 174
-// against 192 us a sweep on 200k vertices.  The same sums.
+// The short rows of a 64-column sweep, a warp per vertex in id order, two
+// columns per lane: 32 registers (FP32), so 64 warps an SM, and 4-byte ids
+// (their reciprocals hit the L1), which web-like graphs -- rows of one length,
+// bound by the L1 and the way to it, or by the FP64 pipe with nothing to gain
+// from a better order -- need more than the side-by-side rows: FP32 174 against
+// 192 us a sweep on 200k vertices, FP64 the
+// 32 registers matter too: 60 vectors on 93k vertices 11.42 against 11.48 ms.  The same sums.
+template <int MODE>
 __global__ void __launch_bounds__(256) k_ppr_flat(PprArgs a) {
+  using S = typename PprType<MODE>::S;
+  using V2 = typename std::conditional<MODE == PPR_S32, float2, double2>::type;
   State* st = a.st;
-  if (ppr_skip<PPR_S32>(st)) return;
-  const int q = st->k32 & 1;
-  const float2* __restrict__ src = reinterpret_cast<const float2*>(a.e[q]);
-  const float* __restrict__ rc = a.rcp32;
+  if (ppr_skip<MODE>(st)) return;
+  const V2* __restrict__ src = reinterpret_cast<const V2*>(ppr_src<MODE>(a, st));
+  const S* __restrict__ rc;
+  if constexpr (MODE == PPR_S32) rc = a.rcp32;
+  else rc = a.rcp;
   const uint32_t lane = lane_id(), warps = (gridDim.x * blockDim.x) >> 5;
-  unsigned int dmax = 0, emag = 0;
+  unsigned long long dmax = 0;
+  unsigned int emag = 0;
   for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < a.n; v += warps) {
     const uint64_t iv = seg_index(v, a.seg_shift);
     const uint32_t s = __ldg(a.xtoff + iv), e = __ldg(a.xtoff + iv + 1);
     if (e - s > a.low_max) continue;
     const uint32_t* __restrict__ edg = seg_edges(a.xtedg, a.xtbase, a.seg_shift, v);
-    float2 acc = make_float2(0.f, 0.f);
+    V2 acc;
+    acc.x = acc.y = S(0);
     uint32_t j = s;
     for (; j + 4 <= e; j += 4) {
       const uint32_t u0 = __ldg(edg + j), u1 = __ldg(edg + j + 1), u2 = __ldg(edg + j + 2), u3 = __ldg(edg + j + 3);
-      const float2 g0 = __ldg(src + (size_t)u0 * 32 + lane), g1 = __ldg(src + (size_t)u1 * 32 + lane);
-      const float2 g2 = __ldg(src + (size_t)u2 * 32 + lane), g3 = __ldg(src + (size_t)u3 * 32 + lane);
-      const float y0 = __ldg(rc + u0), y1 = __ldg(rc + u1), y2 = __ldg(rc + u2), y3 = __ldg(rc + u3);
+      const V2 g0 = __ldg(src + (size_t)u0 * 32 + lane), g1 = __ldg(src + (size_t)u1 * 32 + lane);
+      const V2 g2 = __ldg(src + (size_t)u2 * 32 + lane), g3 = __ldg(src + (size_t)u3 * 32 + lane);
+      const S y0 = __ldg(rc + u0), y1 = __ldg(rc + u1), y2 = __ldg(rc + u2), y3 = __ldg(rc + u3);
       acc.x = fma(g0.x, y0, acc.x); acc.y = fma(g0.y, y0, acc.y);
       acc.x = fma(g1.x, y1, acc.x); acc.y = fma(g1.y, y1, acc.y);
       acc.x = fma(g2.x, y2, acc.x); acc.y = fma(g2.y, y2, acc.y);
@@ -495,20 +503,46 @@ __global__ void __launch_bounds__(256) k_ppr_flat(PprArgs a) {
     }
     for (; j < e; ++j) {
       const uint32_t u = __ldg(edg + j);
-      const float2 g = __ldg(src + (size_t)u * 32 + lane);
-      const float y = __ldg(rc + u);
+      const V2 g = __ldg(src + (size_t)u * 32 + lane);
+      const S y = __ldg(rc + u);
       acc.x = fma(g.x, y, acc.x);
       acc.y = fma(g.y, y, acc.y);
     }
-    const size_t at = (size_t)v * 32 + lane;
-    const float2 r = reinterpret_cast<const float2*>(a.rho)[at], old = src[at];
-    const float P = a.P32;
-    const float2 en = make_float2(fmaf(P, acc.x, r.x), fmaf(P, acc.y, r.y));
-    reinterpret_cast<float2*>(a.e[q ^ 1])[at] = en;
-    emag = max(emag, __float_as_uint(fmaxf(fabsf(en.x), fabsf(en.y))));
-    dmax = max(dmax, __float_as_uint(fmaxf(fabsf(en.x - old.x), fabsf(en.y - old.y))));
+    if constexpr (MODE == PPR_S32) {
+      const int q = st->k32 & 1;
+      const size_t at = (size_t)v * 32 + lane;
+      const float2 r = reinterpret_cast<const float2*>(a.rho)[at], old = src[at];
+      const float P = a.P32;
+      const float2 en = make_float2(fmaf(P, acc.x, r.x), fmaf(P, acc.y, r.y));
+      reinterpret_cast<float2*>(a.e[q ^ 1])[at] = en;
+      emag = max(emag, __float_as_uint(fmaxf(fabsf(en.x), fabsf(en.y))));
+      dmax = max(dmax, (unsigned long long)__float_as_uint(fmaxf(fabsf(en.x - old.x), fabsf(en.y - old.y))));
+    } else {
+      // ppr_finish for two columns, in the 32 registers that the sum has
+      const size_t at = (size_t)v * 32 + lane;
+      double tx = 0.0, ty = 0.0;
+      for (uint32_t i = __ldg(a.toff + v), ie = __ldg(a.toff + v + 1); i < ie; ++i) {
+        const uint32_t col = __ldg(a.tcol + i);
+        if ((col >> 1) == lane) {
+          if (col & 1u) ty += __ldg(a.tmass + i);
+          else tx += __ldg(a.tmass + i);
+        }
+      }
+      const double2 an = make_double2(fma(a.P, acc.x, a.Q * tx), fma(a.P, acc.y, a.Q * ty));
+      const int p = MODE == PPR_J64 ? (st->iter & 1) : 0;
+      const double2 old = reinterpret_cast<const double2*>(a.x[p])[at];
+      reinterpret_cast<double2*>(a.x[p ^ 1])[at] = an;
+      const double dx = an.x - old.x, dy = an.y - old.y;
+      if (MODE == PPR_R64) {
+        const float2 r = make_float2((float)dx, (float)dy);
+        reinterpret_cast<float2*>(a.rho)[at] = r;
+        reinterpret_cast<float2*>(a.e[0])[at] = r;
+      }
+      const unsigned long long d = dbits(fmax(fabs(dx), fabs(dy)));
+      dmax = d > dmax ? d : dmax;
+    }
   }
-  ppr_reduce<PPR_S32>(st, dmax, emag);
+  ppr_reduce<MODE>(st, dmax, emag);
 }
 
 // Long rows: a row's lanes per vertex add its segments in order, a segment
@@ -720,8 +754,8 @@ static void ppr_sweep_c(const PprArgs& a, int sms, cudaStream_t s, uint64_t& lau
   while (b.batch > G && (uint64_t)a.nrows / b.batch < 2ull * 32 * sms) b.batch /= 2;
   // few units in all: no counter (R-MAT 2^16, 5 vectors: 41 us a sweep, 52 with it)
   b.share = (uint64_t)a.nrows / b.batch + a.nparts / G < 2ull * 32 * sms;
-  if (MODE == PPR_S32 && C == 64 && a.flat) {
-    k_ppr_flat<<<grid_for((uint64_t)a.n * 32, 256, sms * 8), 256, 0, s>>>(a);
+  if (C == 64 && a.flat) {
+    k_ppr_flat<MODE><<<grid_for((uint64_t)a.n * 32, 256, sms * 8), 256, 0, s>>>(a);
     ++launches;
     b.nrows = 0;  // the long rows are left
   }
@@ -1095,10 +1129,6 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   if (st) return st;
   PprWs& w = *c->ppr;
   cudaStream_t s = c->stream;
-  const uint64_t slots = g.nseg > 1 ? g.xtpos.back() + (g.m - g.xtseg0.back()) : g.m;
-  TRY_CUDA_ST(grow(&w.pair, w.pair_cap, slots));
-  k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, w.pair);
-  c->launches += 1;
   PprArgs a{};
   a.xtoff = g.xtoff;
   a.xtbase = g.xtbase;
@@ -1106,7 +1136,6 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   a.rcp = g.rcp;
   a.rcp32 = g.rcp32;
   a.xtedg = g.xtedg;
-  a.pair = w.pair;
   a.x[0] = w.x[0];
   a.x[1] = w.x[1];
   a.rho = w.rho;
@@ -1130,6 +1159,13 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   a.rows = by_length ? g.len_list : nullptr;
   a.nrows = by_length ? g.cls_begin[MID] : g.n;
   a.flat = !mixed_lengths(g);
+  if (!a.flat || a.nparts || (nvec % kCols && nvec % kCols <= 48)) {  // not k_ppr_flat alone
+    const uint64_t slots = g.nseg > 1 ? g.xtpos.back() + (g.m - g.xtseg0.back()) : g.m;
+    TRY_CUDA_ST(grow(&w.pair, w.pair_cap, slots));
+    k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, w.pair);
+    c->launches += 1;
+    a.pair = w.pair;
+  }
   double* out = ranks_out;
   const size_t total = (size_t)g.n * nvec;
   if (!device_out) {
