@@ -276,6 +276,9 @@ int run_marking(prx_context* c, const SolveArgs& a, int mode, const uint32_t* du
     c->launches += 1;
     bool pull = a.pull_threshold == 0;
     if (!pull) {
+      // the warps start from the marked vertices, the queue after them
+      TRY_CUDA_ST(cudaMemcpyAsync(&c->st->fcnt[1], &c->st->fcnt[0], sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+      TRY_CUDA_ST(cudaMemcpyAsync(&c->st->q_head, &c->st->fcnt[0], sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
       launch_closure_queue(a, a.pull_threshold, c->sms, s);
       c->launches += 1;
       TRY_CUDA_ST(cudaMemcpyAsync(&c->st_host[1], c->st, sizeof(State), cudaMemcpyDeviceToHost, s));

@@ -73,22 +73,34 @@ __global__ void __launch_bounds__(kThreads) k_frontier_from_bitmap(SolveArgs a) 
 //   queue: frontier 0; its length is fcnt[0] (the tail), q_head counts items
 //   taken, q_done items finished.  A slot is all ones until its producer has
 //   written it (a consumer may take a slot the moment the tail covers it).
-// A warp takes up to 32 items, one per lane.  A lane marks the out-neighbours
-// of a vertex of out-degree <= 32 itself and goes on from one of the newly
-// marked ones (up to kChain steps), so a long path -- the diameter of a road
-// or grid graph -- is walked at one thread's memory latency per step rather
-// than one queue round trip or one kernel launch per level.  The other new
-// vertices wait in shared memory and reach the queue with one atomic per
-// warp; vertices of larger out-degree are expanded by the whole warp.  Tail
-// increments precede the warp's q_done increment (fence), so a warp that
-// reads q_done and then the tail and finds them equal knows nothing is in
-// flight: the closure is done.  Idle warps back off exponentially; every
-// wait is bounded, and running out sets kErrClosureWait and returns.
+//   The vertices it starts with (fcnt[1] of them, q_head is past them) are
+//   claimed in shares by fcnt[2], so that all warps start at once.
+// A warp runs its items, one per lane, for up to kChain steps.  A lane marks
+// the out-neighbours of a vertex of out-degree <= 32 itself and goes on from
+// one of the newly marked ones, so a long path -- the diameter of a road or
+// grid graph -- is walked at one thread's memory latency per step rather than
+// one queue round trip or one kernel launch per level.  The other new vertices
+// wait in shared memory for a lane that has none, and go to the queue, with one
+// atomic per warp, when there are kShare of them (other warps may have nothing
+// to do) or the steps are used up; vertices of larger out-degree are expanded
+// by the whole warp.  Tail increments precede the warp's q_done increment
+// (fence), so a warp that reads q_done and then the tail and finds them equal
+// knows nothing is in flight: the closure is done.  Idle warps back off
+// exponentially; every wait is bounded, and running out sets kErrClosureWait
+// and returns.
+// What bounds it: the latency of a step (offsets, edges, bitmap atomics: 1 us)
+// times the steps that follow one another.  Marking, ms, before (edges one after
+// the other, new vertices to the queue only at the end of a chain, 32 starting
+// vertices a warp) and now: grid 1000^2 from 512 edges 1.61 and 0.48, from 4 26.7
+// and 2.3, grid 2000^2 from 4000 2.02 and 1.09, grid 300^2 from 20 1.70 and 0.30,
+// a path of 200k 196 and 198.  More warps than four an SM queue up for the head:
+// two blocks 2.3 -> 3.9 from 4 edges, four 0.48 -> 4.7 from 512.
 constexpr uint32_t kQueueEmpty = 0xffffffffu;
 constexpr int kClosureSpin = 1 << 20;
 constexpr int kChain = 64;
 constexpr int kQWarps = 4;           // warps per block of the queue kernel
-constexpr uint32_t kQBuf = 2048;     // buffered new vertices per warp (32 KB of shared memory a block)
+constexpr uint32_t kShare = 64;      // buffered new vertices that go to the queue for other warps
+constexpr uint32_t kQBuf = kShare + 32 * 32;  // ... and one more step of every lane (17 KB a block)
 
 __global__ void __launch_bounds__(kQWarps * 32) k_closure_queue(SolveArgs a, uint32_t switch_at) {
   __shared__ uint32_t buf[kQWarps][kQBuf];
@@ -115,6 +127,85 @@ __global__ void __launch_bounds__(kQWarps * 32) k_closure_queue(SolveArgs a, uin
   };
   if (lane == 0) nbuf[w] = 0;
   __syncwarp();
+  // the closure from the lanes' vertices u (none: kQueueEmpty), cnt of them
+  // queue items; what is left after kChain steps goes back to the queue
+  auto run = [&](uint32_t u, uint32_t cnt) {
+    for (int step = 0; step < kChain; ++step) {
+      const unsigned idle = __ballot_sync(0xffffffffu, u == kQueueEmpty);
+      const uint32_t have = nbuf[w];
+      if (idle == 0xffffffffu && !have) break;
+      __syncwarp();
+      if (u == kQueueEmpty) {  // an idle lane takes a buffered vertex
+        const uint32_t k = __popc(idle & ((1u << lane) - 1u));
+        if (k < have) u = buf[w][have - 1 - k];
+      }
+      if (lane == 0 && idle) nbuf[w] = have - min(have, (uint32_t)__popc(idle));
+      __syncwarp();
+      const bool valid = u != kQueueEmpty;
+      uint32_t b = 0, e = 0;
+      if (valid) {
+        const uint64_t iu = seg_index(u, a.seg_shift);
+        b = a.xoff[iu];
+        e = a.xoff[iu + 1];
+      }
+      const bool small = e - b <= 32u;
+      uint32_t next = kQueueEmpty;
+      if (valid && small) {
+        const uint32_t* ed = seg_edges(a.xedg, a.xbase, a.seg_shift, u);
+        const bool look = e - b > 8;  // longer rows (of graphs with hubs) look before they set
+        for (uint32_t j = b; j < e; j += 8) {  // eight edges' loads and atomics in flight
+          uint32_t x[8], was[8];
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) x[k] = ed[min(j + k, e - 1)];
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) was[k] = j + k < e ? (look ? reached[x[k] >> 5] : 0u) : 0xffffffffu;
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) {
+            const uint32_t bit = 1u << (x[k] & 31u);
+            if (!(was[k] & bit)) was[k] = atomicOr(&reached[x[k] >> 5], bit);
+          }
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k) {
+            if ((was[k] >> (x[k] & 31u)) & 1u) continue;
+            if (next == kQueueEmpty) next = x[k];  // this lane goes on from it
+            else buf[w][atomicAdd(&nbuf[w], 1u)] = x[k];
+          }
+        }
+      }
+      unsigned big = __ballot_sync(0xffffffffu, valid && !small);
+      while (big) {
+        const int src = __ffs(big) - 1;
+        big &= big - 1;
+        const uint32_t ub = __shfl_sync(0xffffffffu, u, src);
+        const uint32_t bb = __shfl_sync(0xffffffffu, b, src), eb = __shfl_sync(0xffffffffu, e, src);
+        const uint32_t* ed = seg_edges(a.xedg, a.xbase, a.seg_shift, ub);
+        for (uint32_t j = bb + lane; j < eb; j += 32) {
+          const uint32_t x = ed[j];
+          if (test_and_set(reached, x)) push(queue, &st->fcnt[0], x);
+        }
+      }
+      u = next;
+      __syncwarp();
+      if (nbuf[w] >= kShare) flush();
+    }
+    if (u != kQueueEmpty) buf[w][atomicAdd(&nbuf[w], 1u)] = u;  // chain cut: back to the queue
+    flush();
+    __threadfence();  // this warp's tail increments and slots before its q_done increment
+    __syncwarp();
+    if (lane == 0) atomicAdd(&st->q_done, cnt);
+  };
+  // the vertices the queue starts with, in shares that reach all warps (claimed,
+  // not assigned: no warp waits for one that has not started)
+  const uint32_t first = st->fcnt[1], warps = gridDim.x * kQWarps;
+  const uint32_t share = min(32u, (first + warps - 1) / warps);
+  while (first <= switch_at) {
+    uint32_t i = 0;
+    if (lane == 0) i = atomicAdd(&st->fcnt[2], share);
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if (i >= first) break;
+    const uint32_t cnt = min(share, first - i);
+    run(lane < cnt ? queue[i + lane] : kQueueEmpty, cnt);
+  }
   for (;;) {
     uint32_t h = 0, cnt = 0;
     if (lane == 0) {
@@ -157,48 +248,8 @@ __global__ void __launch_bounds__(kQWarps * 32) k_closure_queue(SolveArgs a, uin
         __nanosleep(64);
       }
     }
-    for (int step = 0; step < kChain; ++step) {
-      const bool valid = u != kQueueEmpty;
-      if (!__any_sync(0xffffffffu, valid)) break;
-      uint32_t b = 0, e = 0;
-      if (valid) {
-        const uint64_t iu = seg_index(u, a.seg_shift);
-        b = a.xoff[iu];
-        e = a.xoff[iu + 1];
-      }
-      const bool small = e - b <= 32u;
-      uint32_t next = kQueueEmpty;
-      if (valid && small) {
-        const uint32_t* ed = seg_edges(a.xedg, a.xbase, a.seg_shift, u);
-        for (uint32_t j = b; j < e; ++j) {
-          const uint32_t x = ed[j];
-          if (test_and_set(reached, x)) {
-            if (next == kQueueEmpty) next = x;  // this lane goes on from x
-            else buf[w][atomicAdd(&nbuf[w], 1u)] = x;
-          }
-        }
-      }
-      unsigned big = __ballot_sync(0xffffffffu, valid && !small);
-      while (big) {
-        const int src = __ffs(big) - 1;
-        big &= big - 1;
-        const uint32_t ub = __shfl_sync(0xffffffffu, u, src);
-        const uint32_t bb = __shfl_sync(0xffffffffu, b, src), eb = __shfl_sync(0xffffffffu, e, src);
-        const uint32_t* ed = seg_edges(a.xedg, a.xbase, a.seg_shift, ub);
-        for (uint32_t j = bb + lane; j < eb; j += 32) {
-          const uint32_t x = ed[j];
-          if (test_and_set(reached, x)) push(queue, &st->fcnt[0], x);
-        }
-      }
-      u = next;
-      __syncwarp();
-      if (nbuf[w] > kQBuf - 32u * 32u) flush();  // room for one more step of every lane
-    }
-    if (u != kQueueEmpty) buf[w][atomicAdd(&nbuf[w], 1u)] = u;  // chain cut: back to the queue
-    flush();
-    __threadfence();  // this warp's tail increments and slots before its q_done increment
     __syncwarp();
-    if (lane == 0) atomicAdd(&st->q_done, cnt);
+    run(u, cnt);
   }
 }
 
@@ -318,7 +369,7 @@ void launch_frontier_from_bitmap(const SolveArgs& a, int sms, cudaStream_t s) {
 }
 
 void launch_closure_queue(const SolveArgs& a, uint32_t switch_at, int sms, cudaStream_t s) {
-  k_closure_queue<<<sms * 2, kQWarps * 32, 0, s>>>(a, switch_at);
+  k_closure_queue<<<sms, kQWarps * 32, 0, s>>>(a, switch_at);
 }
 
 void launch_closure_pull(const SolveArgs& a, uint32_t round, int sms, cudaStream_t s) {
