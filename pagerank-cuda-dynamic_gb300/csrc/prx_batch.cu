@@ -588,13 +588,15 @@ cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd64, ui
   // the cached LOW layouts follow the new version (plain graphs; the hot
   // numbering is kept with them)
   if (!segmented) {
-    const uint64_t low_edges = g.cls_edges[LOW];
+    // room for the new LOW edges: the insertions, and the rest of every row that
+    // a deletion brings down to the LOW bound
+    const uint64_t low_edges = std::min<uint64_t>(m2, g.cls_edges[LOW] + ni + (uint64_t)kLowMax * nd);
     for (auto& l : g.lay) {
       if (!l.width || !l.off || !l.seg_off.empty()) continue;
       const size_t len = (size_t)l.K * ((size_t)n + 1);
       uint32_t *lo = nullptr, *le = nullptr, *ws = nullptr;
       cudaError_t el = graph_alloc(&lo, sizeof(uint32_t) * len, s);
-      if (el == cudaSuccess) el = graph_alloc(&le, sizeof(uint32_t) * edge_slots(low_edges + ni), s);
+      if (el == cudaSuccess) el = graph_alloc(&le, sizeof(uint32_t) * edge_slots(low_edges), s);
       if (el == cudaSuccess) el = graph_alloc(&ws, sizeof(uint32_t) * scan_ws_words((uint32_t)len), s);
       if (el == cudaSuccess)
         el = carry_layout(l, ntoff, ntedg, n, tin, in_list, in_T, nullptr, g.hot_idx, lo, le, ws, sms, s);
