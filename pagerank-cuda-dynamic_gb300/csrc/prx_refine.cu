@@ -23,6 +23,7 @@
 
 namespace prx {
 
+constexpr int kWideBlocks = 5;  // resident blocks an SM of the wide LOW sweep, see wide_rows
 __device__ __forceinline__ unsigned int fbits(float x) { return __float_as_uint(x); }
 
 // New correction of v; returns |change| and raises *mag to |e| (bits).
@@ -42,10 +43,30 @@ __device__ __forceinline__ void reduce32(State* st, unsigned int dl, unsigned in
   block_max_u32(mag, &st->e32max_bits[q]);
 }
 
+// lane_row_sum with eight terms a step: both halves of a 32-byte sector of ids
+// are read together and eight gathers are in flight.  Ids outside the row give
+// +0, which changes no sum that started at +0.
+__device__ __forceinline__ float lane_row_sum8(const float* __restrict__ ce, const uint32_t* __restrict__ edg,
+                                               uint32_t s, uint32_t e, float acc) {
+  for (uint32_t j = s & ~7u; j < e; j += 8) {
+    const uint4 z = make_uint4(0, 0, 0, 0);
+    const uint4 u = j + 3 >= s ? __ldg(reinterpret_cast<const uint4*>(edg + j)) : z;
+    const uint4 w = j + 4 < e ? __ldg(reinterpret_cast<const uint4*>(edg + j + 4)) : z;
+    const uint32_t id[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+    float x[8];
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) x[k] = j + k >= s && j + k < e ? __ldg(ce + id[k]) : 0.f;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) acc += x[k];
+  }
+  return acc;
+}
+
 // LOW: one warp per 32 consecutive ids, one lane per vertex, one launch per
-// source chunk (partial sums carried in acc32), as the FP64 kernel.
-template <bool FIRST, bool LAST>
-__global__ void __launch_bounds__(kThreads) k32_low(SolveArgs a, uint32_t vb, uint32_t ve,
+// source chunk (partial sums carried in acc32), as the FP64 kernel.  WIDE: by
+// lane_row_sum8, see wide_rows.
+template <bool FIRST, bool LAST, bool WIDE>
+__global__ void __launch_bounds__(kThreads, WIDE ? kWideBlocks : 8) k32_low(SolveArgs a, uint32_t vb, uint32_t ve,
                                                     const unsigned long long* __restrict__ base,
                                                     uint32_t shift, const uint32_t* __restrict__ off,
                                                     const uint32_t* __restrict__ edg) {
@@ -63,7 +84,9 @@ __global__ void __launch_bounds__(kThreads) k32_low(SolveArgs a, uint32_t vb, ui
     const uint64_t iv = seg_index(v, shift) - vb;
     const uint32_t s = off[iv], e = off[iv + 1];
     if (!FIRST && !LAST && s == e) continue;
-    const float acc = lane_row_sum(ce, seg_edges(edg, base, shift, v), s, e, FIRST ? 0.f : a.acc32[v]);
+    const uint32_t* __restrict__ ed = seg_edges(edg, base, shift, v);
+    const float from = FIRST ? 0.f : a.acc32[v];
+    const float acc = WIDE ? lane_row_sum8(ce, ed, s, e, from) : lane_row_sum(ce, ed, s, e, from);
     if (LAST) emax = max(emax, finish32(a, v, acc, q, &mag));
     else a.acc32[v] = acc;
   }
@@ -195,17 +218,37 @@ __global__ void k_refine_commit(SolveArgs a) {
 
 static inline int cap_grid32(uint64_t want, int cap) { return (int)(want < (uint64_t)cap ? (want ? want : 1) : cap); }
 
+// Rows of 16 ids and more on average (in one pass) take lane_row_sum8, with five
+// blocks an SM: the L1 and the way to it bound the sweep (74% and 72% of their
+// rates), and fewer rows at a time find more of their sectors' second halves
+// there.  Whole solves, narrow | wide at 3 | 4 | 5 | 6 blocks, ms: web-like 6M
+// vertices 6.30 | 5.56 | 5.45 | 5.39 | 5.45, 12M 11.66 | 10.0 | 9.84 | 9.83 |
+// 10.1; grid 3400^2, rows of five, 2.59 | 3.07 at five.
+static bool wide_rows(const GraphDev& g, int passes) {
+  return g.cls_edges[LOW] / passes >= 16ull * (g.cls_begin[MID] - g.cls_begin[LOW]);
+}
+
+template <bool FIRST, bool LAST>
+static void sweep32_low(const SolveArgs& a, bool wide, uint32_t vb, uint32_t ve, const unsigned long long* base,
+                        uint32_t shift, const uint32_t* off, const uint32_t* edg, int sms, cudaStream_t s) {
+  const uint64_t blocks = ((uint64_t)(ve - vb) + 31) / 32 / 8 + 1;
+  if (wide)
+    k32_low<FIRST, LAST, true><<<cap_grid32(blocks, sms * kWideBlocks), kThreads, 0, s>>>(a, vb, ve, base, shift, off,
+                                                                                        edg);
+  else
+    k32_low<FIRST, LAST, false><<<cap_grid32(blocks, sms * 8), kThreads, 0, s>>>(a, vb, ve, base, shift, off, edg);
+}
+
 bool launch_sweep32(const SolveArgs& a, const GraphDev& g, int cls, const ChunkLayout* lay, int sms, cudaStream_t s) {
   const uint32_t b = g.cls_begin[cls], cnt = g.cls_begin[cls + 1] - b;
   if (!cnt) return false;
   if (cls == LOW) {
     if (!lay || lay->K <= 1) {
-      const uint64_t words = ((uint64_t)g.n + 31) / 32;
-      const int grid = cap_grid32((words + 7) / 8, sms * 8);
-      k32_low<true, true><<<grid, kThreads, 0, s>>>(a, 0, g.n, g.xtbase, g.seg_shift, g.xtoff, g.xtedg);
+      sweep32_low<true, true>(a, wide_rows(g, 1), 0, g.n, g.xtbase, g.seg_shift, g.xtoff, g.xtedg, sms, s);
       return true;
     }
     // one pass per source chunk (per row segment and chunk on segmented rows)
+    const bool wide = wide_rows(g, lay->K);
     const size_t nseg = lay->seg_off.empty() ? 1 : lay->seg_off.size();
     for (size_t q = 0; q < nseg; ++q) {
       const uint32_t v0 = nseg == 1 ? 0 : (uint32_t)(q << g.seg_shift);
@@ -213,12 +256,11 @@ bool launch_sweep32(const SolveArgs& a, const GraphDev& g, int cls, const ChunkL
       const uint32_t* offs = nseg == 1 ? lay->off : lay->seg_off[q];
       const uint32_t* edg = nseg == 1 ? lay->edg : lay->seg_edg[q];
       const size_t row = (size_t)(v1 - v0) + 1;
-      const int grid = cap_grid32(((uint64_t)(v1 - v0) + 31) / 32 / 8 + 1, sms * 8);
       for (int k = 0; k < lay->K; ++k) {
         const uint32_t* off = offs + k * row;
-        if (k == 0) k32_low<true, false><<<grid, kThreads, 0, s>>>(a, v0, v1, nullptr, 32, off, edg);
-        else if (k == lay->K - 1) k32_low<false, true><<<grid, kThreads, 0, s>>>(a, v0, v1, nullptr, 32, off, edg);
-        else k32_low<false, false><<<grid, kThreads, 0, s>>>(a, v0, v1, nullptr, 32, off, edg);
+        if (k == 0) sweep32_low<true, false>(a, wide, v0, v1, nullptr, 32, off, edg, sms, s);
+        else if (k == lay->K - 1) sweep32_low<false, true>(a, wide, v0, v1, nullptr, 32, off, edg, sms, s);
+        else sweep32_low<false, false>(a, wide, v0, v1, nullptr, 32, off, edg, sms, s);
       }
     }
   } else if (cls == MID) {
