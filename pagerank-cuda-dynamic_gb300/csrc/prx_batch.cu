@@ -115,11 +115,35 @@ struct RowMerge {
   const uint32_t* ins;   // its insertions, ascending (none in old)
   uint32_t len, nd, ni;
   uint32_t* out;         // the row's new ids
-  __device__ __forceinline__ void old_id(uint32_t j) const {
-    const uint32_t w = old[j];
-    const uint32_t p = lower_bound_u32(del, nd, w);  // deleted ids below w: all of them precede w
-    if (p < nd && del[p] == w) return;
-    out[j - p + lower_bound_u32(ins, ni, w)] = w;
+  // old ids j, j + 32, ... j + 32 (N - 1) below end, their searches side by side
+  template <int N>
+  __device__ __forceinline__ void old_ids(uint32_t j, uint32_t end) const {
+    uint32_t w[N], p[N], q[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) w[k] = j + 32 * k < end ? old[j + 32 * k] : 0u;
+    lower_bounds(del, nd, w, p);
+    lower_bounds(ins, ni, w, q);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      if (j + 32 * k >= end || (p[k] < nd && del[p[k]] == w[k])) continue;
+      out[j + 32 * k - p[k] + q[k]] = w[k];
+    }
+  }
+  template <int N>
+  __device__ static __forceinline__ void lower_bounds(const uint32_t* a, uint32_t n, const uint32_t (&x)[N],
+                                                      uint32_t (&p)[N]) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) p[k] = 0;
+    if (n == 0) return;
+    uint32_t len = n;
+    while (len > 1) {
+      const uint32_t half = len >> 1;
+#pragma unroll
+      for (int k = 0; k < N; ++k) p[k] += a[p[k] + half - 1] < x[k] ? half : 0u;
+      len -= half;
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) p[k] += a[p[k]] < x[k] ? 1u : 0u;
   }
   __device__ __forceinline__ void ins_id(uint32_t k) const {
     const uint32_t x = ins[k];
@@ -265,7 +289,7 @@ __global__ void __launch_bounds__(kThreads) k_merge_touched(Runs r, const uint32
       }
       continue;
     }
-    for (uint32_t j = lane; j < m.len; j += 32) m.old_id(j);
+    for (uint32_t j = lane; j < m.len; j += 128) m.old_ids<4>(j, m.len);
     for (uint32_t k = lane; k < m.ni; k += 32) m.ins_id(k);
   }
 }
@@ -294,7 +318,8 @@ __global__ void __launch_bounds__(kThreads) k_merge_big(Runs r, const uint32_t* 
     const RowMerge m = touched_merge(r, big[2 * lo], oedg, nedg, dv, dbeg, dend, iv, ibeg, iend);
     const uint32_t c = p - big[2 * lo + 1], po = (m.len + kPiece - 1) / kPiece;
     if (c < po) {
-      for (uint32_t j = c * kPiece + lane; j < min(m.len, (c + 1) * kPiece); j += 32) m.old_id(j);
+      static_assert(kPiece == 8 * 32, "one step");
+      m.old_ids<8>(c * kPiece + lane, min(m.len, (c + 1) * kPiece));
     } else {
       const uint32_t c2 = c - po;
       for (uint32_t k = c2 * kPiece + lane; k < min(m.ni, (c2 + 1) * kPiece); k += 32) m.ins_id(k);
@@ -336,7 +361,9 @@ __global__ void k_layout_counts(const uint32_t* __restrict__ lay_off, const uint
   }
 }
 
-// The touched rows' segments, a thread per row (at most kLowMax ids).
+// The touched rows' segments, a warp per row (at most kLowMax ids): an id's place
+// is the start of its chunk's segment and its rank among the row's ids of the
+// chunk.  A thread per row took 45 us of 11k rows of 36 ids, this 11.
 __global__ void k_layout_touched(const uint32_t* __restrict__ xtoff, const uint32_t* __restrict__ xtedg,
                                  const uint32_t* __restrict__ trow, uint32_t T, const uint32_t* Tp, uint32_t n,
                                  uint32_t width, int K, const uint32_t* __restrict__ off,
@@ -344,15 +371,15 @@ __global__ void k_layout_touched(const uint32_t* __restrict__ xtoff, const uint3
                                  uint32_t hot_words) {
   const size_t row = (size_t)n + 1;
   if (Tp) T = *Tp;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < T; i += gridDim.x * blockDim.x) {
+  const uint32_t lane = lane_id();
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < T; i += (gridDim.x * blockDim.x) >> 5) {
     const uint32_t v = trow[i];
-    uint32_t j = xtoff[v];
-    const uint32_t e = xtoff[v + 1];
-    if (e - j > kLowMax) continue;
-    for (int k = 0; k < K; ++k) {
-      const uint64_t hi = (uint64_t)(k + 1) * width;
-      uint32_t pos = off[k * row + v];
-      while (j < e && xtedg[j] < hi) edg[pos++] = layout_id(hot_idx, hot_words, xtedg[j++]);
+    const uint32_t s = xtoff[v], len = xtoff[v + 1] - s;
+    if (len > kLowMax) continue;
+    for (uint32_t j = lane; j < len; j += 32) {
+      const uint32_t u = xtedg[s + j], k = K == 1 ? 0u : u / width;
+      const uint32_t before = k ? lower_bound_u32(xtedg + s, j, k * width) : 0u;  // the row's ids of lower chunks
+      edg[off[k * row + v] + (j - before)] = layout_id(hot_idx, hot_words, u);
     }
   }
 }
@@ -470,7 +497,7 @@ cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd64, ui
   uint32_t *scratch = nullptr, *noff = nullptr, *ntoff = nullptr, *nedg = nullptr, *ntedg = nullptr, *ndat = nullptr;
   uint32_t *ranges = nullptr, *lists = nullptr;
   const uint32_t* in_list = nullptr;  // the in-CSR's touched rows (plain graphs)
-  uint32_t in_T = 0;
+  const uint32_t* touched_count = nullptr;  // their number, in device memory (plain graphs)
   struct NewLayout {
     ChunkLayout* l;
     uint32_t *off, *edg;
@@ -554,27 +581,31 @@ cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd64, ui
     const std::vector<uint64_t>* opos[2] = {&g.xpos, &g.xtpos};
     std::vector<uint32_t> hb(nseg + 1);
     for (int csr = 0; csr < 2; ++csr) {
-      uint32_t T = 0;
       if (csr == 1) in_list = trow;
       k_word_pop<<<grid, kThreads, 0, s>>>(tch[csr], words, cnt);
       PRX_CU(exclusive_scan_u32(cnt, words + 1, s));
-      PRX_CU(cudaMemcpyAsync(&T, cnt + words, 4, cudaMemcpyDeviceToHost, s));
       k_touched_list<<<grid, kThreads, 0, s>>>(tch[csr], words, cnt, trow);
-      PRX_CU(cudaStreamSynchronize(s));  // T
-      if (csr == 1) in_T = T;
-      k_list_slices<<<(nseg + 256) / 256, 256, 0, s>>>(trow, T, n, S, nseg, bounds);
-      PRX_CU(cudaMemcpyAsync(hb.data(), bounds, 4 * ((size_t)nseg + 1), cudaMemcpyDeviceToHost, s));
+      if (segmented) {
+        uint32_t T = 0;
+        PRX_CU(cudaMemcpyAsync(&T, cnt + words, 4, cudaMemcpyDeviceToHost, s));
+        PRX_CU(cudaStreamSynchronize(s));
+        k_list_slices<<<(nseg + 256) / 256, 256, 0, s>>>(trow, T, n, S, nseg, bounds);
+        PRX_CU(cudaMemcpyAsync(hb.data(), bounds, 4 * ((size_t)nseg + 1), cudaMemcpyDeviceToHost, s));
+        PRX_CU(cudaStreamSynchronize(s));
+      } else {
+        touched_count = cnt + words;  // the kernels read it
+      }
       PRX_CU(cudaMemsetAsync(ranges, 0, sizeof(uint32_t) * 4 * (size_t)n, s));
       if (nd) k_batch_ranges<<<grid, kThreads, 0, s>>>(keys[csr][0], nd, dbeg, dend);
       if (ni) k_batch_ranges<<<grid, kThreads, 0, s>>>(keys[csr][1], ni, ibeg, iend);
-      PRX_CU(cudaStreamSynchronize(s));
       for (uint32_t k = 0; k < nseg; ++k) {
         const uint32_t v0 = segmented ? (uint32_t)((uint64_t)k << S) : 0;
         const uint32_t v1 = segmented ? (uint32_t)std::min<uint64_t>(n, (uint64_t)v0 + (1ull << S)) : n;
         const uint64_t op = segmented ? (*opos[csr])[k] : 0, np = segmented ? pos[csr][k] : 0;
-        const Runs r{ooff[csr] + v0 + k, nof[csr] + v0 + k, trow + hb[k], hb[k + 1] - hb[k], v1 - v0, v0, nullptr};
+        const Runs r{ooff[csr] + v0 + k, nof[csr] + v0 + k, trow + hb[k], hb[k + 1] - hb[k], v1 - v0, v0,
+                     touched_count};
         k_copy_runs<<<grid, kThreads, 0, s>>>(r, oedg[csr] + op, ned[csr] + np);
-        if (r.T) {
+        if (r.T || touched_count) {
           PRX_CU(cudaMemsetAsync(nbig, 0, 8, s));
           k_merge_touched<<<grid, kThreads, 0, s>>>(r, oedg[csr] + op, ned[csr] + np, vals[csr][0], dbeg + v0,
                                                     dend + v0, vals[csr][1], ibeg + v0, iend + v0, big, nbig);
@@ -599,7 +630,7 @@ cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd64, ui
       if (el == cudaSuccess) el = graph_alloc(&le, sizeof(uint32_t) * edge_slots(low_edges), s);
       if (el == cudaSuccess) el = graph_alloc(&ws, sizeof(uint32_t) * scan_ws_words((uint32_t)len), s);
       if (el == cudaSuccess)
-        el = carry_layout(l, ntoff, ntedg, n, tin, in_list, in_T, nullptr, g.hot_idx, lo, le, ws, sms, s);
+        el = carry_layout(l, ntoff, ntedg, n, tin, in_list, 0, touched_count, g.hot_idx, lo, le, ws, sms, s);
       if (ws) cudaFreeAsync(ws, s);
       if (el != cudaSuccess) {
         graph_free({lo, le});

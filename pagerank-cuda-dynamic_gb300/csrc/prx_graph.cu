@@ -195,16 +195,23 @@ __global__ void __launch_bounds__(256) k_cls_edges(const uint32_t* __restrict__ 
   __shared__ unsigned long long acc[NCLS + 1];
   if (threadIdx.x <= NCLS) acc[threadIdx.x] = 0;
   __syncthreads();
-  unsigned long long mine[NCLS + 1] = {0, 0, 0, 0};
+  unsigned long long all = 0, low = 0, high = 0, padded = 0;
   const uint32_t words = (uint32_t)(((uint64_t)n + 31) >> 5);
   for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += (gridDim.x * blockDim.x) >> 5) {
     const uint32_t v = (w << 5) | lane_id();
-    const uint32_t d = v < n ? row_len(xtoff, shift, v) : 0u;
-    mine[d <= kLowMax ? LOW : (d <= mid_max ? MID : HIGH)] += d;
-    mine[NCLS] += __reduce_max_sync(0xffffffffu, d <= kLowMax ? d : 0u);
+    const uint32_t d = v < n ? row_len(xtoff, shift, v) : 0u, l = d <= kLowMax ? d : 0u;
+    all += d;
+    low += l;
+    high += d > kLowMax && d > mid_max ? d : 0u;
+    padded += __reduce_max_sync(0xffffffffu, l);
   }
-  for (int c = 0; c <= NCLS; ++c)
-    if (mine[c]) atomicAdd(&acc[c], mine[c]);
+  unsigned long long mine[NCLS + 1] = {low, all - low - high, high, padded};
+#pragma unroll
+  for (int c = 0; c <= NCLS; ++c) {  // a warp's first: 256 atomics on one word took most of the kernel
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mine[c] += __shfl_xor_sync(0xffffffffu, mine[c], o);
+    if (lane_id() == 0 && mine[c]) atomicAdd(&acc[c], mine[c]);
+  }
   __syncthreads();
   if (threadIdx.x <= NCLS && acc[threadIdx.x]) atomicAdd(&out[threadIdx.x], acc[threadIdx.x]);
 }
@@ -930,15 +937,37 @@ cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, u
 namespace prx {
 
 // ---- exclusive scan of uint32 (in place), three passes ----------------------
+// A tile is kTileV = 8 x 256 words; a warp reads 32 of its 256 at a time (3M
+// words: 6.5 us and, below, 16 at eight consecutive words a thread, 6.0 and
+// 7.0 so).
 __global__ void __launch_bounds__(256) k_scan_tile_sums(const uint32_t* __restrict__ in, uint32_t len,
                                                         uint32_t* __restrict__ sums) {
-  const uint32_t i0 = blockIdx.x * kTileV + threadIdx.x * 8;
+  const uint32_t i0 = blockIdx.x * kTileV + threadIdx.x;
   unsigned long long x = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) x += i0 + k < len ? in[i0 + k] : 0u;
+  for (int k = 0; k < 8; ++k) x += i0 + 256 * k < len ? in[i0 + 256 * k] : 0u;
   unsigned long long tot;
   block_scan_incl(x, &tot);
   if (threadIdx.x == 0) sums[blockIdx.x] = (uint32_t)tot;
+}
+
+// Exclusive sums of a warp's 256 words, v[k] the lane's of the k-th 32;
+// returns their total.
+__device__ __forceinline__ uint32_t warp_scan256(uint32_t v[8], uint32_t lane) {
+  uint32_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    uint32_t x = v[k];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= (uint32_t)o) x += y;
+    }
+    const uint32_t all = __shfl_sync(0xffffffffu, x, 31);
+    v[k] = sum + x - v[k];
+    sum += all;
+  }
+  return sum;
 }
 
 __global__ void __launch_bounds__(1024) k_scan_single(uint32_t* a, uint32_t len) {
@@ -966,18 +995,19 @@ __global__ void __launch_bounds__(1024) k_scan_single(uint32_t* a, uint32_t len)
 
 __global__ void __launch_bounds__(256) k_scan_apply(uint32_t* __restrict__ data, uint32_t len,
                                                     const uint32_t* __restrict__ tile_pre) {
-  const uint32_t i0 = blockIdx.x * kTileV + threadIdx.x * 8;
+  __shared__ uint32_t sums[8];
+  const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const uint32_t b = blockIdx.x * kTileV + 256 * w + lane;
   uint32_t v[8];
-  unsigned long long x = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) { v[k] = i0 + k < len ? data[i0 + k] : 0u; x += v[k]; }
-  unsigned long long tot;
-  uint32_t run = tile_pre[blockIdx.x] + (uint32_t)(block_scan_incl(x, &tot) - x);
+  for (int k = 0; k < 8; ++k) v[k] = b + 32 * k < len ? data[b + 32 * k] : 0u;
+  const uint32_t sum = warp_scan256(v, lane);
+  if (lane == 0) sums[w] = sum;
+  __syncthreads();
+  const uint32_t pre = tile_pre[blockIdx.x] + __reduce_add_sync(0xffffffffu, lane < w ? sums[lane] : 0u);
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    if (i0 + k < len) data[i0 + k] = run;
-    run += v[k];
-  }
+  for (int k = 0; k < 8; ++k)
+    if (b + 32 * k < len) data[b + 32 * k] = pre + v[k];
 }
 
 // The whole scan in one block: 8 words a thread at a time, a running total
@@ -991,21 +1021,10 @@ __global__ void __launch_bounds__(1024) k_scan_block(uint32_t* __restrict__ a, u
   for (uint32_t i0 = 0; i0 < len; i0 += 8192, buf ^= 1) {
     // warp w: the 256 words from i0 + 256 w on, a word of each 32 per lane
     const uint32_t b = i0 + 256 * w + lane;
-    uint32_t v[8], sum = 0;
+    uint32_t v[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) v[k] = b + 32 * k < len ? a[b + 32 * k] : 0u;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {  // v[k]: sum of the warp's words up to and with this one
-      uint32_t x = v[k];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= (uint32_t)o) x += y;
-      }
-      const uint32_t all = __shfl_sync(0xffffffffu, x, 31);
-      v[k] = sum + x - v[k];
-      sum += all;
-    }
+    const uint32_t sum = warp_scan256(v, lane);
     if (lane == 0) sums[buf][w] = sum;
     __syncthreads();
     const uint32_t c = sums[buf][lane];
