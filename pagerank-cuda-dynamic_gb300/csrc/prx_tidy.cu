@@ -18,8 +18,10 @@
 // merged into sorted neighbour sets), adds a self-loop to every vertex
 // (addSelfLoopsOmp, inc/selfLoop.hxx:60-66) and transposes it with the
 // out-degrees (transposeWithDegreeOmp, inc/transpose.hxx:110-134).  Here:
-// keys u * 2^b + v (plus v * 2^b + v for the self-loops), radix sort, unique,
-// row starts from the sorted keys; the transpose the same from v * 2^b + u.
+// counting and row sorts (prx_ingest.cu); of lists with 1024 entries a row and
+// more, keys u * 2^b + v (plus v * 2^b + v for the self-loops), radix sort,
+// unique, row starts from the sorted keys; the transpose the same from
+// v * 2^b + u.
 #include <algorithm>
 #include <vector>
 #include "prx_ctx.h"

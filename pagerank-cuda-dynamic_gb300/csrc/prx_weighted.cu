@@ -21,7 +21,7 @@
 // up to the lines of persist_fits iterate in one cooperative kernel
 // (k_pull_persist), as the FP64 solves do (prx_persist.cu): a sweep of R-MAT
 // 2^18 (4.2M edges, everything in L2) took 83 us in four launches and takes
-// 31 us there.  Larger ones launch the classes one by one.
+// 24 us there.  Larger ones launch the classes one by one.
 //
 // Graphs with row segments (64-bit offsets, see GraphDev): px / pt are laid
 // out like the edge arrays they follow (the same segment bases), and the
