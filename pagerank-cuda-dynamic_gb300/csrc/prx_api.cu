@@ -618,12 +618,21 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
     if (g.hot_n && (st = ensure_ch(c, g.hot_n))) return st;
   }
   const ChunkLayout *lay64 = nullptr, *lay32 = nullptr;
-  if (!persist) TRY_CUDA_ST(ensure_chunks(gr->g, w64, c->sms, c->stream, &lay64, hot_ok && g.hot_n > 0));
-  if (refine && !persist) TRY_CUDA_ST(ensure_chunks(gr->g, w32, c->sms, c->stream, &lay32));
+  // one chunk: the LOW rows by words where rows are long.  A refined solve has
+  // its FP32 sweeps read them too, so without hot sources.
+  const bool by_words = !persist && w64 >= g.n && words_fit(g);
+  const bool hot_words = hot_ok && g.hot_n > 0 && !refine;
+  WordView words;
+  if (by_words) TRY_CUDA_ST(ensure_words(gr->g, hot_words, c->sms, c->stream, &words));
+  if (!persist && !by_words) TRY_CUDA_ST(ensure_chunks(gr->g, w64, c->sms, c->stream, &lay64, hot_ok && g.hot_n > 0));
+  // FP32 contributions by words: one chunk, unless a width was asked for or tuned
+  const bool words32 = words.grp && !o.chunk_vertices && !g.tuned_w32;
+  if (refine && !persist && !words32) TRY_CUDA_ST(ensure_chunks(gr->g, w32, c->sms, c->stream, &lay32));
   cudaStream_t s = c->stream;
   SolveArgs a = make_args(c, g, o);
   a.hot_list = g.hot_list;
-  a.hot_n = (lay64 && lay64->hot) ? g.hot_n : 0;
+  a.words = words;
+  a.hot_n = (lay64 && lay64->hot) || (words.grp && hot_words) ? g.hot_n : 0;
   const int repeat = o.repeat > 0 ? o.repeat : 1;
   float ti = 0, tm = 0, tc = 0, tt = 0;
   const bool timing = o.timing != 0;
@@ -886,7 +895,8 @@ int prx_graph_create(prx_context* c, uint32_t n, uint64_t m, const uint32_t* xof
   if (e == cudaSuccess) e = ensure_hot(g, kDefaultHotCap, c->sms, s);
   if (e == cudaSuccess) {
     const uint32_t width = g.tuned_w64 ? g.tuned_w64 : kDefaultChunk64;
-    e = build_default_layout_pipelined(g, width, g.hot_n > 0, pieces, rows, ev, c->sms, s);
+    if (width < n || !words_fit(g))  // else the first solve lays the rows out by words
+      e = build_default_layout_pipelined(g, width, g.hot_n > 0, pieces, rows, ev, c->sms, s);
   }
   if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ev_done, 0);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -439,4 +439,46 @@ __device__ __forceinline__ double warp_row_sums(const double* c, const uint32_t*
   return len ? acc : init;
 }
 
+// The same sums of a word's rows laid out as WordRows (from group `base` on):
+// len the lane's row, mine whether it is summed.
+template <int K>
+__device__ __forceinline__ double word_row_sums(const double* c, const uint4* __restrict__ grp, uint32_t base,
+                                                uint32_t len, bool mine, const double* ch, bool hot) {
+  const uint32_t want = mine ? len : 0u;
+  const uint32_t L = __reduce_max_sync(0xffffffffu, want);
+  if (L == 0) return 0.0;
+  const uint32_t below = (1u << lane_id()) - 1u;
+  auto ids = [&](uint32_t t) {  // step t's group, called for 0, 4, 8, ...
+    const unsigned rows = __ballot_sync(0xffffffffu, t < len);
+    const uint4 u = t < want ? __ldg(grp + (base + __popc(rows & below))) : make_uint4(0, 0, 0, 0);
+    base += __popc(rows);
+    return u;
+  };
+  auto terms = [&](uint32_t t, const uint4& u, double x[4]) {
+    x[0] = t < want ? gather<double>(c, ch, hot, u.x) : 0.0;
+    x[1] = t + 1 < want ? gather<double>(c, ch, hot, u.y) : 0.0;
+    x[2] = t + 2 < want ? gather<double>(c, ch, hot, u.z) : 0.0;
+    x[3] = t + 3 < want ? gather<double>(c, ch, hot, u.w) : 0.0;
+  };
+  double x[4];
+  uint4 g1 = ids(0), g2 = ids(4);
+  terms(0, g1, x);
+  g1 = g2;
+  g2 = ids(8);
+  const double x0 = __double_as_longlong(x[0]) == (long long)(1ull << 63) ? 0.0 : x[0];  // +0 + -0 = +0
+  double acc = add_step<K, 1>(want ? x0 : 1.0, x, min(4u, L));  // lanes without terms: in soft_add's range
+  uint32_t t = 4;
+  for (; t + 4 <= L; t += 4) {
+    terms(t, g1, x);
+    g1 = g2;
+    g2 = ids(t + 8);
+    acc = add_step<K, 0>(acc, x, 4);
+  }
+  if (t < L) {
+    terms(t, g1, x);
+    acc = add_step<K, 0>(acc, x, L - t);
+  }
+  return want ? acc : 0.0;
+}
+
 }  // namespace prx

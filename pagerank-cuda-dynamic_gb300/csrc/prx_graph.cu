@@ -464,8 +464,10 @@ static void free_layout(ChunkLayout& l) {
   l = ChunkLayout();
 }
 
+static void free_words(GraphDev& g);
 void free_chunks(GraphDev& g) {
   for (auto& l : g.lay) free_layout(l);
+  free_words(g);
 }
 
 // The chunk layout of one CSR of `rows` rows (offsets off[0 .. rows], edges
@@ -650,6 +652,95 @@ cudaError_t build_default_layout_pipelined(GraphDev& g, uint32_t width, bool hot
   return cudaSuccess;
 }
 
+// Groups of four per word of LOW rows (a 0 closing them) and every row's length.
+__global__ void __launch_bounds__(256) k_word_groups(const uint32_t* __restrict__ xtoff,
+                                                     const uint32_t* __restrict__ low_bm, uint32_t n,
+                                                     uint8_t* __restrict__ len, uint32_t* __restrict__ cnt) {
+  const uint32_t words = (n + 31) >> 5, lane = lane_id();
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w <= words; w += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t v = (w << 5) | lane;
+    const bool low = w < words && v < n && ((low_bm[w] >> lane) & 1u);
+    const uint32_t l = low ? xtoff[v + 1] - xtoff[v] : 0u;
+    if (w < words && v < n) len[v] = (uint8_t)l;
+    const uint32_t groups = __reduce_add_sync(0xffffffffu, (l + 3) / 4);
+    if (lane == 0) cnt[w] = groups;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_word_fill(const uint32_t* __restrict__ xtoff,
+                                                   const uint32_t* __restrict__ xtedg,
+                                                   const uint8_t* __restrict__ len, uint32_t n,
+                                                   const uint32_t* __restrict__ base,
+                                                   const uint32_t* __restrict__ hot_idx, uint4* __restrict__ grp) {
+  const uint32_t words = (n + 31) >> 5, lane = lane_id(), below = (1u << lane) - 1u;
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t v = (w << 5) | lane;
+    const uint32_t l = v < n ? len[v] : 0u, s = l ? xtoff[v] : 0u;
+    uint32_t at = base[w];
+    for (uint32_t t = 0;; t += 4) {
+      const unsigned rows = __ballot_sync(0xffffffffu, t < l);
+      if (!rows) break;
+      if (t < l) {
+        uint32_t u[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) u[k] = __ldg(xtedg + s + min(t + k, l - 1));
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) u[k] = layout_id(hot_idx, words, u[k]);
+        grp[at + __popc(rows & below)] = make_uint4(u[0], u[1], u[2], u[3]);
+      }
+      at += __popc(rows);
+    }
+  }
+}
+
+bool words_fit(const GraphDev& g) {
+  return g.nseg == 1 && !g.xtbase && g.cls_begin[MID] && g.cls_edges[LOW] >= 16ull * g.cls_begin[MID];
+}
+
+cudaError_t ensure_words(GraphDev& g, bool hot, int sms, cudaStream_t s, WordView* out) {
+  *out = WordView();
+  const uint32_t nlow = g.cls_begin[MID];
+  WordRows& r = g.words[hot ? 1 : 0];
+  if (!r.built) {
+    const uint32_t words = (g.n + 31) / 32;
+    const uint64_t groups = g.cls_edges[LOW] / 4 + nlow;  // at most
+    cudaError_t e = cudaSuccess;
+    if (!r.len) e = graph_alloc(&r.len, g.n, s);
+    if (e == cudaSuccess && !r.base) e = graph_alloc(&r.base, sizeof(uint32_t) * ((size_t)words + 1), s);
+    if (e == cudaSuccess && r.cap < groups) {
+      if (r.grp) cudaFreeAsync(r.grp, s);
+      r.grp = nullptr;
+      r.cap = 0;
+      const uint64_t cap = groups + groups / 128;  // the next versions' too
+      e = graph_alloc(&r.grp, sizeof(uint4) * cap, s);
+      if (e == cudaSuccess) r.cap = cap;
+    }
+    if (e == cudaSuccess) {
+      k_word_groups<<<sms * 8, 256, 0, s>>>(g.xtoff, g.low_bm, g.n, r.len, r.base);
+      e = exclusive_scan_u32(r.base, words + 1, s);
+      k_word_fill<<<sms * 8, 256, 0, s>>>(g.xtoff, g.xtedg, r.len, g.n, r.base, hot ? g.hot_idx : nullptr, r.grp);
+    }
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      graph_free({r.len, r.base, r.grp});
+      r = WordRows();
+      return cudaSuccess;
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    r.built = true;
+  }
+  *out = {r.len, r.base, r.grp};
+  return cudaSuccess;
+}
+
+static void free_words(GraphDev& g) {
+  for (auto& r : g.words) {
+    graph_free({r.len, r.base, r.grp});
+    r = WordRows();
+  }
+}
+
 cudaError_t ensure_chunks(GraphDev& g, uint32_t width, int sms, cudaStream_t s, const ChunkLayout** out,
                           bool hot) {
   uint64_t& clock = g_layout_clock;
@@ -761,6 +852,7 @@ __global__ void k_hot_list(const uint32_t* __restrict__ bm, const uint32_t* __re
 }
 
 void free_hot(GraphDev& g) {
+  g.words[1].built = false;
   graph_free({g.hot_idx, g.hot_list});
   g.hot_idx = g.hot_list = nullptr;
   g.hot_n = 0;
@@ -829,6 +921,7 @@ cudaError_t ensure_hot(GraphDev& g, uint32_t cap, int sms, cudaStream_t s) {
 cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layouts) {
   const uint32_t n = g.n;
   g.plan_built = g.len_built = g.oplan_built = g.tpos_built = false;
+  g.words[0].built = g.words[1].built = false;
   if (!keep_layouts) {
     free_chunks(g);
     free_hot(g);

@@ -106,7 +106,26 @@ struct ChunkLayout {
   std::vector<uint32_t*> seg_off, seg_edg;
 };
 
+// The LOW rows of a plain graph by 32-id words, for sweeps of one source chunk:
+// word w's ids in groups of four (the last of a row padded), the k-th groups of
+// its rows that have one side by side, from group base[w] on; len[v] the row's
+// length, 0 for a row of another class.  A warp's id loads are then one
+// consecutive piece a step instead of 32 rows' pieces.
+struct WordRows {
+  uint8_t* len = nullptr;
+  uint32_t* base = nullptr;
+  uint4* grp = nullptr;
+  uint64_t cap = 0;               // groups allocated
+  bool built = false;
+};
+struct WordView {
+  const uint8_t* len = nullptr;
+  const uint32_t* base = nullptr;
+  const uint4* grp = nullptr;     // null: not used
+};
+
 struct GraphDev {
+  WordRows words[2];              // plain ids, hot sources encoded (GraphDev::hot_idx)
   int device = 0;                 // device holding the arrays
   uint32_t n = 0;
   uint64_t m = 0;
@@ -211,6 +230,16 @@ constexpr uint32_t kPfTable = 1u << 16;  // out-degrees whose DF-P factor is tab
 constexpr uint32_t kHotFlag = 0x80000000u;
 // The hot sources of g for a cap of `cap` vertices (0: none); graphs of 2^31
 // vertices or more get none (their ids use the flag bit).
+// Whether one-chunk LOW sweeps go by words: plain graphs with rows of 16 in-edges
+// and more on average.  The sweep was bound by the L1 (81% of its wavefronts), and
+// a fifth of those were id loads.  Static solves, ms, rows | words: web-like 3M
+// vertices 3.29 | 2.95, 6M 5.82 | 5.11, 20M 16.2 | 14.4; FP32-refined 3M 2.97 |
+// 2.39, 6M 5.39 | 4.38, 14M 13.7 (two chunks) | 10.5; grid 4096^2, rows of five
+// (padded to eight ids), 3.56 | 3.66.
+bool words_fit(const GraphDev& g);
+// The LOW rows by words for this graph version; a null view when there is no
+// memory for them (the sweeps then read the CSR).
+cudaError_t ensure_words(GraphDev& g, bool hot, int sms, cudaStream_t s, WordView* out);
 cudaError_t ensure_hot(GraphDev& g, uint32_t cap, int sms, cudaStream_t s);
 void free_hot(GraphDev& g);
 
@@ -225,6 +254,7 @@ void free_chunks(GraphDev& g);
 
 // Pointers a solve kernel needs.  Passed by value.
 struct SolveArgs {
+  WordView words;                 // of the FP64 LOW sweeps (null: by off / edg)
   const uint32_t* xoff;
   const uint32_t* xedg;
   const uint32_t* xtoff;

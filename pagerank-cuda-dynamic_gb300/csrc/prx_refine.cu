@@ -93,6 +93,44 @@ __global__ void __launch_bounds__(kThreads, WIDE ? kWideBlocks : 8) k32_low(Solv
   if (LAST) reduce32(st, emax, mag);
 }
 
+// The rows by words (WordRows), two groups a step: eight gathers in flight, and
+// the next two groups' loads behind them.  Terms outside a row are +0.
+__global__ void __launch_bounds__(kThreads, kWideBlocks) k32_words(SolveArgs a) {
+  State* st = a.st;
+  if (st->done || st->inner_done) return;
+  const int q = st->k32 & 1;
+  const float* __restrict__ ce = a.ce[q];
+  const uint32_t words = (uint32_t)(((uint64_t)a.n + 31) >> 5), lane = lane_id(), below = (1u << lane) - 1u;
+  unsigned int emax = 0, mag = 0;
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t v = (w << 5) | lane;
+    const bool low = v < a.n && ((__ldg(a.low_bm + w) >> lane) & 1u);
+    const uint32_t len = v < a.n ? __ldg(a.words.len + v) : 0u;
+    const uint32_t L = __reduce_max_sync(0xffffffffu, len);
+    uint32_t at = __ldg(a.words.base + w);
+    auto ids = [&](uint32_t t) {  // called for 0, 4, 8, ...
+      const unsigned rows = __ballot_sync(0xffffffffu, t < len);
+      const uint4 u = t < len ? __ldg(a.words.grp + (at + __popc(rows & below))) : make_uint4(0, 0, 0, 0);
+      at += __popc(rows);
+      return u;
+    };
+    uint4 g0 = ids(0), g1 = ids(4);
+    float acc = 0.f;
+    for (uint32_t t = 0; t < L; t += 8) {
+      const uint32_t id[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+      float x[8];
+#pragma unroll
+      for (uint32_t k = 0; k < 8; ++k) x[k] = t + k < len ? __ldg(ce + id[k]) : 0.f;
+      g0 = ids(t + 8);
+      g1 = ids(t + 12);
+#pragma unroll
+      for (uint32_t k = 0; k < 8; ++k) acc += x[k];
+    }
+    if (low) emax = max(emax, finish32(a, v, acc, q, &mag));
+  }
+  reduce32(st, emax, mag);
+}
+
 // MID: warp per vertex, lane-strided sums folded by shuffles.
 __global__ void __launch_bounds__(kThreads) k32_mid(SolveArgs a, uint32_t begin, uint32_t count) {
   State* st = a.st;
@@ -243,6 +281,10 @@ bool launch_sweep32(const SolveArgs& a, const GraphDev& g, int cls, const ChunkL
   const uint32_t b = g.cls_begin[cls], cnt = g.cls_begin[cls + 1] - b;
   if (!cnt) return false;
   if (cls == LOW) {
+    if (a.words.grp && !a.hot_n && (!lay || lay->K <= 1)) {
+      k32_words<<<cap_grid32(((uint64_t)g.n + 255) / 256, sms * kWideBlocks), kThreads, 0, s>>>(a);
+      return true;
+    }
     if (!lay || lay->K <= 1) {
       sweep32_low<true, true>(a, wide_rows(g, 1), 0, g.n, g.xtbase, g.seg_shift, g.xtoff, g.xtedg, sms, s);
       return true;

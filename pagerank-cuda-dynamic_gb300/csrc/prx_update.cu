@@ -49,7 +49,7 @@ enum Pass { PASS_ONLY = 0, PASS_FIRST = 1, PASS_INNER = 2, PASS_LAST = 3 };
 // hot: the layout encodes hot sources (the FP64 modes); their contributions
 // are gathered from a.ch[p].
 // K: adds of every step by soft_add (the FP64 modes).
-template <int MODE, int PASS, int K>
+template <int MODE, int PASS, int K, bool WORDS>
 __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
     k_update_low(SolveArgs a, uint32_t vb, uint32_t ve, const unsigned long long* __restrict__ base, uint32_t shift,
                  const uint32_t* __restrict__ off, const uint32_t* __restrict__ edg, bool hot) {
@@ -107,13 +107,22 @@ __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
     // One thread per row: a row's terms must be added front to back (the
     // reference's order), and a whole row per lane keeps the warp's FP64 adds
     // for different rows running side by side.
-    const uint64_t iv = seg_index(v, shift) - vb;
-    const uint32_t s = mine ? off[iv] : 0, e = mine ? off[iv + 1] : 0;
+    uint32_t s = 0, e = 0, wlen = 0;  // the row; by words: its length (0 of another class)
+    if constexpr (WORDS) {
+      wlen = v < ve ? __ldg(a.words.len + v) : 0u;
+      e = wlen;
+    } else {
+      const uint64_t iv = seg_index(v, shift) - vb;
+      s = mine ? off[iv] : 0;
+      e = mine ? off[iv + 1] : 0;
+    }
     mine = low && (FIRST || LAST || s < e);
     bool survive = false, changed = false;
     V acc = V(0);
     if constexpr (T::F32) {
       if (mine) acc = lane_row_sum(c, seg_edges(edg, base, shift, v), s, e, FIRST ? V(0) : carried_of<MODE>(a)[v]);
+    } else if constexpr (WORDS) {
+      acc = word_row_sums<K>(c, a.words.grp, __ldg(a.words.base + w), wlen, mine, ch, hot);
     } else {  // the whole warp sums together
       const V init = (mine && !FIRST) ? carried_of<MODE>(a)[v] : V(0);
       acc = warp_row_sums<false, FIRST, 0, K>(c, seg_edges(edg, base, shift, v), s, mine ? e : s, init, ch, hot);
@@ -463,14 +472,26 @@ void launch_commit_dyn32(const SolveArgs& a, int parity, cudaStream_t s) {
   k_commit_dyn32<<<cap_grid((a.n + kThreads - 1) / kThreads, 152 * 16), kThreads, 0, s>>>(a, parity);
 }
 
+template <int MODE, int PASS, int K>
+static void low_pass_k(int grid, cudaStream_t s, const SolveArgs& a, uint32_t vb, uint32_t ve,
+                       const unsigned long long* base, uint32_t shift, const uint32_t* off, const uint32_t* edg,
+                       bool hot) {
+  if constexpr (PASS == PASS_ONLY && !ModeTraits<MODE>::F32) {
+    if (a.words.grp) {
+      k_update_low<MODE, PASS, K, true><<<grid, kThreads, 0, s>>>(a, vb, ve, base, shift, off, edg, a.hot_n > 0);
+      return;
+    }
+  }
+  k_update_low<MODE, PASS, K, false><<<grid, kThreads, 0, s>>>(a, vb, ve, base, shift, off, edg, hot);
+}
+
 template <int MODE, int PASS>
 static void low_pass(int grid, cudaStream_t s, const SolveArgs& a, uint32_t vb, uint32_t ve,
                      const unsigned long long* base, uint32_t shift, const uint32_t* off, const uint32_t* edg,
                      bool hot) {
-  if (a.int_adds && !ModeTraits<MODE>::F32)
-    k_update_low<MODE, PASS, ModeTraits<MODE>::F32 ? 0 : 1><<<grid, kThreads, 0, s>>>(a, vb, ve, base, shift, off, edg, hot);
-  else
-    k_update_low<MODE, PASS, 0><<<grid, kThreads, 0, s>>>(a, vb, ve, base, shift, off, edg, hot);
+  constexpr int K = ModeTraits<MODE>::F32 ? 0 : 1;
+  if (a.int_adds) low_pass_k<MODE, PASS, K>(grid, s, a, vb, ve, base, shift, off, edg, hot);
+  else low_pass_k<MODE, PASS, 0>(grid, s, a, vb, ve, base, shift, off, edg, hot);
 }
 
 template <int MODE>
