@@ -609,18 +609,23 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   // the plain rows (no hot copy, no source chunks); see launch_persist.
   const bool persist = (!refine || (!dyn && o.max_iterations > 0 && g.mid_max >= kPlanMid)) &&
                        o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase &&
-                       g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) && persist_fits(g);
+                       g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) && persist_fits(g) &&
+                       (mixed_lengths(g) || !words_fit(g) || (uint64_t)g.n <= 32 * kPersistWordUnits);
   if (persist) TRY_CUDA_ST(ensure_plan(gr->g, c->sms, c->stream));
-  const bool hot_ok = o.hot_sources >= 0 && !persist;
+  // one chunk: the LOW rows by words where rows are long.  A refined solve has
+  // its FP32 sweeps read them too, so without hot sources; contributions that L2
+  // holds anyway (64 MB) do without unless they are asked for (Static, web-like
+  // 3M vertices 2.94 ms without and 2.96 with, 6M 5.16 and 5.14, 20M 16.2 and
+  // 14.3), which saves a graph's first solve picking them.
+  const bool by_words = !persist && w64 >= g.n && words_fit(g);
+  const bool hot_ok = o.hot_sources >= 0 && !persist &&
+                      !(by_words && o.hot_sources == 0 && (refine || g.n <= (8u << 20)));
   if (hot_ok) {
     TRY_CUDA_ST(ensure_hot(gr->g, o.hot_sources > 0 ? (uint32_t)o.hot_sources : kDefaultHotCap, c->sms,
                            c->stream));
     if (g.hot_n && (st = ensure_ch(c, g.hot_n))) return st;
   }
   const ChunkLayout *lay64 = nullptr, *lay32 = nullptr;
-  // one chunk: the LOW rows by words where rows are long.  A refined solve has
-  // its FP32 sweeps read them too, so without hot sources.
-  const bool by_words = !persist && w64 >= g.n && words_fit(g);
   const bool hot_words = hot_ok && g.hot_n > 0 && !refine;
   WordView words;
   if (by_words) TRY_CUDA_ST(ensure_words(gr->g, hot_words, c->sms, c->stream, &words));

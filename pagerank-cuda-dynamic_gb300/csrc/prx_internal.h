@@ -348,6 +348,12 @@ constexpr uint64_t kPersistUnits = 48u << 10, kPersistSortedUnits = 1u << 20;
 inline bool plan_fits(uint32_t n, uint32_t low, bool mixed) {
   return ((uint64_t)(mixed ? low : n) + 31) / 32 + (n - low) <= (mixed ? kPersistSortedUnits : kPersistUnits);
 }
+// Graphs whose LOW rows the launched sweep takes by words (words_fit), rows of
+// even length: web-like 0.6M vertices (18,750 units) 76 | 82, 0.8M 98 | 98, 1.1M
+// 134 | 128, 1.5M 178 | 158, FP32 in the same order 62 | 60, 84 | 79, 117 | 101,
+// 156 | 129; but laying the words out costs a graph that is solved once about
+// what is gained at 1.1M.
+constexpr uint64_t kPersistWordUnits = 32u << 10;
 inline bool persist_fits(const GraphDev& g) { return plan_fits(g.n, g.cls_begin[MID], mixed_lengths(g)); }
 cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s);
 // The whole FP64 iteration loop of a plain graph (one row segment) as one
