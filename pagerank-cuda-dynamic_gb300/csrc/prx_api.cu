@@ -631,7 +631,8 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   if (by_words) TRY_CUDA_ST(ensure_words(gr->g, hot_words, c->sms, c->stream, &words));
   if (!persist && !by_words) TRY_CUDA_ST(ensure_chunks(gr->g, w64, c->sms, c->stream, &lay64, hot_ok && g.hot_n > 0));
   // FP32 contributions by words: one chunk, unless a width was asked for or tuned
-  const bool words32 = words.grp && !o.chunk_vertices && !g.tuned_w32;
+  // (the dynamic modes' own FP32 iterations read chunks or the CSR)
+  const bool words32 = words.grp && !dyn && !o.chunk_vertices && !g.tuned_w32;
   if (refine && !persist && !words32) TRY_CUDA_ST(ensure_chunks(gr->g, w32, c->sms, c->stream, &lay32));
   cudaStream_t s = c->stream;
   SolveArgs a = make_args(c, g, o);
