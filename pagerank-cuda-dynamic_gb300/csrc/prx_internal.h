@@ -400,7 +400,8 @@ void launch_frontier_from_bitmap(const SolveArgs& a, int sms, cudaStream_t s);
 // past the count set to all ones): persistent warps take reached vertices
 // and mark their out-neighbours, until nothing is left, or until the queue
 // holds more than switch_at vertices and eight times those done (a closure
-// exploding in few steps, left to pull rounds).
+// exploding in few steps, left to pull rounds; so is one whose marking holds
+// more than switch_at).
 void launch_closure_queue(const SolveArgs& a, uint32_t switch_at, int sms, cudaStream_t s);
 // One DT closure round by pulling: every vertex not yet reached that has a
 // reached in-neighbour joins (no-op once a round added nothing).

@@ -195,10 +195,12 @@ __global__ void __launch_bounds__(kQWarps * 32) k_closure_queue(SolveArgs a, uin
     if (lane == 0) atomicAdd(&st->q_done, cnt);
   };
   // the vertices the queue starts with, in shares that reach all warps (claimed,
-  // not assigned: no warp waits for one that has not started)
+  // not assigned: no warp waits for one that has not started); too many of them
+  // are left to the pull rounds by every warp, for nobody would claim them
   const uint32_t first = st->fcnt[1], warps = gridDim.x * kQWarps;
+  if (first > switch_at) return;
   const uint32_t share = min(32u, (first + warps - 1) / warps);
-  while (first <= switch_at) {
+  for (;;) {
     uint32_t i = 0;
     if (lane == 0) i = atomicAdd(&st->fcnt[2], share);
     i = __shfl_sync(0xffffffffu, i, 0);
