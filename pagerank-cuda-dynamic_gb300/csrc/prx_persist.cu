@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
     auto word_pass = [&](uint32_t w) -> uint32_t {
       const uint32_t v = (w << 5) | lane;
       const uint32_t cw = cur[w], pw = prev[w];
+      __syncwarp();  // every lane has read prev[w] before lane 0 clears it
       if (T::FRONTIER && lane == 0) marked += __popc(cw);
       if (((pw & ~cw) >> lane) & 1u) {  // updated last iteration, not this one: refresh parity p^1
         a.r[p ^ 1][v] = a.r[p][v];

@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kThreads, ModeTraits<MODE>::LOW_BLOCKS)
       if (FIRST) {
         if (T::FRONTIER && lane == 0) marked += __popc(cw);
         const uint32_t pw = prev[w];
+        __syncwarp();  // every lane has read prev[w] before lane 0 clears it
         if (((pw & ~cw) >> lane) & 1u) {  // updated last iteration, not this one: refresh parity p^1
           ranks_of<MODE>(a, p ^ 1)[v] = ranks_of<MODE>(a, p)[v];
           contribs_of<MODE>(a, p ^ 1)[v] = contribs_of<MODE>(a, p)[v];
