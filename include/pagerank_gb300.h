@@ -468,6 +468,11 @@ int prx_autotune(prx_context* ctx, prx_graph* g, const char* cache_path, prx_tun
  * the band where the two are closest. */
 int prx_selftest_division(prx_context* ctx, uint32_t dmax, uint32_t per, unsigned long long* mismatches);
 
+/* Diagnostic with no counterpart in the reference: the nth device allocation
+ * that the library makes for this thread from now on fails as if memory had
+ * run out (0: none).  Returns what was left of the count set before. */
+int64_t prx_selftest_fail_alloc(int64_t nth);
+
 /* Static FP64 PageRank that allocates no memory.  No counterpart in the
  * reference: it serves callers that may not allocate device memory behind
  * their own allocator (a serving process that reserves its HBM up front, a

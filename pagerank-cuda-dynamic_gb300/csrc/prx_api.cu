@@ -72,7 +72,7 @@ int prx_context_create(int device, prx_context** out) {
   c->device = device;
   cudaError_t e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&c->st, sizeof(State));
+  if (e == cudaSuccess) e = device_alloc(&c->st, sizeof(State));
   if (e == cudaSuccess) e = cudaMallocHost(&c->st_host, 2 * sizeof(State));
   for (int i = 0; i < 4 && e == cudaSuccess; ++i) e = cudaEventCreate(&c->ev[i]);
   if (e == cudaSuccess) e = degree_tables(&c->qtab, c->stream);
@@ -143,22 +143,22 @@ int ensure_ws(prx_context* c, uint32_t n, bool dyn) {
   free_ws(c);
   const size_t words = ((size_t)cap + 31) / 32;
   for (int p = 0; p < 2; ++p) {
-    TRY_CUDA_ST(cudaMalloc(&c->r[p], sizeof(double) * cap));
-    TRY_CUDA_ST(cudaMalloc(&c->c[p], sizeof(double) * cap));
+    TRY_CUDA_ST(device_alloc(&c->r[p], sizeof(double) * cap));
+    TRY_CUDA_ST(device_alloc(&c->c[p], sizeof(double) * cap));
   }
-  TRY_CUDA_ST(cudaMalloc(&c->acc64, sizeof(double) * cap));
-  TRY_CUDA_ST(cudaMalloc(&c->acc32, sizeof(float) * cap));
+  TRY_CUDA_ST(device_alloc(&c->acc64, sizeof(double) * cap));
+  TRY_CUDA_ST(device_alloc(&c->acc32, sizeof(float) * cap));
   if (want_dyn) {
-    TRY_CUDA_ST(cudaMalloc(&c->flags, cap));
-    for (auto& b : c->bm) TRY_CUDA_ST(cudaMalloc(&b, sizeof(uint32_t) * words));
-    for (auto& b : c->nf) TRY_CUDA_ST(cudaMalloc(&b, sizeof(uint32_t) * words));
-    TRY_CUDA_ST(cudaMalloc(&c->xb, sizeof(uint32_t) * cap));
-    TRY_CUDA_ST(cudaMalloc(&c->naff, sizeof(uint32_t) * words));
-    TRY_CUDA_ST(cudaMalloc(&c->ever, sizeof(uint32_t) * words));
-    TRY_CUDA_ST(cudaMalloc(&c->pf, sizeof(double) * ((size_t)cap + kPfTable)));  // + the per-degree table
-    TRY_CUDA_ST(cudaMalloc(&c->xl, sizeof(uint32_t) * cap));
-    for (auto& f : c->fr) TRY_CUDA_ST(cudaMalloc(&f, sizeof(uint32_t) * cap));
-    for (int k = MID; k < NCLS; ++k) TRY_CUDA_ST(cudaMalloc(&c->lists[0][k], sizeof(uint32_t) * cap));
+    TRY_CUDA_ST(device_alloc(&c->flags, cap));
+    for (auto& b : c->bm) TRY_CUDA_ST(device_alloc(&b, sizeof(uint32_t) * words));
+    for (auto& b : c->nf) TRY_CUDA_ST(device_alloc(&b, sizeof(uint32_t) * words));
+    TRY_CUDA_ST(device_alloc(&c->xb, sizeof(uint32_t) * cap));
+    TRY_CUDA_ST(device_alloc(&c->naff, sizeof(uint32_t) * words));
+    TRY_CUDA_ST(device_alloc(&c->ever, sizeof(uint32_t) * words));
+    TRY_CUDA_ST(device_alloc(&c->pf, sizeof(double) * ((size_t)cap + kPfTable)));  // + the per-degree table
+    TRY_CUDA_ST(device_alloc(&c->xl, sizeof(uint32_t) * cap));
+    for (auto& f : c->fr) TRY_CUDA_ST(device_alloc(&f, sizeof(uint32_t) * cap));
+    for (int k = MID; k < NCLS; ++k) TRY_CUDA_ST(device_alloc(&c->lists[0][k], sizeof(uint32_t) * cap));
   }
   c->ws_n = cap;
   c->ws_dyn = want_dyn;
@@ -169,7 +169,7 @@ int ensure_ch(prx_context* c, uint32_t hot_n) {
   if (c->ch_n >= hot_n) return PRX_OK;
   for (auto& h : c->ch) { cudaFree(h); h = nullptr; }
   c->ch_n = 0;
-  for (auto& h : c->ch) TRY_CUDA_ST(cudaMalloc(&h, sizeof(double) * hot_n));
+  for (auto& h : c->ch) TRY_CUDA_ST(device_alloc(&h, sizeof(double) * hot_n));
   c->ch_n = hot_n;
   return PRX_OK;
 }
@@ -183,10 +183,10 @@ static int ensure_ws32(prx_context* c, uint32_t n) {
     cudaFree(c->ce32[p]); c->ce32[p] = nullptr;
   }
   c->ws32_n = 0;
-  TRY_CUDA_ST(cudaMalloc(&c->rho, sizeof(float) * n));
+  TRY_CUDA_ST(device_alloc(&c->rho, sizeof(float) * n));
   for (int p = 0; p < 2; ++p) {
-    TRY_CUDA_ST(cudaMalloc(&c->e32[p], sizeof(float) * n));
-    TRY_CUDA_ST(cudaMalloc(&c->ce32[p], sizeof(float) * n));
+    TRY_CUDA_ST(device_alloc(&c->e32[p], sizeof(float) * n));
+    TRY_CUDA_ST(device_alloc(&c->ce32[p], sizeof(float) * n));
   }
   c->ws32_n = n;
   return PRX_OK;
@@ -197,7 +197,7 @@ static int ensure_batch(prx_context* c, size_t elems) {
   cudaFree(c->batch);
   c->batch = nullptr;
   c->batch_cap = 0;
-  TRY_CUDA_ST(cudaMalloc(&c->batch, sizeof(uint32_t) * std::max<size_t>(elems, 1024)));
+  TRY_CUDA_ST(device_alloc(&c->batch, sizeof(uint32_t) * std::max<size_t>(elems, 1024)));
   c->batch_cap = std::max<size_t>(elems, 1024);
   return PRX_OK;
 }
@@ -1017,7 +1017,7 @@ int prx_graph_create64(prx_context* c, uint32_t n, uint64_t m, const uint64_t* x
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the host arrays above are the caller's
     return e;
   };
-  cudaError_t e = cudaMalloc(&tmp, 8 * ((uint64_t)n + 1));
+  cudaError_t e = device_alloc(&tmp, 8 * ((uint64_t)n + 1));
   if (e == cudaSuccess) e = build(xtoff, xtedg, &g.xtoff, &g.xtedg, &g.xtbase, g.xtseg0, g.xtpos);
   if (e == cudaSuccess && xoff) e = build(xoff, xedg, &g.xoff, &g.xedg, &g.xbase, g.xseg0, g.xpos);
   if (e == cudaSuccess) e = graph_alloc(&g.xtdat, 4 * (uint64_t)(n ? n : 1), s);
@@ -1269,6 +1269,8 @@ int prx_solve_device(prx_context* c, prx_graph* gr, int mode, const uint32_t* du
                      double* ranks_out, prx_result* res) {
   return solve_common(c, gr, mode, du, dv, nd, iu, iv, ni, q, o, ranks_out, res, false);
 }
+
+int64_t prx_selftest_fail_alloc(int64_t nth) { return selftest_fail_alloc(nth); }
 
 int prx_selftest_division(prx_context* c, uint32_t dmax, uint32_t per, unsigned long long* mismatches) {
   if (!c || !mismatches) FAIL(PRX_EINVAL, "prx_selftest_division: bad context or NULL output");

@@ -42,15 +42,40 @@ cudaError_t pool_of(int dev, cudaMemPool_t* out) {
 }
 }  // namespace
 
+// The allocation of this thread that prx_selftest_fail_alloc makes fail, counted
+// down (0: none): it asks for more than any device has.
+static thread_local int64_t t_fail_alloc = 0;
+static size_t asked(size_t bytes) {
+  if (t_fail_alloc > 0 && --t_fail_alloc == 0) return (size_t)1 << 60;
+  return bytes ? bytes : 1;
+}
+int64_t selftest_fail_alloc(int64_t nth) {
+  const int64_t left = t_fail_alloc;
+  t_fail_alloc = nth;
+  return left;
+}
+
+// What an allocation that failed leaves: no pointer, and nothing for a later
+// cudaGetLastError to find.
+static cudaError_t allocated(cudaError_t e, void** p) {
+  if (e != cudaSuccess) {
+    *p = nullptr;
+    (void)cudaGetLastError();
+  }
+  return e;
+}
+
 cudaError_t graph_alloc(void** p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   cudaMemPool_t pool = nullptr;
   if (e == cudaSuccess) e = pool_of(dev, &pool);
-  if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, s);
-  return e;
+  if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, asked(bytes), pool, s);
+  return allocated(e, p);
 }
+
+cudaError_t device_alloc(void** p, size_t bytes) { return allocated(cudaMalloc(p, asked(bytes)), p); }
 
 void graph_free(std::initializer_list<void*> ps) {
   bool any = false;

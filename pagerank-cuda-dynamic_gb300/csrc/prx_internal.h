@@ -206,6 +206,7 @@ struct GraphDev {
   bool oplan_built = false, oplan_fits = false;
   uint32_t* tpos = nullptr;       // laid out like xedg; positions relative to the in-CSR's row segment
   bool tpos_built = false;
+  bool weights_set = false;       // px, pt, wsum (and wseg) hold the weights of this version
 };
 
 // Frees the edge weights of g (after a batch, or with the graph).
@@ -513,6 +514,14 @@ template <class T>
 cudaError_t graph_alloc(T** p, size_t bytes, cudaStream_t s) {
   return graph_alloc(reinterpret_cast<void**>(p), bytes, s);
 }
+// cudaMalloc for the arrays outside the pool; *p is null after a failure.
+cudaError_t device_alloc(void** p, size_t bytes);
+template <class T>
+cudaError_t device_alloc(T** p, size_t bytes) {
+  return device_alloc(reinterpret_cast<void**>(p), bytes);
+}
+// prx_selftest_fail_alloc.
+int64_t selftest_fail_alloc(int64_t nth);
 // Returns pool blocks (NULLs skipped) once all work queued on the device has
 // finished, like cudaFree; cudaFree itself would leave the pool counting the
 // blocks as in use.

@@ -791,7 +791,7 @@ static cudaError_t grow(T** p, size_t& cap, size_t want) {
   cudaFree(*p);
   *p = nullptr;
   cap = 0;
-  cudaError_t e = cudaMalloc(p, sizeof(T) * (want ? want : 1));
+  cudaError_t e = device_alloc(p, sizeof(T) * (want ? want : 1));
   if (e == cudaSuccess) cap = want;
   return e;
 }
@@ -812,14 +812,14 @@ static int ppr_ws(prx_context* c, uint32_t n, bool fp32) {
     w.n = 0;
     w.has32 = false;
     const size_t rows = (size_t)n * kCols;
-    for (int i = 0; i < 2; ++i) TRY_CUDA_ST(cudaMalloc(&w.x[i], sizeof(double) * rows));
-    TRY_CUDA_ST(cudaMalloc(&w.toff, sizeof(uint32_t) * ((size_t)n + 1)));
+    for (int i = 0; i < 2; ++i) TRY_CUDA_ST(device_alloc(&w.x[i], sizeof(double) * rows));
+    TRY_CUDA_ST(device_alloc(&w.toff, sizeof(uint32_t) * ((size_t)n + 1)));
     w.n = n;
   }
   if (fp32 && !w.has32) {
     const size_t rows = (size_t)w.n * kCols;
-    TRY_CUDA_ST(cudaMalloc(&w.rho, sizeof(float) * rows));
-    for (int i = 0; i < 2; ++i) TRY_CUDA_ST(cudaMalloc(&w.e[i], sizeof(float) * rows));
+    TRY_CUDA_ST(device_alloc(&w.rho, sizeof(float) * rows));
+    for (int i = 0; i < 2; ++i) TRY_CUDA_ST(device_alloc(&w.e[i], sizeof(float) * rows));
     w.has32 = true;
   }
   return PRX_OK;
@@ -1230,7 +1230,7 @@ int prx_autotune_ppr(prx_context* c, prx_graph* gr, prx_ppr_tune_result* out) {
   }
   off[nvec] = nvec;
   double* ranks = nullptr;
-  TRY_CUDA_ST(cudaMalloc(&ranks, sizeof(double) * (size_t)g.n * nvec));
+  TRY_CUDA_ST(device_alloc(&ranks, sizeof(double) * (size_t)g.n * nvec));
   prx_options o;
   prx_options_default(&o);
   o.precision = PRX_FP32_REFINE;

@@ -144,7 +144,7 @@ int prx_autotune(prx_context* c, prx_graph* gr, const char* cache_path, prx_tune
     return PRX_OK;
   }
   double* ranks = nullptr;
-  TRY_CUDA_ST(cudaMalloc(&ranks, sizeof(double) * g.n));
+  TRY_CUDA_ST(device_alloc(&ranks, sizeof(double) * g.n));
   int st = PRX_OK, trials = 0;
   g.tuned_int_adds = 0;  // steps 1-3 time with the library default
   // 1. MID / HIGH boundary, with the default chunk widths

@@ -42,7 +42,7 @@ void drop_weights(GraphDev& g) {
   g.px = g.pt = g.wsum = nullptr;
   g.wseg = nullptr;
   g.tpos = nullptr;
-  g.tpos_built = false;
+  g.tpos_built = g.weights_set = false;
 }
 
 struct PullArgs {
@@ -548,7 +548,7 @@ static int wk_grow(prx_context* c, size_t doubles) {
   cudaFree(c->wk);
   c->wk = nullptr;
   c->wk_cap = 0;
-  TRY_CUDA_ST(cudaMalloc(&c->wk, sizeof(double) * doubles));
+  TRY_CUDA_ST(device_alloc(&c->wk, sizeof(double) * doubles));
   c->wk_cap = doubles;
   return PRX_OK;
 }
@@ -654,43 +654,29 @@ static int weighted_check(prx_context* c, prx_graph* gr, const char* who) {
     set_error(std::string(who) + ": bad context or graph");
     return PRX_EINVAL;
   }
-  if (!gr->g.px) {
+  if (!gr->g.weights_set) {
     set_error(std::string(who) + ": graph has no edge weights (prx_graph_set_weights)");
     return PRX_ESTATE;
   }
   return PRX_OK;
 }
 
-static void opts_or_default(const prx_options* o, prx_options* out) {
-  if (o) *out = *o;
-  else prx_options_default(out);
-}
-
-extern "C" {
-
-int prx_graph_set_weights(prx_context* c, prx_graph* gr, const float* w) {
-  if (!c || !gr || gr->ctx != c) FAIL(PRX_EINVAL, "prx_graph_set_weights: bad context or graph");
-  GraphDev& g = gr->g;
-  if (!g.xoff) FAIL(PRX_ESTATE, "prx_graph_set_weights: graph has no out-CSR");
-  if (!w && g.m) FAIL(PRX_EINVAL, "prx_graph_set_weights: weights are NULL");
-  TRY_CUDA_ST(cudaSetDevice(c->device));
+static int set_weights(prx_context* c, GraphDev& g, const float* w) {
   cudaStream_t s = c->stream;
   // the arrays stay for the next weights of the same graph version (a batch drops them)
-  if (!g.px) {
-    TRY_CUDA_ST(cudaMalloc(&g.px, sizeof(double) * csr_slots(g, g.xseg0, g.xpos)));
-    TRY_CUDA_ST(cudaMalloc(&g.pt, sizeof(double) * csr_slots(g, g.xtseg0, g.xtpos)));
-    TRY_CUDA_ST(cudaMalloc(&g.wsum, sizeof(double) * (g.n ? g.n : 1)));
-    TRY_CUDA_ST(cudaMalloc(&g.tpos, sizeof(uint32_t) * csr_slots(g, g.xseg0, g.xpos)));
-    if (g.nseg > 1) {  // each out-CSR segment's compact start
-      TRY_CUDA_ST(cudaMalloc(&g.wseg, sizeof(unsigned long long) * g.nseg));
-      TRY_CUDA_ST(cudaMemcpyAsync(g.wseg, g.xseg0.data(), sizeof(unsigned long long) * g.nseg,
-                                  cudaMemcpyHostToDevice, s));
-    }
+  if (!g.px) TRY_CUDA_ST(device_alloc(&g.px, sizeof(double) * csr_slots(g, g.xseg0, g.xpos)));
+  if (!g.pt) TRY_CUDA_ST(device_alloc(&g.pt, sizeof(double) * csr_slots(g, g.xtseg0, g.xtpos)));
+  if (!g.wsum) TRY_CUDA_ST(device_alloc(&g.wsum, sizeof(double) * (g.n ? g.n : 1)));
+  if (!g.tpos) TRY_CUDA_ST(device_alloc(&g.tpos, sizeof(uint32_t) * csr_slots(g, g.xseg0, g.xpos)));
+  if (!g.wseg && g.nseg > 1) {  // each out-CSR segment's compact start
+    TRY_CUDA_ST(device_alloc(&g.wseg, sizeof(unsigned long long) * g.nseg));
+    TRY_CUDA_ST(cudaMemcpyAsync(g.wseg, g.xseg0.data(), sizeof(unsigned long long) * g.nseg, cudaMemcpyHostToDevice,
+                                s));
   }
   if (!g.oplan_built) {
     const size_t ids = sizeof(uint32_t) * (g.n ? g.n : 1);
-    if (!g.ocls_list) TRY_CUDA_ST(cudaMalloc(&g.ocls_list, ids));
-    if (!g.oplan_list) TRY_CUDA_ST(cudaMalloc(&g.oplan_list, ids));
+    if (!g.ocls_list) TRY_CUDA_ST(device_alloc(&g.ocls_list, ids));
+    if (!g.oplan_list) TRY_CUDA_ST(device_alloc(&g.oplan_list, ids));
     uint64_t padded = 0, edges[NCLS];
     TRY_CUDA_ST(build_class_lists(g.xoff, g.seg_shift, g.n, g.mid_max, g.ocls_list, g.ocls_begin, g.ocls_edges,
                                   c->sms, s, &padded));
@@ -722,13 +708,30 @@ int prx_graph_set_weights(prx_context* c, prx_graph* gr, const float* w) {
   TRY_CUDA_ST(cudaMemcpyAsync(&c->st_host[1], c->st, sizeof(State), cudaMemcpyDeviceToHost, s));
   TRY_CUDA_ST(cudaStreamSynchronize(s));
   const uint32_t err = c->st_host[1].err;
-  if (err) {
-    drop_weights(g);
-    if (err & 1u) FAIL(PRX_EINVAL, "prx_graph_set_weights: every weight must be positive and finite");
-    FAIL(PRX_EINVAL, "prx_graph_set_weights: an out-edge is missing from the in-CSR");
-  }
+  if (err & 1u) FAIL(PRX_EINVAL, "prx_graph_set_weights: every weight must be positive and finite");
+  if (err) FAIL(PRX_EINVAL, "prx_graph_set_weights: an out-edge is missing from the in-CSR");
   g.tpos_built = true;
   return PRX_OK;
+}
+
+static void opts_or_default(const prx_options* o, prx_options* out) {
+  if (o) *out = *o;
+  else prx_options_default(out);
+}
+
+extern "C" {
+
+int prx_graph_set_weights(prx_context* c, prx_graph* gr, const float* w) {
+  if (!c || !gr || gr->ctx != c) FAIL(PRX_EINVAL, "prx_graph_set_weights: bad context or graph");
+  GraphDev& g = gr->g;
+  if (!g.xoff) FAIL(PRX_ESTATE, "prx_graph_set_weights: graph has no out-CSR");
+  if (!w && g.m) FAIL(PRX_EINVAL, "prx_graph_set_weights: weights are NULL");
+  TRY_CUDA_ST(cudaSetDevice(c->device));
+  g.weights_set = false;
+  const int st = set_weights(c, g, w);
+  if (st) drop_weights(g);  // whatever failed: no weights, and nothing half allocated for the next call to use
+  else g.weights_set = true;
+  return st;
 }
 
 int prx_solve_weighted(prx_context* c, prx_graph* gr, const double* t, const double* r0, const prx_options* opt,

@@ -416,6 +416,12 @@ def selftest_division(ctx, dmax, per):
     return bad.value
 
 
+def selftest_fail_alloc(nth):
+    """Make this thread's nth device allocation from now on fail (0: none);
+    returns what was left of the count set before."""
+    return load().prx_selftest_fail_alloc(int(nth))
+
+
 # ---- the reference's five entry points ------------------------------------
 def pagerank_static(ctx, g, opts=None):
     return solve(ctx, g, _lib.STATIC, opts=opts)
