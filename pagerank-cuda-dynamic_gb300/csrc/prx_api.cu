@@ -607,11 +607,11 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   // contributions
   // A small or medium graph runs its FP64 loop as one cooperative kernel on
   // the plain rows (no hot copy, no source chunks); see launch_persist.
-  const bool persist = (!refine || (!dyn && o.max_iterations > 0 && g.mid_max >= kPlanMid)) &&
-                       o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase &&
-                       g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) && persist_fits(g) &&
-                       (mixed_lengths(g) || !words_fit(g) || (uint64_t)g.n <= 32 * kPersistWordUnits);
-  if (persist) TRY_CUDA_ST(ensure_plan(gr->g, c->sms, c->stream));
+  bool persist = (!refine || (!dyn && o.max_iterations > 0 && g.mid_max >= kPlanMid)) &&
+                 o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase &&
+                 g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) && persist_fits(g) &&
+                 (mixed_lengths(g) || !words_fit(g) || (uint64_t)g.n <= 32 * kPersistWordUnits);
+  if (persist) TRY_CUDA_ST(ensure_plan(gr->g, c->sms, c->stream, &persist));
   // one chunk: the LOW rows by words where rows are long.  A refined solve has
   // its FP32 sweeps read them too, so without hot sources; contributions that L2
   // holds anyway (64 MB) do without unless they are asked for (Static, web-like

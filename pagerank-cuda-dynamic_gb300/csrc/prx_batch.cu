@@ -452,9 +452,8 @@ cudaError_t batch_by_target(const uint32_t* u, const uint32_t* v, uint32_t count
   if (e == cudaSuccess) e = radix_sort_u64(key, tmp, count, 32, 32 + vbits, hist, sms, s, &sorted);
   if (e == cudaSuccess) k_target_split<<<grid, kThreads, 0, s>>>(sorted, count, tk, tv);
   if (e == cudaSuccess) e = cudaGetLastError();
-  cudaFreeAsync(key, s);
-  cudaFreeAsync(tmp, s);
-  cudaFreeAsync(hist, s);
+  for (void* p : {(void*)key, (void*)tmp, (void*)hist})
+    if (p) cudaFreeAsync(p, s);
   return e;
 }
 
@@ -634,16 +633,20 @@ cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd64, ui
       if (ws) cudaFreeAsync(ws, s);
       if (el != cudaSuccess) {
         graph_free({lo, le});
-        err = el;
-        goto done;
+        lo = le = nullptr;
+        if (el != cudaErrorMemoryAllocation) {
+          err = el;
+          goto done;
+        }
       }
-      layouts_new.push_back({&l, lo, le});
+      layouts_new.push_back({&l, lo, le});  // null: no memory, the next solve that wants it builds it
     }
   }
   PRX_CU(cudaGetLastError());
   PRX_CU(cudaStreamSynchronize(s));
   for (auto& x : layouts_new) {
     graph_free({x.l->off, x.l->edg});
+    if (!x.off) *x.l = ChunkLayout();
     x.l->off = x.off;
     x.l->edg = x.edg;
   }

@@ -1022,7 +1022,7 @@ cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s) {
   return e;
 }
 
-cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s) {
+static cudaError_t build_plan(GraphDev& g, int sms, cudaStream_t s) {
   if (g.n == 0) return cudaSuccess;
   if (mixed_lengths(g)) {
     const cudaError_t e = ensure_len_list(g, sms, s);
@@ -1038,6 +1038,21 @@ cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s) {
     e = sort_by_length(g.xtoff, g.seg_shift, mid, g.plan_begin[HIGH] - g.plan_begin[MID], kPlanMid, mid, sms, s);
   g.plan_built = e == cudaSuccess;
   return e;
+}
+
+cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s, bool* have) {
+  const cudaError_t e = build_plan(g, sms, s);
+  *have = e == cudaSuccess;
+  if (e != cudaErrorMemoryAllocation) return e;
+  if (!g.plan_built) {
+    graph_free({g.plan_list});
+    g.plan_list = nullptr;
+  }
+  if (!g.len_built) {
+    graph_free({g.len_list});
+    g.len_list = nullptr;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, uint32_t mid_max, uint32_t* list,

@@ -197,10 +197,11 @@ struct GraphDev {
   // of the out-CSR, built on the first weights of a graph version: ids by
   // row-length class with mid_max and (oplan) with kPlanMid as the MID / HIGH
   // boundary, LOW ids by length where they mix; each out-edge's position among
-  // the in-edges
+  // the in-edges.  Without memory for them the weights do with ocls and searches.
   uint32_t* ocls_list = nullptr;
   uint32_t ocls_begin[NCLS + 1] = {0, 0, 0, 0};
   uint64_t ocls_edges[NCLS] = {0, 0, 0};
+  uint32_t ocls_mid = 0;          // the mid_max they were built with
   uint32_t* oplan_list = nullptr;
   uint32_t oplan_begin[NCLS + 1] = {0, 0, 0, 0};
   bool oplan_built = false, oplan_fits = false;
@@ -335,9 +336,11 @@ inline bool mixed_lengths(const GraphDev& g) { return g.low_padded > 2 * g.cls_e
 // first (ties in the given order), into out (may be list).
 cudaError_t sort_by_length(const uint32_t* off, uint32_t shift, const uint32_t* list, uint32_t count, uint32_t top,
                            uint32_t* out, int sms, cudaStream_t s);
-// GraphDev::len_list, and the persistent loop's rows: plan_list,
-// and len_list where the lengths mix.
-cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s);
+cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s);  // GraphDev::len_list
+// The persistent loop's rows: plan_list, and len_list where the lengths mix.
+// *have: they are there; not so when there is no memory for them (the sweeps
+// are launched class by class then).
+cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s, bool* have);
 constexpr uint32_t kPlanMid = 1024;
 // Largest graphs it takes, in units of a MID row or 32 LOW rows: in id order
 // and by length.
@@ -356,7 +359,6 @@ inline bool plan_fits(uint32_t n, uint32_t low, bool mixed) {
 // what is gained at 1.1M.
 constexpr uint64_t kPersistWordUnits = 32u << 10;
 inline bool persist_fits(const GraphDev& g) { return plan_fits(g.n, g.cls_begin[MID], mixed_lengths(g)); }
-cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s);
 // The whole FP64 iteration loop of a plain graph (one row segment) as one
 // cooperative kernel from the ranks in parity 0 (prx_persist.cu); ensure_plan
 // first.

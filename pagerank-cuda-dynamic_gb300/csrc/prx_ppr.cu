@@ -1153,9 +1153,14 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   a.per = a.seg / kSegParts;
   if ((st = ppr_segments(c, g, a))) return st;
   // The LOW rows in order of length (rows side by side in a warp then end
-  // together); by id with another bound or with row segments.
-  const bool by_length = a.low_max == kLowMax && g.nseg == 1;
-  if (by_length) TRY_CUDA_ST(ensure_len_list(gr->g, c->sms, s));
+  // together); by id with another bound, with row segments, or without memory
+  // for the list.
+  bool by_length = a.low_max == kLowMax && g.nseg == 1;
+  if (by_length) {
+    const cudaError_t e = ensure_len_list(gr->g, c->sms, s);
+    if (e != cudaErrorMemoryAllocation) TRY_CUDA_ST(e);
+    by_length = e == cudaSuccess;
+  }
   a.rows = by_length ? g.len_list : nullptr;
   a.nrows = by_length ? g.cls_begin[MID] : g.n;
   a.flat = !mixed_lengths(g);

@@ -351,7 +351,7 @@ struct WeightCsr {
   const uint32_t *xoff, *xedg, *xtoff, *xtedg;
   const unsigned long long *xbase, *xtbase, *wseg;
   uint32_t shift;
-  uint32_t* tpos;   // GraphDev::tpos
+  uint32_t* tpos;   // GraphDev::tpos (null: no memory for it, every call searches)
 };
 
 // p = w / W_u of an out-edge to its places in px and pt; its position among
@@ -376,7 +376,7 @@ __device__ __forceinline__ void put_weight(const WeightCsr& c, uint32_t u, uint6
   }
   if (lo < end && row[lo] == u) {
     pt[bv + lo] = p;
-    c.tpos[at] = lo;
+    if (c.tpos) c.tpos[at] = lo;
   } else {
     atomicOr(err, 2u);
   }
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(256) k_weight_edges(WeightCsr c, const float* 
 
 // ---- gradients -------------------------------------------------------------------
 // dL/dw_uv = (r_u / W_u) (alpha lambda_v - lambda_u + g_u): a warp per source
-// of up to kPlanMid edges, the pieces of the longer rows (list) by block as in
+// of up to mid_max edges, the pieces of the longer rows (list) by block as in
 // k_weight_edges.
 __device__ __forceinline__ void grad_row(const WeightCsr& cs, uint32_t u, uint32_t first, uint32_t step,
                                          const double* __restrict__ wsum, const double* __restrict__ r,
@@ -497,9 +497,9 @@ __device__ __forceinline__ void grad_row(const WeightCsr& cs, uint32_t u, uint32
 __global__ void __launch_bounds__(256) k_grad_w(WeightCsr cs, const double* __restrict__ wsum,
                                                 const double* __restrict__ r, const double* __restrict__ lam,
                                                 const double* __restrict__ g, double alpha, uint32_t n,
-                                                double* __restrict__ out) {
+                                                uint32_t mid_max, double* __restrict__ out) {
   for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += (gridDim.x * blockDim.x) >> 5)
-    if (row_len(cs.xoff, cs.shift, u) <= kPlanMid) grad_row(cs, u, lane_id(), 32, wsum, r, lam, g, alpha, out);
+    if (row_len(cs.xoff, cs.shift, u) <= mid_max) grad_row(cs, u, lane_id(), 32, wsum, r, lam, g, alpha, out);
 }
 __global__ void __launch_bounds__(256) k_grad_w_long(WeightCsr cs, const uint32_t* __restrict__ list,
                                                      const double* __restrict__ wsum, const double* __restrict__ r,
@@ -565,6 +565,36 @@ static uint64_t csr_slots(const GraphDev& g, const std::vector<uint64_t>& seg0, 
 
 // Blocks per long row of k_weight_edges and k_grad_w_long.
 constexpr int kLongPieces = 8;
+
+// The out-rows by class that the weights and their gradients go by: oplan_list,
+// or ocls_list when there was no memory for it.
+struct OutRows {
+  const uint32_t *list, *begin;
+  uint32_t mid_max;
+};
+static OutRows out_rows(const GraphDev& g) {
+  return g.oplan_built ? OutRows{g.oplan_list, g.oplan_begin, kPlanMid}
+                       : OutRows{g.ocls_list, g.ocls_begin, g.ocls_mid};
+}
+
+// GraphDev::oplan_list, its order and oplan_fits; ocls_list is there.
+static cudaError_t build_out_plan(GraphDev& g, uint64_t padded, int sms, cudaStream_t s) {
+  cudaError_t e = g.oplan_list ? cudaSuccess : device_alloc(&g.oplan_list, sizeof(uint32_t) * (g.n ? g.n : 1));
+  uint64_t edges[NCLS] = {0, 0, 0};
+  if (e == cudaSuccess)
+    e = build_class_lists(g.xoff, g.seg_shift, g.n, kPlanMid, g.oplan_list, g.oplan_begin, edges, sms, s);
+  const bool mixed = padded > 2 * edges[LOW];  // as for the in-edges
+  if (e == cudaSuccess && mixed)
+    e = sort_by_length(g.xoff, g.seg_shift, g.ocls_list, g.ocls_begin[MID], kLowMax, g.oplan_list, sms, s);
+  if (e == cudaSuccess) {
+    uint32_t* mid_rows = g.oplan_list + g.oplan_begin[MID];
+    e = sort_by_length(g.xoff, g.seg_shift, mid_rows, g.oplan_begin[HIGH] - g.oplan_begin[MID], kPlanMid, mid_rows,
+                       sms, s);
+  }
+  g.oplan_fits = plan_fits(g.n, g.oplan_begin[MID], mixed);
+  g.oplan_built = e == cudaSuccess;
+  return e;
+}
 
 // The persistent loop's rows of a, for graphs up to the lines of persist_fits.
 static void take_plan(PullArgs& a, const uint32_t* list, const uint32_t* low, const uint32_t begin[NCLS + 1]) {
@@ -667,38 +697,34 @@ static int set_weights(prx_context* c, GraphDev& g, const float* w) {
   if (!g.px) TRY_CUDA_ST(device_alloc(&g.px, sizeof(double) * csr_slots(g, g.xseg0, g.xpos)));
   if (!g.pt) TRY_CUDA_ST(device_alloc(&g.pt, sizeof(double) * csr_slots(g, g.xtseg0, g.xtpos)));
   if (!g.wsum) TRY_CUDA_ST(device_alloc(&g.wsum, sizeof(double) * (g.n ? g.n : 1)));
-  if (!g.tpos) TRY_CUDA_ST(device_alloc(&g.tpos, sizeof(uint32_t) * csr_slots(g, g.xseg0, g.xpos)));
+  if (!g.tpos) {
+    const cudaError_t e = device_alloc(&g.tpos, sizeof(uint32_t) * csr_slots(g, g.xseg0, g.xpos));
+    if (e != cudaErrorMemoryAllocation) TRY_CUDA_ST(e);
+  }
   if (!g.wseg && g.nseg > 1) {  // each out-CSR segment's compact start
     TRY_CUDA_ST(device_alloc(&g.wseg, sizeof(unsigned long long) * g.nseg));
     TRY_CUDA_ST(cudaMemcpyAsync(g.wseg, g.xseg0.data(), sizeof(unsigned long long) * g.nseg, cudaMemcpyHostToDevice,
                                 s));
   }
   if (!g.oplan_built) {
-    const size_t ids = sizeof(uint32_t) * (g.n ? g.n : 1);
-    if (!g.ocls_list) TRY_CUDA_ST(device_alloc(&g.ocls_list, ids));
-    if (!g.oplan_list) TRY_CUDA_ST(device_alloc(&g.oplan_list, ids));
-    uint64_t padded = 0, edges[NCLS];
+    if (!g.ocls_list) TRY_CUDA_ST(device_alloc(&g.ocls_list, sizeof(uint32_t) * (g.n ? g.n : 1)));
+    uint64_t padded = 0;
     TRY_CUDA_ST(build_class_lists(g.xoff, g.seg_shift, g.n, g.mid_max, g.ocls_list, g.ocls_begin, g.ocls_edges,
                                   c->sms, s, &padded));
-    TRY_CUDA_ST(build_class_lists(g.xoff, g.seg_shift, g.n, kPlanMid, g.oplan_list, g.oplan_begin, edges, c->sms, s));
-    const bool mixed = padded > 2 * edges[LOW];  // as for the in-edges
-    if (mixed)
-      TRY_CUDA_ST(sort_by_length(g.xoff, g.seg_shift, g.ocls_list, g.ocls_begin[MID], kLowMax, g.oplan_list, c->sms, s));
-    uint32_t* mid_rows = g.oplan_list + g.oplan_begin[MID];
-    TRY_CUDA_ST(sort_by_length(g.xoff, g.seg_shift, mid_rows, g.oplan_begin[HIGH] - g.oplan_begin[MID], kPlanMid,
-                               mid_rows, c->sms, s));
-    g.oplan_fits = plan_fits(g.n, g.oplan_begin[MID], mixed);
-    g.oplan_built = true;
+    g.ocls_mid = g.mid_max;
+    const cudaError_t e = build_out_plan(g, padded, c->sms, s);
+    if (e != cudaErrorMemoryAllocation) TRY_CUDA_ST(e);
   }
   launch_state_reset(c->st, 0, 0.0, s);
   if (g.n) {
     const bool found = g.tpos_built;
-    const WeightRows by_class = {g.oplan_list, g.oplan_begin[MID], g.oplan_begin[HIGH] - g.oplan_begin[MID]};
+    const OutRows out = out_rows(g);
+    const WeightRows by_class = {out.list, out.begin[MID], out.begin[HIGH] - out.begin[MID]};
     const uint64_t units = by_class.nmid + (by_class.nlow + 31ull) / 32;
     k_set_weights<<<pull_grid(units * 32, 256, c->sms * 8), 256, 0, s>>>(weight_csr(g), by_class, w, found, g.wsum,
                                                                          g.px, g.pt, &c->st->err);
-    if (const uint32_t nl = g.oplan_begin[NCLS] - g.oplan_begin[HIGH]) {
-      const uint32_t* rows = g.oplan_list + g.oplan_begin[HIGH];
+    if (const uint32_t nl = out.begin[NCLS] - out.begin[HIGH]) {
+      const uint32_t* rows = out.list + out.begin[HIGH];
       k_weight_sums<<<nl, 256, 0, s>>>(weight_csr(g), w, rows, g.wsum, &c->st->err);
       k_weight_edges<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), w, rows, found, g.wsum, g.px, g.pt,
                                                           &c->st->err);
@@ -710,7 +736,7 @@ static int set_weights(prx_context* c, GraphDev& g, const float* w) {
   const uint32_t err = c->st_host[1].err;
   if (err & 1u) FAIL(PRX_EINVAL, "prx_graph_set_weights: every weight must be positive and finite");
   if (err) FAIL(PRX_EINVAL, "prx_graph_set_weights: an out-edge is missing from the in-CSR");
-  g.tpos_built = true;
+  g.tpos_built = g.tpos != nullptr;
   return PRX_OK;
 }
 
@@ -752,10 +778,9 @@ int prx_solve_weighted(prx_context* c, prx_graph* gr, const double* t, const dou
   if ((st = wk_grow(c, 2 * (size_t)g.n))) return st;
   cudaStream_t s = c->stream;
   PullArgs a = forward_args(g, t, o.damping);
-  if (persist_fits(g)) {
-    TRY_CUDA_ST(ensure_plan(gr->g, c->sms, s));
-    take_plan(a, g.plan_list, mixed_lengths(g) ? g.len_list : g.plan_list, g.plan_begin);
-  }
+  bool plan = persist_fits(g);
+  if (plan) TRY_CUDA_ST(ensure_plan(gr->g, c->sms, s, &plan));
+  if (plan) take_plan(a, g.plan_list, mixed_lengths(g) ? g.len_list : g.plan_list, g.plan_begin);
   a.x[0] = c->wk;
   a.x[1] = c->wk + g.n;
   const uint64_t l0 = c->launches;
@@ -812,7 +837,7 @@ int prx_adjoint(prx_context* c, prx_graph* gr, const double* t, const double* r,
   a.shift = g.seg_shift;
   a.list = g.ocls_list;
   for (int k = 0; k <= NCLS; ++k) a.begin[k] = g.ocls_begin[k];
-  if (g.oplan_fits) take_plan(a, g.oplan_list, g.oplan_list, g.oplan_begin);
+  if (g.oplan_built && g.oplan_fits) take_plan(a, g.oplan_list, g.oplan_list, g.oplan_begin);
   a.base = gl;
   a.base_scale = 1.0;
   a.alpha = alpha;
@@ -830,11 +855,12 @@ int prx_adjoint(prx_context* c, prx_graph* gr, const double* t, const double* r,
   if (lambda) TRY_CUDA_ST(cudaMemcpyAsync(lambda, lam, sizeof(double) * g.n, cudaMemcpyDeviceToDevice, s));
   const int grid = pull_grid((uint64_t)g.n * 32, 256, c->sms * 16);
   if (grad_w) {
-    k_grad_w<<<grid, 256, 0, s>>>(weight_csr(g), g.wsum, r, lam, gl, alpha, g.n, grad_w);
+    const OutRows out = out_rows(g);
+    k_grad_w<<<grid, 256, 0, s>>>(weight_csr(g), g.wsum, r, lam, gl, alpha, g.n, out.mid_max, grad_w);
     c->launches += 1;
-    if (const uint32_t nl = g.oplan_begin[NCLS] - g.oplan_begin[HIGH]) {
-      k_grad_w_long<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), g.oplan_list + g.oplan_begin[HIGH], g.wsum, r,
-                                                         lam, gl, alpha, grad_w);
+    if (const uint32_t nl = out.begin[NCLS] - out.begin[HIGH]) {
+      k_grad_w_long<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), out.list + out.begin[HIGH], g.wsum, r, lam, gl,
+                                                         alpha, grad_w);
       c->launches += 1;
     }
   }
