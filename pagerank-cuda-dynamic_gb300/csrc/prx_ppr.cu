@@ -68,7 +68,7 @@ struct PprWs {
   double* x[2] = {nullptr, nullptr};   // FP64 ranks, [n][64], ping-pong (refinement: base, sweep output)
   float* rho = nullptr;                // FP32 refinement: residual [n][64]
   float* e[2] = {nullptr, nullptr};    // FP32 corrections, ping-pong
-  double* part = nullptr;              // partial rows of the long rows' parts [nparts][C]
+  double* part = nullptr;              // partial rows of the long rows' parts (or segments) [nparts][C]
   size_t part_cap = 0;
   uint2* parts = nullptr;              // vertex, first edge
   size_t parts_cap = 0;
@@ -80,7 +80,7 @@ struct PprWs {
   uint32_t* tent = nullptr;            // entries: vertex, column (sorted)
   double* tmass = nullptr;             // entry mass 1/|S_k|
   size_t t_cap = 0, tm_cap = 0;
-  uint2* pair = nullptr;               // the graph's in-edges as pairs (PprArgs::pair), for one call
+  uint2* pair = nullptr;               // the graph's in-edges as pairs (PprArgs::pair), for one FP32 call
   size_t pair_cap = 0;
   double* out = nullptr;               // device staging of the host output
   size_t out_cap = 0;
@@ -114,6 +114,7 @@ struct PprArgs {
   const float* rcp32;
   const uint32_t* xtedg;
   const uint2* pair;              // per in-edge, laid out like xtedg: source, bits of its FP32 reciprocal out-degree
+                                  // (FP32 sweeps; null: no memory for it, they read ids and gather reciprocals)
   const uint32_t* toff;
   const uint32_t* tcol;           // column of each teleport entry
   const double* tmass;
@@ -125,10 +126,11 @@ struct PprArgs {
   uint32_t low_max;               // rows up to this in-degree: one warp per vertex
   uint32_t seg;                   // in-edges per segment of a longer row (a multiple of kSegParts)
   uint32_t per;                   // in-edges per part: seg / kSegParts
-  const uint32_t* partstart;      // [nbig + 1]: each long row's first part
+  uint32_t group;                 // partial rows a segment: kSegParts, or 1 when there is no memory for its parts'
+  const uint32_t* partstart;      // [nbig + 1]: each long row's first partial row
   const uint2* parts;             // vertex, first edge (relative to its row segment)
   uint32_t nparts;
-  double* part;                   // the parts' partial rows
+  double* part;                   // the partial rows
   State* st;
   uint32_t n;
   const uint32_t* rows;           // the vertices of the short rows in the order they are taken (null: by id)
@@ -212,23 +214,42 @@ __device__ __forceinline__ const typename PprType<MODE>::S* ppr_src(const PprArg
   else if constexpr (MODE == PPR_R64) return a.x[0];
   else return a.e[st->k32 & 1];
 }
-// acc += row(u) / outdeg(u) over the edges [s, s + len) of pair, by the LPR
-// lanes of a row (every lane of the warp calls it; rows may differ in
-// length), one edge after the other.  A pair is an edge's source and the bits
-// of its FP32 reciprocal, read by all lanes of the row at once: for the FP32
-// sweeps, which the L1 bounds, half the wavefronts of an id, a reciprocal
-// gather and the row.  first: the pairs of the first U edges, loaded by the
-// caller.  Up to U rows are in flight.
-template <int MODE, int C>
-__device__ __forceinline__ void ppr_pairs(const uint2* __restrict__ ed, uint32_t len, uint2 pr[PprShape<MODE, C>::U]) {
-#pragma unroll
-  for (int k = 0; k < PprShape<MODE, C>::U; ++k) pr[k] = (uint32_t)k < len ? __ldg(ed + k) : make_uint2(0, 0);
+// An in-edge as a sweep reads it, by all lanes of its row at once: with PAIRS
+// (the FP32 sweeps, which the L1 bounds) the source and the bits of its FP32
+// reciprocal, half the wavefronts of an id, a reciprocal gather and the row;
+// else the source's id.
+template <bool PAIRS> struct PprEdge {
+  using T = uint32_t;
+  __device__ static __forceinline__ const T* base(const PprArgs& a) { return a.xtedg; }
+  __device__ static __forceinline__ T none() { return 0; }
+  __device__ static __forceinline__ uint32_t source(T e) { return e; }
+};
+template <> struct PprEdge<true> {
+  using T = uint2;
+  __device__ static __forceinline__ const T* base(const PprArgs& a) { return a.pair; }
+  __device__ static __forceinline__ T none() { return make_uint2(0, 0); }
+  __device__ static __forceinline__ uint32_t source(T e) { return e.x; }
+};
+// The reciprocals of a mode's precision.
+template <int MODE>
+__device__ __forceinline__ const typename PprType<MODE>::S* ppr_rcp(const PprArgs& a) {
+  if constexpr (MODE == PPR_S32) return a.rcp32;
+  else return a.rcp;
 }
-template <int MODE, int C>
+// acc += row(u) / outdeg(u) over the len edges at ed, by the LPR lanes of a row
+// (every lane of the warp calls it; rows may differ in length), one edge after
+// the other.  pr: the first U edges, loaded by the caller (ppr_edges).  Up to U
+// rows are in flight.
+template <int MODE, int C, bool PAIRS, class T>
+__device__ __forceinline__ void ppr_edges(const T* __restrict__ ed, uint32_t len, T pr[PprShape<MODE, C>::U]) {
+#pragma unroll
+  for (int k = 0; k < PprShape<MODE, C>::U; ++k) pr[k] = (uint32_t)k < len ? __ldg(ed + k) : PprEdge<PAIRS>::none();
+}
+template <int MODE, int C, bool PAIRS, class T>
 __device__ __forceinline__ void ppr_gather(const typename PprType<MODE>::S* __restrict__ src,
-                                           const double* __restrict__ rcp, const uint2* __restrict__ ed, uint32_t len,
-                                           uint2 pr[PprShape<MODE, C>::U], uint32_t sub,
-                                           typename PprShape<MODE, C>::V& acc) {
+                                           const typename PprType<MODE>::S* __restrict__ rcp,
+                                           const T* __restrict__ ed, uint32_t len, T pr[PprShape<MODE, C>::U],
+                                           uint32_t sub, typename PprShape<MODE, C>::V& acc) {
   using Sh = PprShape<MODE, C>;
   using S = typename Sh::S;
   using V = typename Sh::V;
@@ -240,16 +261,17 @@ __device__ __forceinline__ void ppr_gather(const typename PprType<MODE>::S* __re
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       if (base + k < len) {
-        g[k] = Sh::template load<true>(src, pr[k].x, sub);
-        if constexpr (MODE == PPR_S32) w[k] = __uint_as_float(pr[k].y);
-        else w[k] = __ldg(rcp + pr[k].x);
+        const uint32_t u = PprEdge<PAIRS>::source(pr[k]);
+        g[k] = Sh::template load<true>(src, u, sub);
+        if constexpr (PAIRS) w[k] = __uint_as_float(pr[k].y);
+        else w[k] = __ldg(rcp + u);
       } else {  // + 0 * 0 leaves the sum
 #pragma unroll
         for (int i = 0; i < Sh::N; ++i) g[k][i] = S(0);
         w[k] = S(0);
       }
     }
-    if (base + U < longest) ppr_pairs<MODE, C>(ed + base + U, len > base + U ? len - base - U : 0u, pr);
+    if (base + U < longest) ppr_edges<MODE, C, PAIRS>(ed + base + U, len > base + U ? len - base - U : 0u, pr);
     auto add = [&](int k) {
 #pragma unroll
       for (int i = 0; i < Sh::N; ++i) acc[i] = fma(g[k][i], w[k], acc[i]);
@@ -370,10 +392,11 @@ __device__ __forceinline__ void ppr_reduce(State* st, unsigned long long dmax, u
 // One sweep's rows.  A warp takes units: first G parts of long rows (partial
 // sums of a.per in-edges each, added up by k_ppr_combine), then batches of
 // short rows (in-degree <= low_max), LPR lanes per vertex and G vertices side
-// by side; a batch's bounds are loaded by a lane each, and the first pairs of
+// by side; a batch's bounds are loaded by a lane each, and the first edges of
 // the next G vertices while it sums these.  No warp waits for another.
-template <int MODE, int C>
+template <int MODE, int C, bool PAIRS>
 __global__ void __launch_bounds__(256, PprShape<MODE, C>::BLOCKS) k_ppr_rows(PprArgs a) {
+  using Ed = PprEdge<PAIRS>;
   using Sh = PprShape<MODE, C>;
   using S = typename Sh::S;
   using V = typename Sh::V;
@@ -382,6 +405,7 @@ __global__ void __launch_bounds__(256, PprShape<MODE, C>::BLOCKS) k_ppr_rows(Ppr
   State* st = a.st;
   if (ppr_skip<MODE>(st)) return;
   const S* __restrict__ src = ppr_src<MODE>(a, st);
+  const S* __restrict__ rcp = ppr_rcp<MODE>(a);
   const uint32_t lane = lane_id(), sub = lane % LPR, grp = lane / LPR;
   unsigned long long dmax = 0;
   unsigned int emag = 0;
@@ -402,7 +426,7 @@ __global__ void __launch_bounds__(256, PprShape<MODE, C>::BLOCKS) k_ppr_rows(Ppr
     else if (lane == 0) next = atomicAdd(&st->work, 1u);
   };
   if (!a.share) take();
-  uint2 pr[U];
+  typename Ed::T pr[U];
   for (;;) {
     const uint32_t b = __shfl_sync(0xffffffffu, next, 0);
     if (b >= np + nb) break;
@@ -410,17 +434,17 @@ __global__ void __launch_bounds__(256, PprShape<MODE, C>::BLOCKS) k_ppr_rows(Ppr
     if (b < np) {
       const uint32_t i = b * G + grp;
       uint32_t len = 0;
-      const uint2* ed = a.pair;
+      const typename Ed::T* ed = Ed::base(a);
       if (i < a.nparts) {
         const uint2 w = __ldg(a.parts + i);  // vertex, first edge
         const uint32_t end = __ldg(a.xtoff + seg_index(w.x, a.seg_shift) + 1);
         len = min(a.per, end - w.y);
         ed += w.y + (a.xtbase ? a.xtbase[(uint64_t)w.x >> a.seg_shift] : 0ull);
       }
-      ppr_pairs<MODE, C>(ed, len, pr);
+      ppr_edges<MODE, C, PAIRS>(ed, len, pr);
       V acc;
       zero(acc);
-      ppr_gather<MODE, C>(src, a.rcp, ed, len, pr, sub, acc);
+      ppr_gather<MODE, C, PAIRS>(src, rcp, ed, len, pr, sub, acc);
       if (i < a.nparts) Sh::store(reinterpret_cast<S*>(a.part), i, sub, acc);
       continue;
     }
@@ -437,21 +461,21 @@ __global__ void __launch_bounds__(256, PprShape<MODE, C>::BLOCKS) k_ppr_rows(Ppr
     }
     const uint32_t cnt = min(a.batch, a.nrows - i0);
     uint32_t v, len;
-    const uint2* ed;
+    const typename Ed::T* ed;
     auto fetch = [&](uint32_t i) {  // vertex i + grp of the batch and its first edges
       const uint32_t k = i + grp;
       v = __shfl_sync(0xffffffffu, mv, k & 31);
-      ed = a.pair + __shfl_sync(0xffffffffu, ms, k & 31);
+      ed = Ed::base(a) + __shfl_sync(0xffffffffu, ms, k & 31);
       len = __shfl_sync(0xffffffffu, ml, k & 31);
       if (k >= cnt) len = 0xffffffffu;
-      ppr_pairs<MODE, C>(ed, len == 0xffffffffu ? 0u : len, pr);
+      ppr_edges<MODE, C, PAIRS>(ed, len == 0xffffffffu ? 0u : len, pr);
     };
     fetch(0);
     for (uint32_t i = 0; i < cnt; i += G) {
       const uint32_t cv = v, cl = len;
       V acc;
       zero(acc);
-      ppr_gather<MODE, C>(src, a.rcp, ed, cl == 0xffffffffu ? 0u : cl, pr, sub, acc);
+      ppr_gather<MODE, C, PAIRS>(src, rcp, ed, cl == 0xffffffffu ? 0u : cl, pr, sub, acc);
       if (i + G < cnt) fetch(i + G);
       if (cl == 0xffffffffu) continue;
       unsigned int em = 0;
@@ -477,9 +501,7 @@ __global__ void __launch_bounds__(256) k_ppr_flat(PprArgs a) {
   State* st = a.st;
   if (ppr_skip<MODE>(st)) return;
   const V2* __restrict__ src = reinterpret_cast<const V2*>(ppr_src<MODE>(a, st));
-  const S* __restrict__ rc;
-  if constexpr (MODE == PPR_S32) rc = a.rcp32;
-  else rc = a.rcp;
+  const S* __restrict__ rc = ppr_rcp<MODE>(a);
   const uint32_t lane = lane_id(), warps = (gridDim.x * blockDim.x) >> 5;
   unsigned long long dmax = 0;
   unsigned int emag = 0;
@@ -545,9 +567,52 @@ __global__ void __launch_bounds__(256) k_ppr_flat(PprArgs a) {
   ppr_reduce<MODE>(st, dmax, emag);
 }
 
-// Long rows: a row's lanes per vertex add its segments in order, a segment
-// being its kSegParts parts (fewer in the last) added in order.
+// The long rows' segments without memory for their parts' partial rows (a.group
+// 1): a row's lanes sum a segment's parts one after the other and add them up as
+// k_ppr_combine would, the same bits, and leave one partial row a segment.
 template <int MODE, int C>
+__global__ void __launch_bounds__(256) k_ppr_segments(PprArgs a) {
+  using Sh = PprShape<MODE, C>;
+  using S = typename Sh::S;
+  using V = typename Sh::V;
+  State* st = a.st;
+  if (ppr_skip<MODE>(st)) return;
+  const S* __restrict__ src = ppr_src<MODE>(a, st);
+  const S* __restrict__ rcp = ppr_rcp<MODE>(a);
+  const uint32_t lane = lane_id(), sub = lane % Sh::LPR, grp = lane / Sh::LPR;
+  for (uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < (a.nparts + Sh::G - 1) / Sh::G;
+       b += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t i = b * Sh::G + grp;
+    uint32_t rest = 0;  // edges of the segment left
+    const uint32_t* ed = a.xtedg;
+    if (i < a.nparts) {
+      const uint2 w = __ldg(a.parts + i);  // vertex, first edge
+      rest = min(a.seg, __ldg(a.xtoff + seg_index(w.x, a.seg_shift) + 1) - w.y);
+      ed += w.y + (a.xtbase ? a.xtbase[(uint64_t)w.x >> a.seg_shift] : 0ull);
+    }
+    V acc;
+#pragma unroll 1
+    for (uint32_t q = 0; q < kSegParts; ++q) {
+      const uint32_t len = min(a.per, rest);
+      uint32_t pr[Sh::U];
+      V x;
+#pragma unroll
+      for (int k = 0; k < Sh::N; ++k) x[k] = S(0);
+      ppr_edges<MODE, C, false>(ed, len, pr);
+      ppr_gather<MODE, C, false>(src, rcp, ed, len, pr, sub, x);
+#pragma unroll
+      for (int k = 0; k < Sh::N; ++k) acc[k] = q == 0 ? x[k] : (len ? acc[k] + x[k] : acc[k]);
+      ed += len;
+      rest -= len;
+    }
+    if (i < a.nparts) Sh::store(reinterpret_cast<S*>(a.part), i, sub, acc);
+  }
+}
+
+// Long rows: a row's lanes per vertex add its segments in order, a segment
+// being its GROUP parts (fewer in the last) added in order: kSegParts, or one
+// partial row that holds their sum.
+template <int MODE, int C, uint32_t GROUP>
 __global__ void __launch_bounds__(256) k_ppr_combine(PprArgs a) {
   using Sh = PprShape<MODE, C>;
   using S = typename Sh::S;
@@ -564,10 +629,10 @@ __global__ void __launch_bounds__(256) k_ppr_combine(PprArgs a) {
 #pragma unroll
     for (int k = 0; k < Sh::N; ++k) acc[k] = S(0);
     const uint32_t end = a.partstart[i + 1];
-    for (uint32_t g = a.partstart[i]; g < end; g += kSegParts) {
-      V x[kSegParts];
+    for (uint32_t g = a.partstart[i]; g < end; g += GROUP) {
+      V x[GROUP];
 #pragma unroll
-      for (uint32_t k = 0; k < kSegParts; ++k) {
+      for (uint32_t k = 0; k < GROUP; ++k) {
         if (g + k < end) {
           x[k] = Sh::template load<false>(part, g + k, sub);
         } else {
@@ -576,7 +641,7 @@ __global__ void __launch_bounds__(256) k_ppr_combine(PprArgs a) {
         }
       }
 #pragma unroll
-      for (uint32_t k = 1; k < kSegParts; ++k)
+      for (uint32_t k = 1; k < GROUP; ++k)
         if (g + k < end) {
 #pragma unroll
           for (int j = 0; j < Sh::N; ++j) x[0][j] += x[k][j];
@@ -759,13 +824,26 @@ static void ppr_sweep_c(const PprArgs& a, int sms, cudaStream_t s, uint64_t& lau
     ++launches;
     b.nrows = 0;  // the long rows are left
   }
-  const uint64_t units = ((uint64_t)b.nrows + b.batch - 1) / b.batch + (a.nparts + G - 1) / G;
+  if (a.nparts && a.group == 1) {
+    k_ppr_segments<MODE, C><<<grid_for((uint64_t)a.nparts * (32 / G), 256, sms * 8), 256, 0, s>>>(a);
+    ++launches;
+    b.nparts = 0;
+  }
+  const uint64_t units = ((uint64_t)b.nrows + b.batch - 1) / b.batch + (b.nparts + G - 1) / G;
   if (units) {
-    k_ppr_rows<MODE, C><<<grid_for(units * 32, 256, sms * PprShape<MODE, C>::BLOCKS), 256, 0, s>>>(b);
+    const int grid = grid_for(units * 32, 256, sms * PprShape<MODE, C>::BLOCKS);
+    if constexpr (MODE == PPR_S32) {
+      if (a.pair) k_ppr_rows<MODE, C, true><<<grid, 256, 0, s>>>(b);
+      else k_ppr_rows<MODE, C, false><<<grid, 256, 0, s>>>(b);
+    } else {
+      k_ppr_rows<MODE, C, false><<<grid, 256, 0, s>>>(b);
+    }
     ++launches;
   }
   if (a.nparts) {
-    k_ppr_combine<MODE, C><<<grid_for((uint64_t)a.nbig * (32 / G), 256, sms * 8), 256, 0, s>>>(a);
+    const int grid = grid_for((uint64_t)a.nbig * (32 / G), 256, sms * 8);
+    if (a.group == 1) k_ppr_combine<MODE, C, 1><<<grid, 256, 0, s>>>(a);
+    else k_ppr_combine<MODE, C, kSegParts><<<grid, 256, 0, s>>>(a);
     ++launches;
   }
 }
@@ -818,6 +896,9 @@ static int ppr_ws(prx_context* c, uint32_t n, bool fp32) {
   }
   if (fp32 && !w.has32) {
     const size_t rows = (size_t)w.n * kCols;
+    cudaFree(w.rho);  // of a call that ended here
+    cudaFree(w.e[0]);
+    w.rho = w.e[0] = nullptr;
     TRY_CUDA_ST(device_alloc(&w.rho, sizeof(float) * rows));
     for (int i = 0; i < 2; ++i) TRY_CUDA_ST(device_alloc(&w.e[i], sizeof(float) * rows));
     w.has32 = true;
@@ -825,8 +906,31 @@ static int ppr_ws(prx_context* c, uint32_t n, bool fp32) {
   return PRX_OK;
 }
 
-// The long rows of graph g (in-degree above a.low_max) and their parts of
-// a.per edges into the workspace.
+// The partial rows of the long rows a.big: a.group per segment of a.seg edges.
+static cudaError_t ppr_parts(prx_context* c, const GraphDev& g, PprArgs& a) {
+  PprWs& w = *c->ppr;
+  cudaStream_t s = c->stream;
+  const uint32_t per = a.seg / a.group;
+  k_ppr_partcount<<<grid_for(a.nbig, 256, c->sms * 4), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, a.nbig, per,
+                                                                    w.partstart);
+  cudaError_t e = exclusive_scan_u32(w.partstart, a.nbig + 1, s);
+  uint32_t nparts = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&nparts, w.partstart + a.nbig, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = grow(&w.parts, w.parts_cap, (size_t)nparts);
+  if (e == cudaSuccess) e = grow(&w.part, w.part_cap, (size_t)nparts * kCols);
+  if (e != cudaSuccess) return e;
+  k_ppr_partfill<<<grid_for((uint64_t)a.nbig * 32, 256, c->sms * 8), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, a.nbig,
+                                                                                  per, w.partstart, w.parts);
+  a.partstart = w.partstart;
+  a.parts = w.parts;
+  a.nparts = nparts;
+  a.part = w.part;
+  return cudaGetLastError();
+}
+
+// The long rows of graph g (in-degree above a.low_max) and their partial rows
+// into the workspace: a part each, or, without memory for those, a segment each.
 static int ppr_segments(prx_context* c, const GraphDev& g, PprArgs& a) {
   PprWs& w = *c->ppr;
   cudaStream_t s = c->stream;
@@ -848,19 +952,13 @@ static int ppr_segments(prx_context* c, const GraphDev& g, PprArgs& a) {
   a.nparts = 0;
   if (!nbig) return PRX_OK;
   TRY_CUDA_ST(grow(&w.partstart, w.partstart_cap, (size_t)nbig + 1));
-  k_ppr_partcount<<<grid_for(nbig, 256, c->sms * 4), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, nbig, a.per, w.partstart);
-  TRY_CUDA_ST(exclusive_scan_u32(w.partstart, nbig + 1, s));
-  uint32_t nparts = 0;
-  TRY_CUDA_ST(cudaMemcpyAsync(&nparts, w.partstart + nbig, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  TRY_CUDA_ST(cudaStreamSynchronize(s));
-  TRY_CUDA_ST(grow(&w.parts, w.parts_cap, (size_t)nparts));
-  TRY_CUDA_ST(grow(&w.part, w.part_cap, (size_t)nparts * kCols));
-  k_ppr_partfill<<<grid_for((uint64_t)nbig * 32, 256, c->sms * 8), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, nbig, a.per,
-                                                                                w.partstart, w.parts);
-  a.partstart = w.partstart;
-  a.parts = w.parts;
-  a.nparts = nparts;
-  a.part = w.part;
+  a.group = kSegParts;
+  cudaError_t e = ppr_parts(c, g, a);
+  if (e == cudaErrorMemoryAllocation) {
+    a.group = 1;
+    e = ppr_parts(c, g, a);
+  }
+  TRY_CUDA_ST(e);
   return PRX_OK;
 }
 
@@ -1164,12 +1262,15 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   a.rows = by_length ? g.len_list : nullptr;
   a.nrows = by_length ? g.cls_begin[MID] : g.n;
   a.flat = !mixed_lengths(g);
-  if (!a.flat || a.nparts || (nvec % kCols && nvec % kCols <= 48)) {  // not k_ppr_flat alone
+  if (fp32 && (!a.flat || a.nparts || (nvec % kCols && nvec % kCols <= 48))) {  // not k_ppr_flat alone
     const uint64_t slots = g.nseg > 1 ? g.xtpos.back() + (g.m - g.xtseg0.back()) : g.m;
-    TRY_CUDA_ST(grow(&w.pair, w.pair_cap, slots));
-    k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, w.pair);
-    c->launches += 1;
-    a.pair = w.pair;
+    const cudaError_t e = grow(&w.pair, w.pair_cap, slots);
+    if (e != cudaErrorMemoryAllocation) TRY_CUDA_ST(e);
+    if (e == cudaSuccess) {
+      k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, w.pair);
+      c->launches += 1;
+      a.pair = w.pair;
+    }
   }
   double* out = ranks_out;
   const size_t total = (size_t)g.n * nvec;

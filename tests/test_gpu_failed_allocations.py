@@ -171,3 +171,48 @@ def test_apply_batch_without_its_layout(pg, ctx):
         x = fresh()
     assert passed >= 3   # the layout's offsets, ids and scan
     x.close()
+
+
+@pytest.mark.parametrize("vectors", [5, 24, 64])
+@pytest.mark.parametrize("refine", [False, True])
+@pytest.mark.parametrize("kind", ["hubs", "web"])
+def test_personalized_solve(pg, kind, refine, vectors):
+    xoff, xedg = {"hubs": lambda: pg.graphs.rmat(12, 48, a=0.7, b=0.1, c=0.1, seed=3),   # rows of several segments
+                  "web": lambda: pg.graphs.weblike(3001, dmax=900, window=512, seed=9)}[kind]()
+    n = len(xoff) - 1
+    xt = O.transpose(xoff, xedg)
+    rng = np.random.default_rng(4)
+    seeds = [rng.integers(0, n, 1 + k % 5) for k in range(vectors)]
+    opts = pg.options(tolerance=1e-9, precision=pg.FP32_REFINE if refine else pg.FP64)
+
+    def fresh():
+        c = pg.Context(0)
+        return c, pg.Graph(c, *xt, xoff, xedg)
+
+    def solve(c, g):
+        return pg.solve_ppr_batched(c, g, seeds, opts)
+
+    c, g = fresh()
+    want, res = solve(c, g)
+    passed, failed, got = 0, 0, []
+    c.close()
+    g.close()
+    c, g = fresh()
+    for error in failing(pg, lambda: got.append(solve(c, g))):
+        if error is None:
+            passed += 1
+            r, again = got.pop()
+            assert np.array_equal(r, want) and again["iterations"] == res["iterations"]
+        else:
+            failed += 1
+        r, again = solve(c, g)
+        assert np.array_equal(r, want) and again["iterations"] == res["iterations"]
+        g.close()
+        c.close()
+        c, g = fresh()
+    # the length list and its sort, the partial rows and where they start (graphs with
+    # long rows), and the pairs of the FP32 sweeps
+    long_rows = bool((np.diff(xt[0].astype(np.int64)) > 64).any())
+    assert passed >= 2 + 2 * long_rows + (refine and vectors < 64), (passed, failed)
+    g.close()
+    c.close()
