@@ -1250,6 +1250,14 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   r.seg_edges = a.seg;
   a.per = a.seg / kSegParts;
   if ((st = ppr_segments(c, g, a))) return st;
+  double* out = ranks_out;
+  const size_t total = (size_t)g.n * nvec;
+  if (!device_out) {
+    TRY_CUDA_ST(grow(&w.out, w.out_cap, total));
+    out = w.out;
+  }
+  const uint64_t l0 = c->launches;
+  TRY_CUDA_ST(cudaEventRecord(c->ev[0], s));
   // The LOW rows in order of length (rows side by side in a warp then end
   // together); by id with another bound, with row segments, or without memory
   // for the list.
@@ -1272,14 +1280,6 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
       a.pair = w.pair;
     }
   }
-  double* out = ranks_out;
-  const size_t total = (size_t)g.n * nvec;
-  if (!device_out) {
-    TRY_CUDA_ST(grow(&w.out, w.out_cap, total));
-    out = w.out;
-  }
-  const uint64_t l0 = c->launches;
-  TRY_CUDA_ST(cudaEventRecord(c->ev[0], s));
   for (uint32_t c0 = 0; c0 < nvec; c0 += kCols) {
     const uint32_t cols = std::min<uint32_t>(kCols, nvec - c0);
     for (int w : {64, 48, 32, 24, 16, 8})
