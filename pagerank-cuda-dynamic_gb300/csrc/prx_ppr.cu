@@ -80,8 +80,6 @@ struct PprWs {
   uint32_t* tent = nullptr;            // entries: vertex, column (sorted)
   double* tmass = nullptr;             // entry mass 1/|S_k|
   size_t t_cap = 0, tm_cap = 0;
-  uint2* pair = nullptr;               // the graph's in-edges as pairs (PprArgs::pair), for one FP32 call
-  size_t pair_cap = 0;
   double* out = nullptr;               // device staging of the host output
   size_t out_cap = 0;
 };
@@ -101,7 +99,6 @@ void ppr_free(PprWs* w) {
   cudaFree(w->toff);
   cudaFree(w->tent);
   cudaFree(w->tmass);
-  cudaFree(w->pair);
   cudaFree(w->out);
   delete w;
 }
@@ -874,6 +871,15 @@ static cudaError_t grow(T** p, size_t& cap, size_t want) {
   return e;
 }
 
+// PprArgs::pair: a block of the graph pool for the length of one call.
+struct PprPairs {
+  cudaStream_t s;
+  uint2* p = nullptr;
+  ~PprPairs() {
+    if (p) cudaFreeAsync(p, s);
+  }
+};
+
 static int ppr_ws(prx_context* c, uint32_t n, bool fp32) {
   if (!c->ppr) {
     c->ppr = new PprWs();
@@ -1227,6 +1233,7 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   if (st) return st;
   PprWs& w = *c->ppr;
   cudaStream_t s = c->stream;
+  PprPairs pair{s};
   PprArgs a{};
   a.xtoff = g.xtoff;
   a.xtbase = g.xtbase;
@@ -1272,12 +1279,12 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   a.flat = !mixed_lengths(g);
   if (fp32 && (!a.flat || a.nparts || (nvec % kCols && nvec % kCols <= 48))) {  // not k_ppr_flat alone
     const uint64_t slots = g.nseg > 1 ? g.xtpos.back() + (g.m - g.xtseg0.back()) : g.m;
-    const cudaError_t e = grow(&w.pair, w.pair_cap, slots);
+    const cudaError_t e = graph_alloc(&pair.p, sizeof(uint2) * slots, s);
     if (e != cudaErrorMemoryAllocation) TRY_CUDA_ST(e);
     if (e == cudaSuccess) {
-      k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, w.pair);
+      k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, pair.p);
       c->launches += 1;
-      a.pair = w.pair;
+      a.pair = pair.p;
     }
   }
   for (uint32_t c0 = 0; c0 < nvec; c0 += kCols) {
