@@ -42,8 +42,8 @@ struct PersistRows {
 
 // Expansion of the changed vertices (nf[p]) into nxt, whichever way
 // k_expand_push / k_expand_pull would go.  The out-edges of the changed
-// vertices of a word are spread over the warp's lanes, those of more than
-// kWarpExpand out-edges were queued in xb and get a block each.
+// vertices of a word are spread over the warp's lanes, those of out-degree
+// above kWarpExpand were queued in xb and get a block each.
 constexpr uint32_t kWarpExpand = 1024;
 
 __device__ __forceinline__ void persist_push(const SolveArgs& a, const uint32_t* nf, uint32_t* nxt, uint32_t nbig,
@@ -57,7 +57,8 @@ __device__ __forceinline__ void persist_push(const SolveArgs& a, const uint32_t*
       const uint32_t u = (w << 5) | lane;
       b = a.xoff[u];
       len = a.xoff[u + 1] - b;
-      if (len > kWarpExpand) len = 0;  // queued
+      // queued, by the degree given with the graph, which may differ from the row's
+      if (len > kWarpExpand && __ldg(a.xtdat + u) > kWarpExpand) len = 0;
     }
     uint32_t incl = len;
 #pragma unroll
