@@ -577,6 +577,43 @@ static int run_refine_loop(prx_context* c, const prx_graph* gr, const SolveArgs&
   }
 }
 
+// The FP64 source-chunk width of a solve.
+static uint32_t chunk64(const GraphDev& g, const prx_options& o) {
+  return o.chunk_vertices ? o.chunk_vertices : g.tuned_w64 ? g.tuned_w64 : kDefaultChunk64;
+}
+
+// What a solve reads, and so what has to be built for it (a new graph builds it
+// for the default options).
+struct Route {
+  // A small or medium graph runs its FP64 loop as one cooperative kernel on
+  // the plain rows (no hot copy, no source chunks); see launch_persist.
+  bool persist;
+  // one chunk: the LOW rows by words where rows are long.
+  bool by_words;
+  // Hot sources (the FP64 sweeps of every mode): a layout whose edges from
+  // the highest out-degree vertices gather from a dense copy of their
+  // contributions.  A refined solve has its FP32 sweeps read the rows by words
+  // too, so without hot sources; contributions that L2 holds anyway (64 MB) do
+  // without unless they are asked for (Static, web-like 3M vertices 2.94 ms
+  // without and 2.96 with, 6M 5.16 and 5.14, 20M 16.2 and 16.6), which saves a
+  // graph's first solve picking them.
+  bool hot;
+};
+static Route route_without(const GraphDev& g, const prx_options& o) {  // ... the cooperative kernel
+  const bool by_words = chunk64(g, o) >= g.n && words_fit(g);
+  const bool refine = o.precision == PRX_FP32_REFINE;
+  return {false, by_words,
+          o.hot_sources >= 0 && !(by_words && o.hot_sources == 0 && (refine || g.n <= (8u << 20)))};
+}
+static Route route_of(const GraphDev& g, const prx_options& o, bool dyn) {
+  const bool refine = o.precision == PRX_FP32_REFINE;
+  const bool persist = (!refine || (!dyn && o.max_iterations > 0 && g.mid_max >= kPlanMid)) &&
+                       o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase && g.nseg == 1 &&
+                       (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) && persist_fits(g) &&
+                       (mixed_lengths(g) || !words_fit(g) || (uint64_t)g.n <= 32 * kPersistWordUnits);
+  return persist ? Route{true, false, false} : route_without(g, o);
+}
+
 // Core solve; q_dev/batch arrays are device pointers.  On success *final_ranks
 // points at the device buffer holding the ranks.
 static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* du, const uint32_t* dv, uint64_t nd,
@@ -596,30 +633,17 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   // FP64 sweep (bound by GB300's FP64 add rate as much as by HBM) gains from
   // two chunks only (200 MB of contributions each), the FP32 sweep from
   // 48 MB chunks.
-  const uint32_t w64 = o.chunk_vertices ? o.chunk_vertices
-                      : g.tuned_w64          ? g.tuned_w64
-                                             : kDefaultChunk64;
+  const uint32_t w64 = chunk64(g, o);
   const uint32_t w32 = o.chunk_vertices ? o.chunk_vertices
                       : g.tuned_w32          ? g.tuned_w32
                                              : (48u << 20) / sizeof(float);
-  // Hot sources (the FP64 sweeps of every mode): a layout whose edges from
-  // the highest out-degree vertices gather from a dense copy of their
-  // contributions
-  // A small or medium graph runs its FP64 loop as one cooperative kernel on
-  // the plain rows (no hot copy, no source chunks); see launch_persist.
-  bool persist = (!refine || (!dyn && o.max_iterations > 0 && g.mid_max >= kPlanMid)) &&
-                 o.loop == PRX_LOOP_AUTO && !o.timing && o.hot_sources <= 0 && !g.xtbase &&
-                 g.nseg == 1 && (o.chunk_vertices == 0 || o.chunk_vertices >= g.n) && persist_fits(g) &&
-                 (mixed_lengths(g) || !words_fit(g) || (uint64_t)g.n <= 32 * kPersistWordUnits);
-  if (persist) TRY_CUDA_ST(ensure_plan(gr->g, c->sms, c->stream, &persist));
-  // one chunk: the LOW rows by words where rows are long.  A refined solve has
-  // its FP32 sweeps read them too, so without hot sources; contributions that L2
-  // holds anyway (64 MB) do without unless they are asked for (Static, web-like
-  // 3M vertices 2.94 ms without and 2.96 with, 6M 5.16 and 5.14, 20M 16.2 and
-  // 14.3), which saves a graph's first solve picking them.
-  const bool by_words = !persist && w64 >= g.n && words_fit(g);
-  const bool hot_ok = o.hot_sources >= 0 && !persist &&
-                      !(by_words && o.hot_sources == 0 && (refine || g.n <= (8u << 20)));
+  Route route = route_of(g, o, dyn);
+  if (route.persist) {
+    bool have = false;
+    TRY_CUDA_ST(ensure_plan(gr->g, c->sms, c->stream, &have));
+    if (!have) route = route_without(g, o);
+  }
+  const bool persist = route.persist, by_words = route.by_words, hot_ok = route.hot;
   if (hot_ok) {
     TRY_CUDA_ST(ensure_hot(gr->g, o.hot_sources > 0 ? (uint32_t)o.hot_sources : kDefaultHotCap, c->sms,
                            c->stream));
@@ -898,12 +922,14 @@ int prx_graph_create(prx_context* c, uint32_t n, uint64_t m, const uint32_t* xof
   if (e == cudaSuccess) e = build_classes(g, c->sms, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) e = tune_apply_cached(g, c->sms, s);
-  if (e == cudaSuccess) e = ensure_hot(g, kDefaultHotCap, c->sms, s);
-  if (e == cudaSuccess) {
-    const uint32_t width = g.tuned_w64 ? g.tuned_w64 : kDefaultChunk64;
-    if (width < n || !words_fit(g))  // else the first solve lays the rows out by words
-      e = build_default_layout_pipelined(g, width, g.hot_n > 0, pieces, rows, ev, c->sms, s);
-  }
+  // what the default solves read, but for the plans and the rows by words, which
+  // the first solve builds
+  prx_options defaults;
+  prx_options_default(&defaults);
+  const Route route = route_of(g, defaults, false);
+  if (e == cudaSuccess && route.hot) e = ensure_hot(g, kDefaultHotCap, c->sms, s);
+  if (e == cudaSuccess && !route.persist && !route.by_words)
+    e = build_default_layout_pipelined(g, chunk64(g, defaults), g.hot_n > 0, pieces, rows, ev, c->sms, s);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ev_done, 0);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) cudaStreamSynchronize(cs);  // no copy may still write into freed arrays
