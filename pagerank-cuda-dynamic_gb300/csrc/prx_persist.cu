@@ -674,7 +674,8 @@ cudaError_t launch_persist_refine(const SolveArgs& a, const GraphDev& g, int sms
   const PersistRows rows = persist_rows(g);
   const uint64_t units = (uint64_t)rows.nmid + ((uint64_t)(rows.sorted ? rows.nlow : a.n) + 31) / 32;
   const uint64_t want = std::max<uint64_t>(1, rows.nlong + (units + kThreads / 32 - 1) / (kThreads / 32));
-  return launch_resident(k_persist_refine<2>, want, kThreads, sms, s, a, rows);
+  return a.int_adds ? launch_resident(k_persist_refine<2>, want, kThreads, sms, s, a, rows)
+                    : launch_resident(k_persist_refine<0>, want, kThreads, sms, s, a, rows);
 }
 
 cudaError_t launch_persist(const SolveArgs& a, const GraphDev& g, int mode, int sms, cudaStream_t s) {

@@ -26,3 +26,14 @@ def test_equals_launched_loop(ctx, case):
             for key in ("iterations", "refinements", "last_delta", "edges_processed"):
                 assert a[key] == b[key], (mode, kw, key)
     g.close()
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_same_bits_without_integer_adds(ctx, case):
+    import pagerank_gb300 as pg
+    xoff, xedg = CASES[case](pg)
+    g = pg.Graph(ctx, *O.transpose(xoff, xedg), xoff, xedg)
+    want, b = pg.solve(ctx, g, pg.STATIC, opts=pg.options(precision=pg.FP32_REFINE))
+    r, a = pg.solve(ctx, g, pg.STATIC, opts=pg.options(precision=pg.FP32_REFINE, int_adds=-1))
+    assert np.array_equal(r, want) and a["iterations"] == b["iterations"]
+    g.close()
