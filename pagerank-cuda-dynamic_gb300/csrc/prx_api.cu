@@ -594,8 +594,8 @@ struct Route {
   // the highest out-degree vertices gather from a dense copy of their
   // contributions.  A refined solve has its FP32 sweeps read the rows by words
   // too, so without hot sources; contributions that L2 holds anyway (64 MB) do
-  // without unless they are asked for (Static, web-like 3M vertices 2.94 ms
-  // without and 2.96 with, 6M 5.16 and 5.14, 20M 16.2 and 16.6), which saves a
+  // without unless they are asked for (Static, web-like 3M vertices 2.97 ms
+  // without and 2.97 with, 6M 5.08 and 5.04, 20M 19.0 and 16.4), which saves a
   // graph's first solve picking them.
   bool hot;
 };
@@ -872,9 +872,9 @@ int prx_graph_create(prx_context* c, uint32_t n, uint64_t m, const uint32_t* xof
   g.m_cap = m;
   cudaStream_t s = c->stream;
   // The in-edges go up on a copy stream in row-range pieces; meanwhile the
-  // degree classes, the hot sources and the default LOW layout are built on
-  // the context's stream, each piece's part of the layout as soon as that
-  // piece has landed.  The out-CSR (dynamic modes) follows the in-edges.
+  // degree classes and what the default solves read of the hot sources and the
+  // LOW layout (route_of) are built on the context's stream, each piece's part
+  // of the layout as soon as that piece has landed.  The out-CSR (dynamic modes) follows the in-edges.
   auto alloc = [&](uint32_t** dst, size_t cnt, size_t slots = 0) -> cudaError_t {
     return graph_alloc(dst, sizeof(uint32_t) * (slots > cnt ? slots : (cnt ? cnt : 1)), s);
   };

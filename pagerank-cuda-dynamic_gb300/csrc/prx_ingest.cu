@@ -21,7 +21,7 @@
 // the in-rows (their targets' sectors come and go 4 bytes at a time; grouping
 // the entries by windows that stay in L2 first cost what it saved), 3 0.9 and
 // 0.6, the radix sort of the rows that need it 0.9, 4 0.4.  Radix sorts of all
-// keys took 11.9 in nine passes, the whole build 12.0 then and 8.8 now.
+// keys took 11.9 in nine passes, the whole build 12.0 then and 8.3 now.
 #include <algorithm>
 #include "prx_ctx.h"
 #include "prx_device.cuh"

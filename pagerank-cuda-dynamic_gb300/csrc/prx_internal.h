@@ -230,18 +230,18 @@ constexpr uint32_t kQuotTable = 1u << 16;  // out-degrees whose 64-bit reciproca
 cudaError_t degree_tables(const uint64_t** out, cudaStream_t s);
 constexpr uint32_t kPfTable = 1u << 16;  // out-degrees whose DF-P factor is tabulated
 constexpr uint32_t kHotFlag = 0x80000000u;
-// The hot sources of g for a cap of `cap` vertices (0: none); graphs of 2^31
-// vertices or more get none (their ids use the flag bit).
 // Whether one-chunk LOW sweeps go by words: plain graphs with rows of 16 in-edges
 // and more on average.  The sweep was bound by the L1 (81% of its wavefronts), and
 // a fifth of those were id loads.  Static solves, ms, rows | words: web-like 3M
-// vertices 3.29 | 2.95, 6M 5.82 | 5.11, 20M 16.2 | 14.4; FP32-refined 3M 2.97 |
+// vertices 3.29 | 2.95, 6M 5.82 | 5.11, 20M 18.8 | 16.6; FP32-refined 3M 2.97 |
 // 2.39, 6M 5.39 | 4.38, 14M 13.7 (two chunks) | 10.5; grid 4096^2, rows of five
 // (padded to eight ids), 3.56 | 3.66.
 bool words_fit(const GraphDev& g);
 // The LOW rows by words for this graph version; a null view when there is no
 // memory for them (the sweeps then read the CSR).
 cudaError_t ensure_words(GraphDev& g, bool hot, int sms, cudaStream_t s, WordView* out);
+// The hot sources of g for a cap of `cap` vertices (0: none); graphs of 2^31
+// vertices or more get none (their ids use the flag bit).
 cudaError_t ensure_hot(GraphDev& g, uint32_t cap, int sms, cudaStream_t s);
 void free_hot(GraphDev& g);
 

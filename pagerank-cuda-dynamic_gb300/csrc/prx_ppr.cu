@@ -37,7 +37,9 @@
 // Longer rows are cut into segments of `seg` in-edges (512 by default) of
 // eight contiguous parts; a part's sum is a partial row, and a second kernel
 // adds a segment's parts, and a vertex's segments, in order and finishes the
-// vertex.  Every sum has a fixed order for given low_max / seg,
+// vertex.  Where memory for the parts' partial rows or for the FP32 sweeps'
+// pairs is short, a segment's parts are summed one after the other and ids are
+// read instead: the same bits, slower.  Every sum has a fixed order for given low_max / seg,
 // so results are deterministic; prx_autotune_ppr picks both per graph.
 //
 // Loop: by default the whole iteration loop of a column block is one CUDA
@@ -120,7 +122,7 @@ struct PprArgs {
   float* e[2];
   const uint32_t* big;            // vertices with in-degree > low_max
   uint32_t nbig;
-  uint32_t low_max;               // rows up to this in-degree: one warp per vertex
+  uint32_t low_max;               // rows up to this in-degree are summed whole, LPR lanes per vertex
   uint32_t seg;                   // in-edges per segment of a longer row (a multiple of kSegParts)
   uint32_t per;                   // in-edges per part: seg / kSegParts
   uint32_t group;                 // partial rows a segment: kSegParts, or 1 when there is no memory for its parts'
@@ -152,7 +154,7 @@ template <int MODE, int C> struct PprShape {
   static constexpr int N = VEC ? 16 / (int)sizeof(S) : 3;
   static constexpr int LPR = C / N;
   static constexpr int G = 32 / LPR;
-  static constexpr int U = 4;       // rows a lane has in flight
+  static constexpr int U = 4;       // rows a lane has in flight (ppr_gather's branches are for four)
   static constexpr int BLOCKS = 4;  // resident blocks of 256 per SM
   using Raw = typename std::conditional<sizeof(S) == 8, double2, float4>::type;
   struct V {
@@ -283,19 +285,6 @@ __device__ __forceinline__ void ppr_gather(const typename PprType<MODE>::S* __re
       if (n >= 4) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) add(k);
-        if constexpr (U == 8) {
-          if (n >= 8) {
-#pragma unroll
-            for (int k = 4; k < 8; ++k) add(k);
-          } else {
-            switch (n) {
-              case 5: add(4); break;
-              case 6: add(4); add(5); break;
-              case 7: add(4); add(5); add(6); break;
-              default: break;
-            }
-          }
-        }
       } else {
         switch (n) {
           case 1: add(0); break;

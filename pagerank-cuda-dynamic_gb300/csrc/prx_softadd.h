@@ -33,7 +33,8 @@ namespace prx {
 constexpr uint32_t kSoftAddHiLimit = 2000u << 20;
 
 // Bits of RN(x + y) for the bit patterns x, y of two doubles whose high words
-// are below kSoftAddHiLimit (zeros and subnormals included).
+// are below kSoftAddHiLimit (zeros and subnormals included): the method in one
+// function, as the host test checks it.  The kernels take soft_add below.
 PRX_HD uint64_t add_nonneg_bits(uint64_t x, uint64_t y) {
   // non-negative doubles order as their bit patterns
   const uint64_t h = x > y ? x : y, l = x > y ? y : x;
@@ -67,7 +68,7 @@ PRX_HD uint64_t add_nonneg_bits(uint64_t x, uint64_t y) {
 // bit, which is always 0, and one comparison decides both.  A shift of 63 or
 // more leaves F below 1/2 whatever the operand was, so an addend that is zero
 // or subnormal needs no case of its own as long as the running sum is at
-// least 2^kSoftMinExp.
+// least 2^-895 (kSoftMinHi).
 //
 // Measured on GB300 (cycles per warp-wide addition and SM, throughput /
 // latency): DADD 20 / 65, add_nonneg_bits 22 / 110, soft_add 14 / 79, and 10
