@@ -1244,6 +1244,7 @@ static int solve_common(prx_context* c, prx_graph* gr, int mode, const uint32_t*
   TRY_CUDA_ST(cudaSetDevice(c->device));
   const uint32_t *ddu = du, *ddv = dv, *diu = iu;
   const double* dq = q;
+  PoolBlock start{c->stream};
   int st;
   if (host) {
     if (dyn) {
@@ -1261,9 +1262,15 @@ static int solve_common(prx_context* c, prx_graph* gr, int mode, const uint32_t*
     st = ensure_ws(c, g.n, dyn);
     if (st) return st;
     if (q && mode != PRX_STATIC) {
-      // stage q in r[1]: init reads it before anything writes r[1]
-      TRY_CUDA_ST(cudaMemcpyAsync(c->r[1], q, sizeof(double) * g.n, cudaMemcpyHostToDevice, c->stream));
-      dq = c->r[1];
+      // stage q in r[1]: init reads it before anything writes r[1]; repetitions
+      // start from it again, so it has a place of its own
+      double* stage = c->r[1];
+      if (opt.repeat > 1) {
+        TRY_CUDA_ST(graph_alloc(&start.p, sizeof(double) * g.n, c->stream));
+        stage = static_cast<double*>(start.p);
+      }
+      TRY_CUDA_ST(cudaMemcpyAsync(stage, q, sizeof(double) * g.n, cudaMemcpyHostToDevice, c->stream));
+      dq = stage;
     } else {
       dq = nullptr;
     }

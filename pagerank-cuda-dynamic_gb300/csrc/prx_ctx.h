@@ -118,6 +118,15 @@ inline cudaError_t capture_conditional(cudaStream_t s, cudaStream_t s2, cudaGrap
 
 }  // namespace prx
 
+// A block of the graph pool (graph_alloc) for the length of one call.
+struct PoolBlock {
+  cudaStream_t s;
+  void* p = nullptr;
+  ~PoolBlock() {
+    if (p) cudaFreeAsync(p, s);
+  }
+};
+
 #define TRY_CUDA_ST(x)                                                                   \
   do {                                                                                   \
     cudaError_t e_ = (x);                                                                \

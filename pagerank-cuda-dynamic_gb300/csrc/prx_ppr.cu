@@ -860,15 +860,6 @@ static cudaError_t grow(T** p, size_t& cap, size_t want) {
   return e;
 }
 
-// PprArgs::pair: a block of the graph pool for the length of one call.
-struct PprPairs {
-  cudaStream_t s;
-  uint2* p = nullptr;
-  ~PprPairs() {
-    if (p) cudaFreeAsync(p, s);
-  }
-};
-
 static int ppr_ws(prx_context* c, uint32_t n, bool fp32) {
   if (!c->ppr) {
     c->ppr = new PprWs();
@@ -1222,7 +1213,7 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   if (st) return st;
   PprWs& w = *c->ppr;
   cudaStream_t s = c->stream;
-  PprPairs pair{s};
+  PoolBlock pairs{s};  // PprArgs::pair
   PprArgs a{};
   a.xtoff = g.xtoff;
   a.xtbase = g.xtbase;
@@ -1268,12 +1259,13 @@ static int ppr_common(prx_context* c, prx_graph* gr, uint32_t nvec, const uint32
   a.flat = !mixed_lengths(g);
   if (fp32 && (!a.flat || a.nparts || (nvec % kCols && nvec % kCols <= 48))) {  // not k_ppr_flat alone
     const uint64_t slots = g.nseg > 1 ? g.xtpos.back() + (g.m - g.xtseg0.back()) : g.m;
-    const cudaError_t e = graph_alloc(&pair.p, sizeof(uint2) * slots, s);
+    const cudaError_t e = graph_alloc(&pairs.p, sizeof(uint2) * slots, s);
     if (e != cudaErrorMemoryAllocation) TRY_CUDA_ST(e);
     if (e == cudaSuccess) {
-      k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, pair.p);
+      uint2* pair = static_cast<uint2*>(pairs.p);
+      k_ppr_pairs<<<grid_for(slots, 256, c->sms * 32), 256, 0, s>>>(g.xtedg, slots, g.n, g.rcp32, pair);
       c->launches += 1;
-      a.pair = pair.p;
+      a.pair = pair;
     }
   }
   for (uint32_t c0 = 0; c0 < nvec; c0 += kCols) {
