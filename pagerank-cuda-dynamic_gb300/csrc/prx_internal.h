@@ -204,7 +204,8 @@ struct GraphDev {
   uint32_t ocls_mid = 0;          // the mid_max they were built with
   uint32_t* oplan_list = nullptr;
   uint32_t oplan_begin[NCLS + 1] = {0, 0, 0, 0};
-  bool oplan_built = false, oplan_fits = false;
+  bool oplan_built = false;       // for this version of the classes
+  bool oplan_have = false, oplan_fits = false;  // of the weights that are set
   uint32_t* tpos = nullptr;       // laid out like xedg; positions relative to the in-CSR's row segment
   bool tpos_built = false;
   bool weights_set = false;       // px, pt, wsum (and wseg) hold the weights of this version

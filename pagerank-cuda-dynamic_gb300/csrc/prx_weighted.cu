@@ -573,8 +573,8 @@ struct OutRows {
   uint32_t mid_max;
 };
 static OutRows out_rows(const GraphDev& g) {
-  return g.oplan_built ? OutRows{g.oplan_list, g.oplan_begin, kPlanMid}
-                       : OutRows{g.ocls_list, g.ocls_begin, g.ocls_mid};
+  return g.oplan_have ? OutRows{g.oplan_list, g.oplan_begin, kPlanMid}
+                      : OutRows{g.ocls_list, g.ocls_begin, g.ocls_mid};
 }
 
 // GraphDev::oplan_list, its order and oplan_fits; ocls_list is there.
@@ -592,7 +592,7 @@ static cudaError_t build_out_plan(GraphDev& g, uint64_t padded, int sms, cudaStr
                        sms, s);
   }
   g.oplan_fits = plan_fits(g.n, g.oplan_begin[MID], mixed);
-  g.oplan_built = e == cudaSuccess;
+  g.oplan_built = g.oplan_have = e == cudaSuccess;
   return e;
 }
 
@@ -837,7 +837,7 @@ int prx_adjoint(prx_context* c, prx_graph* gr, const double* t, const double* r,
   a.shift = g.seg_shift;
   a.list = g.ocls_list;
   for (int k = 0; k <= NCLS; ++k) a.begin[k] = g.ocls_begin[k];
-  if (g.oplan_built && g.oplan_fits) take_plan(a, g.oplan_list, g.oplan_list, g.oplan_begin);
+  if (g.oplan_have && g.oplan_fits) take_plan(a, g.oplan_list, g.oplan_list, g.oplan_begin);
   a.base = gl;
   a.base_scale = 1.0;
   a.alpha = alpha;

@@ -67,3 +67,20 @@ def test_loop_equals_launched_sweeps(pg, ctx, case):
         assert both[0][1]["iterations"] == both[1][1]["iterations"] == cap
         assert float((both[0][0] - both[1][0]).abs().max()) <= 1e-12 * float(t.max())
     g.close()
+
+
+def test_plan_stays_after_autotune(pg, ctx):
+    import torch
+    from pagerank_gb300 import autograd as A
+    g = pg.Graph.from_out_csr(ctx, *pg.graphs.rmat(12, 16, seed=3))
+    n, m = g.size()
+    A.set_weights(ctx, g, 0.5 + torch.rand(m, generator=torch.Generator(device="cuda").manual_seed(5), device="cuda"))
+    goal = torch.ones(n, dtype=torch.float64, device="cuda")
+    r, _ = A.solve_weighted(ctx, g)
+    before = A.adjoint(ctx, g, r, goal)
+    pg.autotune(ctx, g)
+    after = A.adjoint(ctx, g, r, goal)
+    assert torch.equal(before["grad_w"], after["grad_w"])
+    # one kernel for the loop, not three a sweep
+    assert after["result"]["kernel_launches"] < before["result"]["kernel_launches"] + after["result"]["iterations"]
+    g.close()
