@@ -495,6 +495,7 @@ cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd64, ui
   const int grid = sms * 8;
   uint32_t *scratch = nullptr, *noff = nullptr, *ntoff = nullptr, *nedg = nullptr, *ntedg = nullptr, *ndat = nullptr;
   uint32_t *ranges = nullptr, *lists = nullptr;
+  void* class_ws = nullptr;  // taken before the graph is changed: nothing may fail for memory after
   const uint32_t* in_list = nullptr;  // the in-CSR's touched rows (plain graphs)
   const uint32_t* touched_count = nullptr;  // their number, in device memory (plain graphs)
   struct NewLayout {
@@ -615,6 +616,7 @@ cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd64, ui
     }
   }
   k_out_degree<<<grid, kThreads, 0, s>>>(noff, S, n, ndat);
+  PRX_CU(graph_alloc(&class_ws, class_ws_bytes(n), s));
   // the cached LOW layouts follow the new version (plain graphs; the hot
   // numbering is kept with them)
   if (!segmented) {
@@ -662,12 +664,13 @@ cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd64, ui
   }
   g.m = m2;
   g.m_cap = m2;
-  PRX_CU(build_classes(g, sms, s, !segmented));
+  PRX_CU(build_classes(g, sms, s, !segmented, class_ws));
 done:
   for (auto& x : layouts_new) graph_free({x.off, x.edg});
   if (scratch) cudaFreeAsync(scratch, s);
   if (ranges) cudaFreeAsync(ranges, s);
   if (lists) cudaFreeAsync(lists, s);
+  if (class_ws) cudaFreeAsync(class_ws, s);
   if (segd) cudaFreeAsync(segd, s);
   graph_free({noff, ntoff, nedg, ntedg, ndat});
   graph_free({nbase, ntbase});

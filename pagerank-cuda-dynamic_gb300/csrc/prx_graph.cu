@@ -943,7 +943,7 @@ cudaError_t ensure_hot(GraphDev& g, uint32_t cap, int sms, cudaStream_t s) {
   return cudaSuccess;
 }
 
-cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layouts) {
+cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layouts, void* ws) {
   const uint32_t n = g.n;
   g.plan_built = g.len_built = g.oplan_built = g.tpos_built = false;
   g.words[0].built = g.words[1].built = false;
@@ -969,7 +969,7 @@ cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layout
     if (e != cudaSuccess) return e;
   }
   return build_class_lists(g.xtoff, g.seg_shift, n, g.mid_max, g.cls_list, g.cls_begin, g.cls_edges, sms, s,
-                           &g.low_padded);
+                           &g.low_padded, ws);
 }
 
 void launch_vertex_tables(const uint32_t* xtoff, uint32_t shift, const uint32_t* xtdat, uint32_t n, uint32_t* low_bm,
@@ -1055,9 +1055,16 @@ cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s, bool* have) {
   return cudaSuccess;
 }
 
+// [class-major tile counts | 4 bounds | pad | 4 u64 sums]
+static size_t class_sums_at(uint32_t n) {
+  const size_t words = (size_t)NCLS * (((size_t)n + kTileV - 1) / kTileV) + NCLS + 1;
+  return (words * sizeof(uint32_t) + 7) & ~(size_t)7;
+}
+size_t class_ws_bytes(uint32_t n) { return class_sums_at(n) + (NCLS + 1) * sizeof(unsigned long long); }
+
 cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, uint32_t mid_max, uint32_t* list,
                               uint32_t begin[NCLS + 1], uint64_t edges_out[NCLS], int sms, cudaStream_t s,
-                              uint64_t* low_padded) {
+                              uint64_t* low_padded, void* ws) {
   if (low_padded) *low_padded = 0;
   if (n == 0) {
     for (int c = 0; c <= NCLS; ++c) begin[c] = 0;
@@ -1065,14 +1072,11 @@ cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, u
     return cudaSuccess;
   }
   const uint32_t ntiles = (n + kTileV - 1) / kTileV;
-  uint32_t* cnt = nullptr;
-  // [class-major tile counts | 4 bounds | pad | 4 u64 sums]
-  const size_t words = (size_t)NCLS * ntiles + NCLS + 1;
-  const size_t bytes = ((words * sizeof(uint32_t) + 7) & ~(size_t)7) + (NCLS + 1) * sizeof(unsigned long long);
-  cudaError_t e = graph_alloc(&cnt, bytes, s);
+  uint32_t* cnt = static_cast<uint32_t*>(ws);
+  cudaError_t e = ws ? cudaSuccess : graph_alloc(&cnt, class_ws_bytes(n), s);
   if (e != cudaSuccess) return e;
   uint32_t* bounds = cnt + (size_t)NCLS * ntiles;
-  unsigned long long* edges = (unsigned long long*)((char*)cnt + ((words * sizeof(uint32_t) + 7) & ~(size_t)7));
+  unsigned long long* edges = (unsigned long long*)((char*)cnt + class_sums_at(n));
   e = cudaMemsetAsync(edges, 0, (NCLS + 1) * sizeof(unsigned long long), s);
   k_cls_count<<<ntiles, 256, 0, s>>>(off, shift, n, mid_max, ntiles, cnt);
   k_cls_scan<<<1, 1024, 0, s>>>(cnt, ntiles, bounds);
@@ -1083,7 +1087,7 @@ cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, u
   if (e == cudaSuccess) e = cudaMemcpyAsync(hb, bounds, sizeof(hb), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(he, edges, sizeof(he), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFreeAsync(cnt, s);
+  if (!ws) cudaFreeAsync(cnt, s);
   if (e != cudaSuccess) return e;
   for (int c = 0; c <= NCLS; ++c) begin[c] = hb[c];
   for (int c = 0; c < NCLS; ++c) edges_out[c] = he[c];

@@ -418,7 +418,10 @@ void launch_state_reset(State* st, int max_iter, double tol, cudaStream_t s);
 // Degree classes, LOW bitmap and reciprocals of g's current arrays; the
 // cached layouts and hot sources are dropped unless keep_layouts (a batch
 // apply that carried them to the new version).
-cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layouts = false);
+// ws: class_ws_bytes(n) of device memory, or null: it allocates them.  With it,
+// for a graph that had classes before, nothing is allocated.
+cudaError_t build_classes(GraphDev& g, int sms, cudaStream_t s, bool keep_layouts = false, void* ws = nullptr);
+size_t class_ws_bytes(uint32_t n);
 // The LOW-class bitmap and the reciprocal out-degrees (FP64 and FP32) of a
 // graph version, by kernels alone (build_classes runs them too).
 void launch_vertex_tables(const uint32_t* xtoff, uint32_t shift, const uint32_t* xtdat, uint32_t n, uint32_t* low_bm,
@@ -430,7 +433,7 @@ cudaError_t tune_apply_cached(GraphDev& g, int sms, cudaStream_t s);
 // into list (n), their bounds and the edges of each class.
 cudaError_t build_class_lists(const uint32_t* off, uint32_t shift, uint32_t n, uint32_t mid_max, uint32_t* list,
                               uint32_t begin[NCLS + 1], uint64_t edges[NCLS], int sms, cudaStream_t s,
-                              uint64_t* low_padded = nullptr);
+                              uint64_t* low_padded = nullptr, void* ws = nullptr);
 // b: device array [du | dv | iu | iv | tdk | tdv | tik | tiv]; t* = batch sorted by (v, u)
 cudaError_t apply_batch_device(GraphDev& g, const uint32_t* b, uint64_t nd, uint64_t ni, int sms, cudaStream_t s);
 // The arrays of one graph version (a plain CSR pair and the out-degrees).

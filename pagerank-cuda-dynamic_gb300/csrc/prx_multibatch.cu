@@ -229,6 +229,8 @@ extern "C" int prx_solve_batches_device(prx_context* c, prx_graph* gr, int mode,
   MbControl* ctl = nullptr;
   MB_TRY(alloc((void**)&rec, sizeof(MbRecord) * K));
   MB_TRY(alloc((void**)&ctl, sizeof(MbControl)));
+  void* class_ws = nullptr;
+  MB_TRY(alloc(&class_ws, class_ws_bytes(n)));
   MB_TRY(cudaStreamSynchronize(s));
 
   // the sequence as one graph
@@ -360,7 +362,7 @@ extern "C" int prx_solve_batches_device(prx_context* c, prx_graph* gr, int mode,
                     (void*)set[keep].xtdat})
       owned.erase(std::find(owned.begin(), owned.end(), p));
     drop_weights(g);
-    MB_TRY(build_classes(g, c->sms, s));
+    MB_TRY(build_classes(g, c->sms, s, false, class_ws));
   }
   MB_TRY(cudaMemcpyAsync(ranks_out, qbuf, 8 * (size_t)n, cudaMemcpyDeviceToDevice, s));
   MB_TRY(cudaStreamSynchronize(s));

@@ -216,3 +216,29 @@ def test_personalized_solve(pg, kind, refine, vectors):
     assert passed >= 2 + 2 * long_rows + (refine and vectors < 64), (passed, failed)
     g.close()
     c.close()
+
+
+@pytest.mark.parametrize("seg_shift", [0, 10])
+def test_apply_batch_is_all_or_nothing(pg, ctx, seg_shift):
+    xoff, xedg = pg.graphs.rmat(12, 16, seed=3)
+    old, it_old = O.solve("static", None, None, *O.transpose(xoff, xedg))
+    batch = pg.graphs.random_batch(xoff, xedg, 40, 100, seed=2)
+    yoff, yedg = pg.graphs.apply_batch(xoff, xedg, *batch)
+    want, it = O.solve("static", None, None, *O.transpose(yoff, yedg))
+
+    def holds(x, ranks, iterations):
+        for kw in ({}, {"loop": pg.LOOP_GRAPH}):
+            r, res = pg.pagerank_static(ctx, x, pg.options(**kw))
+            assert res["iterations"] == iterations and np.array_equal(r, ranks)
+
+    x, failed = graph(pg, ctx, "rmat", seg_shift), 0
+    for error in failing(pg, lambda: x.apply_batch(*batch)):
+        if error:
+            failed += 1
+            holds(x, old, it_old)     # unchanged, and the batch still applies
+            x.apply_batch(*batch)
+        holds(x, want, it)
+        x.close()
+        x = graph(pg, ctx, "rmat", seg_shift)
+    assert failed >= 8
+    x.close()
