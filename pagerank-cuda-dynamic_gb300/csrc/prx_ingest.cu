@@ -45,10 +45,12 @@ struct LongRows {
 
 // cnt[at] += 1 for the lanes of a full warp that have a row (at != kNoId), and
 // the lane's own place among its row's.  One atomic per run of equal rows (lists
-// in row order), or per distinct row when a row that two lanes are asked for
-// comes back in three runs (a hub): one counter takes an atomic every 0.65 ns.
-// Matching every warp took 346 us where this takes 317 (17M entries, both ways).
-__device__ __forceinline__ uint32_t add_one(uint32_t* cnt, uint32_t at) {
+// in row order), or per distinct row once a row that two lanes are asked for
+// came back in three runs (a hub): one counter takes an atomic every 0.65 ns.
+// Matching every warp took 346 us where this takes 317 (17M entries, both ways);
+// asking anew each time took 1515 us of 20M entries whose largest row had a sixth
+// of them, and hubs, kept over the warp's entries, takes 713.
+__device__ __forceinline__ uint32_t add_one(uint32_t* cnt, uint32_t at, bool& hubs) {
   const uint32_t lane = lane_id(), upto = 0xffffffffu >> (31 - lane);
   const uint32_t before = __shfl_up_sync(0xffffffffu, at, 1);
   const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || at != before);
@@ -56,7 +58,8 @@ __device__ __forceinline__ uint32_t add_one(uint32_t* cnt, uint32_t at) {
   const unsigned hub1 = __ballot_sync(0xffffffffu, at == __shfl_sync(0xffffffffu, at, 16)) & heads;
   unsigned same;
   uint32_t leader;
-  if (__popc(hub0) > 2 || __popc(hub1) > 2) {
+  hubs = hubs || __popc(hub0) > 2 || __popc(hub1) > 2;
+  if (hubs) {
     same = __match_any_sync(0xffffffffu, at);
     leader = __ffs(same) - 1;
   } else {
@@ -85,13 +88,14 @@ __global__ void __launch_bounds__(256) k_ing_count(const uint32_t* __restrict__ 
                                                    uint32_t* __restrict__ out, uint32_t* __restrict__ in, uint32_t* __restrict__ at_out,
                                                    uint32_t* __restrict__ at_in, uint32_t* __restrict__ bad) {
   const uint32_t step = gridDim.x * blockDim.x;
+  bool out_hubs = false, in_hubs = false;
   for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < count; i0 += step) {
     const uint32_t i = i0 + lane_id();
     const uint32_t a = i < count ? u[i] : kNoId, b = i < count ? v[i] : kNoId;
     const bool ok = a < n && b < n;
     if (i < count && !ok) *bad = 1u;
-    const uint32_t p = add_one(out, ok ? counter_of(a, bits) : kNoId);
-    const uint32_t q = add_one(in, ok ? counter_of(b, bits) : kNoId);
+    const uint32_t p = add_one(out, ok ? counter_of(a, bits) : kNoId, out_hubs);
+    const uint32_t q = add_one(in, ok ? counter_of(b, bits) : kNoId, in_hubs);
     if (ok) {
       at_out[i] = p;
       at_in[i] = q;
