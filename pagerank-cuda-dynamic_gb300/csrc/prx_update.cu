@@ -171,12 +171,20 @@ __device__ __forceinline__ void list_of(const SolveArgs& a, int cls, uint32_t be
   }
 }
 
+// What finish_listed reads besides the sum, loaded before the row by the thread
+// that will hold it (the reciprocal waits for the degree).
+template <int MODE>
+__device__ __forceinline__ VertexIn listed_in(const SolveArgs& a, uint32_t v, int p, bool mine) {
+  VertexIn in{};
+  if constexpr (!ModeTraits<MODE>::F32) {
+    if (mine) in = load_vertex(a, v, p);
+  }
+  return in;
+}
 template <int MODE>
 __device__ __forceinline__ void finish_listed(const SolveArgs& a, uint32_t v, typename ModeTraits<MODE>::V x, int p,
-                                              unsigned long long& emax, unsigned int& mag) {
+                                              const VertexIn& in, unsigned long long& emax, unsigned int& mag) {
   bool survive, changed;
-  VertexIn in{};
-  if constexpr (!ModeTraits<MODE>::F32) in = load_vertex(a, v, p);
   const unsigned long long ev = finish_vertex<MODE>(a, v, x, p, survive, changed, mag, in);
   emax = ev > emax ? ev : emax;
   if (ModeTraits<MODE>::DYN && survive) atomicOr(&a.bm[(a.st->iter + 1) % 3][v >> 5], 1u << (v & 31u));
@@ -207,9 +215,10 @@ __global__ void __launch_bounds__(kThreads) k_update_mid(SolveArgs a, uint32_t b
     const uint64_t iv = seg_index(v, a.seg_shift);
     const uint32_t s = a.xtoff[iv], d = a.xtoff[iv + 1] - s;
     const uint32_t* __restrict__ ed = seg_edges(a.xtedg, a.xtbase, a.seg_shift, v) + s;
+    const VertexIn in = listed_in<MODE>(a, v, p, lane == 0);
     const V x = mid_row_sum<V, false, false>(c, ed, d, lane);
     if (lane == 0) {
-      finish_listed<MODE>(a, v, x, p, emax, mag);
+      finish_listed<MODE>(a, v, x, p, in, emax, mag);
       edges += d;
     }
   }
@@ -238,9 +247,10 @@ __global__ void __launch_bounds__(256) k_update_high(SolveArgs a, uint32_t begin
     const uint64_t iv = seg_index(v, a.seg_shift);
     const uint32_t s = a.xtoff[iv], d = a.xtoff[iv + 1] - s;
     const uint32_t* __restrict__ ed = seg_edges(a.xtedg, a.xtbase, a.seg_shift, v) + s;
+    const VertexIn in = listed_in<MODE>(a, v, p, t == 0);
     const V x = high_row_sum<V, false, false>(c, ed, d, t, part);
     if (t == 0) {
-      finish_listed<MODE>(a, v, x, p, emax, mag);
+      finish_listed<MODE>(a, v, x, p, in, emax, mag);
       edges += d;
     }
   }

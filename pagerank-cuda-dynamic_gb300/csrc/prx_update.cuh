@@ -164,7 +164,7 @@ __device__ __forceinline__ V load_c(const V* c) {
   else return __ldg(c);
 }
 
-// The integer pipes take about half of the FP64 adds of the MID and HIGH sums
+// The integer pipes take about half of the FP64 adds of the MID sums
 // (soft_add): GB300's FP64 pipe needs 20 cycles a warp-wide add, soft_add 14
 // of the integer pipes'.  It needs every term to be normal and below 2^977;
 // sums that meet another one (zero, negative, subnormal, huge: a caller's
@@ -218,6 +218,8 @@ struct RowTree {
 // none: of 28 warp-wide adds for a row of 275 terms, 12 are left.
 // PRE: the ids of the next 256 terms are loaded behind the gathers of these
 // (few warps, where the latency of the two loads counts; 8 more registers).
+// The loads of 256 terms and more stand under one branch: a predicate each kept
+// them from being in flight together (R-MAT 2^16 launched, us: 34 so, 19 now).
 // mid_lane_sums: the partial sums of virtual threads 0 .. 31 (after the halving
 // tree's first three levels), one per lane.
 template <class V, bool COH, bool SOFT, bool PRE>
@@ -226,26 +228,40 @@ __device__ __forceinline__ V mid_lane_sums(const V* c, const uint32_t* __restric
   V ps[8];
   uint32_t u[8];
   auto ids = [&](uint32_t base) {
+    if (base + 256 <= d) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint32_t t = base + lane + 32u * k;
-      u[k] = t < d ? __ldg(ed + t) : 0u;
+      for (int k = 0; k < 8; ++k) u[k] = __ldg(ed + base + lane + 32u * k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) u[k] = base + lane + 32u * k < d ? __ldg(ed + base + lane + 32u * k) : 0u;
     }
   };
   if (PRE) ids(0);
   for (uint32_t base = 0; base < d; base += 256) {
     if (!PRE) ids(base);
     V x[8];
+    const bool full = base + 256 <= d;
+    if (full) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = base + lane + 32u * k < d ? load_c<COH>(c + u[k]) : V(0);
+      for (int k = 0; k < 8; ++k) x[k] = load_c<COH>(c + u[k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[k] = base + lane + 32u * k < d ? load_c<COH>(c + u[k]) : V(0);
+    }
     if (PRE) ids(base + 256);
     if (SOFT) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) bad = bad || (base + lane + 32u * k < d && soft_out_of_range(x[k]));
+      for (int k = 0; k < 8; ++k) bad = bad || ((full || base + lane + 32u * k < d) && soft_out_of_range(x[k]));
     }
     if (base == 0) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) ps[k] = SOFT ? x[k] : V(0) + x[k];
+    } else if (full) {
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        ps[k] += x[k];
+        ps[k + 1] = plus<SOFT>(ps[k + 1], x[k + 1]);
+      }
     } else {
 #pragma unroll
       for (int k = 0; k < 8; k += 2) {
@@ -302,53 +318,50 @@ __device__ __forceinline__ V mid_row_sum(const V* c, const uint32_t* __restrict_
 }
 
 // HIGH: the same sum by a block of 256 (thread t of the reference's block);
-// part: 256 values of shared memory.  The sum is in thread 0.  Eight gathers
-// are in flight, in the last batch too (empty slots add +0.0).
-template <class V, bool COH, bool SOFT, bool PRE>
-__device__ __forceinline__ V high_thread_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t t,
-                                             bool& bad) {
+// part: 256 values of shared memory.  The sum is in thread 0.  Eight gathers are
+// in flight, in the last batch too (empty slots add +0.0).  By FP64 adds alone: a
+// thread's adds wait for one another, and soft_add's take longer (79 cycles against
+// 65).  Static with half of them soft | so, ms: a star of 1M in the cooperative loop
+// 13.2 | 9.0, launched 20.3 | 10.8, R-MAT 2^18 with 64 edges a vertex 4.8 | 5.1 (5.2
+// and 3.7 once its rows of 1025 to 4096 go by warp).
+template <class V, bool COH, bool PRE>
+__device__ __forceinline__ V high_thread_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t t) {
   V acc = V(0);
   uint32_t u[8];
   auto ids = [&](uint32_t base) {
+    if (base + 8 * 256 <= d) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint32_t j = base + 256 * k + t;
-      u[k] = j < d ? __ldg(ed + j) : 0u;
+      for (int k = 0; k < 8; ++k) u[k] = __ldg(ed + base + 256 * k + t);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) u[k] = base + 256 * k + t < d ? __ldg(ed + base + 256 * k + t) : 0u;
     }
   };
   if (PRE) ids(0);
-  for (uint32_t base = 0; base < d; base += 8 * 256) {
+  uint32_t base = 0;
+  for (; base + 8 * 256 <= d; base += 8 * 256) {
+    if (!PRE) ids(base);
+    V x[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = load_c<COH>(c + u[k]);
+    if (PRE) ids(base + 8 * 256);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) acc += x[k];
+  }
+  if (base < d) {
     if (!PRE) ids(base);
     V x[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) x[k] = base + 256 * k + t < d ? load_c<COH>(c + u[k]) : V(0);
-    if (PRE) ids(base + 8 * 256);
-    if (SOFT) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k) bad = bad || (base + 256 * k + t < d && soft_out_of_range(x[k]));
-    }
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      if (base + 256 * k < d) {
-        if (SOFT && k < 4) acc = plus<SOFT>(acc, x[k]);
-        else acc += x[k];
-      }
+      if (base + 256 * k < d) acc += x[k];
   }
   return acc;
 }
 template <class V, bool COH, bool PRE>
 __device__ __forceinline__ V high_row_sum(const V* c, const uint32_t* __restrict__ ed, uint32_t d, uint32_t t, V* part) {
-  constexpr bool SOFT = std::is_same<V, double>::value;
-  bool bad = false;
-  V acc = high_thread_sum<V, COH, SOFT, PRE>(c, ed, d, t, bad);
-  if constexpr (SOFT) {
-    if (__syncthreads_or(bad)) {
-      acc = 0.0;
-#pragma unroll 1
-      for (uint32_t j = t; j < d; j += 256) acc += load_c<COH>(c + __ldg(ed + j));
-    }
-  }
-  part[t] = acc;
+  part[t] = high_thread_sum<V, COH, PRE>(c, ed, d, t);
   __syncthreads();
   if (t < 128) part[t] += part[t + 128];
   __syncthreads();
