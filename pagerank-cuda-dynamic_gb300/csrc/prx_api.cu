@@ -641,7 +641,8 @@ static int solve_core(prx_context* c, prx_graph* gr, int mode, const uint32_t* d
   if (route.persist) {
     bool have = false;
     TRY_CUDA_ST(ensure_plan(gr->g, c->sms, c->stream, &have));
-    if (!have) route = route_without(g, o);
+    // (the refinement sums rows of up to mid_max ids as a warp does)
+    if (!have || (refine && g.mid_max < g.plan_info.mid_max)) route = route_without(g, o);
   }
   const bool persist = route.persist, by_words = route.by_words, hot_ok = route.hot;
   if (hot_ok) {

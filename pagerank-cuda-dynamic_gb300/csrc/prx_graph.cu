@@ -1022,6 +1022,26 @@ cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s) {
   return e;
 }
 
+cudaError_t build_plan_lists(const uint32_t* off, uint32_t shift, uint32_t n, uint32_t* list,
+                             uint32_t begin[NCLS + 1], PlanInfo* info, int sms, cudaStream_t s) {
+  uint64_t edges[NCLS] = {0, 0, 0};
+  *info = PlanInfo();
+  info->mid_max = kPlanMid;
+  cudaError_t e = build_class_lists(off, shift, n, kPlanMid, list, begin, edges, sms, s);
+  if (e != cudaSuccess) return e;
+  const uint32_t nlong = begin[NCLS] - begin[HIGH];
+  if (nlong > kPlanManyLong * (uint32_t)sms) {
+    info->mid_max = kPlanMidMany;
+    e = build_class_lists(off, shift, n, kPlanMidMany, list, begin, edges, sms, s);
+    if (e != cudaSuccess) return e;
+    info->mid_long = nlong - (begin[NCLS] - begin[HIGH]);
+  }
+  info->solo = edges[HIGH] > (uint64_t)kSoloRow * (begin[NCLS] - begin[HIGH]);
+  info->low_edges = edges[LOW];
+  uint32_t* mid = list + begin[MID];
+  return sort_by_length(off, shift, mid, begin[HIGH] - begin[MID], info->mid_max, mid, sms, s);
+}
+
 static cudaError_t build_plan(GraphDev& g, int sms, cudaStream_t s) {
   if (g.n == 0) return cudaSuccess;
   if (mixed_lengths(g)) {
@@ -1030,12 +1050,8 @@ static cudaError_t build_plan(GraphDev& g, int sms, cudaStream_t s) {
   }
   if (g.plan_built) return cudaSuccess;
   cudaError_t e = g.plan_list ? cudaSuccess : graph_alloc(&g.plan_list, sizeof(uint32_t) * g.n, s);
-  uint64_t edges[NCLS];
   if (e == cudaSuccess)
-    e = build_class_lists(g.xtoff, g.seg_shift, g.n, kPlanMid, g.plan_list, g.plan_begin, edges, sms, s);
-  uint32_t* mid = g.plan_list + g.plan_begin[MID];
-  if (e == cudaSuccess)
-    e = sort_by_length(g.xtoff, g.seg_shift, mid, g.plan_begin[HIGH] - g.plan_begin[MID], kPlanMid, mid, sms, s);
+    e = build_plan_lists(g.xtoff, g.seg_shift, g.n, g.plan_list, g.plan_begin, &g.plan_info, sms, s);
   g.plan_built = e == cudaSuccess;
   return e;
 }

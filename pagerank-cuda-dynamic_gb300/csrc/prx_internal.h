@@ -124,6 +124,14 @@ struct WordView {
   const uint4* grp = nullptr;     // null: not used
 };
 
+// What a plan's rows are like (build_plan_lists).
+struct PlanInfo {
+  uint32_t mid_max = 0;           // the MID / HIGH boundary taken
+  uint32_t mid_long = 0;          // MID rows longer than kPlanMid, the first of them
+  bool solo = false;              // the HIGH rows are longer than kSoloRow on average (see WarpShare)
+  uint64_t low_edges = 0;
+};
+
 struct GraphDev {
   WordRows words[2];              // plain ids, hot sources encoded (GraphDev::hot_idx)
   int device = 0;                 // device holding the arrays
@@ -184,6 +192,7 @@ struct GraphDev {
   bool len_built = false;
   uint32_t* plan_list = nullptr;
   uint32_t plan_begin[NCLS + 1] = {0, 0, 0, 0};
+  PlanInfo plan_info;
   bool plan_built = false;
   // batched personalized PageRank picks of prx_autotune_ppr (0: defaults):
   // rows of in-degree above ppr_low_max are cut into ppr_seg-edge segments
@@ -204,6 +213,7 @@ struct GraphDev {
   uint32_t ocls_mid = 0;          // the mid_max they were built with
   uint32_t* oplan_list = nullptr;
   uint32_t oplan_begin[NCLS + 1] = {0, 0, 0, 0};
+  PlanInfo oplan_info;
   bool oplan_built = false;       // for this version of the classes
   bool oplan_have = false, oplan_fits = false;  // of the weights that are set
   uint32_t* tpos = nullptr;       // laid out like xedg; positions relative to the in-CSR's row segment
@@ -343,6 +353,17 @@ cudaError_t ensure_len_list(GraphDev& g, int sms, cudaStream_t s);  // GraphDev:
 // are launched class by class then).
 cudaError_t ensure_plan(GraphDev& g, int sms, cudaStream_t s, bool* have);
 constexpr uint32_t kPlanMid = 1024;
+// Rows of 1025 to 4096 go by warp like the MID ones where more than kPlanManyLong
+// an SM are longer than kPlanMid: a block synchronizes five times a row, which pays
+// while there are few.  Static, ms, by block | by warp: 20000 rows of 1500 0.66 |
+// 0.35 (the adjoint 19.6 | 7.2), R-MAT 2^18 of 64 edges a vertex 4.8 | 3.7, 2^20 of
+// 16 6.9 | 6.2; R-MAT 2^16 of 64 (a few hundred of them) 1.58 | 1.93, of 16 0.88 |
+// 1.27.
+constexpr uint32_t kPlanMidMany = 4096, kPlanManyLong = 6, kSoloRow = 16384;
+// The ids of the rows of `off` by class with that boundary, the MID ones longest
+// first.
+cudaError_t build_plan_lists(const uint32_t* off, uint32_t shift, uint32_t n, uint32_t* list,
+                             uint32_t begin[NCLS + 1], PlanInfo* info, int sms, cudaStream_t s);
 // Largest graphs it takes, in units of a MID row or 32 LOW rows: in id order
 // and by length.
 // Static, us an iteration, launched | persistent: in id order web-like 200k 40 |

@@ -38,6 +38,7 @@ struct PersistRows {
   const uint32_t* list;  // nmid MID ids, then nlong longer ones (GraphDev::plan_list)
   uint32_t nlow, nmid, nlong;
   bool sorted;           // whether the LOW rows go by `low`, or word by word
+  bool solo;             // see WarpShare
 };
 
 // Expansion of the changed vertices (nf[p]) into nxt, whichever way
@@ -151,8 +152,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
   if (st->done) return;
   const uint32_t lane = lane_id(), t = threadIdx.x;
   const RowTree tree{s_tree[t >> 5]};
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t warp = warps - 1 - ((blockIdx.x * blockDim.x + t) >> 5);
+  const WarpShare share(rows.nlong, rows.solo);
+  const uint32_t warps = share.warps, warp = share.warp;
   const uint32_t words = (a.n + 31) >> 5;
   const uint32_t units = rows.nmid + (rows.sorted ? (rows.nlow + 31) / 32 : words);
   const int max_iter = st->max_iter;
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
       }
       return cw;
     };
-    for (uint32_t i = blockIdx.x; i < rows.nlong; i += gridDim.x) {
+    for (uint32_t i = share.row; i < rows.nlong; i += gridDim.x) {
       const uint32_t v = __ldg(rows.list + rows.nmid + i);
       if (!affected(v)) continue;
       const uint32_t s = __ldg(a.xtoff + v), d = __ldg(a.xtoff + v + 1) - s;
@@ -335,8 +336,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist(SolveArgs a, PersistRow
       break;
     }
     if (T::FRONTIER && s_nf) {  // no vertex to expand: no second barrier either
-      if (expand_by_pull(s_nf, s_marked, a.n, a.pull_threshold)) persist_pull(a, rows, a.nf[p], nxt, warp, warps);
-      else persist_push(a, a.nf[p], nxt, s_xb, warp, warps);
+      if (expand_by_pull(s_nf, s_marked, a.n, a.pull_threshold)) persist_pull(a, rows, a.nf[p], nxt, share.any, share.all);
+      else persist_push(a, a.nf[p], nxt, s_xb, share.any, share.all);
       if (!bar.sync([] {})) return;
     }
   }
@@ -391,8 +392,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist_refine(SolveArgs a, Per
   if (st->done) return;
   const uint32_t lane = lane_id(), t = threadIdx.x;
   const RowTree tree{s_tree[t >> 5]};
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t warp = warps - 1 - ((blockIdx.x * blockDim.x + t) >> 5);
+  const WarpShare share(rows.nlong, rows.solo);
+  const uint32_t warps = share.warps, warp = share.warp;
   const uint32_t words = (a.n + 31) >> 5;
   const uint32_t units = rows.nmid + (rows.sorted ? (rows.nlow + 31) / 32 : words);
   const int max_iter = st->max_iter;
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist_refine(SolveArgs a, Per
       const unsigned long long ev = finish_vertex<MODE_REFINE64>(a, v, x, 0, survive, changed, mag, in);
       emax = ev > emax ? ev : emax;
     };
-    for (uint32_t i = blockIdx.x; i < rows.nlong; i += gridDim.x) {
+    for (uint32_t i = share.row; i < rows.nlong; i += gridDim.x) {
       const uint32_t v = __ldg(rows.list + rows.nmid + i);
       const uint32_t s = __ldg(a.xtoff + v), d = __ldg(a.xtoff + v + 1) - s;
       const VertexIn in{__ldg(a.xtdat + v), 0ull, a.r[0][v]};
@@ -505,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_persist_refine(SolveArgs a, Per
       emax = max(emax, __float_as_uint(fabsf(en - old)));
       mag = max(mag, __float_as_uint(fabsf(en)));
     };
-    for (uint32_t i = blockIdx.x; i < rows.nlong; i += gridDim.x) {
+    for (uint32_t i = share.row; i < rows.nlong; i += gridDim.x) {
       const uint32_t v = __ldg(rows.list + rows.nmid + i);
       const uint32_t s = __ldg(a.xtoff + v), d = __ldg(a.xtoff + v + 1) - s;
       const uint32_t* __restrict__ ed = a.xtedg + s;
@@ -667,7 +668,7 @@ static cudaError_t persist_t(const SolveArgs& a, const PersistRows& rows, int sm
 
 static PersistRows persist_rows(const GraphDev& g) {
   return {g.len_list, g.plan_list + g.plan_begin[MID], g.plan_begin[MID], g.plan_begin[HIGH] - g.plan_begin[MID],
-          g.plan_begin[NCLS] - g.plan_begin[HIGH], mixed_lengths(g)};
+          g.plan_begin[NCLS] - g.plan_begin[HIGH], mixed_lengths(g), g.plan_info.solo};
 }
 
 cudaError_t launch_persist_refine(const SolveArgs& a, const GraphDev& g, int sms, cudaStream_t s) {

@@ -66,6 +66,7 @@ struct PullArgs {
   const uint32_t* plan;
   const uint32_t* plan_low;
   uint32_t plan_begin[NCLS + 1];
+  bool solo;
 };
 
 __device__ __forceinline__ const double* pull_src(const PullArgs& a) {
@@ -199,8 +200,8 @@ __global__ void __launch_bounds__(256, 3) k_pull_persist(PullArgs a, const uint3
   if (st->done) return;
   const uint32_t lane = lane_id(), t = threadIdx.x;
   const RowTree tree{s_tree[t >> 5]};
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t warp = warps - 1 - ((blockIdx.x * blockDim.x + t) >> 5);
+  const WarpShare share(a.begin[NCLS] - a.begin[HIGH], a.solo);
+  const uint32_t warps = share.warps, warp = share.warp;
   const uint32_t nlow = a.begin[MID] - a.begin[LOW], nmid = a.begin[HIGH] - a.begin[MID];
   const uint32_t units = nmid + (nlow + 31) / 32;
   const uint32_t low0 = warp < nmid ? warp + (nmid - warp + warps - 1) / warps * warps : warp;
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(256, 3) k_pull_persist(PullArgs a, const uint3
       }
       return acc;
     };
-    for (uint32_t i = a.begin[HIGH] + blockIdx.x; i < a.begin[NCLS]; i += gridDim.x) {
+    for (uint32_t i = a.begin[HIGH] + share.row; i < a.begin[NCLS]; i += gridDim.x) {
       const PullRow r = pull_row(a, __ldg(a.list + i));
       double acc = strided(r, t, 256, (r.len + 255) / 256);
 #pragma unroll
@@ -406,10 +407,9 @@ __device__ __forceinline__ double checked_weight(float x, uint32_t* err) {
 // average), and one hub's row kept its warp busy for 2.5 ms.  Now rows of up
 // to 64 edges go by thread (in order of length where they mix), the next ones
 // by warp, longer ones by block (k_weight_sums, k_weight_edges), with one
-// reciprocal per row and three FP64 operations per edge.  list: the row ids by
-// class, begin: their bounds.
+// reciprocal per row and three FP64 operations per edge.
 struct WeightRows {
-  const uint32_t* list;
+  const uint32_t *low, *mid;
   uint32_t nlow, nmid;
 };
 
@@ -420,9 +420,9 @@ __global__ void __launch_bounds__(256) k_set_weights(WeightCsr c, WeightRows row
   const uint32_t units = rows.nmid + (rows.nlow + 31) / 32;
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < units; i += warps) {
     const bool mid = i < rows.nmid;
-    const uint32_t at = mid ? rows.nlow + i : 32 * (i - rows.nmid) + lane;
+    const uint32_t at = mid ? i : 32 * (i - rows.nmid) + lane;
     if (!mid && at >= rows.nlow) continue;
-    const uint32_t u = rows.list[at], first = mid ? lane : 0, step = mid ? 32 : 1;
+    const uint32_t u = (mid ? rows.mid : rows.low)[at], first = mid ? lane : 0, step = mid ? 32 : 1;
     const uint64_t iu = seg_index(u, c.shift);
     const uint32_t s = c.xoff[iu], e = c.xoff[iu + 1];
     const uint64_t bu = c.xbase ? c.xbase[(uint64_t)u >> c.shift] : 0;  // device position of the row's segment
@@ -568,36 +568,38 @@ constexpr int kLongPieces = 8;
 
 // The out-rows by class that the weights and their gradients go by: oplan_list,
 // or ocls_list when there was no memory for it.
+// LOW ids, MID ones up to mid_max, then the longer ones in two pieces (of oplan_list
+// the first MID rows and the HIGH ones).
 struct OutRows {
-  const uint32_t *list, *begin;
+  const uint32_t *low, *mid, *longs[2];
+  uint32_t nlow, nmid, nlong[2];
   uint32_t mid_max;
 };
 static OutRows out_rows(const GraphDev& g) {
-  return g.oplan_have ? OutRows{g.oplan_list, g.oplan_begin, kPlanMid}
-                      : OutRows{g.ocls_list, g.ocls_begin, g.ocls_mid};
+  const uint32_t* list = g.oplan_have ? g.oplan_list : g.ocls_list;
+  const uint32_t* begin = g.oplan_have ? g.oplan_begin : g.ocls_begin;
+  const uint32_t skip = g.oplan_have ? g.oplan_info.mid_long : 0, nmid = begin[HIGH] - begin[MID];
+  return {list, list + begin[MID] + skip, {list + begin[MID], list + begin[HIGH]}, begin[MID], nmid - skip,
+          {skip, begin[NCLS] - begin[HIGH]}, g.oplan_have ? kPlanMid : g.ocls_mid};
 }
 
 // GraphDev::oplan_list, its order and oplan_fits; ocls_list is there.
 static cudaError_t build_out_plan(GraphDev& g, uint64_t padded, int sms, cudaStream_t s) {
   cudaError_t e = g.oplan_list ? cudaSuccess : device_alloc(&g.oplan_list, sizeof(uint32_t) * (g.n ? g.n : 1));
-  uint64_t edges[NCLS] = {0, 0, 0};
   if (e == cudaSuccess)
-    e = build_class_lists(g.xoff, g.seg_shift, g.n, kPlanMid, g.oplan_list, g.oplan_begin, edges, sms, s);
-  const bool mixed = padded > 2 * edges[LOW];  // as for the in-edges
+    e = build_plan_lists(g.xoff, g.seg_shift, g.n, g.oplan_list, g.oplan_begin, &g.oplan_info, sms, s);
+  const bool mixed = padded > 2 * g.oplan_info.low_edges;  // as for the in-edges
   if (e == cudaSuccess && mixed)
     e = sort_by_length(g.xoff, g.seg_shift, g.ocls_list, g.ocls_begin[MID], kLowMax, g.oplan_list, sms, s);
-  if (e == cudaSuccess) {
-    uint32_t* mid_rows = g.oplan_list + g.oplan_begin[MID];
-    e = sort_by_length(g.xoff, g.seg_shift, mid_rows, g.oplan_begin[HIGH] - g.oplan_begin[MID], kPlanMid, mid_rows,
-                       sms, s);
-  }
   g.oplan_fits = plan_fits(g.n, g.oplan_begin[MID], mixed);
   g.oplan_built = g.oplan_have = e == cudaSuccess;
   return e;
 }
 
 // The persistent loop's rows of a, for graphs up to the lines of persist_fits.
-static void take_plan(PullArgs& a, const uint32_t* list, const uint32_t* low, const uint32_t begin[NCLS + 1]) {
+static void take_plan(PullArgs& a, const uint32_t* list, const uint32_t* low, const uint32_t begin[NCLS + 1],
+                      bool solo) {
+  a.solo = solo;
   a.plan = list;
   a.plan_low = low;
   for (int k = 0; k <= NCLS; ++k) a.plan_begin[k] = begin[k];
@@ -719,14 +721,15 @@ static int set_weights(prx_context* c, GraphDev& g, const float* w) {
   if (g.n) {
     const bool found = g.tpos_built;
     const OutRows out = out_rows(g);
-    const WeightRows by_class = {out.list, out.begin[MID], out.begin[HIGH] - out.begin[MID]};
+    const WeightRows by_class = {out.low, out.mid, out.nlow, out.nmid};
     const uint64_t units = by_class.nmid + (by_class.nlow + 31ull) / 32;
     k_set_weights<<<pull_grid(units * 32, 256, c->sms * 8), 256, 0, s>>>(weight_csr(g), by_class, w, found, g.wsum,
                                                                          g.px, g.pt, &c->st->err);
-    if (const uint32_t nl = out.begin[NCLS] - out.begin[HIGH]) {
-      const uint32_t* rows = out.list + out.begin[HIGH];
-      k_weight_sums<<<nl, 256, 0, s>>>(weight_csr(g), w, rows, g.wsum, &c->st->err);
-      k_weight_edges<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), w, rows, found, g.wsum, g.px, g.pt,
+    for (int k = 0; k < 2; ++k) {
+      const uint32_t nl = out.nlong[k];
+      if (!nl) continue;
+      k_weight_sums<<<nl, 256, 0, s>>>(weight_csr(g), w, out.longs[k], g.wsum, &c->st->err);
+      k_weight_edges<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), w, out.longs[k], found, g.wsum, g.px, g.pt,
                                                           &c->st->err);
     }
   }
@@ -780,7 +783,7 @@ int prx_solve_weighted(prx_context* c, prx_graph* gr, const double* t, const dou
   PullArgs a = forward_args(g, t, o.damping);
   bool plan = persist_fits(g);
   if (plan) TRY_CUDA_ST(ensure_plan(gr->g, c->sms, s, &plan));
-  if (plan) take_plan(a, g.plan_list, mixed_lengths(g) ? g.len_list : g.plan_list, g.plan_begin);
+  if (plan) take_plan(a, g.plan_list, mixed_lengths(g) ? g.len_list : g.plan_list, g.plan_begin, g.plan_info.solo);
   a.x[0] = c->wk;
   a.x[1] = c->wk + g.n;
   const uint64_t l0 = c->launches;
@@ -837,7 +840,7 @@ int prx_adjoint(prx_context* c, prx_graph* gr, const double* t, const double* r,
   a.shift = g.seg_shift;
   a.list = g.ocls_list;
   for (int k = 0; k <= NCLS; ++k) a.begin[k] = g.ocls_begin[k];
-  if (g.oplan_have && g.oplan_fits) take_plan(a, g.oplan_list, g.oplan_list, g.oplan_begin);
+  if (g.oplan_have && g.oplan_fits) take_plan(a, g.oplan_list, g.oplan_list, g.oplan_begin, g.oplan_info.solo);
   a.base = gl;
   a.base_scale = 1.0;
   a.alpha = alpha;
@@ -858,9 +861,11 @@ int prx_adjoint(prx_context* c, prx_graph* gr, const double* t, const double* r,
     const OutRows out = out_rows(g);
     k_grad_w<<<grid, 256, 0, s>>>(weight_csr(g), g.wsum, r, lam, gl, alpha, g.n, out.mid_max, grad_w);
     c->launches += 1;
-    if (const uint32_t nl = out.begin[NCLS] - out.begin[HIGH]) {
-      k_grad_w_long<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), out.list + out.begin[HIGH], g.wsum, r, lam, gl,
-                                                         alpha, grad_w);
+    for (int k = 0; k < 2; ++k) {
+      const uint32_t nl = out.nlong[k];
+      if (!nl) continue;
+      k_grad_w_long<<<dim3(nl, kLongPieces), 256, 0, s>>>(weight_csr(g), out.longs[k], g.wsum, r, lam, gl, alpha,
+                                                         grad_w);
       c->launches += 1;
     }
   }
