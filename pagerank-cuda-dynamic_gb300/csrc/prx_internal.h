@@ -211,6 +211,7 @@ struct GraphDev {
   uint32_t ocls_begin[NCLS + 1] = {0, 0, 0, 0};
   uint64_t ocls_edges[NCLS] = {0, 0, 0};
   uint32_t ocls_mid = 0;          // the mid_max they were built with
+  bool oside = false;             // weights of LOW rows by eight lanes (k_set_weights)
   uint32_t* oplan_list = nullptr;
   uint32_t oplan_begin[NCLS + 1] = {0, 0, 0, 0};
   PlanInfo oplan_info;

@@ -407,24 +407,31 @@ __device__ __forceinline__ double checked_weight(float x, uint32_t* err) {
 // average), and one hub's row kept its warp busy for 2.5 ms.  Now rows of up
 // to 64 edges go by thread (in order of length where they mix), the next ones
 // by warp, longer ones by block (k_weight_sums, k_weight_edges), with one
-// reciprocal per row and three FP64 operations per edge.
+// reciprocal per row and three FP64 operations per edge.  L lanes take a row of up
+// to 64: eight where they are four edges long and more (a lane alone reads its row
+// piece by piece: 31M edges in even rows of 30 5.1 ms, R-MAT 2^18 0.29; by eight
+// 1.29 and 0.18), one for shorter ones (rows of 3 0.09 | 0.26) and for rows of
+// mixed lengths past L2 (R-MAT 2^20 0.70 | 0.78).
+constexpr uint32_t kSideMixed = 1u << 19;
 struct WeightRows {
   const uint32_t *low, *mid;
   uint32_t nlow, nmid;
 };
 
+template <uint32_t L>
 __global__ void __launch_bounds__(256) k_set_weights(WeightCsr c, WeightRows rows, const float* __restrict__ w,
                                                      bool found, double* __restrict__ wsum, double* __restrict__ px,
                                                      double* __restrict__ pt, uint32_t* err) {
   const uint32_t lane = lane_id(), warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t units = rows.nmid + (rows.nlow + 31) / 32;
+  constexpr uint32_t G = 32 / L;  // LOW rows side by side
+  const uint32_t units = rows.nmid + (rows.nlow + G - 1) / G;
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < units; i += warps) {
     const bool mid = i < rows.nmid;
-    const uint32_t at = mid ? i : 32 * (i - rows.nmid) + lane;
-    if (!mid && at >= rows.nlow) continue;
-    const uint32_t u = (mid ? rows.mid : rows.low)[at], first = mid ? lane : 0, step = mid ? 32 : 1;
+    const uint32_t at = mid ? i : G * (i - rows.nmid) + lane / L;
+    const bool row = mid || at < rows.nlow;
+    const uint32_t u = row ? (mid ? rows.mid : rows.low)[at] : 0u, first = mid ? lane : lane % L, step = mid ? 32 : L;
     const uint64_t iu = seg_index(u, c.shift);
-    const uint32_t s = c.xoff[iu], e = c.xoff[iu + 1];
+    const uint32_t s = row ? c.xoff[iu] : 0u, e = row ? c.xoff[iu + 1] : 0u;
     const uint64_t bu = c.xbase ? c.xbase[(uint64_t)u >> c.shift] : 0;  // device position of the row's segment
     const uint64_t wu = c.wseg ? c.wseg[(uint64_t)u >> c.shift] : 0;    // its compact position
     double acc = 0.0;
@@ -432,8 +439,11 @@ __global__ void __launch_bounds__(256) k_set_weights(WeightCsr c, WeightRows row
     if (mid) {
 #pragma unroll
       for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    } else {
+#pragma unroll
+      for (int o = L / 2; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     }
-    if (!mid || lane == 0) wsum[u] = acc;
+    if (row && first == 0) wsum[u] = acc;
     const double y = 1.0 / acc;
     for (uint32_t j = s + first; j < e; j += step)
       put_weight(c, u, bu + j, div_by(widen(w[wu + j]), acc, y), found, px, pt, err);
@@ -714,6 +724,8 @@ static int set_weights(prx_context* c, GraphDev& g, const float* w) {
     TRY_CUDA_ST(build_class_lists(g.xoff, g.seg_shift, g.n, g.mid_max, g.ocls_list, g.ocls_begin, g.ocls_edges,
                                   c->sms, s, &padded));
     g.ocls_mid = g.mid_max;
+    g.oside = g.ocls_edges[LOW] >= 4ull * g.ocls_begin[MID] &&
+              (padded <= 2 * g.ocls_edges[LOW] || g.n <= kSideMixed);
     const cudaError_t e = build_out_plan(g, padded, c->sms, s);
     if (e != cudaErrorMemoryAllocation) TRY_CUDA_ST(e);
   }
@@ -722,9 +734,10 @@ static int set_weights(prx_context* c, GraphDev& g, const float* w) {
     const bool found = g.tpos_built;
     const OutRows out = out_rows(g);
     const WeightRows by_class = {out.low, out.mid, out.nlow, out.nmid};
-    const uint64_t units = by_class.nmid + (by_class.nlow + 31ull) / 32;
-    k_set_weights<<<pull_grid(units * 32, 256, c->sms * 8), 256, 0, s>>>(weight_csr(g), by_class, w, found, g.wsum,
-                                                                         g.px, g.pt, &c->st->err);
+    const uint64_t units = by_class.nmid + (by_class.nlow + (g.oside ? 3ull : 31ull)) / (g.oside ? 4 : 32);
+    const int grid = pull_grid(units * 32, 256, c->sms * 8);
+    if (g.oside) k_set_weights<8><<<grid, 256, 0, s>>>(weight_csr(g), by_class, w, found, g.wsum, g.px, g.pt, &c->st->err);
+    else k_set_weights<1><<<grid, 256, 0, s>>>(weight_csr(g), by_class, w, found, g.wsum, g.px, g.pt, &c->st->err);
     for (int k = 0; k < 2; ++k) {
       const uint32_t nl = out.nlong[k];
       if (!nl) continue;
