@@ -372,8 +372,17 @@ cudaError_t build_plan_lists(const uint32_t* off, uint32_t shift, uint32_t n, ui
 // (31,000) 30 | 25, 1400^2 (61,000) 51 | 58; by length R-MAT 2^16 47 | 14, 2^18
 // 78 | 29, 2^21 (145,000) 375 | 219, 2^23 (630,000) 1254 | 991.
 constexpr uint64_t kPersistUnits = 48u << 10, kPersistSortedUnits = 1u << 20;
-inline bool plan_fits(uint32_t n, uint32_t low, bool mixed) {
-  return ((uint64_t)(mixed ? low : n) + 31) / 32 + (n - low) <= (mixed ? kPersistSortedUnits : kPersistUnits);
+// Past kPersistUnits the order by length costs a row scattered offsets and ranks
+// and pays only where it saves many steps: padded is what the LOW edges (edges)
+// would be, had every row of 32 neighbours the longest one's length (2.1 to 2.3
+// times as many for in-degrees of 2 and 3 at random, 3.8 to 4.4 for R-MAT).
+// Static, ms, launched | persistent: 12M vertices of 1 random edge 9.7 | 20.2, of 2
+// edges 12.7 | 30.5; 2^21 vertices 2.33 | 2.60, 2.88 | 3.61; 2^20 1.31 | 0.92, 1.73 |
+// 1.29.  R-MAT 2^23 of 2 edges 27.3 | 18.6, 2^21 9.7 | 4.4.
+inline bool plan_fits(uint32_t n, uint32_t low, uint64_t edges, uint64_t padded) {
+  const bool mixed = padded > 2 * edges;  // mixed_lengths
+  return ((uint64_t)(mixed ? low : n) + 31) / 32 + (n - low) <=
+         (padded > 3 * edges ? kPersistSortedUnits : kPersistUnits);
 }
 // Graphs whose LOW rows the launched sweep takes by words (words_fit), rows of
 // even length: web-like 0.6M vertices (18,750 units) 76 | 82, 0.8M 98 | 98, 1.1M
@@ -381,7 +390,7 @@ inline bool plan_fits(uint32_t n, uint32_t low, bool mixed) {
 // 156 | 129; but laying the words out costs a graph that is solved once about
 // what is gained at 1.1M.
 constexpr uint64_t kPersistWordUnits = 32u << 10;
-inline bool persist_fits(const GraphDev& g) { return plan_fits(g.n, g.cls_begin[MID], mixed_lengths(g)); }
+inline bool persist_fits(const GraphDev& g) { return plan_fits(g.n, g.cls_begin[MID], g.cls_edges[LOW], g.low_padded); }
 // The whole FP64 iteration loop of a plain graph (one row segment) as one
 // cooperative kernel from the ranks in parity 0 (prx_persist.cu); ensure_plan
 // first.

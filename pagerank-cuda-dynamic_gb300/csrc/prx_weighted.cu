@@ -601,7 +601,7 @@ static cudaError_t build_out_plan(GraphDev& g, uint64_t padded, int sms, cudaStr
   const bool mixed = padded > 2 * g.oplan_info.low_edges;  // as for the in-edges
   if (e == cudaSuccess && mixed)
     e = sort_by_length(g.xoff, g.seg_shift, g.ocls_list, g.ocls_begin[MID], kLowMax, g.oplan_list, sms, s);
-  g.oplan_fits = plan_fits(g.n, g.oplan_begin[MID], mixed);
+  g.oplan_fits = plan_fits(g.n, g.oplan_begin[MID], g.oplan_info.low_edges, padded);
   g.oplan_built = g.oplan_have = e == cudaSuccess;
   return e;
 }
