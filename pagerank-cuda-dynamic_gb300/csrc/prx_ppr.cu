@@ -60,6 +60,8 @@ namespace prx {
 constexpr int kCols = 64;         // vectors per column block at most
 constexpr uint32_t kSeg = 512;    // default in-edges per segment of a long row
 constexpr uint32_t kSegParts = 8; // parts of a segment, summed side by side
+constexpr uint32_t kSpread = 4;   // segments of a row past which blocks combine it
+constexpr uint32_t kSlice = 8;    // lanes of a row that such a block takes
 
 enum PprMode { PPR_J64 = 0, PPR_R64 = 1, PPR_S32 = 2 };
 
@@ -74,7 +76,7 @@ struct PprWs {
   size_t part_cap = 0;
   uint2* parts = nullptr;              // vertex, first edge
   size_t parts_cap = 0;
-  uint32_t* partstart = nullptr;       // first part of each long vertex (+ total)
+  uint32_t* partstart = nullptr;       // first part of each long vertex (+ total), PprArgs::longs
   size_t partstart_cap = 0;
   uint32_t* big = nullptr;             // vertices above a low_max other than 64, and their scan
   size_t big_cap = 0;
@@ -129,6 +131,8 @@ struct PprArgs {
   const uint32_t* partstart;      // [nbig + 1]: each long row's first partial row
   const uint2* parts;             // vertex, first edge (relative to its row segment)
   uint32_t nparts;
+  const uint32_t* longs;          // positions in big of the rows of more than spread partial rows
+  uint32_t nlong, spread;
   double* part;                   // the partial rows
   State* st;
   uint32_t n;
@@ -597,48 +601,94 @@ __global__ void __launch_bounds__(256) k_ppr_segments(PprArgs a) {
 
 // Long rows: a row's lanes per vertex add its segments in order, a segment
 // being its GROUP parts (fewer in the last) added in order: kSegParts, or one
-// partial row that holds their sum.
+// partial row that holds their sum.  Of rows of more than a.spread partial rows
+// (a.longs) the first blocks take kSlice lanes' columns each: their groups of
+// lanes form segments side by side and leave them in shared memory to the first
+// group, which adds them in the same order.  Solves, ms, every row by a group of
+// lanes | so, of 5 vectors in FP32, 40 in FP32 and 64 in FP64: R-MAT 2^19 8.3 | 5.3,
+// 18.2 | 15.3, 57.1 | 54.2; 100 hubs of 15,000 1.85 | 0.90, 2.56 | 1.84, 5.09 | 4.51;
+// a star of 64k 3.69 | 0.91, 3.67 | 1.36, 4.92 | 2.31.  With the line at 8 | 16
+// segments (5 vectors) R-MAT 2^19 5.4 | 5.4, 2^17 2.1 | 2.5.
 template <int MODE, int C, uint32_t GROUP>
-__global__ void __launch_bounds__(256) k_ppr_combine(PprArgs a) {
+__global__ void __launch_bounds__(256) k_ppr_combine(PprArgs a, uint32_t long_blocks) {
   using Sh = PprShape<MODE, C>;
   using S = typename Sh::S;
   using V = typename Sh::V;
   constexpr uint32_t LPR = Sh::LPR;
+  constexpr uint32_t SLICE = LPR < kSlice ? LPR : kSlice, SLICES = LPR / SLICE, SEGS = 256 / SLICE - 1;
   State* st = a.st;
   if (ppr_skip<MODE>(st)) return;
   const S* part = reinterpret_cast<const S*>(a.part);
-  const uint32_t sub = threadIdx.x % LPR;
+  uint32_t sub = threadIdx.x % LPR;
   unsigned long long dmax = 0;
   unsigned int emag = 0;
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / LPR; i < a.nbig; i += gridDim.x * blockDim.x / LPR) {
-    V acc;
+  auto segment = [&](uint32_t g, uint32_t end) {  // the sum of partial rows g .. g + GROUP - 1 (g < end)
+    V x[GROUP];
 #pragma unroll
-    for (int k = 0; k < Sh::N; ++k) acc[k] = S(0);
-    const uint32_t end = a.partstart[i + 1];
-    for (uint32_t g = a.partstart[i]; g < end; g += GROUP) {
-      V x[GROUP];
+    for (uint32_t k = 0; k < GROUP; ++k) {
+      if (g + k < end) {
+        x[k] = Sh::template load<false>(part, g + k, sub);
+      } else {
 #pragma unroll
-      for (uint32_t k = 0; k < GROUP; ++k) {
-        if (g + k < end) {
-          x[k] = Sh::template load<false>(part, g + k, sub);
-        } else {
-#pragma unroll
-          for (int j = 0; j < Sh::N; ++j) x[k][j] = S(0);
-        }
+        for (int j = 0; j < Sh::N; ++j) x[k][j] = S(0);
       }
-#pragma unroll
-      for (uint32_t k = 1; k < GROUP; ++k)
-        if (g + k < end) {
-#pragma unroll
-          for (int j = 0; j < Sh::N; ++j) x[0][j] += x[k][j];
-        }
-#pragma unroll
-      for (int k = 0; k < Sh::N; ++k) acc[k] += x[0][k];
     }
+#pragma unroll
+    for (uint32_t k = 1; k < GROUP; ++k)
+      if (g + k < end) {
+#pragma unroll
+        for (int j = 0; j < Sh::N; ++j) x[0][j] += x[k][j];
+      }
+    return x[0];
+  };
+  auto finish = [&](uint32_t i, const V& acc) {
     unsigned int em = 0;
     const unsigned long long d = ppr_finish<MODE, C>(a, st, a.big[i], acc, sub, &em);
     dmax = d > dmax ? d : dmax;
     emag = em > emag ? em : emag;
+  };
+  if (blockIdx.x < long_blocks) {
+    __shared__ V sums[2][256];
+    const uint32_t row = threadIdx.x / SLICE;  // 0: adds the segments, the others form them
+    for (uint32_t k = blockIdx.x; k < a.nlong * SLICES; k += long_blocks) {
+      const uint32_t i = a.longs[k / SLICES], end = a.partstart[i + 1];
+      sub = k % SLICES * SLICE + threadIdx.x % SLICE;
+      V acc;
+#pragma unroll
+      for (int j = 0; j < Sh::N; ++j) acc[j] = S(0);
+      uint32_t b = 0;
+      for (uint32_t g = a.partstart[i]; g < end; g += GROUP * SEGS, b ^= 1u) {
+        const uint32_t mine = g + (row - 1) * GROUP;
+        if (row && mine < end) sums[b][threadIdx.x] = segment(mine, end);
+        __syncthreads();  // (b is added up while b ^ 1 is filled)
+        if (row == 0) {
+          const uint32_t m = min(SEGS, (end - g + GROUP - 1) / GROUP);
+#pragma unroll 4
+          for (uint32_t q = 1; q <= m; ++q) {
+            const V x = sums[b][q * SLICE + threadIdx.x];
+#pragma unroll
+            for (int j = 0; j < Sh::N; ++j) acc[j] += x[j];
+          }
+        }
+      }
+      if (row == 0) finish(i, acc);
+      __syncthreads();  // before the next row's first sums
+    }
+  } else {
+    for (uint32_t i = ((blockIdx.x - long_blocks) * blockDim.x + threadIdx.x) / LPR; i < a.nbig;
+         i += (gridDim.x - long_blocks) * blockDim.x / LPR) {
+      const uint32_t end = a.partstart[i + 1], start = a.partstart[i];
+      if (end - start > a.spread) continue;
+      V acc;
+#pragma unroll
+      for (int k = 0; k < Sh::N; ++k) acc[k] = S(0);
+      for (uint32_t g = start; g < end; g += GROUP) {
+        const V x = segment(g, end);
+#pragma unroll
+        for (int k = 0; k < Sh::N; ++k) acc[k] += x[k];
+      }
+      finish(i, acc);
+    }
   }
   ppr_reduce<MODE>(st, dmax, emag);
 }
@@ -746,6 +796,13 @@ __global__ void k_ppr_partcount(const uint32_t* __restrict__ xtoff, uint32_t shi
     cnt[i] = (row_len(xtoff, shift, big[i]) + per - 1) / per;
 }
 
+// The long rows of more than `most` parts, in any order: positions and count.
+__global__ void k_ppr_longs(const uint32_t* __restrict__ start, uint32_t nbig, uint32_t most, uint32_t* count,
+                            uint32_t* __restrict__ longs) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += gridDim.x * blockDim.x)
+    if (start[i + 1] - start[i] > most) longs[atomicAdd(count, 1u)] = i;
+}
+
 // Vertices of in-degree above t: flags (n + 1 entries, the last 0) for the
 // scan, then the ascending list.
 __global__ void k_ppr_bigflags(const uint32_t* __restrict__ xtoff, uint32_t shift, uint32_t n, uint32_t t,
@@ -827,9 +884,10 @@ static void ppr_sweep_c(const PprArgs& a, int sms, cudaStream_t s, uint64_t& lau
     ++launches;
   }
   if (a.nparts) {
-    const int grid = grid_for((uint64_t)a.nbig * (32 / G), 256, sms * 8);
-    if (a.group == 1) k_ppr_combine<MODE, C, 1><<<grid, 256, 0, s>>>(a);
-    else k_ppr_combine<MODE, C, kSegParts><<<grid, 256, 0, s>>>(a);
+    const uint32_t lb = std::min<uint32_t>(a.nlong * std::max(1u, 32 / G / kSlice), 8 * sms);
+    const int grid = grid_for((uint64_t)a.nbig * (32 / G), 256, sms * 8) + lb;
+    if (a.group == 1) k_ppr_combine<MODE, C, 1><<<grid, 256, 0, s>>>(a, lb);
+    else k_ppr_combine<MODE, C, kSegParts><<<grid, 256, 0, s>>>(a, lb);
     ++launches;
   }
 }
@@ -900,15 +958,24 @@ static cudaError_t ppr_parts(prx_context* c, const GraphDev& g, PprArgs& a) {
   k_ppr_partcount<<<grid_for(a.nbig, 256, c->sms * 4), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, a.nbig, per,
                                                                     w.partstart);
   cudaError_t e = exclusive_scan_u32(w.partstart, a.nbig + 1, s);
-  uint32_t nparts = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&nparts, w.partstart + a.nbig, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+  // parts in all, rows of many of them, those rows
+  uint32_t* count = w.partstart + a.nbig;
+  a.spread = kSpread * a.group;
+  if (e == cudaSuccess) e = cudaMemsetAsync(count + 1, 0, sizeof(uint32_t), s);
+  if (e != cudaSuccess) return e;
+  k_ppr_longs<<<grid_for(a.nbig, 256, c->sms * 4), 256, 0, s>>>(w.partstart, a.nbig, a.spread, count + 1, count + 2);
+  uint32_t host[2] = {0, 0};
+  e = cudaMemcpyAsync(host, count, sizeof host, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  const uint32_t nparts = host[0];
   if (e == cudaSuccess) e = grow(&w.parts, w.parts_cap, (size_t)nparts);
   if (e == cudaSuccess) e = grow(&w.part, w.part_cap, (size_t)nparts * kCols);
   if (e != cudaSuccess) return e;
   k_ppr_partfill<<<grid_for((uint64_t)a.nbig * 32, 256, c->sms * 8), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, a.nbig,
                                                                                   per, w.partstart, w.parts);
   a.partstart = w.partstart;
+  a.longs = count + 2;
+  a.nlong = host[1];
   a.parts = w.parts;
   a.nparts = nparts;
   a.part = w.part;
@@ -937,7 +1004,7 @@ static int ppr_segments(prx_context* c, const GraphDev& g, PprArgs& a) {
   a.nbig = nbig;
   a.nparts = 0;
   if (!nbig) return PRX_OK;
-  TRY_CUDA_ST(grow(&w.partstart, w.partstart_cap, (size_t)nbig + 1));
+  TRY_CUDA_ST(grow(&w.partstart, w.partstart_cap, 2 * (size_t)nbig + 2));
   a.group = kSegParts;
   cudaError_t e = ppr_parts(c, g, a);
   if (e == cudaErrorMemoryAllocation) {
