@@ -86,7 +86,9 @@ __device__ __forceinline__ uint32_t counter_of(uint32_t v, int bits) {
 __global__ void __launch_bounds__(256) k_ing_count(const uint32_t* __restrict__ u, const uint32_t* __restrict__ v,
                                                    uint32_t count, uint32_t n, int bits,
                                                    uint32_t* __restrict__ out, uint32_t* __restrict__ in, uint32_t* __restrict__ at_out,
-                                                   uint32_t* __restrict__ at_in, uint32_t* __restrict__ bad) {
+                                                   uint32_t* __restrict__ at_in, uint32_t* __restrict__ bad,
+                                                   const uint32_t* __restrict__ heavy, uint32_t least) {
+  if (heavy && *heavy >= least) return;  // radix keys instead
   const uint32_t step = gridDim.x * blockDim.x;
   bool out_hubs = false, in_hubs = false;
   for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < count; i0 += step) {
@@ -500,7 +502,7 @@ static cudaError_t build_csr(uint32_t* raw_off, const uint32_t* u, const uint32_
 }
 
 cudaError_t build_csr_pair(GraphDev& g, const uint32_t* u, const uint32_t* v, uint32_t count, bool self_loops,
-                           bool* bad_id, int sms, cudaStream_t s) {
+                           bool* bad_id, int sms, cudaStream_t s, HeavyRows* heavy) {
   const uint32_t n = g.n;
   const uint32_t total = count + (self_loops ? n : 0);
   *bad_id = false;
@@ -525,8 +527,18 @@ cudaError_t build_csr_pair(GraphDev& g, const uint32_t* u, const uint32_t* v, ui
     k_ing_fill<<<ing_grid(2 * counters, sms), 256, 0, s>>>(cnt, 2 * counters, self_loops ? 1u : 0u);
     if (count)
       k_ing_count<<<ing_grid(count, sms), 256, 0, s>>>(u, v, count, n, bits, cnt, cnt + counters, at_out, at_in,
-                                                        lr.count + 4);
+                                                        lr.count + 4, heavy ? heavy->share : nullptr,
+                                                        heavy ? heavy->least : 0u);
     k_ing_lengths<<<ing_grid(rows, sms), 256, 0, s>>>(cnt, cnt + counters, n, bits, out, in);
+    if (e == cudaSuccess && heavy && heavy->share) {
+      e = cudaEventSynchronize(heavy->ready);  // (while the entries are counted)
+      heavy->found = e == cudaSuccess && *heavy->host >= heavy->least;
+    }
+    if (heavy && heavy->found) {
+      graph_free({ws, g.xoff, g.xtoff, g.xtdat});
+      g.xoff = g.xtoff = g.xtdat = nullptr;
+      return e;
+    }
     if (e == cudaSuccess)
       e = build_csr(out, u, v, count, n, self_loops, at_out, lr, g.xoff, g.xtdat, &g.xedg, &m, bad_id, sms, s);
     if (e == cudaSuccess && !*bad_id)

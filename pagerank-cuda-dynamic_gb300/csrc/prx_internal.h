@@ -526,8 +526,19 @@ cudaError_t exclusive_scan_u32_ws(uint32_t* data, uint32_t len, uint32_t* sums, 
 // Both CSRs and the out-degrees of g (n set, its arrays not allocated) from an
 // edge list in device memory (prx_ingest.cu), a loop on every vertex with
 // self_loops.  *bad_id: an id was out of range (the CSRs are incomplete then).
+// heavy: a sample of the list on its way; when it finds rows that radix keys are
+// faster for, nothing is built and found is set.
+struct HeavyRows {
+  uint32_t* slots = nullptr;
+  const uint32_t* share = nullptr;  // samples in such rows (null: no sample)
+  uint32_t least = 0;               // of them for the keys
+  const uint32_t* host = nullptr;   // share, after ready
+  cudaEvent_t ready = nullptr;
+  bool found = false;
+};
 cudaError_t build_csr_pair(GraphDev& g, const uint32_t* u, const uint32_t* v, uint32_t count, bool self_loops,
-                           bool* bad_id, int sms, cudaStream_t s);
+                           bool* bad_id, int sms, cudaStream_t s,
+                           HeavyRows* heavy = nullptr);
 
 // Stable LSD radix sort of keys[0 .. count) on their bits [lo, hi), 8 at a
 // time, ping-ponging with tmp (both with 2 keys of slack past count: the
