@@ -251,7 +251,10 @@ __global__ void __launch_bounds__(kThreads) k_copy_runs(Runs r, const uint32_t* 
 // A warp's 32 ids wait for three chains of dependent loads (the id, its place
 // among the deletions and among the insertions), 1 us together: rows up to 4096
 // and pieces of 1024 made the two kernels 164 us on a batch of 11k edges
-// whose sources' rows go to 100k ids, these 63.
+// whose sources' rows go to 100k ids, these 63.  Two ids a lane side by side (one in
+// rows of up to 32) leave 32 registers, so that the whole grid is resident: with
+// four, 40 registers and six of eight blocks, a million rows of 3 took 626 us
+// instead of 326.
 constexpr uint32_t kBigRow = 512;
 constexpr uint32_t kPiece = 256;
 
@@ -267,13 +270,13 @@ __device__ __forceinline__ uint32_t merge_pieces(const RowMerge& m) {
   return (m.len + kPiece - 1) / kPiece + (m.ni + kPiece - 1) / kPiece;
 }
 
-__global__ void __launch_bounds__(kThreads) k_merge_touched(Runs r, const uint32_t* __restrict__ oedg,
-                                                            uint32_t* __restrict__ nedg, const uint32_t* dv,
-                                                            const uint32_t* __restrict__ dbeg,
-                                                            const uint32_t* __restrict__ dend, const uint32_t* iv,
-                                                            const uint32_t* __restrict__ ibeg,
-                                                            const uint32_t* __restrict__ iend, uint32_t* big,
-                                                            unsigned long long* nbig) {
+__global__ void __launch_bounds__(kThreads, 8) k_merge_touched(Runs r, const uint32_t* __restrict__ oedg,
+                                                               uint32_t* __restrict__ nedg, const uint32_t* dv,
+                                                               const uint32_t* __restrict__ dbeg,
+                                                               const uint32_t* __restrict__ dend, const uint32_t* iv,
+                                                               const uint32_t* __restrict__ ibeg,
+                                                               const uint32_t* __restrict__ iend, uint32_t* big,
+                                                               unsigned long long* nbig) {
   r.load_T();
   const uint32_t lane = lane_id();
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -289,7 +292,11 @@ __global__ void __launch_bounds__(kThreads) k_merge_touched(Runs r, const uint32
       }
       continue;
     }
-    for (uint32_t j = lane; j < m.len; j += 128) m.old_ids<4>(j, m.len);
+    if (m.len <= 32) {
+      if (lane < m.len) m.old_ids<1>(lane, m.len);
+    } else {
+      for (uint32_t j = lane; j < m.len; j += 64) m.old_ids<2>(j, m.len);
+    }
     for (uint32_t k = lane; k < m.ni; k += 32) m.ins_id(k);
   }
 }
