@@ -368,9 +368,10 @@ __global__ void k_layout_counts(const uint32_t* __restrict__ lay_off, const uint
   }
 }
 
-// The touched rows' segments, a warp per row (at most kLowMax ids): an id's place
-// is the start of its chunk's segment and its rank among the row's ids of the
-// chunk.  A thread per row took 45 us of 11k rows of 36 ids, this 11.
+// The touched rows' segments, eight lanes a row (at most kLowMax ids): an id's
+// place is the start of its chunk's segment and its rank among the row's ids of the
+// chunk.  A thread per row took 45 us of 11k rows of 36 ids, a warp 11; of a million
+// rows of 3 a thread took 89, a warp 335, eight lanes 106.
 __global__ void k_layout_touched(const uint32_t* __restrict__ xtoff, const uint32_t* __restrict__ xtedg,
                                  const uint32_t* __restrict__ trow, uint32_t T, const uint32_t* Tp, uint32_t n,
                                  uint32_t width, int K, const uint32_t* __restrict__ off,
@@ -378,12 +379,12 @@ __global__ void k_layout_touched(const uint32_t* __restrict__ xtoff, const uint3
                                  uint32_t hot_words) {
   const size_t row = (size_t)n + 1;
   if (Tp) T = *Tp;
-  const uint32_t lane = lane_id();
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < T; i += (gridDim.x * blockDim.x) >> 5) {
+  const uint32_t lane = threadIdx.x & 7u;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / 8; i < T; i += gridDim.x * blockDim.x / 8) {
     const uint32_t v = trow[i];
     const uint32_t s = xtoff[v], len = xtoff[v + 1] - s;
     if (len > kLowMax) continue;
-    for (uint32_t j = lane; j < len; j += 32) {
+    for (uint32_t j = lane; j < len; j += 8) {
       const uint32_t u = xtedg[s + j], k = K == 1 ? 0u : u / width;
       const uint32_t before = k ? lower_bound_u32(xtedg + s, j, k * width) : 0u;  // the row's ids of lower chunks
       edg[off[k * row + v] + (j - before)] = layout_id(hot_idx, hot_words, u);
