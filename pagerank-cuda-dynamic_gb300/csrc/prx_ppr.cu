@@ -791,16 +791,13 @@ __global__ void k_ppr_init(PprArgs a) {
 
 // Part counts of the long vertices (ceil(indeg / per)), then the parts.
 __global__ void k_ppr_partcount(const uint32_t* __restrict__ xtoff, uint32_t shift, const uint32_t* __restrict__ big,
-                                uint32_t nbig, uint32_t per, uint32_t* __restrict__ cnt) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += gridDim.x * blockDim.x)
-    cnt[i] = (row_len(xtoff, shift, big[i]) + per - 1) / per;
-}
-
-// The long rows of more than `most` parts, in any order: positions and count.
-__global__ void k_ppr_longs(const uint32_t* __restrict__ start, uint32_t nbig, uint32_t most, uint32_t* count,
-                            uint32_t* __restrict__ longs) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += gridDim.x * blockDim.x)
-    if (start[i + 1] - start[i] > most) longs[atomicAdd(count, 1u)] = i;
+                                uint32_t nbig, uint32_t per, uint32_t most, uint32_t* __restrict__ cnt) {
+  uint32_t* longs = cnt + nbig + 1;  // their number, then they, in any order
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbig; i += gridDim.x * blockDim.x) {
+    const uint32_t parts = (row_len(xtoff, shift, big[i]) + per - 1) / per;
+    cnt[i] = parts;
+    if (parts > most) longs[1 + atomicAdd(longs, 1u)] = i;
+  }
 }
 
 // Vertices of in-degree above t: flags (n + 1 entries, the last 0) for the
@@ -955,15 +952,14 @@ static cudaError_t ppr_parts(prx_context* c, const GraphDev& g, PprArgs& a) {
   PprWs& w = *c->ppr;
   cudaStream_t s = c->stream;
   const uint32_t per = a.seg / a.group;
-  k_ppr_partcount<<<grid_for(a.nbig, 256, c->sms * 4), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, a.nbig, per,
-                                                                    w.partstart);
-  cudaError_t e = exclusive_scan_u32(w.partstart, a.nbig + 1, s);
-  // parts in all, rows of many of them, those rows
-  uint32_t* count = w.partstart + a.nbig;
   a.spread = kSpread * a.group;
-  if (e == cudaSuccess) e = cudaMemsetAsync(count + 1, 0, sizeof(uint32_t), s);
+  uint32_t* count = w.partstart + a.nbig;  // parts in all, rows of more than a.spread, those rows
+  cudaError_t e = cudaMemsetAsync(count + 1, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
-  k_ppr_longs<<<grid_for(a.nbig, 256, c->sms * 4), 256, 0, s>>>(w.partstart, a.nbig, a.spread, count + 1, count + 2);
+  k_ppr_partcount<<<grid_for(a.nbig, 256, c->sms * 4), 256, 0, s>>>(g.xtoff, g.seg_shift, a.big, a.nbig, per, a.spread,
+                                                                    w.partstart);
+  e = exclusive_scan_u32(w.partstart, a.nbig + 1, s);
+  if (e != cudaSuccess) return e;
   uint32_t host[2] = {0, 0};
   e = cudaMemcpyAsync(host, count, sizeof host, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
